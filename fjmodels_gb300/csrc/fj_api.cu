@@ -55,6 +55,8 @@ struct fj_ctx {
     DevBuf batch;                                      // batched launch: MomentArgs[n] | block_start | point_start
     std::vector<char> batch_host;                      // what `batch` holds (re-uploaded only when it changes)
     DevBuf delta_ws;                                   // GPU focal-distance tables: views | Eg ptrs | Dg ptrs | flags
+    DevBuf trig;                                       // FP64 form: quadrature-angle table (MomentArgs::trig)
+    DevBuf plain;                                      // FP64 form: work counter | blocks' scratch (PlainWork)
     DevBuf queue;                                      // mixed kernel's work queue: counter | order | costs
     int q_total = 0;                                   // items of the launch whose costs the queue holds
     bool q_costs = false, q_order = false;             // costs recorded / order taken from them
@@ -173,6 +175,36 @@ int queue_setup(fj_ctx *ctx, long long total, ItemQueue &q)
     q.total = n;
     ctx->q_costs = true;  // this launch records them
     ctx->q_launches++;
+    return FJ_OK;
+}
+
+// Work queue and block scratch of a persistent FP64 launch of `total` items whose
+// kernel fits `resident` blocks on the GPU at once.  One buffer per context,
+// grown on demand: a context's launches are ordered on its stream.
+int plain_setup(fj_ctx *ctx, long long total, int resident, int chunk, PlainWork &w)
+{
+    if (total < 1 || total > 0x7fffffffLL) return fail(ctx, FJ_ERR_ARG, "moments: too many work items");
+    if (resident < 1) return fail(ctx, FJ_ERR_CUDA, "moments: tables exceed shared memory");
+    w.total = (int)total;
+    w.grid = (int)(total < resident ? total : resident);
+    w.per_block = plain_scratch_bytes(chunk);
+    int rc = ensure(ctx, ctx->plain, 256 + w.grid * w.per_block);
+    if (rc) return rc;
+    w.next = (unsigned *)ctx->plain.p;
+    w.scratch = (char *)ctx->plain.p + 256;
+    return FJ_OK;
+}
+
+// the FP64 solver's angle table, made on first use
+int trig_table(fj_ctx *ctx, const double2 **t)
+{
+    if (!ctx->trig.p) {
+        int rc = ensure(ctx, ctx->trig, kTrigTableEntries * sizeof(double2));
+        if (rc) return rc;
+        FJ_CUDA(launch_trig_table((double2 *)ctx->trig.p, ctx->stream));
+        FJ_CUDA(cudaStreamSynchronize(ctx->stream));  // a later call may use another stream
+    }
+    *t = (const double2 *)ctx->trig.p;
     return FJ_OK;
 }
 
@@ -341,8 +373,10 @@ int build_args(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delta
     }
     const long long nq3 = (long long)rule->nq * rule->nq * rule->nq;
     a.mixed_chunk = ctx->mixed_chunk;
+    if (!mixed && (rc = trig_table(ctx, &a.trig))) return rc;
+    a.plain_chunk = plain_chunk(npts, nq3);
     a.blocks_per_point =
-        mixed ? mixed_blocks_per_point(nq3, a.mixed_chunk) : (int)((nq3 + kPlainChunk - 1) / kPlainChunk);
+        mixed ? mixed_blocks_per_point(nq3, a.mixed_chunk) : (int)((nq3 + a.plain_chunk - 1) / a.plain_chunk);
     a.out6 = out6;
     a.jout = nullptr;
     return FJ_OK;
@@ -390,11 +424,16 @@ int run_moments(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delt
         a.jout = ctx->jout;
         FJ_CUDA(cudaMemsetAsync(a.jout, 0xFF, (size_t)npts * nq3 * 2 * sizeof(float), ctx->stream));
     }
+    PlainWork pw{};
+    if (!mixed && (rc = plain_setup(ctx, (long long)npts * a.blocks_per_point, moments_resident(moment_smem_bytes(a)),
+                                    kPlainChunk, pw)))
+        return rc;
     FJ_CUDA(cudaMemsetAsync(a.counters, 0, kNumCounters * sizeof(unsigned long long), ctx->stream));
     FJ_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
     ItemQueue q{};
     if (mixed && (rc = queue_setup(ctx, (long long)npts * a.blocks_per_point, q))) return rc;
-    FJ_CUDA(mixed ? launch_moments_mixed(a, ctx->mixed_variant, dw, q, ctx->stream) : launch_moments(a, ctx->stream));
+    FJ_CUDA(mixed ? launch_moments_mixed(a, ctx->mixed_variant, dw, q, ctx->stream)
+                  : launch_moments(a, pw, ctx->stream));
     FJ_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
     return stats ? read_stats(ctx, nq3 * npts, stats) : FJ_OK;
 }
@@ -463,7 +502,8 @@ int fj_ctx_destroy(fj_ctx *ctx)
     if (!ctx) return FJ_OK;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
-    for (DevBuf *b : {&ctx->partial, &ctx->counters, &ctx->rule, &ctx->misc, &ctx->defer, &ctx->queue})
+    for (DevBuf *b : {&ctx->partial, &ctx->counters, &ctx->rule, &ctx->misc, &ctx->defer, &ctx->queue, &ctx->trig,
+                      &ctx->plain, &ctx->batch, &ctx->delta_ws})
         if (b->p) cudaFree(b->p);
     for (auto &kv : ctx->gauss_nodes) cudaFree(kv.second.p);
     for (auto &kv : ctx->poly) cudaFree(kv.second.p);
@@ -570,10 +610,12 @@ int fj_moments_batch(fj_ctx *ctx, int n, const fj_batch_item *items, const fj_qu
     const MomentBatch b{(const MomentArgs *)db, (const int *)(db + n * sizeof(MomentArgs)),
                         (const int *)(db + n * sizeof(MomentArgs) + (n + 1) * sizeof(int)), n};
     FJ_CUDA(cudaMemsetAsync(ctx->counters.p, 0, kNumCounters * sizeof(unsigned long long), ctx->stream));
+    PlainWork pw{};
+    if (!mixed && (rc = plain_setup(ctx, bs[n], moments_resident(smem), kPlainChunk, pw))) return rc;
     FJ_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
     ItemQueue q{};
     if (mixed && (rc = queue_setup(ctx, bs[n], q))) return rc;
-    FJ_CUDA(launch_moments_batch(args[0], b, bs[n], smem, mixed, ctx->mixed_variant, dw, q, ctx->stream));
+    FJ_CUDA(launch_moments_batch(args[0], b, bs[n], smem, mixed, ctx->mixed_variant, dw, q, pw, ctx->stream));
     FJ_CUDA(launch_moments_finalize_batch(b, ps[n], ctx->stream));
     FJ_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
     return stats ? read_stats(ctx, nodes, stats) : FJ_OK;
@@ -699,7 +741,18 @@ int fj_actions(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delta
         return fail(ctx, FJ_ERR_ARG, "actions: bad arguments");
     GLRule gl;
     if ((rc = gl_rule(ctx, jquad, &gl))) return rc;
-    FJ_CUDA(launch_actions(view(pot), delta->Egrid, delta->Dgrid, delta->ngrid, gl, pts, n, out, ctx->stream));
+    if (n == 0) return FJ_OK;
+    const double2 *trig = nullptr;
+    if ((rc = trig_table(ctx, &trig))) return rc;
+    // points per work item: as plain_chunk, a share of the GPU's blocks each
+    int chunk = kActionChunk;
+    while (chunk > 32 && (n + chunk - 1) / chunk < (size_t)kPlainItems) chunk >>= 1;
+    PlainWork pw{};
+    if ((rc = plain_setup(ctx, (long long)((n + chunk - 1) / chunk),
+                          actions_resident(actions_smem_bytes(pot->nr, pot->npoly, delta->ngrid)), kActionChunk, pw)))
+        return rc;
+    FJ_CUDA(launch_actions(view(pot), delta->Egrid, delta->Dgrid, delta->ngrid, gl, trig, pts, n, chunk, out, pw,
+                           ctx->stream));
     return FJ_OK;
 }
 
@@ -765,13 +818,22 @@ int fj_los(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delta, co
     a.m.counters = (unsigned long long *)ctx->counters.p;
     a.rhl = rhl; a.kind = kind; a.Rzv = Rzv; a.n = n; a.out = out;
     fj_tanh_sinh01(a.x01, a.w01);
-    a.blocks_per_item = los_blocks_per_item(kind, rule->nq);
+    const int nodes = los_nodes(kind, rule->nq);
+    a.blocks_per_item = 1;
+    if (kind != FJ_LOS_SIGMA) {
+        const int chunk = plain_chunk(n, nodes);
+        static_assert(kLosChunk == kPlainChunk, "one chunk rule");
+        a.blocks_per_item = (nodes + chunk - 1) / chunk;
+    }
     if ((long long)n * a.blocks_per_item > 0x7fffffffLL) return fail(ctx, FJ_ERR_ARG, "los: too many values");
+    PlainWork pw{};
+    if ((rc = plain_setup(ctx, (long long)n * a.blocks_per_item, los_resident(los_smem_bytes(a.m)), kLosChunk, pw)))
+        return rc;
     if ((rc = ensure(ctx, ctx->partial, (size_t)n * a.blocks_per_item * sizeof(double)))) return rc;
     a.partial = (double *)ctx->partial.p;
     FJ_CUDA(cudaMemsetAsync(ctx->counters.p, 0, kNumCounters * sizeof(unsigned long long), ctx->stream));
     FJ_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
-    FJ_CUDA(launch_los(a, ctx->stream));
+    FJ_CUDA(launch_los(a, pw, ctx->stream));
     FJ_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
     if (stats) {
         const long long nq = rule->nq;

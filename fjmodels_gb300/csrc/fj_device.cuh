@@ -56,7 +56,65 @@ FJ_HD double dmax(double a, double b) { return a > b ? a : b; }  // MAX of inclu
 struct PotView {
     int nr, npoly;
     const double *ar, *phil, *Pr, *Pr2;
+    const double *itab;  // interpolation constants (interp_table), or null: divide in place
 };
+
+// a / b for a divisor whose correctly rounded reciprocal y is at hand: the
+// quotient estimate corrected once by its exact remainder (Markstein, IBM J.
+// Res. Dev. 34, 1990).  It is the correctly rounded quotient in all but ~2^-50
+// of the cases (a tie of the corrected estimate with a rounding boundary), for
+// three FP64 operations instead of a division's nine or more: on the GB300 an
+// FP64 instruction occupies an SM's FP64 pipe for ~18 cycles whatever the
+// number of active lanes, so the kernels that use it are bound by their count.
+FJ_HD double div_by(double a, double b, double y)
+{
+#ifdef __CUDA_ARCH__
+    const double q = __dmul_rn(a, y);
+    return __fma_rn(__fma_rn(-q, b, a), y, q);
+#else
+    (void)y;
+    return a / b;
+#endif
+}
+
+// correctly rounded reciprocal of b (the y of div_by)
+FJ_HD double recip(double b)
+{
+#ifdef __CUDA_ARCH__
+    return __drcp_rn(b);
+#else
+    return 1.0 / b;
+#endif
+}
+
+// Interpolation constants of a radial grid (PotView::itab): two floats for the
+// interval guess, then {1 / (ar[n+1] - ar[n])} per interval, then for the
+// intervals whose top node is below 10 and each third point (below, above)
+// {den, 1/den, f3}, den = (ar[thr]-ar[top]) (ar[thr]-ar[bot]).
+constexpr int kQuadTab = 9;
+FJ_HD int interp_table_size(int nr) { return 1 + nr + 6 * kQuadTab; }
+
+// entries i0, i0 + stride, .. (a block's threads share the work)
+FJ_HD void interp_table(int nr, const double *ar, double *tab, int i0, int stride)
+{
+    if (i0 == 0) {
+        float *g = (float *)tab;
+        const float l0 = log2f((float)ar[0]);
+        g[0] = l0;
+        g[1] = (nr - 1) / (log2f((float)ar[nr - 1]) - l0);
+    }
+    for (int n = i0; n < nr - 1; n += stride) tab[1 + n] = recip(ar[n + 1] - ar[n]);
+    for (int i = i0; i < 2 * kQuadTab; i += stride) {
+        const int n = i >> 1, thr = (i & 1) ? n + 2 : n - 1;
+        double *q = tab + 1 + nr + 3 * i;
+        q[0] = q[1] = q[2] = 0.0;
+        if (thr >= 0 && thr < nr && n + 1 < nr) {
+            q[0] = (ar[thr] - ar[n + 1]) * (ar[thr] - ar[n]);
+            q[1] = recip(q[0]);
+            q[2] = (ar[thr] - ar[n]) / (ar[n + 1] - ar[n]);
+        }
+    }
+}
 
 // bracketing search with the semantics of topbottom (include/Utils.h:103-119)
 FJ_HD int topbottom(const double *xm, int n, double x, int &bot, int &top)
@@ -92,6 +150,37 @@ FJ_HD void interp_setup(const PotView &P, double r, Interp &I)
     I.x = 0.0;
     if (r >= ar[nr - 1]) { I.ext = true; I.quad = false; I.x = ar[nr - 1] / r; return; }
     I.ext = false;
+#ifdef __CUDA_ARCH__
+    if (P.itab && __double_as_longlong(r) >= __double_as_longlong(ar[0])) {
+        const double *tab = P.itab;
+        const float2 g = *(const float2 *)tab;
+        // interval from the logarithmic spacing (log2 of the leading bits, no
+        // FP64 operation), corrected by neighbour tests on the bit patterns
+        // (ordered like the positive values): any increasing grid gives the
+        // bracketing interval.  A radius on a grid node may take either
+        // neighbour, which give the same value.
+        const long long rb = __double_as_longlong(r);
+        const int hi = (int)(rb >> 32);
+        const float m = __int_as_float(0x3f800000 | ((hi & 0xfffff) << 3) | (int)(((unsigned)rb) >> 29));
+        const float lr = (float)((hi >> 20) - 1023) + __log2f(m);
+        int b = (int)((lr - g.x) * g.y);
+        b = b < 0 ? 0 : (b > nr - 2 ? nr - 2 : b);
+        while (b > 0 && rb < __double_as_longlong(ar[b])) --b;
+        while (b < nr - 2 && rb > __double_as_longlong(ar[b + 1])) ++b;
+        const double ab = ar[b], at = ar[b + 1], db = r - ab;
+        I.f1 = div_by(db, at - ab, tab[1 + b]);
+        I.bot = b; I.top = b + 1; I.thr = b + 1;
+        I.quad = b < kQuadTab;
+        if (I.quad) {
+            const bool up = !(I.f1 < 0.5 && b > 0);
+            I.thr = up ? b + 2 : b - 1;
+            const double *q = tab + 1 + nr + 3 * (2 * b + (up ? 1 : 0));
+            I.f2 = div_by((r - at) * db, q[0], q[1]);
+            I.f3 = q[2];
+        }
+        return;
+    }
+#endif
     int top = 0, bot = 0;
     topbottom(ar, nr, r, bot, top);
     const double db = r - ar[bot];
@@ -121,13 +210,59 @@ FJ_HD double interp_in(const Interp &I, const double *T, int npoly, int k)
 }
 
 // next even Legendre polynomial P_{2np} from P_{2np-4}, P_{2np-2} (UtilsLeg.h:68-79), np >= 2
+// (on the device the divisions by functions of np come from a table: one
+// corrected product and two products instead of three divisions)
+struct LegCoef { double l, lm1, D, rD, B, C; };
+struct LegTable { LegCoef c[kMaxPoly]; };
+constexpr LegTable make_leg_table()
+{
+    LegTable t{};
+    for (int np = 2; np < kMaxPoly; np++) {
+        const int l = 2 * (np - 1), l2 = 2 * l;
+        LegCoef &o = t.c[np];
+        o.l = l; o.lm1 = l - 1;
+        o.D = (double)((l2 + 1) * (l2 - 1));
+        o.rD = 1.0 / o.D;
+        o.B = (l2 * l + l2 - 1) / (double)((l2 - 1) * (l2 + 3));
+        o.C = (l2 + 1) * (l2 + 3) / (double)((l + 1) * (l + 2));
+    }
+    return t;
+}
+// reciprocals of the small integers (the full recurrence divides by its degree)
+struct IntRecip { double y[2 * kMaxPoly + 2]; };
+constexpr IntRecip make_int_recip()
+{
+    IntRecip t{};
+    for (int i = 1; i < 2 * kMaxPoly + 2; i++) t.y[i] = 1.0 / i;
+    return t;
+}
+#if defined(__CUDACC__)
+static __constant__ LegTable kLeg_d = make_leg_table();
+static __constant__ IntRecip kIntRecip_d = make_int_recip();
+#endif
+
 FJ_HD double evenleg_next(int np, double c2, double pm2, double pm1)
 {
+#ifdef __CUDA_ARCH__
+    const LegCoef &t = kLeg_d.c[np];
+    return (div_by(-pm2 * t.l * t.lm1, t.D, t.rD) + pm1 * (c2 - t.B)) * t.C;
+#endif
     const int l = 2 * (np - 1), l2 = 2 * l;
     double p = -pm2 * l * (l - 1) / (double)((l2 + 1) * (l2 - 1)) +
                pm1 * (c2 - (l2 * l + l2 - 1) / (double)((l2 - 1) * (l2 + 3)));
     p *= (l2 + 1) * (l2 + 3) / (double)((l + 1) * (l + 2));
     return p;
+}
+
+// P_i of the full Legendre recurrence from P_{i-1}, P_{i-2} (dlegend, UtilsLeg.h:43-57), i >= 2
+FJ_HD double fullleg_next(int i, double c, double Pl, double Pl_m1)
+{
+    const double a = (2 * i - 1) * c * Pl - (i - 1) * Pl_m1;
+#ifdef __CUDA_ARCH__
+    return div_by(a, (double)i, kIntRecip_d.y[i]);
+#else
+    return a / (double)i;
+#endif
 }
 
 // Phi(R,z): Potential::operator() (pot/Potential.cpp:206-219)
@@ -164,29 +299,33 @@ FJ_HDNI void pot_grad(const PotView &P, double R, double z, double &phi, double 
     const double *ar = P.ar;
     const int np_ = P.npoly, nr = P.nr;
     const double r0 = sqrt(R * R + z * z);
-    const double cphi = z / r0;
     double r = r0;
     if (r < ar[0]) r = ar[0];
-    const double s = R / r;
-    double c = z / r;
+    // the four quotients by r share its reciprocal while that is a normal number
+    const bool near = r < 1e150;
+    const double ir = near ? recip(r) : 1.0;
+    auto over_r = [&](double a) { return near ? div_by(a, r, ir) : a / r; };
+    const double s = over_r(R);
+    double c = over_r(z);
+    const double cphi = r == r0 ? c : z / r0;
     if (c == 1) c -= 1e-8;
     Interp I;
     interp_setup(P, r, I);
     const double x2 = I.ext ? I.x * I.x : 0.0;
     double xp = I.x;
-    const double cp2 = cphi * cphi, cc2 = c * c;
+    const double cp2 = cphi * cphi, cc2 = c * c, omc = 1 - c * c, iomc = recip(omc);
+    const bool same = cp2 == cc2;  // inside the grid: one even recurrence serves both
     // even polys at cphi (potential) and at c (radial derivative)
     double ep2 = 1, ep1 = 0, ec2 = 1, ec1 = 0;
     // full recurrence at c: Pl_m1 = P_{n-1}, Pl = P_n
     double Pl_m1 = 0, Pl = 1;
-    int nfull = 0;
     double gphi = 0, gdr = 0, gdth = 0;
     for (int k = 0; k < np_; k++) {
         double ph, dph;
         if (I.ext) {
             const double t = P.phil[(nr - 1) * np_ + k];
             ph = t * xp;
-            dph = -(2 * k + 1) * t * xp / r;
+            dph = over_r(-(2 * k + 1) * t * xp);
             xp *= x2;
         } else {
             ph = interp_in(I, P.phil, np_, k);
@@ -197,29 +336,27 @@ FJ_HDNI void pot_grad(const PotView &P, double R, double z, double &phi, double 
         else if (k == 1) { pe_phi = 1.5 * cp2 - .5; pe_c = 1.5 * cc2 - .5; ep1 = pe_phi; ec1 = pe_c; }
         else {
             pe_phi = evenleg_next(k, cp2, ep2, ep1); ep2 = ep1; ep1 = pe_phi;
-            pe_c = evenleg_next(k, cc2, ec2, ec1); ec2 = ec1; ec1 = pe_c;
+            if (same) pe_c = pe_phi;
+            else pe_c = evenleg_next(k, cc2, ec2, ec1);
+            ec2 = ec1; ec1 = pe_c;
         }
         // advance the full recurrence to n = 2k
         double dleg = 0;
         if (k > 0) {
             const int n = 2 * k;
-            while (nfull < n) {
-                const int i = nfull + 1;
-                double Pn;
-                if (i == 1) Pn = c;
-                else Pn = ((2 * i - 1) * c * Pl - (i - 1) * Pl_m1) / (double)i;
-                Pl_m1 = Pl; Pl = Pn; nfull = i;
-            }
-            dleg = (n * Pl_m1 - n * c * Pl) / (1 - c * c);
+            const double P1 = k == 1 ? c : fullleg_next(n - 1, c, Pl, Pl_m1);
+            const double P2 = fullleg_next(n, c, P1, Pl);
+            Pl_m1 = P1; Pl = P2;
+            dleg = div_by(n * Pl_m1 - n * c * Pl, omc, iomc);
         }
         if (k == 0) gphi = ph; else gphi += ph * pe_phi;
         gdr += dph * pe_c;
         gdth += ph * dleg;
     }
-    gdth *= -sqrt(1 - c * c);
+    gdth *= -sqrt(omc);
     phi = gphi;
-    dR = gdth * (c / r) + gdr * s;
-    dz = gdth * (-s / r) + gdr * c;
+    dR = gdth * over_r(c) + gdr * s;
+    dz = gdth * over_r(-s) + gdr * c;
 }
 
 // Potential::dr with its second derivative (pot/Potential.cpp:224-234); r not clamped
@@ -271,7 +408,7 @@ FJ_HD void pot_theta_sums(const PotView &P, double r, double c, double &s1, doub
         if (k > 0) {
             while (nfull < n) {
                 const int i = nfull + 1;
-                const double Pn = (i == 1) ? c : ((2 * i - 1) * c * Pl - (i - 1) * Pl_m1) / (double)i;
+                const double Pn = (i == 1) ? c : fullleg_next(i, c, Pl, Pl_m1);
                 Pl_m1 = Pl; Pl = Pn; nfull = i;
             }
             d1 = (n * Pl_m1 - n * c * Pl) / (1 - c * c);
@@ -367,7 +504,11 @@ FJ_HD double rescale_err(double err, double resabs, double resasc)
 {
     err = fabs(err);
     if (resasc != 0 && err != 0) {
+#ifdef __CUDA_ARCH__
+        const double ratio = 200 * err / resasc, scale = ratio * sqrt(ratio);  // an estimate: its last bit decides nothing
+#else
         const double scale = pow(200 * err / resasc, 1.5);
+#endif
         err = scale < 1 ? resasc * scale : resasc;
     }
     if (resabs > DBL_MIN / (50 * DBL_EPSILON)) {
@@ -777,7 +918,22 @@ struct Fudge {
     double sinhu, coshu;   // sinh(u), cosh(u) of the point
     double sh1sq, ch1sq, Phiu1, PhivPIH;
     double uinner, uouter, umid, vturn, ubar, Deltau;
+    // what the u and v equations repeat at every evaluation (set by prepare)
+    double LzD2, ish1, Erch, B0, C0, hL, DD, Dshu, Dchu;
     unsigned fail;
+
+    FJ_HD void prepare()
+    {
+        DD = Delta * Delta;
+        hL = .5 * Lzsq;
+        LzD2 = hL / DD;
+        ish1 = 1 / sh1sq;
+        Erch = Er * ch1sq;
+        B0 = (sh1sq + sv2) * Phiu1;
+        C0 = (1 + shu2) * PhivPIH;
+        Dshu = Delta * sinhu;
+        Dchu = Delta * coshu;
+    }
 
     FJ_HD double Phiu(double shu, double chu) const { return pot_phi(P, Delta * shu * sinv, Delta * chu * cosv); }
     FJ_HD double dU(double u_) const
@@ -791,14 +947,14 @@ struct Fudge {
         double sn, cs;
         sincos(v_, &sn, &cs);
         const double s2 = sn * sn;
-        const double dV = (1 + shu2) * PhivPIH - (shu2 + s2) * Phiv(sn, cs);
-        return E * s2 + Iv + dV - .5 * Lzsq / (Delta * Delta * s2);
+        const double dV = C0 - (shu2 + s2) * pot_phi(P, Dshu * sn, Dchu * cs);
+        return E * s2 + Iv + dV - hL / (DD * s2);
     }
     FJ_HD double uturnfn(double u_) const
     {
         const double shu = sinh(u_), chu = cosh(u_), s2 = shu * shu;
-        const double dUv = (s2 + sv2) * Phiu(shu, chu) - (sh1sq + sv2) * Phiu1;
-        return E * (s2 - sh1sq) + Er * ch1sq - dUv - .5 * Lzsq / (Delta * Delta) * (1 / s2 - 1 / sh1sq);
+        const double dUv = (s2 + sv2) * Phiu(shu, chu) - B0;
+        return E * (s2 - sh1sq) + Erch - dUv - LzD2 * (1 / s2 - ish1);
     }
     FJ_HD double duturnfn(double u_) const
     {
@@ -971,14 +1127,12 @@ struct SerialMomInt {
     FJ_HD double operator()(F &f, double b, unsigned &fail) const { return mom_integral(f, b, *gl, fail); }
 };
 
-// Actions of one phase-space point: uvOrb ctor (uvOrb.cpp:15-36), Ju, Jv, the
-// momentum integrals by mi(integrand, upper limit, fail).
-// Returns false for an unbound orbit (Jr = Jz = 1e31).
-template <class MI>
-FJ_HDNI bool fudge_actions_with(const PotView &P, double Delta, double R, double z, double Phi, double pR,
-                                double vphi, double pz, const MI &mi, double &Jr, double &Jz, unsigned &fail)
+// One phase-space point: uvOrb ctor (uvOrb.cpp:15-36) and the turning points of
+// Ju and Jv into o (umid, uinner, uouter, ubar, Deltau, vturn; o.fail).
+// Returns false for an unbound orbit.
+FJ_HDNI bool fudge_turning_points(const PotView &P, double Delta, double R, double z, double Phi, double pR,
+                                  double vphi, double pz, Fudge &o)
 {
-    Fudge o;
     o.P = P;
     o.fail = 0;
     o.Delta = Delta;
@@ -1002,7 +1156,7 @@ FJ_HDNI bool fudge_actions_with(const PotView &P, double Delta, double R, double
     const double pu = Delta * (pR * chu * o.sv + pz * shu * cv);
     const double pv = Delta * (pR * shu * cv - pz * chu * o.sv);
     o.E = .5 * p2 + .5 * o.Lzsq / (R * R) + Phi;
-    if (o.E >= 0 || isnan(o.E)) { Jr = Jz = 1e31; return false; }
+    if (o.E >= 0 || isnan(o.E)) return false;
     sincos(o.v, &o.sinv, &o.cosv);
     o.sinhu = sinh(o.u);
     o.coshu = cosh(o.u);
@@ -1026,22 +1180,39 @@ FJ_HDNI bool fudge_actions_with(const PotView &P, double Delta, double R, double
         const double dVv = (1 + o.shu2) * o.PhivPIH - (o.shu2 + sn * sn) * o.Phiv(sn, cs);
         o.Iv = .5 * (pv * pv) / Delta2 - o.E * o.sv2 + .5 * o.Lzsq / (Delta2 * o.sv2) - dVv;
     }
-    const double rtwo = sqrt(2.0);
-    // Ju (uvOrb.cpp:226-239)
+    o.prepare();
     get_turn_u(o, 1);
-    if (fabs(o.uouter - o.uinner) < kTINY) Jr = 0;
-    else {
-        o.ubar = .5 * (o.uinner + o.uouter);
-        o.Deltau = .5 * (o.uouter - o.uinner);
-        JuIntF fju{&o};
-        Jr = rtwo * Delta * o.Deltau * mi(fju, kPI, o.fail) / kPI;
-    }
-    // Jv (uvOrb.cpp:247-257)
+    o.ubar = .5 * (o.uinner + o.uouter);
+    o.Deltau = .5 * (o.uouter - o.uinner);
     o.vturn = get_turn_v(o, .5 * kPIH);
-    if (fabs(o.vturn - kPIH) < kTINY) Jz = 0;
+    return true;
+}
+
+// whether Ju and Jv vanish (uvOrb.cpp:226-229, 247-249), and their factors
+// before the integrals (uvOrb.cpp:238, 256)
+FJ_HD bool fudge_ju_zero(const Fudge &o) { return fabs(o.uouter - o.uinner) < kTINY; }
+FJ_HD bool fudge_jv_zero(const Fudge &o) { return fabs(o.vturn - kPIH) < kTINY; }
+FJ_HD double fudge_ju_factor(const Fudge &o) { return sqrt(2.0) * o.Delta * o.Deltau; }
+FJ_HD double fudge_jv_factor(const Fudge &o) { return 2 * sqrt(2.0) * o.Delta * (kPIH - o.vturn); }
+
+// Actions of one phase-space point: the turning points, Ju and Jv with the
+// momentum integrals by mi(integrand, upper limit, fail).
+// Returns false for an unbound orbit (Jr = Jz = 1e31).
+template <class MI>
+FJ_HDNI bool fudge_actions_with(const PotView &P, double Delta, double R, double z, double Phi, double pR,
+                                double vphi, double pz, const MI &mi, double &Jr, double &Jz, unsigned &fail)
+{
+    Fudge o;
+    if (!fudge_turning_points(P, Delta, R, z, Phi, pR, vphi, pz, o)) { Jr = Jz = 1e31; return false; }
+    if (fudge_ju_zero(o)) Jr = 0;
+    else {
+        JuIntF fju{&o};
+        Jr = fudge_ju_factor(o) * mi(fju, kPI, o.fail) / kPI;
+    }
+    if (fudge_jv_zero(o)) Jz = 0;
     else {
         JvIntF fjv{&o};
-        Jz = 2 * rtwo * Delta * (kPIH - o.vturn) * mi(fjv, kPIH, o.fail) / kPI;
+        Jz = fudge_jv_factor(o) * mi(fjv, kPIH, o.fail) / kPI;
     }
     fail |= o.fail;
     return true;

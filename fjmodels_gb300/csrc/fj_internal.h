@@ -22,7 +22,18 @@ enum : int {
     kCntBound = 0, kCntFailed = 1, kCntPoisson = 2, kCntEscalated = 3,
     kCntFailQuad = 4, kCntFailBracket = 5, kCntFailRoot = 6, kCntResolved64 = 7, kNumCounters = 8
 };
-constexpr int kPlainChunk = 1024;  // velocity nodes of one point per block (FP64 form)
+constexpr int kPlainChunk = 1024;  // most velocity nodes of one point per work item (FP64 form)
+// Nodes per work item of a model of npts points, nq3 nodes each: as large as
+// possible (a long node list keeps the lanes of a block busy to its end) while
+// there are enough items to fill the GPU and balance their uneven cost.  By the
+// model's own size alone, so that a batched launch sums in the same order.
+constexpr int kPlainItems = 1216;  // 8 per SM
+inline int plain_chunk(long long npts, long long nq3)
+{
+    int c = kPlainChunk;
+    while (c > 128 && npts * ((nq3 + c - 1) / c) < kPlainItems) c >>= 1;
+    return c;
+}
 // per-thread stack the kernels need: the QAGS interval list (kQagsCap entries
 // of four doubles and an int), the epsilon table and the call frames
 constexpr size_t kStackBytes = 8192;
@@ -43,6 +54,8 @@ struct MomentArgs {
     const double *Rz;        // point mode: [npts][2]; else NULL
     int npts;
     int blocks_per_point;
+    int plain_chunk;         // FP64 form: nodes per work item (<= kPlainChunk)
+    const double2 *trig;     // FP64 form: sines and cosines of the quadrature angles (launch_trig_table)
     int mixed_chunk;         // mixed form: nodes per block (<= kMixedMaxNodes)
     float *jout;             // mixed form, optional: (Jr, Jz) of every bound node [npts][nq^3][2]
     double *partial;         // [npts][blocks_per_point][6]
@@ -57,6 +70,24 @@ struct MomentArgs {
 // n values at Rzv [n][3] (R, z, v) of one kind (FJ_LOS_*), on m's potential,
 // focal-distance table, [-1,1] rule and DF, with the 22-point [0,1] table
 constexpr int kLos01 = 22;
+// Work queue and scratch of a persistent FP64 launch (k_moments, k_los,
+// k_actions): items 0 .. total-1 from a device counter that the launch zeroes,
+// scratch of per_block bytes for each of its blocks
+struct PlainWork {
+    unsigned *next;
+    char *scratch;
+    size_t per_block;
+    int total, grid;
+};
+size_t plain_scratch_bytes(int chunk);  // per block, for items of at most chunk points
+// blocks of a persistent launch resident at once
+int moments_resident(size_t smem);
+int los_resident(size_t smem);
+int actions_resident(size_t smem);
+// the table of MomentArgs::trig, kTrigTableEntries entries
+constexpr size_t kTrigTableEntries = 2 * 1024 * 21;
+cudaError_t launch_trig_table(double2 *trig, cudaStream_t s);
+
 struct LosArgs {
     MomentArgs m;
     const double *rhl;  // [nr*npoly] density multipoles (SigmaDF)
@@ -68,9 +99,10 @@ struct LosArgs {
     int blocks_per_item;  // blocks sharing one value's nodes (kLosChunk nodes each)
     double *partial;      // [n][blocks_per_item] block sums, added in order by k_los_finalize
 };
-constexpr int kLosChunk = 1024;  // nodes of one value per block
-cudaError_t launch_los(const LosArgs &a, cudaStream_t s);
-int los_blocks_per_item(int kind, int nq);
+constexpr int kLosChunk = 1024;  // most nodes of one value per work item
+size_t los_smem_bytes(const MomentArgs &m);
+cudaError_t launch_los(const LosArgs &a, const PlainWork &w, cudaStream_t s);
+int los_nodes(int kind, int nq);  // a value's nodes
 size_t los_local_bytes();
 
 // Focal-distance tables of n models (fj_delta.cu): one thread per (model,
@@ -131,7 +163,7 @@ __device__ __forceinline__ int batch_model(const int *start, int n, int i)
 }
 
 size_t moment_smem_bytes(const MomentArgs &a);
-cudaError_t launch_moments(const MomentArgs &a, cudaStream_t s);
+cudaError_t launch_moments(const MomentArgs &a, const PlainWork &w, cudaStream_t s);
 // batched forms: grid = total blocks, smem = the largest model's
 // work queue of the persistent mixed kernel: item i is block order[i] (order
 // NULL: block i) of the launch's layout; cost[b] receives block b's cycles
@@ -142,7 +174,8 @@ struct ItemQueue {
     int total;
 };
 cudaError_t launch_moments_batch(const MomentArgs &a0, const MomentBatch &b, int nblocks, size_t smem, bool mixed,
-                                 int variant, const DeferWork &dw, const ItemQueue &q, cudaStream_t s);
+                                 int variant, const DeferWork &dw, const ItemQueue &q, const PlainWork &w,
+                                 cudaStream_t s);
 cudaError_t launch_moments_finalize_batch(const MomentBatch &b, int npoints, cudaStream_t s);
 // dst6[q][idx[t]] = src6[q][t] (moments of n points into a grid of npts)
 cudaError_t launch_scatter6(int n, const int *idx, const double *src6, int npts, double *dst6, cudaStream_t s);
@@ -177,8 +210,10 @@ int mixed_blocks_per_point(long long nq3, int chunk);
 cudaError_t launch_moments_mixed(const MomentArgs &a, int variant, const DeferWork &dw, const ItemQueue &q,
                                  cudaStream_t s);
 
-cudaError_t launch_actions(PotView P, const double *Eg, const double *Dg, int ngrid, GLRule gl,
-                           const double *pts, size_t n, double *out, cudaStream_t s);
+constexpr int kActionChunk = 256;  // most points per work item of the action batch
+size_t actions_smem_bytes(int nr, int npoly, int ngrid);
+cudaError_t launch_actions(PotView P, const double *Eg, const double *Dg, int ngrid, GLRule gl, const double2 *trig,
+                           const double *pts, size_t n, int chunk, double *out, const PlainWork &w, cudaStream_t s);
 cudaError_t launch_potential_eval(PotView P, const double *Rz, size_t n, double *out, cudaStream_t s);
 
 // projection: poly [npoly][ngauss] = 2 P_2l(c_g) w_g

@@ -3,14 +3,14 @@
 // the phase-space kernel's node body (Staeckel-fudge actions + DF, plain FP64)
 // under 3-D and 2-D tensor rules.
 //
-// A value's nodes are split into ranges of kLosChunk nodes, one block each
-// (a line profile's 22^3 nodes: 11 blocks), so a few hundred values fill the
-// GPU.  As in the phase-space kernels, a block compacts its bound nodes,
-// orders them by the cost proxy of fj_order.cuh and hands them to threads as
-// they free up, storing each node's DF; thread t then sums list entries t,
-// t + kLosBlock, .. from the stored DFs, the block adds the thread sums in a
-// fixed order and k_los_finalize adds the blocks' sums in order, so a value
-// is the same run to run.
+// A value's nodes are split into ranges of at most kLosChunk nodes, the work
+// items of a persistent launch (a line profile's 22^3 nodes: 11 items), so a few
+// hundred values fill the GPU; of few values the ranges are shorter.  As in the
+// phase-space kernel, a block compacts an item's bound nodes, orders them by the
+// cost proxy of fj_order.cuh and solves their orbits together (fj_solve64.cuh);
+// thread t sums list entries t, t + kLosBlock, .., the block adds the thread
+// sums in a fixed order and k_los_finalize adds the items' sums in order, so a
+// value is the same run to run.
 //   SIGMA  SigmaDF(R, z) = 2 sum_i w01_i (rmax - R) rho(R + x01_i (rmax - R), z),
 //          rho from the density multipoles (ev_dens, UtilsLeg.h:285-298, 323-334)
 //   LINE   line_profile(R, z, vx): [-1,1]^3 rule over (vy, x, vz), the DF at the
@@ -24,12 +24,14 @@
 #include "../../include/fjgpu.h"
 #include "fj_internal.h"
 #include "fj_order.cuh"
+#include "fj_solve64.cuh"
 
 namespace fj {
 
 namespace {
 
-constexpr int kLosBlock = 128;
+constexpr int kLosBlock = kSolveBlock;
+static_assert(kLosChunk <= kPlainChunk, "an item's orbits fit the solver's scratch");
 
 __device__ __forceinline__ double los_warp_sum(double v)
 {
@@ -69,34 +71,41 @@ __device__ double sigma_df(const PotView &P, const double *rhl, const LosArgs &a
     return 2 * s;
 }
 
-__global__ void __launch_bounds__(kLosBlock) k_los(LosArgs a)
+__global__ void __launch_bounds__(kLosBlock, 2) k_los(LosArgs a, PlainWork work)
 {
     extern __shared__ double sm[];
+    __shared__ int s_item;
     const MomentArgs &m = a.m;
     const int nr = m.P.nr, npoly = m.P.npoly, nt = nr * npoly;
-    double *s_ar = sm, *s_phil = s_ar + nr, *s_Pr = s_phil + nt, *s_Pr2 = s_Pr + nt;
-    double *s_Eg = s_Pr2 + nt, *s_Dg = s_Eg + m.ngrid, *s_xq = s_Dg + m.ngrid, *s_wq = s_xq + m.nq;
-    double *s_glx = s_wq + m.nq, *s_glw = s_glx + m.gl.n, *s_rhl = s_glw + m.gl.n, *s_red = s_rhl + nt;
-    double *s_df = s_red + kLosBlock / 32;                          // [kLosChunk] DF of the list entries
-    float *s_key = (float *)(s_df + kLosChunk);                       // [kLosChunk] cost keys
-    unsigned short *s_list = (unsigned short *)(s_key + kLosChunk);   // [kLosChunk] bound nodes
-    int *s_wc = (int *)(s_list + kLosChunk), *s_next = s_wc + kLosBlock / 32;
+    double *s_ar = sm, *s_phil = s_ar + nr, *s_Pr = s_phil + nt, *s_it = s_Pr + nt;
+    double *s_Eg = s_it + interp_table_size(nr), *s_Dg = s_Eg + m.ngrid, *s_xq = s_Dg + m.ngrid, *s_wq = s_xq + m.nq;
+    double *s_glx = s_wq + m.nq, *s_glw = s_glx + m.gl.n, *s_red = s_glw + m.gl.n;
+    SolveShared *s_solve = (SolveShared *)(s_red + kLosBlock / 32);
+    float *s_key = (float *)s_solve->vals;                            // cost keys, until the solves
+    unsigned short *s_list = (unsigned short *)(s_solve + 1);         // [kLosChunk] bound nodes
+    int *s_wc = (int *)(s_list + kLosChunk);
     for (int i = threadIdx.x; i < nr; i += blockDim.x) s_ar[i] = m.P.ar[i];
-    for (int i = threadIdx.x; i < nt; i += blockDim.x) {
-        s_phil[i] = m.P.phil[i]; s_Pr[i] = m.P.Pr[i]; s_Pr2[i] = m.P.Pr2[i];
-        s_rhl[i] = a.rhl ? a.rhl[i] : 0.;
-    }
+    for (int i = threadIdx.x; i < nt; i += blockDim.x) { s_phil[i] = m.P.phil[i]; s_Pr[i] = m.P.Pr[i]; }
     for (int i = threadIdx.x; i < m.ngrid; i += blockDim.x) { s_Eg[i] = m.Eg[i]; s_Dg[i] = m.Dg[i]; }
     for (int i = threadIdx.x; i < m.nq; i += blockDim.x) { s_xq[i] = m.xq[i]; s_wq[i] = m.wq[i]; }
     for (int i = threadIdx.x; i < m.gl.n; i += blockDim.x) { s_glx[i] = m.gl.x01[i]; s_glw[i] = m.gl.w01[i]; }
     __syncthreads();
-    const PotView P{nr, npoly, s_ar, s_phil, s_Pr, s_Pr2};
+    interp_table(nr, s_ar, s_it, threadIdx.x, blockDim.x);
+    const PotView P{nr, npoly, s_ar, s_phil, s_Pr, m.P.Pr2, s_it};
     const GLRule gl{m.gl.n, s_glx, s_glw};
-    const int B = a.blocks_per_item, item = blockIdx.x / B, chunk = blockIdx.x % B;
+    const SolveScratch S = solve_scratch(work.scratch + blockIdx.x * work.per_block, kPlainChunk);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_item = (int)atomicAdd(work.next, 1u);
+    __syncthreads();
+    const int bid = s_item;
+    if (bid >= work.total) return;
+    const int B = a.blocks_per_item, item = bid / B, chunk = bid % B;
     const double R = a.Rzv[3 * item], z = a.Rzv[3 * item + 1], v = a.Rzv[3 * item + 2];
     if (a.kind == FJ_LOS_SIGMA) {
-        if (threadIdx.x == 0) a.out[item] = sigma_df(P, s_rhl, a, R, z);
-        return;
+        if (threadIdx.x == 0) a.out[item] = sigma_df(P, a.rhl, a, R, z);
+        continue;
     }
     const double rmax = s_ar[nr - 1];
     const double Phi = pot_phi(P, R, z), Ve = sqrt(-2 * (Phi - pot_phi(P, 10 * rmax, 10 * rmax)));
@@ -128,9 +137,8 @@ __global__ void __launch_bounds__(kLosBlock) k_los(LosArgs a)
             w = a.w01[i] * s_wq[j];
         }
     };
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // bound nodes of [n0, n1) in node order, then ordered by the cost proxy of
-    // the phase-space kernels (most expensive first), taken as threads free up
+    // the phase-space kernels (most expensive first)
     int nbound = 0;
     for (int base = n0; base < n1; base += kLosBlock) {
         const int node = base + threadIdx.x;
@@ -159,28 +167,25 @@ __global__ void __launch_bounds__(kLosBlock) k_los(LosArgs a)
         s_key[q] = node_cost_key((float)(V[0] * iVe), (float)(V[1] * iVe), (float)(V[2] * iVe));
     }
     sort_list(s_list, s_key, nbound);
-    if (threadIdx.x == 0) *s_next = kLosBlock;
-    __syncthreads();
+    solve_orbits64(P, gl, m.trig, nbound, S, *s_solve,
+                   [&](int q, double &Delta, double &R_, double &z_, double &Phi_, double &V0, double &V1, double &V2) {
+                       double V[3], w, jacob;
+                       node_vel(n0 + s_list[q], V, w, jacob);
+                       V0 = V[0]; V1 = V[1]; V2 = V[2];
+                       Delta = deltafn(s_Eg, s_Dg, m.ngrid, .5 * (V0 * V0 + V1 * V1 + V2 * V2) + Phi);
+                       R_ = R; z_ = z; Phi_ = Phi;
+                   });
     unsigned failed = 0;
-    for (int q = threadIdx.x; q < nbound;) {  // df(), DF.cpp:78-124
+    double sum = 0;  // fixed order: thread t adds list entries t, t + kLosBlock, ..
+    for (int q = threadIdx.x; q < nbound; q += kLosBlock) {  // df(), DF.cpp:78-124
         double V[3], w, jacob;
         node_vel(n0 + s_list[q], V, w, jacob);
-        const double H = .5 * (V[0] * V[0] + V[1] * V[1] + V[2] * V[2]) + Phi;
-        unsigned fail = 0;
-        double Jr, Jz;
-        fudge_actions(P, deltafn(s_Eg, s_Dg, m.ngrid, H), R, z, Phi, V[0], V[1], V[2], gl, Jr, Jz, fail);
-        double DF = df_value(m.df, P, R, Jr, Jz, R * V[1], fail);
+        const OrbitRec &o = S.rec[q];
+        unsigned fail = o.status();
+        double DF = df_value(m.df, P, R, o.Jr, o.Jz, R * V[1], fail);
         if (fail & (kFailBracket | kFailRoot)) DF = 0.;
         failed += fail ? 1u : 0u;
-        s_df[q] = DF;
-        q = atomicAdd(s_next, 1);
-    }
-    __syncthreads();
-    double sum = 0;  // fixed order: thread t adds list entries t, t + kLosBlock, ..
-    for (int q = threadIdx.x; q < nbound; q += kLosBlock) {
-        double V[3], w, jacob;
-        node_vel(n0 + s_list[q], V, w, jacob);
-        sum += w * (jacob * s_df[q]);
+        sum += w * (jacob * DF);
     }
     const double ws = los_warp_sum(sum);
     unsigned nfw = failed;
@@ -192,11 +197,12 @@ __global__ void __launch_bounds__(kLosBlock) k_los(LosArgs a)
         double s = 0;
         unsigned nf = 0;
         for (int q = 0; q < kLosBlock / 32; q++) { s += s_red[q]; nf += (unsigned)s_wc[q]; }
-        a.partial[blockIdx.x] = s;
+        a.partial[bid] = s;
         if (a.m.counters) {
             if (nbound) atomicAdd(&a.m.counters[kCntBound], (unsigned long long)nbound);
             if (nf) atomicAdd(&a.m.counters[kCntFailed], (unsigned long long)nf);
         }
+    }
     }
 }
 
@@ -215,18 +221,29 @@ __global__ void k_los_finalize(LosArgs a)
 
 }  // namespace
 
-int los_blocks_per_item(int kind, int nq)
+int los_nodes(int kind, int nq)
 {
-    const long long nnodes = kind == FJ_LOS_LINE ? (long long)nq * nq * nq
-                             : kind == FJ_LOS_PVPHI ? (long long)kLos01 * kLos01 : (long long)kLos01 * nq;
-    return kind == FJ_LOS_SIGMA ? 1 : (int)((nnodes + kLosChunk - 1) / kLosChunk);
+    return kind == FJ_LOS_LINE ? nq * nq * nq : kind == FJ_LOS_PVPHI ? kLos01 * kLos01 : kLos01 * nq;
 }
 
 size_t los_smem_bytes(const MomentArgs &m)
 {
     const size_t nt = (size_t)m.P.nr * m.P.npoly;
-    return (m.P.nr + 4 * nt + 2 * m.ngrid + 2 * m.nq + 2 * m.gl.n + kLosBlock / 32 + kLosChunk) * sizeof(double) +
-           kLosChunk * (sizeof(float) + sizeof(unsigned short)) + (kLosBlock / 32 + 1) * sizeof(int);
+    return (m.P.nr + 2 * nt + interp_table_size(m.P.nr) + 2 * m.ngrid + 2 * m.nq + 2 * m.gl.n + kLosBlock / 32) *
+               sizeof(double) +
+           sizeof(SolveShared) + kLosChunk * sizeof(unsigned short) + (kLosBlock / 32 + 1) * sizeof(int);
+}
+
+int los_resident(size_t smem)
+{
+    int dev = 0, nsm = 0, per_sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        (smem > 48 * 1024 &&
+         cudaFuncSetAttribute(k_los, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_los, kLosBlock, smem) != cudaSuccess)
+        return 0;
+    return per_sm * nsm;
 }
 
 size_t los_local_bytes()
@@ -235,15 +252,13 @@ size_t los_local_bytes()
     return cudaFuncGetAttributes(&at, k_los) == cudaSuccess ? at.localSizeBytes : 0;
 }
 
-cudaError_t launch_los(const LosArgs &a, cudaStream_t s)
+cudaError_t launch_los(const LosArgs &a, const PlainWork &w, cudaStream_t s)
 {
-    const size_t smem = los_smem_bytes(a.m);
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(k_los, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
-    k_los<<<(unsigned)((long long)a.n * a.blocks_per_item), kLosBlock, smem, s>>>(a);
-    cudaError_t e = cudaGetLastError();
+    if (w.grid < 1) return cudaErrorInvalidConfiguration;
+    cudaError_t e = cudaMemsetAsync(w.next, 0, sizeof(unsigned), s);
+    if (e != cudaSuccess) return e;
+    k_los<<<(unsigned)w.grid, kLosBlock, los_smem_bytes(a.m), s>>>(a, w);
+    e = cudaGetLastError();
     if (e != cudaSuccess || a.kind == FJ_LOS_SIGMA) return e;
     k_los_finalize<<<(a.n + 127) / 128, 128, 0, s>>>(a);
     return cudaGetLastError();

@@ -954,6 +954,7 @@ FJ_HDNI void fudge64_at_point(Fudge &o, const PotView &P, double Delta, double L
     sincos(v, &sn, &cs);
     const double dVv = (1 + shu2) * o.PhivPIH - (shu2 + sn * sn) * o.Phiv(sn, cs);
     o.Iv = .5 * (pv * pv) / D2 - E * sv2 + .5 * Lzsq / (D2 * sv2) - dVv;
+    o.prepare();
 }
 
 // FP32 tables of PotViewF for the phase point whose potential is Phi_h;

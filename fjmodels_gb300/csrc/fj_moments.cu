@@ -5,16 +5,17 @@
 //
 // Work unit: node q = (i, j, k) of the nq^3 tensor rule (integ/GaussQuad.cpp:
 // 160-180), velocity V = 1e-6 + Ve*(x_i, x_j, x_k) (integ/Integ.cpp:46-62).
-// A block takes kPlainChunk consecutive nodes of one point, compacts the bound
-// ones (H < 0) into a shared list, orders it by the cost proxy of fj_order.cuh
-// and its threads take the entries as they free up; each node's DF goes to a
-// shared array, and after the list thread t sums the moments of entries t,
-// t + 128, .. in order.  The per-block sums go to a scratch array and a second
-// kernel adds them in a fixed order, so results are deterministic run to run.
+// A work item is a range of at most kPlainChunk consecutive nodes of one point;
+// a persistent block compacts its bound ones (H < 0) into a shared list, orders
+// it by the cost proxy of fj_order.cuh, solves the list's orbits together
+// (fj_solve64.cuh), and thread t sums the moments of entries t, t + 128, .. in
+// order.  The per-item sums go to a scratch array and a second kernel adds them
+// in a fixed order, so results are deterministic run to run.
 #include <cstdint>
 
 #include "fj_internal.h"
 #include "fj_order.cuh"
+#include "fj_solve64.cuh"
 
 namespace fj {
 
@@ -25,140 +26,202 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
+static_assert(kTrigTableEntries == 2 * kTrigPanels * 21, "trig table size");
+static_assert(sizeof(SolveShared::vals) >= kPlainChunk * sizeof(float), "the cost keys share the panel values' memory");
+static_assert(kMomentBlock == kSolveBlock, "the moment blocks run the orbit solver");
+
+size_t plain_scratch_bytes(int chunk) { return (solve_scratch_bytes(chunk) + 255) / 256 * 256; }
+
+// panels of the bisection trees of [0, pi] (Ju) and [0, pi/2] (Jv): interval
+// `heap` by halving from the root, as the quadrature does
+__global__ void k_trig_table(double2 *trig)
+{
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= kTrigTableEntries) return;
+    const bool kv = t >= kTrigTableEntries / 2;
+    const unsigned heap = (t / 21) % kTrigPanels;
+    const int e = t % 21;
+    if (heap == 0) { trig[t] = make_double2(0., 0.); return; }
+    double a = 0., b = kv ? kPIH : kPI;
+    for (int bit = 30 - __clz((int)heap); bit >= 0; bit--) {
+        const double m = 0.5 * (a + b);
+        if ((heap >> bit) & 1u) a = m; else b = m;
+    }
+    double sn, cs;
+    sincos(gk_abscissa<21>(a, b, e), &sn, &cs);
+    trig[t] = make_double2(sn, cs);
+}
+
+cudaError_t launch_trig_table(double2 *trig, cudaStream_t s)
+{
+    k_trig_table<<<(unsigned)((kTrigTableEntries + 127) / 128), 128, 0, s>>>(trig);
+    return cudaGetLastError();
+}
+
+// shared memory of a model's tables: radii, potential and its radial derivative
+// (the second one, which only the quasi-isothermal DF reads, stays in device
+// memory), interpolation constants, focal distances, velocity and momentum rules
+static size_t table_doubles(int nr, int npoly, int ngrid, int nq, int ngl)
+{
+    return nr + 2 * (size_t)nr * npoly + interp_table_size(nr) + 2 * ngrid + 2 * nq + 2 * ngl;
+}
+
 size_t moment_smem_bytes(const MomentArgs &a)
 {
-    const size_t nd = a.P.nr + 3 * (size_t)a.P.nr * a.P.npoly + 2 * a.ngrid + 2 * a.nq + 2 * a.gl.n;
-    return nd * sizeof(double) + 6 * (kMomentBlock / 32) * sizeof(double) + 4 * sizeof(double) +
-           kPlainChunk * (sizeof(double) + sizeof(float) + sizeof(unsigned short)) + (kMomentBlock / 32 + 1) * sizeof(int) +
-           16;
+    const size_t nd = table_doubles(a.P.nr, a.P.npoly, a.ngrid, a.nq, a.gl.n);
+    return nd * sizeof(double) + 6 * (kMomentBlock / 32) * sizeof(double) + 4 * sizeof(double) + sizeof(SolveShared) +
+           kPlainChunk * sizeof(unsigned short) + (kMomentBlock / 32) * sizeof(int) + 16;
 }
 
-__global__ void __launch_bounds__(kMomentBlock) k_moments(MomentArgs a0, MomentBatch batch)
+__global__ void __launch_bounds__(kMomentBlock, 2) k_moments(MomentArgs a0, MomentBatch batch, PlainWork work)
 {
     extern __shared__ double sm[];
-    MomentArgs a = a0;
-    int bid = blockIdx.x;
-    if (batch.n > 0) {
-        const int m = batch_model(batch.block_start, batch.n, bid);
-        a = batch.args[m];
-        bid -= batch.block_start[m];
-    }
-    const int nr = a.P.nr, npoly = a.P.npoly, nt = nr * npoly;
-    double *s_ar = sm, *s_phil = s_ar + nr, *s_Pr = s_phil + nt, *s_Pr2 = s_Pr + nt;
-    double *s_Eg = s_Pr2 + nt, *s_Dg = s_Eg + a.ngrid, *s_xq = s_Dg + a.ngrid, *s_wq = s_xq + a.nq;
-    double *s_glx = s_wq + a.nq, *s_glw = s_glx + a.gl.n, *s_red = s_glw + a.gl.n;
-    double *s_pt = s_red + 6 * (kMomentBlock / 32), *s_df = s_pt + 4;
-    float *s_key = (float *)(s_df + kPlainChunk);
-    unsigned short *s_list = (unsigned short *)(s_key + kPlainChunk);
-    int *s_wc = (int *)(((uintptr_t)(s_list + kPlainChunk) + 15) & ~(uintptr_t)15), *s_next = s_wc + kMomentBlock / 32;
-    for (int i = threadIdx.x; i < nr; i += blockDim.x) s_ar[i] = a.P.ar[i];
-    for (int i = threadIdx.x; i < nt; i += blockDim.x) {
-        s_phil[i] = a.P.phil[i]; s_Pr[i] = a.P.Pr[i]; s_Pr2[i] = a.P.Pr2[i];
-    }
-    for (int i = threadIdx.x; i < a.ngrid; i += blockDim.x) { s_Eg[i] = a.Eg[i]; s_Dg[i] = a.Dg[i]; }
-    for (int i = threadIdx.x; i < a.nq; i += blockDim.x) { s_xq[i] = a.xq[i]; s_wq[i] = a.wq[i]; }
-    for (int i = threadIdx.x; i < a.gl.n; i += blockDim.x) { s_glx[i] = a.gl.x01[i]; s_glw[i] = a.gl.w01[i]; }
-    __syncthreads();
-
-    const PotView P{nr, npoly, s_ar, s_phil, s_Pr, s_Pr2};
-    const GLRule gl{a.gl.n, s_glx, s_glw};
-    const int B = a.blocks_per_point;
-    const int p = bid / B, chunk = bid % B;
-    const int nq = a.nq, nq2 = nq * nq, nq3 = nq2 * nq;
-    const int n0 = chunk * kPlainChunk, n1 = min(n0 + kPlainChunk, nq3);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) {  // the point (integ/Integ.cpp:150-151)
-        double R, z;
-        if (a.Rz) { R = a.Rz[2 * p]; z = a.Rz[2 * p + 1]; }
-        else {
-            const int n = p / a.ngauss, g = p % a.ngauss;
-            const double c = a.ci[g], si = sqrt(1 - c * c);
-            R = s_ar[n] * si; z = s_ar[n] * c;
+    __shared__ int s_item;
+    int model = -1;  // whose tables are in shared memory
+    for (;;) {
+        __syncthreads();  // every thread is done with the previous item's shared data
+        if (threadIdx.x == 0) s_item = (int)atomicAdd(work.next, 1u);
+        __syncthreads();
+        int bid = s_item;
+        if (bid >= work.total) return;
+        int m = 0;
+        if (batch.n > 0) {
+            m = batch_model(batch.block_start, batch.n, bid);
+            bid -= batch.block_start[m];
         }
-        const double Phi_h = pot_phi(P, R, z), rmax = s_ar[nr - 1];
-        s_pt[0] = R; s_pt[1] = z; s_pt[2] = Phi_h;
-        s_pt[3] = sqrt(-2 * (Phi_h - pot_phi(P, 10 * rmax, 10 * rmax)));
-        *s_next = kMomentBlock;
-    }
-    __syncthreads();
-    const double R = s_pt[0], z = s_pt[1], Phi_h = s_pt[2], Ve = s_pt[3];
-    auto velocity = [&](int node, double &V0, double &V1, double &V2) {
-        V0 = 1e-6 + Ve * s_xq[node / nq2]; V1 = 1e-6 + Ve * s_xq[(node / nq) % nq]; V2 = 1e-6 + Ve * s_xq[node % nq];
-    };
-    // bound nodes of [n0, n1) in node order
-    int nbound = 0;
-    for (int base = n0; base < n1; base += kMomentBlock) {
-        const int node = base + threadIdx.x;
-        bool b = false;
-        if (node < n1) {
+        const MomentArgs &a = batch.n > 0 ? batch.args[m] : a0;
+        const int nr = a.P.nr, npoly = a.P.npoly, nt = nr * npoly;
+        double *s_ar = sm, *s_phil = s_ar + nr, *s_Pr = s_phil + nt, *s_it = s_Pr + nt;
+        double *s_Eg = s_it + interp_table_size(nr), *s_Dg = s_Eg + a.ngrid,
+               *s_xq = s_Dg + a.ngrid, *s_wq = s_xq + a.nq;
+        double *s_glx = s_wq + a.nq, *s_glw = s_glx + a.gl.n, *s_red = s_glw + a.gl.n;
+        double *s_pt = s_red + 6 * (kMomentBlock / 32);
+        SolveShared *s_solve = (SolveShared *)(s_pt + 4);
+        float *s_key = (float *)s_solve->vals;  // until the solves
+        unsigned short *s_list = (unsigned short *)(s_solve + 1);
+        int *s_wc = (int *)(((uintptr_t)(s_list + kPlainChunk) + 15) & ~(uintptr_t)15);
+        if (m != model) {
+            model = m;
+            for (int i = threadIdx.x; i < nr; i += blockDim.x) s_ar[i] = a.P.ar[i];
+            for (int i = threadIdx.x; i < nt; i += blockDim.x) { s_phil[i] = a.P.phil[i]; s_Pr[i] = a.P.Pr[i]; }
+            for (int i = threadIdx.x; i < a.ngrid; i += blockDim.x) { s_Eg[i] = a.Eg[i]; s_Dg[i] = a.Dg[i]; }
+            for (int i = threadIdx.x; i < a.nq; i += blockDim.x) { s_xq[i] = a.xq[i]; s_wq[i] = a.wq[i]; }
+            for (int i = threadIdx.x; i < a.gl.n; i += blockDim.x) { s_glx[i] = a.gl.x01[i]; s_glw[i] = a.gl.w01[i]; }
+            __syncthreads();
+            interp_table(nr, s_ar, s_it, threadIdx.x, blockDim.x);
+            __syncthreads();
+        }
+        const PotView P{nr, npoly, s_ar, s_phil, s_Pr, a.P.Pr2, s_it};
+        const GLRule gl{a.gl.n, s_glx, s_glw};
+        const int B = a.blocks_per_point;
+        const int p = bid / B, chunk = bid % B;
+        const int nq = a.nq, nq2 = nq * nq, nq3 = nq2 * nq;
+        const int n0 = chunk * a.plain_chunk, n1 = min(n0 + a.plain_chunk, nq3);
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        if (threadIdx.x == 0) {  // the point (integ/Integ.cpp:150-151)
+            double R, z;
+            if (a.Rz) { R = a.Rz[2 * p]; z = a.Rz[2 * p + 1]; }
+            else {
+                const int n = p / a.ngauss, g = p % a.ngauss;
+                const double c = a.ci[g], si = sqrt(1 - c * c);
+                R = s_ar[n] * si; z = s_ar[n] * c;
+            }
+            const double Phi_h = pot_phi(P, R, z), rmax = s_ar[nr - 1];
+            s_pt[0] = R; s_pt[1] = z; s_pt[2] = Phi_h;
+            s_pt[3] = sqrt(-2 * (Phi_h - pot_phi(P, 10 * rmax, 10 * rmax)));
+        }
+        __syncthreads();
+        const double R = s_pt[0], z = s_pt[1], Phi_h = s_pt[2], Ve = s_pt[3];
+        auto velocity = [&](int node, double &V0, double &V1, double &V2) {
+            V0 = 1e-6 + Ve * s_xq[node / nq2]; V1 = 1e-6 + Ve * s_xq[(node / nq) % nq]; V2 = 1e-6 + Ve * s_xq[node % nq];
+        };
+        // bound nodes of [n0, n1) in node order
+        int nbound = 0;
+        for (int base = n0; base < n1; base += kMomentBlock) {
+            const int node = base + threadIdx.x;
+            bool b = false;
+            if (node < n1) {
+                double V0, V1, V2;
+                velocity(node, V0, V1, V2);
+                b = .5 * (V0 * V0 + V1 * V1 + V2 * V2) + Phi_h < 0;
+            }
+            const unsigned bal = __ballot_sync(0xffffffffu, b);
+            if (lane == 0) s_wc[warp] = __popc(bal);
+            __syncthreads();
+            int off = nbound, tot = 0;
+            for (int w = 0; w < kMomentBlock / 32; w++) {
+                if (w < warp) off += s_wc[w];
+                tot += s_wc[w];
+            }
+            if (b) s_list[off + __popc(bal & ((1u << lane) - 1u))] = (unsigned short)(node - n0);
+            __syncthreads();
+            nbound += tot;
+        }
+        for (int q = threadIdx.x; q < nbound; q += kMomentBlock) {
+            const int node = n0 + s_list[q];
+            s_key[q] = node_cost_key((float)s_xq[node / nq2], (float)s_xq[(node / nq) % nq], (float)s_xq[node % nq]);
+        }
+        sort_list(s_list, s_key, nbound);
+        // the orbits of the list
+        const SolveScratch S = solve_scratch(work.scratch + blockIdx.x * work.per_block, kPlainChunk);
+        solve_orbits64(P, gl, a.trig, nbound, S, *s_solve,
+                       [&](int q, double &Delta, double &R_, double &z_, double &Phi_, double &V0, double &V1, double &V2) {
+                           velocity(n0 + s_list[q], V0, V1, V2);
+                           const double H = .5 * (V0 * V0 + V1 * V1 + V2 * V2) + Phi_h;
+                           Delta = deltafn(s_Eg, s_Dg, a.ngrid, H);
+                           R_ = R; z_ = z; Phi_ = Phi_h;
+                       });
+        FailTally tally;
+        double mm[6] = {0, 0, 0, 0, 0, 0};
+        const double jacob = Ve * Ve * Ve;
+        for (int q = threadIdx.x; q < nbound; q += kMomentBlock) {
+            const int node = n0 + s_list[q];
             double V0, V1, V2;
             velocity(node, V0, V1, V2);
-            b = .5 * (V0 * V0 + V1 * V1 + V2 * V2) + Phi_h < 0;
+            const OrbitRec &o = S.rec[q];
+            unsigned fail = o.status();
+            double DF = df_value(a.df, P, R, o.Jr, o.Jz, R * V1, fail);
+            if (fail & (kFailBracket | kFailRoot)) DF = 0.;
+            tally.add(fail);
+            const double w = s_wq[node / nq2] * s_wq[(node / nq) % nq] * s_wq[node % nq];
+            const double jd = jacob * DF;
+            mm[0] += w * jd;
+            mm[1] += w * (jd * V1);
+            mm[2] += w * (jd * V0 * V0);
+            mm[3] += w * (jd * V1 * V1);
+            mm[4] += w * (jd * V2 * V2);
+            mm[5] += w * (jd * V0 * V2);
         }
-        const unsigned bal = __ballot_sync(0xffffffffu, b);
-        if (lane == 0) s_wc[warp] = __popc(bal);
-        __syncthreads();
-        int off = nbound, tot = 0;
-        for (int w = 0; w < kMomentBlock / 32; w++) {
-            if (w < warp) off += s_wc[w];
-            tot += s_wc[w];
-        }
-        if (b) s_list[off + __popc(bal & ((1u << lane) - 1u))] = (unsigned short)(node - n0);
-        __syncthreads();
-        nbound += tot;
-    }
-    for (int q = threadIdx.x; q < nbound; q += kMomentBlock) {
-        const int node = n0 + s_list[q];
-        s_key[q] = node_cost_key((float)s_xq[node / nq2], (float)s_xq[(node / nq) % nq], (float)s_xq[node % nq]);
-    }
-    sort_list(s_list, s_key, nbound);
-    // the solves, nodes taken as threads free up
-    FailTally tally;
-    for (int q = threadIdx.x; q < nbound;) {
-        const int node = n0 + s_list[q];
-        double V0, V1, V2;
-        velocity(node, V0, V1, V2);
-        const double H = .5 * (V0 * V0 + V1 * V1 + V2 * V2) + Phi_h;
-        unsigned fail = 0;
-        double Jr, Jz;
-        fudge_actions(P, deltafn(s_Eg, s_Dg, a.ngrid, H), R, z, Phi_h, V0, V1, V2, gl, Jr, Jz, fail);
-        double DF = df_value(a.df, P, R, Jr, Jz, R * V1, fail);
-        if (fail & (kFailBracket | kFailRoot)) DF = 0.;
-        tally.add(fail);
-        s_df[q] = DF;
-        q = atomicAdd(s_next, 1);
-    }
-    __syncthreads();
-    double m[6] = {0, 0, 0, 0, 0, 0};
-    const double jacob = Ve * Ve * Ve;
-    for (int q = threadIdx.x; q < nbound; q += kMomentBlock) {
-        const int node = n0 + s_list[q];
-        double V0, V1, V2;
-        velocity(node, V0, V1, V2);
-        const double w = s_wq[node / nq2] * s_wq[(node / nq) % nq] * s_wq[node % nq];
-        const double jd = jacob * s_df[q];
-        m[0] += w * jd;
-        m[1] += w * (jd * V1);
-        m[2] += w * (jd * V0 * V0);
-        m[3] += w * (jd * V1 * V1);
-        m[4] += w * (jd * V2 * V2);
-        m[5] += w * (jd * V0 * V2);
-    }
-    // block reduction in a fixed order
+        // block reduction in a fixed order
 #pragma unroll
-    for (int q = 0; q < 6; q++) {
-        const double v = warp_sum(m[q]);
-        if (lane == 0) s_red[warp * 6 + q] = v;
+        for (int q = 0; q < 6; q++) {
+            const double v = warp_sum(mm[q]);
+            if (lane == 0) s_red[warp * 6 + q] = v;
+        }
+        warp_count_fails(a.counters, tally);
+        __syncthreads();
+        if (threadIdx.x < 6) {
+            double s = 0;
+            for (int w = 0; w < kMomentBlock / 32; w++) s += s_red[w * 6 + threadIdx.x];
+            a.partial[((size_t)p * B + chunk) * 6 + threadIdx.x] = s;
+        }
+        if (threadIdx.x == 0 && nbound) atomicAdd(&a.counters[kCntBound], (unsigned long long)nbound);
     }
-    warp_count_fails(a.counters, tally);
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        double s = 0;
-        for (int w = 0; w < kMomentBlock / 32; w++) s += s_red[w * 6 + threadIdx.x];
-        a.partial[((size_t)p * B + chunk) * 6 + threadIdx.x] = s;
-    }
-    if (threadIdx.x == 0 && nbound) atomicAdd(&a.counters[kCntBound], (unsigned long long)nbound);
 }
+
+static int resident_blocks(const void *kernel, size_t smem)
+{
+    int dev = 0, nsm = 0, per_sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        (smem > 48 * 1024 &&
+         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSolveBlock, smem) != cudaSuccess)
+        return 0;
+    return per_sm * nsm;
+}
+
+int moments_resident(size_t smem) { return resident_blocks((const void *)k_moments, smem); }
 
 // sums the per-block partials of each point and normalises as rhofDF does
 // (integ/Integ.cpp:160-162)
@@ -210,29 +273,21 @@ cudaError_t launch_moments_finalize_batch(const MomentBatch &b, int npoints, cud
     return cudaGetLastError();
 }
 
-cudaError_t launch_moments(const MomentArgs &a, cudaStream_t s)
-{
-    const size_t smem = moment_smem_bytes(a);
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_moments, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
-    const long long nblocks = (long long)a.npts * a.blocks_per_point;
-    k_moments<<<(unsigned)nblocks, kMomentBlock, smem, s>>>(a, MomentBatch{nullptr, nullptr, nullptr, 0});
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    return launch_moments_finalize(a, s);
-}
-
-cudaError_t launch_moments_plain_batch(const MomentArgs &a0, const MomentBatch &b, int nblocks, size_t smem,
+cudaError_t launch_moments_plain_batch(const MomentArgs &a0, const MomentBatch &b, size_t smem, const PlainWork &w,
                                       cudaStream_t s)
 {
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_moments, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
-    k_moments<<<(unsigned)nblocks, kMomentBlock, smem, s>>>(a0, b);
+    if (w.grid < 1) return cudaErrorInvalidConfiguration;
+    const cudaError_t e = cudaMemsetAsync(w.next, 0, sizeof(unsigned), s);
+    if (e != cudaSuccess) return e;
+    k_moments<<<(unsigned)w.grid, kMomentBlock, smem, s>>>(a0, b, w);
     return cudaGetLastError();
+}
+
+cudaError_t launch_moments(const MomentArgs &a, const PlainWork &w, cudaStream_t s)
+{
+    const cudaError_t e =
+        launch_moments_plain_batch(a, MomentBatch{nullptr, nullptr, nullptr, 0}, moment_smem_bytes(a), w, s);
+    return e == cudaSuccess ? launch_moments_finalize(a, s) : e;
 }
 
 cudaError_t launch_moments_finalize(const MomentArgs &a, cudaStream_t s)
@@ -242,46 +297,137 @@ cudaError_t launch_moments_finalize(const MomentArgs &a, cudaStream_t s)
 }
 
 // ---------------------------------------------------------------- actions
-__global__ void k_actions(PotView P, const double *Eg, const double *Dg, int ngrid, GLRule gl,
-                          const double *pts, size_t n, double *out)
+// Work items of `chunk` consecutive points; unbound points (H >= 0) give -1, -1
+__global__ void __launch_bounds__(kSolveBlock, 2) k_actions(PotView P0, const double *Eg, const double *Dg, int ngrid,
+                                                            GLRule gl0, const double2 *trig, const double *pts,
+                                                            size_t n, int chunk, double *out, bool staged,
+                                                            PlainWork work)
 {
-    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    const double R = pts[5 * t], z = pts[5 * t + 1], vR = pts[5 * t + 2], vp = pts[5 * t + 3], vz = pts[5 * t + 4];
-    const double Phi = pot_phi(P, R, z);
-    const double H = .5 * (vR * vR + vp * vp + vz * vz) + Phi;
-    if (H >= 0) { out[2 * t] = -1; out[2 * t + 1] = -1; return; }
-    double Jr, Jz;
-    unsigned fail = 0;
-    fudge_actions(P, deltafn(Eg, Dg, ngrid, H), R, z, Phi, vR, vp, vz, gl, Jr, Jz, fail);
-    out[2 * t] = Jr;
-    out[2 * t + 1] = Jz;
+    extern __shared__ double sm[];  // solver | tables (staged: of a size that fits; else read in device memory)
+    __shared__ int s_item, s_n;
+    __shared__ unsigned short s_list[kActionChunk];
+    __shared__ double s_pot[kActionChunk];
+    const int nr = P0.nr, npoly = P0.npoly, nt = nr * npoly;
+    SolveShared *s_solve = (SolveShared *)sm;
+    double *s_ar = (double *)(s_solve + 1), *s_phil = s_ar + nr, *s_Pr = s_phil + nt, *s_it = s_Pr + nt,
+           *s_Eg = s_it + interp_table_size(nr), *s_Dg = s_Eg + ngrid;
+    PotView P = P0;
+    if (staged) {
+        for (int i = threadIdx.x; i < nr; i += blockDim.x) s_ar[i] = P0.ar[i];
+        for (int i = threadIdx.x; i < nt; i += blockDim.x) { s_phil[i] = P0.phil[i]; s_Pr[i] = P0.Pr[i]; }
+        for (int i = threadIdx.x; i < ngrid; i += blockDim.x) { s_Eg[i] = Eg[i]; s_Dg[i] = Dg[i]; }
+        __syncthreads();
+        interp_table(nr, s_ar, s_it, threadIdx.x, blockDim.x);
+        P = PotView{nr, npoly, s_ar, s_phil, s_Pr, P0.Pr2, s_it};
+        Eg = s_Eg; Dg = s_Dg;
+    }
+    const SolveScratch S = solve_scratch(work.scratch + blockIdx.x * work.per_block, kActionChunk);
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) { s_item = (int)atomicAdd(work.next, 1u); s_n = 0; }
+        __syncthreads();
+        const int item = s_item;
+        if (item >= work.total) return;
+        const size_t t0 = (size_t)item * chunk;
+        const int m = (int)(n - t0 < (size_t)chunk ? n - t0 : (size_t)chunk);
+        for (int i = threadIdx.x; i < m; i += blockDim.x) {
+            const double *x = pts + 5 * (t0 + i);
+            const double Phi = pot_phi(P, x[0], x[1]);
+            if (.5 * (x[2] * x[2] + x[3] * x[3] + x[4] * x[4]) + Phi >= 0) {
+                out[2 * (t0 + i)] = -1;
+                out[2 * (t0 + i) + 1] = -1;
+            } else {
+                s_pot[i] = Phi;
+                s_list[atomicAdd(&s_n, 1)] = (unsigned short)i;
+            }
+        }
+        __syncthreads();
+        solve_orbits64(P, gl0, trig, s_n, S, *s_solve,
+                       [&](int q, double &Delta, double &R, double &z, double &Phi, double &vR, double &vp, double &vz) {
+                           const double *x = pts + 5 * (t0 + s_list[q]);
+                           R = x[0]; z = x[1]; vR = x[2]; vp = x[3]; vz = x[4];
+                           Phi = s_pot[s_list[q]];
+                           Delta = deltafn(Eg, Dg, ngrid, .5 * (vR * vR + vp * vp + vz * vz) + Phi);
+                       });
+        for (int q = threadIdx.x; q < s_n; q += blockDim.x) {
+            const size_t t = t0 + s_list[q];
+            out[2 * t] = S.rec[q].Jr;
+            out[2 * t + 1] = S.rec[q].Jz;
+        }
+    }
 }
 
-cudaError_t launch_actions(PotView P, const double *Eg, const double *Dg, int ngrid, GLRule gl,
-                           const double *pts, size_t n, double *out, cudaStream_t s)
+// tables beyond this size stay in device memory (two blocks per SM still fit)
+constexpr size_t kStagedTables = 96 * 1024;
+static size_t actions_table_bytes(int nr, int npoly, int ngrid)
+{
+    return (nr + 2 * (size_t)nr * npoly + interp_table_size(nr) + 2 * (size_t)ngrid) * sizeof(double);
+}
+size_t actions_smem_bytes(int nr, int npoly, int ngrid)
+{
+    const size_t t = actions_table_bytes(nr, npoly, ngrid);
+    return sizeof(SolveShared) + (t <= kStagedTables ? t : 0);
+}
+
+int actions_resident(size_t smem) { return resident_blocks((const void *)k_actions, smem); }
+
+cudaError_t launch_actions(PotView P, const double *Eg, const double *Dg, int ngrid, GLRule gl, const double2 *trig,
+                           const double *pts, size_t n, int chunk, double *out, const PlainWork &w, cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
-    k_actions<<<(unsigned)((n + 63) / 64), 64, 0, s>>>(P, Eg, Dg, ngrid, gl, pts, n, out);
+    if (w.grid < 1 || chunk > kActionChunk) return cudaErrorInvalidConfiguration;
+    const cudaError_t e = cudaMemsetAsync(w.next, 0, sizeof(unsigned), s);
+    if (e != cudaSuccess) return e;
+    const bool staged = actions_table_bytes(P.nr, P.npoly, ngrid) <= kStagedTables;
+    k_actions<<<(unsigned)w.grid, kSolveBlock, actions_smem_bytes(P.nr, P.npoly, ngrid), s>>>(
+        P, Eg, Dg, ngrid, gl, trig, pts, n, chunk, out, staged, w);
     return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------- potential
-__global__ void k_potential_eval(PotView P, const double *Rz, size_t n, double *out)
+// Grid-stride over the points; the tables and interpolation constants staged in
+// shared memory once per block where they fit (the FP64 pipe is the bound: ~400
+// FP64 instructions per point at l <= 12).  200 003 points, 80 x 7 tables: 367
+// us with a division per recurrence step and a bisection search per point, 253
+// us with the reciprocals and the interval guess of interp_setup.
+constexpr int kPotBlock = 256;
+constexpr size_t kPotStaged = 40 * 1024;
+static size_t potential_smem_bytes(const PotView &P)
 {
-    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    double phi, dR, dz;
-    pot_grad(P, Rz[2 * t], Rz[2 * t + 1], phi, dR, dz);
-    out[3 * t] = phi;
-    out[3 * t + 1] = dR;
-    out[3 * t + 2] = dz;
+    return (P.nr + 2 * (size_t)P.nr * P.npoly + interp_table_size(P.nr)) * sizeof(double);
+}
+
+__global__ void __launch_bounds__(kPotBlock) k_potential_eval(PotView P, const double *Rz, size_t n, double *out,
+                                                              bool staged)
+{
+    extern __shared__ double sm[];
+    if (staged) {
+        const int nr = P.nr, nt = nr * P.npoly;
+        double *s_ar = sm, *s_phil = s_ar + nr, *s_Pr = s_phil + nt, *s_it = s_Pr + nt;
+        for (int i = threadIdx.x; i < nr; i += blockDim.x) s_ar[i] = P.ar[i];
+        for (int i = threadIdx.x; i < nt; i += blockDim.x) { s_phil[i] = P.phil[i]; s_Pr[i] = P.Pr[i]; }
+        __syncthreads();
+        interp_table(nr, s_ar, s_it, threadIdx.x, blockDim.x);
+        __syncthreads();
+        P = PotView{nr, P.npoly, s_ar, s_phil, s_Pr, P.Pr2, s_it};
+    }
+    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
+        double phi, dR, dz;
+        pot_grad(P, Rz[2 * t], Rz[2 * t + 1], phi, dR, dz);
+        out[3 * t] = phi;
+        out[3 * t + 1] = dR;
+        out[3 * t + 2] = dz;
+    }
 }
 
 cudaError_t launch_potential_eval(PotView P, const double *Rz, size_t n, double *out, cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
-    k_potential_eval<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(P, Rz, n, out);
+    const size_t tab = potential_smem_bytes(P), blocks = (n + kPotBlock - 1) / kPotBlock;
+    const bool staged = tab <= kPotStaged;
+    const size_t most = staged ? 4 * 152 : 0x7fffffff;  // staged: one wave, each block's tables serve all its points
+    k_potential_eval<<<(unsigned)(blocks < most ? blocks : most), kPotBlock, staged ? tab : 0, s>>>(P, Rz, n, out,
+                                                                                                 staged);
     return cudaGetLastError();
 }
 

@@ -583,13 +583,14 @@ cudaError_t launch_moments_mixed(const MomentArgs &a, int variant, const DeferWo
     return launch_moments_finalize(a, s);
 }
 
-cudaError_t launch_moments_plain_batch(const MomentArgs &a0, const MomentBatch &b, int nblocks, size_t smem,
+cudaError_t launch_moments_plain_batch(const MomentArgs &a0, const MomentBatch &b, size_t smem, const PlainWork &w,
                                       cudaStream_t s);
 
 cudaError_t launch_moments_batch(const MomentArgs &a0, const MomentBatch &b, int nblocks, size_t smem, bool mixed,
-                                 int variant, const DeferWork &dw, const ItemQueue &q, cudaStream_t s)
+                                 int variant, const DeferWork &dw, const ItemQueue &q, const PlainWork &w,
+                                 cudaStream_t s)
 {
-    if (!mixed) return launch_moments_plain_batch(a0, b, nblocks, smem, s);
+    if (!mixed) return launch_moments_plain_batch(a0, b, smem, w, s);
     if (q.total != nblocks) return cudaErrorInvalidValue;
     const cudaError_t e = launch_mixed_any(a0, b, q, smem, variant, s);
     return e == cudaSuccess ? launch_deferred(a0, b, nblocks, dw, s) : e;

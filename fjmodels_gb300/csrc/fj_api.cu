@@ -49,13 +49,14 @@ struct fj_ctx {
     std::map<int, DevBuf> gl_rules;                    // jquad -> [2][n]
     std::vector<double> rule_host;                     // last uploaded velocity rule
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    int mixed_variant = 0, mixed_chunk = kMixedMaxNodes;  // mixed kernel configuration (fj_autotune_mixed)
+    int mixed_variant = 7, mixed_chunk = 1024;         // mixed kernel configuration (fj_autotune_mixed)
     int poisson = FJ_POISSON_QAGS;                     // radial integrals of fj_poisson (fj_set_poisson)
     float *jout = nullptr;                             // mixed form: actions of every bound node (fj_set_action_output)
     DevBuf batch;                                      // batched launch: MomentArgs[n] | block_start | point_start
     std::vector<char> batch_host;                      // what `batch` holds (re-uploaded only when it changes)
     DevBuf delta_ws;                                   // GPU focal-distance tables: views | Eg ptrs | Dg ptrs | flags
     DevBuf trig;                                       // FP64 form: quadrature-angle table (MomentArgs::trig)
+    DevBuf mixed_ws;                                   // mixed form: blocks' scratch
     DevBuf plain;                                      // FP64 form: work counter | blocks' scratch (PlainWork)
     DevBuf queue;                                      // mixed kernel's work queue: counter | order | costs
     int q_total = 0;                                   // items of the launch whose costs the queue holds
@@ -100,23 +101,23 @@ int ensure(fj_ctx *ctx, DevBuf &b, size_t bytes)
 }
 
 // Scratch of the mixed form's FP64 pass over capped nodes for a launch of
-// nblocks blocks (nw bitmap words each) and `nodes` phase-space nodes, in one
+// nblocks blocks (`words` bitmap words together) and `nodes` phase-space nodes, in one
 // buffer: bitmaps | counts | offsets | scan carries | list (nodes, blocks,
 // moments).  The list holds 1/256 of the nodes (at least 64 Ki, at most 4 Mi
 // entries); a launch that leaves more is still exact (the extra nodes are
 // solved by their block's adding thread), only slower.
-int defer_setup(fj_ctx *ctx, long long nblocks, int nw, long long nodes, DeferWork &dw, unsigned *&bitmaps)
+int defer_setup(fj_ctx *ctx, long long nblocks, size_t words, long long nodes, DeferWork &dw, unsigned *&bitmaps)
 {
     const long long nchunks = (nblocks + kScanChunk - 1) / kScanChunk;
     long long cap = nodes / 256;
     cap = cap < 65536 ? 65536 : (cap > (4ll << 20) ? (4ll << 20) : cap);
-    const size_t ints = (size_t)nblocks * nw + 2 * (size_t)nblocks + nchunks + 2 + 2 * (size_t)cap;
+    const size_t ints = words + 2 * (size_t)nblocks + nchunks + 2 + 2 * (size_t)cap;
     const size_t off_mom = (ints * sizeof(int) + 15) / 16 * 16;
     int rc = ensure(ctx, ctx->defer, off_mom + (size_t)cap * 6 * sizeof(double));
     if (rc) return rc;
     int *base = (int *)ctx->defer.p;
     bitmaps = (unsigned *)base;
-    dw.count = base + (size_t)nblocks * nw;
+    dw.count = base + words;
     dw.offset = dw.count + nblocks;
     dw.chunk_sum = dw.offset + nblocks;
     dw.node = dw.chunk_sum + nchunks + 2;
@@ -152,7 +153,7 @@ int refresh_queue_order(fj_ctx *ctx)
     return FJ_OK;
 }
 
-int queue_setup(fj_ctx *ctx, long long total, ItemQueue &q)
+int queue_setup(fj_ctx *ctx, long long total, int stride, const MixedSmem &sm, ItemQueue &q)
 {
     if (total < 1 || total > 0x7fffffffLL) return fail(ctx, FJ_ERR_ARG, "moments: too many work items");
     const int n = (int)total;
@@ -173,6 +174,21 @@ int queue_setup(fj_ctx *ctx, long long total, ItemQueue &q)
     q.order = ctx->q_order ? order : nullptr;
     q.cost = (float *)(order + n);
     q.total = n;
+    int turn, integrate;
+    mixed_resident(ctx->mixed_variant, sm, turn, integrate);
+    if (turn < 1 || integrate < 1) return fail(ctx, FJ_ERR_CUDA, "moments: tables exceed shared memory");
+    q.grid_turn = n < turn ? n : turn;
+    q.grid = n < integrate ? n : integrate;
+    q.stride = stride;
+    q.per_slice = (int)std::min<long long>(n, std::max<long long>(1, kMixedSliceNodes / stride));
+    const size_t rec = (size_t)q.per_slice * stride * mixed_rec_bytes(), pt = (size_t)q.per_slice * 4 * sizeof(double),
+                 nb = ((size_t)q.per_slice * sizeof(int) + 15) / 16 * 16;
+    int rc = ensure(ctx, ctx->mixed_ws, rec + pt + nb + q.grid * mixed_scratch_bytes());
+    if (rc) return rc;
+    q.rec = (char *)ctx->mixed_ws.p;
+    q.point = (double *)(q.rec + rec);
+    q.nbound = (int *)(q.rec + rec + pt);
+    q.scratch = q.rec + rec + pt + nb;
     ctx->q_costs = true;  // this launch records them
     ctx->q_launches++;
     return FJ_OK;
@@ -372,7 +388,7 @@ int build_args(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delta
         a.ci = gn;
     }
     const long long nq3 = (long long)rule->nq * rule->nq * rule->nq;
-    a.mixed_chunk = ctx->mixed_chunk;
+    a.mixed_chunk = plain_chunk(npts, nq3, ctx->mixed_chunk);
     if (!mixed && (rc = trig_table(ctx, &a.trig))) return rc;
     a.plain_chunk = plain_chunk(npts, nq3);
     a.blocks_per_point =
@@ -414,7 +430,7 @@ int run_moments(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delt
     DeferWork dw{};
     if (mixed) {
         const long long nb = (long long)npts * a.blocks_per_point;
-        if ((rc = defer_setup(ctx, nb, defer_words(a.mixed_chunk), (long long)npts * nq3, dw, a.defer))) return rc;
+        if ((rc = defer_setup(ctx, nb, (size_t)nb * defer_words(a.mixed_chunk), (long long)npts * nq3, dw, a.defer))) return rc;
         a.defer_count = dw.count;
     }
     if ((rc = ensure(ctx, ctx->counters, kNumCounters * sizeof(unsigned long long)))) return rc;
@@ -431,7 +447,8 @@ int run_moments(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delt
     FJ_CUDA(cudaMemsetAsync(a.counters, 0, kNumCounters * sizeof(unsigned long long), ctx->stream));
     FJ_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
     ItemQueue q{};
-    if (mixed && (rc = queue_setup(ctx, (long long)npts * a.blocks_per_point, q))) return rc;
+    if (mixed && (rc = queue_setup(ctx, (long long)npts * a.blocks_per_point,
+                                   (int)((nq3 + a.blocks_per_point - 1) / a.blocks_per_point), mixed_smem(a), q))) return rc;
     FJ_CUDA(mixed ? launch_moments_mixed(a, ctx->mixed_variant, dw, q, ctx->stream)
                   : launch_moments(a, pw, ctx->stream));
     FJ_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
@@ -503,7 +520,7 @@ int fj_ctx_destroy(fj_ctx *ctx)
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     for (DevBuf *b : {&ctx->partial, &ctx->counters, &ctx->rule, &ctx->misc, &ctx->defer, &ctx->queue, &ctx->trig,
-                      &ctx->plain, &ctx->batch, &ctx->delta_ws})
+                      &ctx->plain, &ctx->mixed_ws, &ctx->batch, &ctx->delta_ws})
         if (b->p) cudaFree(b->p);
     for (auto &kv : ctx->gauss_nodes) cudaFree(kv.second.p);
     for (auto &kv : ctx->poly) cudaFree(kv.second.p);
@@ -554,6 +571,8 @@ int fj_moments_batch(fj_ctx *ctx, int n, const fj_batch_item *items, const fj_qu
     std::vector<MomentArgs> args(n);
     std::vector<int> bs(n + 1, 0), ps(n + 1, 0);
     size_t smem = 0, partial = 0, defer_words_total = 0;
+    MixedSmem msm{0, 0};
+    int stride = 1;
     bool mixed = false;
     long long nodes = 0;
     const long long nq3 = (long long)rule->nq * rule->nq * rule->nq;
@@ -576,15 +595,21 @@ int fj_moments_batch(fj_ctx *ctx, int n, const fj_batch_item *items, const fj_qu
             args[m].defer_count = reinterpret_cast<int *>((size_t)bs[m]);
             defer_words_total += (size_t)nb * defer_words(args[m].mixed_chunk);
         }
-        const size_t sm = mixed ? moment_mixed_smem_bytes(args[m]) : moment_smem_bytes(args[m]);
-        smem = sm > smem ? sm : smem;
+        if (mixed) {
+            const MixedSmem sm = mixed_smem(args[m]);
+            msm.turn = std::max(msm.turn, sm.turn);
+            msm.integrate = std::max(msm.integrate, sm.integrate);
+            stride = std::max(stride, (int)((nq3 + args[m].blocks_per_point - 1) / args[m].blocks_per_point));
+        } else {
+            smem = std::max(smem, moment_smem_bytes(args[m]));
+        }
         nodes += nq3 * npts;
     }
     int rc;
     if ((rc = ensure(ctx, ctx->partial, partial * sizeof(double)))) return rc;
     DeferWork dw{};
     unsigned *bitmaps = nullptr;
-    if (mixed && (rc = defer_setup(ctx, bs[n], defer_words(ctx->mixed_chunk), nodes, dw, bitmaps))) return rc;
+    if (mixed && (rc = defer_setup(ctx, bs[n], defer_words_total, nodes, dw, bitmaps))) return rc;
     if ((rc = ensure(ctx, ctx->counters, kNumCounters * sizeof(unsigned long long)))) return rc;
     for (int m = 0; m < n; m++) {
         args[m].partial = (double *)ctx->partial.p + reinterpret_cast<size_t>(args[m].partial);
@@ -614,8 +639,8 @@ int fj_moments_batch(fj_ctx *ctx, int n, const fj_batch_item *items, const fj_qu
     if (!mixed && (rc = plain_setup(ctx, bs[n], moments_resident(smem), kPlainChunk, pw))) return rc;
     FJ_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
     ItemQueue q{};
-    if (mixed && (rc = queue_setup(ctx, bs[n], q))) return rc;
-    FJ_CUDA(launch_moments_batch(args[0], b, bs[n], smem, mixed, ctx->mixed_variant, dw, q, pw, ctx->stream));
+    if (mixed && (rc = queue_setup(ctx, bs[n], stride, msm, q))) return rc;
+    FJ_CUDA(launch_moments_batch(args[0], b, bs[n], smem, msm, mixed, ctx->mixed_variant, dw, q, pw, ctx->stream));
     FJ_CUDA(launch_moments_finalize_batch(b, ps[n], ctx->stream));
     FJ_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
     return stats ? read_stats(ctx, nodes, stats) : FJ_OK;

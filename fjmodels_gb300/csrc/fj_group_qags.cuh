@@ -39,11 +39,12 @@ template <class T> struct alignas(4 * sizeof(T)) QagsEntry { T a, b, r, e; };
 
 // interval list, order and epsilon table of one group (in device memory, where
 // the entries in use stay in L1)
-template <class T, int CAP>
+template <class T, int CAP, bool HEAP = false>
 struct QagsList {
+    static constexpr bool kHeap = HEAP;  // whether the intervals carry their number in the bisection tree
     QagsEntry<T> iv[CAP];
     T eps[52], res3[3];
-    unsigned heap[CAP];       // interval number in the bisection tree (root 1), 0 beyond 2^31
+    unsigned heap[HEAP ? CAP : 1];  // root 1, halves of h: 2h and 2h + 1; 0 beyond 2^30
     unsigned char iord[CAP];
 };
 
@@ -102,17 +103,18 @@ __device__ __noinline__ void group_qelg(T *tab, int &n_io, T *res3, int &nres, T
 }
 
 // The state of one integral after its first panel (the first lane's registers)
-template <class T, int CAP>
+template <class T, int CAP, bool HEAP = false>
 struct GroupQags {
+    using List = QagsList<T, CAP, HEAP>;
     T area, errsum, errmax, res_ext, err_ext, correc, ertest, erlarg, small, len;
     int maxerr, nrmax, last, numrl2, nres, ktmin, ierro, iroff1, iroff2, iroff3;
     bool extrap, noext;
 
     // res0, err0: the first panel on [a, b], which did not finish the integral
-    __device__ void begin(QagsList<T, CAP> &L, T a, T b, T res0, T err0)
+    __device__ void begin(List &L, T a, T b, T res0, T err0)
     {
         L.iv[0] = QagsEntry<T>{a, b, res0, err0};
-        L.heap[0] = 1;
+        if (HEAP) L.heap[0] = 1;
         L.iord[0] = 0;
         L.eps[0] = res0;
         area = res0; errsum = err0; errmax = err0;
@@ -124,7 +126,7 @@ struct GroupQags {
         extrap = noext = false;
     }
 
-    __device__ T list_sum(const QagsList<T, CAP> &L, int n) const
+    __device__ T list_sum(const List &L, int n) const
     {
         T s = 0;
         for (int k = 0; k <= n; k++) s += L.iv[k].r;
@@ -134,13 +136,13 @@ struct GroupQags {
     // The two half panels [a1, b1], [b1, b2] of interval maxerr: results, errors
     // and their resasc.  Returns true when the integral is finished (result, and
     // full if the list had no room left), else maxerr is the next interval.
-    __device__ bool update(QagsList<T, CAP> &L, T area1, T error1, T rasc1, T area2, T error2, T rasc2, T epsabs,
+    __device__ bool update(List &L, T area1, T error1, T rasc1, T area2, T error2, T rasc2, T epsabs,
                            T epsrel, T &result, bool &full)
     {
         constexpr T EPS = QagsNum<T>::eps, TINY_ = QagsNum<T>::tiny, HUGE_ = QagsNum<T>::huge;
         const QagsEntry<T> top = L.iv[maxerr];
         const T a1 = top.a, b1 = T(0.5) * (top.a + top.b), a2 = b1, b2 = top.b;
-        const unsigned h = L.heap[maxerr], h1 = h < (1u << 30) ? 2 * h : 0u, h2 = h1 ? h1 + (h ? 1u : 0u) : 0u;
+        const unsigned h = HEAP ? L.heap[maxerr] : 0u, h1 = h < (1u << 30) ? 2 * h : 0u, h2 = h1 ? h1 + 1u : 0u;
         const T erlast = errmax;
         const T area12 = area1 + area2, erro12 = error1 + error2;
         int ier = 0;  // a class set in one bisection always ends the loop there
@@ -159,11 +161,11 @@ struct GroupQags {
         if (!(error2 > error1)) {
             L.iv[maxerr] = QagsEntry<T>{a1, b1, area1, error1};
             L.iv[last] = QagsEntry<T>{a2, b2, area2, error2};
-            L.heap[maxerr] = h1; L.heap[last] = h2;
+            if (HEAP) { L.heap[maxerr] = h1; L.heap[last] = h2; }
         } else {
             L.iv[maxerr] = QagsEntry<T>{a2, b2, area2, error2};
             L.iv[last] = QagsEntry<T>{a1, b1, area1, error1};
-            L.heap[maxerr] = h2; L.heap[last] = h1;
+            if (HEAP) { L.heap[maxerr] = h2; L.heap[last] = h1; }
         }
         {   // DQPSRT with 1-based positions
             unsigned char *iord = L.iord;

@@ -28,10 +28,10 @@ constexpr int kPlainChunk = 1024;  // most velocity nodes of one point per work 
 // there are enough items to fill the GPU and balance their uneven cost.  By the
 // model's own size alone, so that a batched launch sums in the same order.
 constexpr int kPlainItems = 1216;  // 8 per SM
-inline int plain_chunk(long long npts, long long nq3)
+inline int plain_chunk(long long npts, long long nq3, int most = kPlainChunk)
 {
-    int c = kPlainChunk;
-    while (c > 128 && npts * ((nq3 + c - 1) / c) < kPlainItems) c >>= 1;
+    int c = most;
+    while (c > 128 && npts * ((nq3 + c - 1) / c) < kPlainItems) c = c / 2 < 128 ? 128 : c / 2;
     return c;
 }
 // per-thread stack the kernels need: the QAGS interval list (kQagsCap entries
@@ -165,16 +165,26 @@ __device__ __forceinline__ int batch_model(const int *start, int n, int i)
 size_t moment_smem_bytes(const MomentArgs &a);
 cudaError_t launch_moments(const MomentArgs &a, const PlainWork &w, cudaStream_t s);
 // batched forms: grid = total blocks, smem = the largest model's
-// work queue of the persistent mixed kernel: item i is block order[i] (order
-// NULL: block i) of the launch's layout; cost[b] receives block b's cycles
+// Work queue and workspace of the mixed form's persistent kernels.  Item i is
+// block order[i] (order NULL: block i) of the launch's layout; cost[b] receives
+// block b's cycles.  The launch goes through its items in slices of per_slice,
+// whose nodes' records fit the workspace.
 struct ItemQueue {
-    unsigned *next;    // device counter, zeroed by the launch
+    unsigned *next;    // [2] device counters, zeroed by the launch
     const int *order;  // [total] or NULL
     float *cost;       // [total] or NULL
-    int total;
+    char *scratch;     // mixed_scratch_bytes() for each of the `grid` blocks
+    char *rec;         // [per_slice][stride] node records (mixed_rec_bytes() each)
+    double *point;     // [per_slice][4] R, z, Phi, escape speed of the items' points
+    int *nbound;       // [per_slice] bound nodes of the items
+    int stride;        // most nodes of an item
+    int total, per_slice;
+    int grid_turn, grid;  // blocks of the two kernels
+    int first, count;     // the slice (set per launch)
 };
-cudaError_t launch_moments_batch(const MomentArgs &a0, const MomentBatch &b, int nblocks, size_t smem, bool mixed,
-                                 int variant, const DeferWork &dw, const ItemQueue &q, const PlainWork &w,
+struct MixedSmem { size_t turn, integrate; };  // dynamic shared memory of the two kernels
+cudaError_t launch_moments_batch(const MomentArgs &a0, const MomentBatch &b, int nblocks, size_t smem,
+                                 const MixedSmem &msm, bool mixed, int variant, const DeferWork &dw, const ItemQueue &q, const PlainWork &w,
                                  cudaStream_t s);
 cudaError_t launch_moments_finalize_batch(const MomentBatch &b, int npoints, cudaStream_t s);
 // dst6[q][idx[t]] = src6[q][t] (moments of n points into a grid of npts)
@@ -205,7 +215,12 @@ constexpr int kScanChunk = 1024;  // blocks per chunk of the count scan
 constexpr int kMixedMaxNodes = 8192; // largest node range of one block (shared-memory list)
 FJ_HD int defer_words(int chunk) { return (chunk + 31) / 32; }  // bitmap words of one block
 constexpr int kMixedVariants = 8;    // builds of the mixed kernel (2 forms x 4 register budgets)
-size_t moment_mixed_smem_bytes(const MomentArgs &a);
+MixedSmem mixed_smem(const MomentArgs &a);
+size_t mixed_rec_bytes();      // per node of a slice
+size_t mixed_scratch_bytes();  // per block of the integration kernel
+void mixed_resident(int variant, const MixedSmem &sm, int &turn, int &integrate);  // blocks resident at once
+// nodes whose records a workspace holds: 2.2 GB of records at most per context
+constexpr long long kMixedSliceNodes = 20ll << 20;
 int mixed_blocks_per_point(long long nq3, int chunk);
 cudaError_t launch_moments_mixed(const MomentArgs &a, int variant, const DeferWork &dw, const ItemQueue &q,
                                  cudaStream_t s);

@@ -45,6 +45,12 @@ struct PotViewF {
     float out0, shift, lr0, idl;
     float c2pt;         // cos^2 of the polar angle of the grid point
     const float *pyl;   // P_2k(c2pt), k < npoly
+    // the kernels' tables for the evaluator (evaluator_tables_f): per radius and
+    // multipole {phil, its difference to the next radius}, and per interval with a
+    // quadratic correction and side of the third point (below, above)
+    // phil[thr] - phil[b] - f3 (phil[b+1] - phil[b])
+    const float *pd;    // [nr][npoly][2]
+    const float *pe;    // [2 kQuadIntervals][npoly]
 };
 
 // even-Legendre recurrence P_2k from P_2k-2, P_2k-4 (include/UtilsLeg.h:43-50)
@@ -70,6 +76,35 @@ FJ_HD const LegCoefF &leg_f()
     return kLegF_d;
 #else
     return kLegF_h;
+#endif
+}
+
+// FP32 products, sums and fused multiply-adds that the compiler neither
+// contracts nor takes apart: the evaluator and the panel abscissas have the same
+// bits wherever and however they are inlined (the host build has no FMA: fma_rn
+// is a product and a sum there, as everywhere in that build).
+FJ_HD float mul_rn(float x, float y)
+{
+#ifdef __CUDA_ARCH__
+    return __fmul_rn(x, y);
+#else
+    return x * y;
+#endif
+}
+FJ_HD float add_rn(float x, float y)
+{
+#ifdef __CUDA_ARCH__
+    return __fadd_rn(x, y);
+#else
+    return x + y;
+#endif
+}
+FJ_HD float fma_rn(float x, float y, float z)
+{
+#ifdef __CUDA_ARCH__
+    return __fmaf_rn(x, y, z);
+#else
+    return x * y + z;
 #endif
 }
 
@@ -123,14 +158,14 @@ FJ_HD void interp_setup_f(const PotViewF &P, float r, InterpF &I)
     while (b > 0 && r < ar[b]) --b;
     while (b < nr - 2 && r > ar[b + 1]) ++b;
     I.bot = b;
-    I.f1 = (r - ar[b]) * P.ih[b];
+    I.f1 = mul_rn(add_rn(r, -ar[b]), P.ih[b]);
     I.quad = b < kQuadIntervals;
     if (I.quad) {
         const bool lo = I.f1 < 0.5f && b > 0;
         I.thr = lo ? b - 1 : b + 2;
         const float *q = P.qc + 4 * b + (lo ? 0 : 2);
         I.q = q[0];
-        I.f2 = (r - ar[b + 1]) * (r - ar[b]) * q[0];
+        I.f2 = mul_rn(mul_rn(add_rn(r, -ar[b + 1]), add_rn(r, -ar[b])), q[0]);
         I.f3 = q[1];
     }
 }
@@ -248,9 +283,12 @@ struct DState {
     float f1, f2, f3, f1p, f2p, df1, df2, x, dc2, xe2, xp1, sum0, phipt;
 };
 
+// The arithmetic is written in explicit products, sums and FMAs: the values
+// are the same in the turning-point searches (out of line) and in the momentum
+// integrals (inlined), on any path through the optimiser.
 FJ_HD void dphi_setup(const PotViewF &P, float R, float z, float rpt, float dr2, float dc2, float Phipt, DState &s)
 {
-    const float r = sqrtf(R * R + z * z);
+    const float r = sqrtf(fma_rn(R, R, mul_rn(z, z)));
     const float *ar = P.ar;
     const int nr = P.nr;
     const float a0 = ar[0], rmax = ar[nr - 1];
@@ -261,9 +299,9 @@ FJ_HD void dphi_setup(const PotViewF &P, float R, float z, float rpt, float dr2,
     if (r >= rmax) {  // phi_l = phil[nr-1][l] (rmax/r)^(2l+1); the monopole from the unshifted table value
         s.mode = 2;
         const float xe = rmax / r;
-        s.xe2 = xe * xe;
-        s.xp1 = xe * s.xe2;
-        s.sum0 = P.out0 * xe - P.shift;
+        s.xe2 = mul_rn(xe, xe);
+        s.xp1 = mul_rn(xe, s.xe2);
+        s.sum0 = fma_rn(P.out0, xe, -P.shift);
     } else {
         const float re = fmaxf(r, a0), rpe = fmaxf(rpt, a0);
         InterpF I;
@@ -272,19 +310,19 @@ FJ_HD void dphi_setup(const PotViewF &P, float R, float z, float rpt, float dr2,
         const float ab = ar[s.b], at = ar[s.b + 1];
         s.mode = 1;
         if (rpt < rmax && rpe >= ab && rpe <= at) {
-            const float fp = (rpe - ab) * P.ih[s.b];
+            const float fp = mul_rn(add_rn(rpe, -ab), P.ih[s.b]);
             const int thr_p = (fp < 0.5f && s.b > 0) ? s.b - 1 : s.b + 2;
             if (!s.quad || thr_p == s.thr || rpe == ab || rpe == at) {
                 s.mode = 0;
                 s.f1p = fp;
-                s.f2p = s.quad ? (rpe - at) * (rpe - ab) * I.q : 0.f;
-                const float dr = (r >= a0 && rpt >= a0) ? dr2 / (r + rpt) : re - rpe;
-                s.df1 = dr * P.ih[s.b];
-                s.df2 = s.quad ? I.q * dr * (re + rpe - ab - at) : 0.f;
+                s.f2p = s.quad ? mul_rn(mul_rn(add_rn(rpe, -at), add_rn(rpe, -ab)), I.q) : 0.f;
+                const float dr = (r >= a0 && rpt >= a0) ? dr2 / add_rn(r, rpt) : add_rn(re, -rpe);
+                s.df1 = mul_rn(dr, P.ih[s.b]);
+                s.df2 = s.quad ? mul_rn(mul_rn(I.q, dr), add_rn(add_rn(add_rn(re, rpe), -ab), -at)) : 0.f;
             }
         }
     }
-    s.x = s.mode == 0 ? P.c2pt + dc2 : (z * z) / (r * r);
+    s.x = s.mode == 0 ? add_rn(P.c2pt, dc2) : mul_rn(z, z) / mul_rn(r, r);
 }
 
 // the term of multipole k: px = P_k(x), dk = P_k(x) - P_k(y), xp the
@@ -292,18 +330,25 @@ FJ_HD void dphi_setup(const PotViewF &P, float R, float z, float rpt, float dr2,
 FJ_HD void dphi_acc(const PotViewF &P, const DState &s, float &sum, int k, float px, float dk, float xp)
 {
     const int np_ = P.npoly;
+#ifdef __CUDA_ARCH__
+    const float2 vd = *(const float2 *)(P.pd + 2 * (s.b * np_ + k));
+    const float vb = vd.x, d = vd.y;
+    const float e = s.quad ? P.pe[(2 * s.b + (s.thr > s.b ? 1 : 0)) * np_ + k] : 0.f;
+#else
     const float *T = P.phil;
     const float vb = T[s.b * np_ + k], d = T[(s.b + 1) * np_ + k] - vb;
     const float e = s.quad ? T[s.thr * np_ + k] - vb - s.f3 * d : 0.f;
-    const float t = xp * px;
+#endif
+    const float t = mul_rn(xp, px);
     const bool m0 = s.mode == 0, m1 = s.mode == 1;
     const float ca = m0 ? dk : t;
-    const float cb = m0 ? s.df1 * px + s.f1p * dk : (m1 ? s.f1 * px : t);
-    const float cg = m0 ? s.df2 * px + s.f2p * dk : s.f2 * px;
-    sum += vb * ca + d * cb + e * cg;
+    const float cb = m0 ? (k == 1 ? fma_rn(s.f1p, dk, mul_rn(s.df1, px)) : fma_rn(s.df1, px, mul_rn(s.f1p, dk)))
+                        : (m1 ? mul_rn(s.f1, px) : t);
+    const float cg = m0 ? fma_rn(s.df2, px, mul_rn(s.f2p, dk)) : mul_rn(s.f2, px);
+    sum = add_rn(sum, fma_rn(e, cg, fma_rn(vb, ca, mul_rn(d, cb))));
 }
 
-FJ_HD float dphi_end(const DState &s, float sum) { return s.mode == 0 ? sum : sum - s.phipt; }
+FJ_HD float dphi_end(const DState &s, float sum) { return s.mode == 0 ? sum : add_rn(sum, -s.phipt); }
 
 // one multipole chain: Legendre recurrences of x and of the difference
 struct DChain {
@@ -314,18 +359,19 @@ struct DChain {
         dphi_acc(P, s, sum, 0, 1.f, 0.f, s.mode == 2 ? 0.f : 1.f);  // the extrapolated monopole is in sum0
         px2 = 1.f; d2 = 0.f;
         if (P.npoly > 1) {
-            px1 = 1.5f * s.x - .5f;
-            d1 = 1.5f * s.dc2;
+            px1 = fma_rn(1.5f, s.x, -.5f);
+            d1 = mul_rn(1.5f, s.dc2);
             dphi_acc(P, s, sum, 1, px1, d1, s.xp1);
         }
-        xp = s.xp1 * s.xe2;
+        xp = mul_rn(s.xp1, s.xe2);
     }
     FJ_HD void step(const PotViewF &P, const LegCoefF &L, const DState &s, int k)
     {
-        const float px = ((s.x - L.B[k]) * px1 - L.A[k] * px2) * L.C[k];
-        const float dk = ((s.x - L.B[k]) * d1 + s.dc2 * P.pyl[k - 1] - L.A[k] * d2) * L.C[k];
+        const float xb = add_rn(s.x, -L.B[k]), A = L.A[k], C = L.C[k];
+        const float px = mul_rn(fma_rn(xb, px1, -mul_rn(A, px2)), C);
+        const float dk = mul_rn(fma_rn(-A, d2, fma_rn(xb, d1, mul_rn(s.dc2, P.pyl[k - 1]))), C);
         dphi_acc(P, s, sum, k, px, dk, xp);
-        xp *= s.xe2;
+        xp = mul_rn(xp, s.xe2);
         px2 = px1; px1 = px; d2 = d1; d1 = dk;
     }
 };
@@ -409,25 +455,6 @@ FJ_HD float rescale_err_f(float err, float resabs, float resasc)
 }
 
 struct GK21f { float xgk[11], wgk[11], wg[5]; };
-
-// FP32 products and sums that are never contracted into an FMA: the panel
-// abscissas have the same bits wherever the code is compiled (device, host)
-FJ_HD float mul_rn(float x, float y)
-{
-#ifdef __CUDA_ARCH__
-    return __fmul_rn(x, y);
-#else
-    return x * y;
-#endif
-}
-FJ_HD float add_rn(float x, float y)
-{
-#ifdef __CUDA_ARCH__
-    return __fadd_rn(x, y);
-#else
-    return x + y;
-#endif
-}
 
 // The e-th (0..20) abscissa of the 21-point Gauss-Kronrod panel on [a, b], in
 // the evaluation order of gk21_f: the centre, then -/+ the Gauss-point
@@ -733,6 +760,7 @@ struct FudgeF {
     float Delta, D2, K, EC, C0, Lt, shu2, sv2, swp, svp, sinv, cosv, sinhu, coshu, pvterm;
     float rpt, Phipt;  // the point: radius and FP32 potential
     double u_pt;
+    float u_f;     // (float)u_pt
     float tb, Dt;  // Ju: centre and half-width of [t_in, t_out]
     float wt;      // Jv: turning point in w
 };
@@ -755,61 +783,66 @@ FJ_HD void fudge_geom(const FudgeF &o, int mode, float x, FGeo &G)
         float sn, cs;
         sincos_psi(x, &sn, &cs);
         fac = sn;
-        if (mode == kEvJu) { x = o.tb - o.Dt * cs; m = kEvU; }
+        if (mode == kEvJu) { x = fma_rn(-o.Dt, cs, o.tb); m = kEvU; }
         else {
-            const float w = o.wt * cs;
+            const float w = mul_rn(o.wt, cs);
             if (w <= .5f * kPIHf) { x = w; m = kEvVw; }
-            else { x = kPIHf - w; m = kEvVv; }
+            else { x = add_rn(kPIHf, -w); m = kEvVv; }
         }
     }
     G.fac = fac;
     if (m == kEvU) {
         float s, c, Ds, KE;
-        if (fabsf(x) < .5f) {  // offsets: no cancellation for |t| < 1/2
-            float st, cm1;
-            sinh_coshm1(x, st, cm1);
-            const float ds = o.sinhu * cm1 + o.coshu * st;  // sinh(u_pt + t) - sinh(u_pt)
-            s = o.sinhu + ds;
-            c = o.coshu + o.coshu * cm1 + o.sinhu * st;
-            Ds = ds * (s + o.sinhu);
-            KE = Ds * o.K + o.EC;
-        } else {  // far from the point the direct form has no cancellation
-            float cm1;
-            sinh_coshm1((float)o.u_pt + x, s, cm1);
-            c = 1.f + cm1;
-            Ds = s * s - o.shu2;
-            KE = s * s * o.K + o.C0;
+        // sinh and cosh - 1 from one expm1: of the offset t for |t| < 1/2 (no
+        // cancellation), of u_pt + t far from the point
+        const bool near = fabsf(x) < .5f;
+        const float em = expm1f(near ? x : add_rn(o.u_f, x)), h = em / mul_rn(2.f, add_rn(em, 1.f));
+        const float sh = mul_rn(h, add_rn(em, 2.f));
+        if (near) {
+            const float cm1 = mul_rn(h, em);
+            const float ds = fma_rn(o.sinhu, cm1, mul_rn(o.coshu, sh));  // sinh(u_pt + t) - sinh(u_pt)
+            s = add_rn(o.sinhu, ds);
+            c = fma_rn(o.sinhu, sh, fma_rn(o.coshu, cm1, o.coshu));
+            Ds = mul_rn(ds, add_rn(s, o.sinhu));
+            KE = fma_rn(Ds, o.K, o.EC);
+        } else {  // the direct form
+            s = sh;
+            c = fma_rn(h, em, 1.f);
+            const float ss = mul_rn(s, s);
+            Ds = add_rn(ss, -o.shu2);
+            KE = fma_rn(ss, o.K, o.C0);
         }
-        const float s2 = s * s, cv2 = o.swp * o.swp;
-        G.R = o.Delta * s * o.sinv;
-        G.z = o.Delta * c * o.cosv;
-        G.dr2 = o.D2 * Ds;
-        G.dc2 = -cv2 * o.sv2 * Ds / ((s2 + cv2) * (o.shu2 + cv2));
-        G.A = KE + (o.Lt > 0.f ? o.Lt * Ds / (s2 * o.shu2) : 0.f);
-        G.Bc = -(s2 + o.sv2);
+        const float s2 = mul_rn(s, s), cv2 = mul_rn(o.swp, o.swp);
+        G.R = mul_rn(mul_rn(o.Delta, s), o.sinv);
+        G.z = mul_rn(mul_rn(o.Delta, c), o.cosv);
+        G.dr2 = mul_rn(o.D2, Ds);
+        G.dc2 = mul_rn(mul_rn(-cv2, o.sv2), Ds) / mul_rn(add_rn(s2, cv2), add_rn(o.shu2, cv2));
+        G.A = add_rn(KE, o.Lt > 0.f ? mul_rn(o.Lt, Ds) / mul_rn(s2, o.shu2) : 0.f);
+        G.Bc = -add_rn(s2, o.sv2);
     } else {
         float sn, cs, Dv;
         sincosf(x, &sn, &cs);
         if (m == kEvVw) {  // x = w: sin v = cos w, cos v = sin w
-            Dv = (o.swp - sn) * (o.swp + sn);  // cos^2 v_pt - sin^2 w
+            Dv = mul_rn(add_rn(o.swp, -sn), add_rn(o.swp, sn));  // cos^2 v_pt - sin^2 w
             const float t_ = sn; sn = cs; cs = t_;
         } else {
-            Dv = (sn - o.svp) * (sn + o.svp);  // sin^2 v - sin^2 v_pt
+            Dv = mul_rn(add_rn(sn, -o.svp), add_rn(sn, o.svp));  // sin^2 v - sin^2 v_pt
         }
-        const float s2 = sn * sn;
-        G.R = o.Delta * o.sinhu * sn;
-        G.z = o.Delta * o.coshu * cs;
-        G.dr2 = -o.D2 * Dv;
-        G.dc2 = -(1.f + o.shu2) * o.shu2 * Dv / ((o.shu2 + cs * cs) * (o.shu2 + o.swp * o.swp));
-        G.A = Dv * (o.K + (o.Lt > 0.f ? o.Lt / (o.sv2 * s2) : 0.f)) + o.pvterm;
-        G.Bc = -(o.shu2 + s2);
+        const float s2 = mul_rn(sn, sn);
+        G.R = mul_rn(mul_rn(o.Delta, o.sinhu), sn);
+        G.z = mul_rn(mul_rn(o.Delta, o.coshu), cs);
+        G.dr2 = mul_rn(-o.D2, Dv);
+        G.dc2 = mul_rn(mul_rn(-add_rn(1.f, o.shu2), o.shu2), Dv) /
+                mul_rn(fma_rn(cs, cs, o.shu2), fma_rn(o.swp, o.swp, o.shu2));
+        G.A = fma_rn(Dv, add_rn(o.K, o.Lt > 0.f ? o.Lt / mul_rn(o.sv2, s2) : 0.f), o.pvterm);
+        G.Bc = -add_rn(o.shu2, s2);
     }
 }
 
 FJ_HD float fudge_finish(int mode, const FGeo &G, float dphi)
 {
-    const float val = G.A + G.Bc * dphi;
-    return mode >= kEvJu ? sqrtf(fmaxf(0.f, val)) * G.fac : val;
+    const float val = fma_rn(G.Bc, dphi, G.A);
+    return mode >= kEvJu ? mul_rn(sqrtf(fmaxf(0.f, val)), G.fac) : val;
 }
 
 // The one evaluator of every FP32 turning-point search and momentum
@@ -980,8 +1013,8 @@ FJ_HD void point_legendre_f(float y, int npoly, float *pyl)
 }
 
 // FP32 tables of one grid point (R, z): radii, potential multipoles shifted by
-// Phi_h, interval reciprocals, quadratic-correction constants and P_2k(c2pt);
-// threads i0, i0 + stride, ... share the work
+// Phi_h, interval reciprocals, quadratic-correction constants and P_2k(c2pt)
+// (fPr may be null: the momentum integrals need no radial derivative); threads i0, i0 + stride, ... share the work
 FJ_HD void mixed_tables_f(int nr, int npoly, const double *ar, const double *phil, const double *Pr, double Phi_h,
                           double R, double z, float *far, float *fphil, float *fPr, float *ih, float *qc, float *pyl,
                           int i0, int stride)
@@ -997,7 +1030,7 @@ FJ_HD void mixed_tables_f(int nr, int npoly, const double *ar, const double *phi
     }
     for (int i = i0; i < nr * npoly; i += stride) {
         fphil[i] = (float)(i % npoly == 0 ? phil[i] - Phi_h : phil[i]);
-        fPr[i] = (float)Pr[i];
+        if (fPr) fPr[i] = (float)Pr[i];
     }
     if (i0 == 0) point_legendre_f(point_c2_f(R, z), npoly, pyl);
 }
@@ -1015,19 +1048,41 @@ FJ_HD PotViewF mixed_view_f(int nr, int npoly, const double *ar, const double *p
     v.idl = (float)((nr - 1) / log(ar[nr - 1] / ar[0]));
     v.c2pt = point_c2_f(R, z);
     v.pyl = pyl;
+    v.pd = v.pe = nullptr;
     return v;
 }
 
-// One velocity node of the mixed form: the prolate-spheroidal transform of
-// the phase point (Uvpt.cpp:11-24) in FP64, Ju and Jv (uvOrb.cpp:226-257)
-// with FP32 turning points and QAGS, FP64 turning points at the limits, and
-// the double-power-law DF (DF.cpp:65-76,108-119) in FP32.  PF is shifted by
-// PF.shift = Phi_h (mixed_tables_f); the node's energy enters shifted too.
-// Returns the DF (NaN -> 0 as DF.cpp:105); fail gets the kFail* bits,
-// esc = 1 when the FP64 turning-point path ran; J (optional) the actions.
-FJ_HDNI double mixed_node_df(const PotView &P, const PotViewF &PF, const GK21f &K, const DFDev &d, double Delta,
-                             double R, double z, double Phi_h, double V0, double V1, double V2, unsigned &fail,
-                             unsigned &esc, double *J = nullptr)
+// The kernels' evaluator tables of PotViewF (pd, pe) from its FP32 tables, which
+// must be complete; threads i0, i0 + stride, ... share the work
+FJ_HD void evaluator_tables_f(const PotViewF &P, float *pd, float *pe, int i0, int stride)
+{
+    const int nr = P.nr, np_ = P.npoly;
+    const float *T = P.phil;
+    for (int i = i0; i < nr * np_; i += stride) {
+        pd[2 * i] = T[i];
+        pd[2 * i + 1] = i < (nr - 1) * np_ ? add_rn(T[i + np_], -T[i]) : 0.f;
+    }
+    for (int i = i0; i < 2 * kQuadIntervals * np_; i += stride) {
+        const int n = i / (2 * np_), up = (i / np_) & 1, k = i % np_, thr = up ? n + 2 : n - 1;
+        float e = 0.f;
+        if (thr >= 0 && thr < nr && n + 1 < nr) {
+            const float vb = T[n * np_ + k], d = add_rn(T[(n + 1) * np_ + k], -vb);
+            e = fma_rn(-P.qc[4 * n + (up ? 3 : 1)], d, add_rn(T[thr * np_ + k], -vb));
+        }
+        pe[i] = e;
+    }
+}
+
+// One velocity node of the mixed form up to its turning points: the
+// prolate-spheroidal transform of the phase point (Uvpt.cpp:11-24) in FP64, the
+// FP32 u and v turning points (uvOrb.cpp:131-224), in FP64 where the FP32 search
+// gives up.  PF is shifted by PF.shift = Phi_h (mixed_tables_f); the node's
+// energy enters shifted too.  o gets what the integrands need (tb, Dt, wt; Dt and
+// wt as they are, zero orbits told by ju, jv = false); fail the kFail* bits,
+// esc = 1 when the FP64 search ran.  Returns false for an unbound node.
+FJ_HDNI bool mixed_turning_points(const PotView &P, const PotViewF &PF, double Delta, double R, double z, double Phi_h,
+                                  double V0, double V1, double V2, FudgeF &o, bool &ju, bool &jv, unsigned &fail,
+                                  unsigned &esc)
 {
     const double Lz = R * V1, Lzsq = Lz * Lz;
     const double D2 = Delta * Delta, R2 = R * R, z2 = z * z, r2 = R2 + z2;
@@ -1041,71 +1096,94 @@ FJ_HDNI double mixed_node_df(const PotView &P, const PotViewF &PF, const GK21f &
     const double pu = Delta * (V0 * chu * sv + V2 * shu * cv);
     const double pv = Delta * (V0 * shu * cv - V2 * chu * sv);
     const double E = .5 * (V0 * V0 + V2 * V2) + .5 * Lzsq / R2 + Phi_h;
-    double Jr = 1e31, Jz = 1e31;
-    if (!(E >= 0 || isnan(E))) {
-        FudgeF o;
-        o.P = PF;
-        o.Delta = (float)Delta;
-        o.D2 = (float)D2;
-        o.K = (float)(.5 * (V0 * V0 + V2 * V2) + .5 * Lzsq / R2);
-        o.EC = (float)(.5 * (pu * pu) / D2);
-        o.C0 = (float)(.5 * (pu * pu) / D2 - shu2 * (.5 * (V0 * V0 + V2 * V2) + .5 * Lzsq / R2));
-        o.Lt = (float)(.5 * Lzsq / D2);
-        o.shu2 = (float)shu2;
-        o.sv2 = (float)sv2;
-        o.swp = (float)fabs(cv);
-        o.svp = (float)sqrt(sv2);
-        double sn, cs;
-        sincos(v, &sn, &cs);
-        o.sinv = (float)sn; o.cosv = (float)cs;
-        o.sinhu = (float)shu; o.coshu = (float)chu;
-        o.pvterm = (float)(.5 * (pv * pv) / D2);
-        o.u_pt = u;
-        o.rpt = (float)(Delta * sqrt(shu2 + cv2));
-        o.Phipt = pot_phi_f(PF, o.Delta * o.sinhu * o.sinv, o.Delta * o.coshu * o.cosv);
-        Fudge o64;
-        bool have64 = false;
-        const float rtwo = 1.41421356237309505f;
-        float tin, tout;
-        if (!get_turn_u_f(o, 1.0, tin, tout, fail)) {  // u limit: FP64 (uvOrb.cpp:131-201)
-            fudge64_at_point(o64, P, Delta, Lzsq, E, u, v, shu2, sv, cv, sv2, pu, pv);
-            have64 = true;
-            get_turn_u(o64, 1);
-            fail |= o64.fail;
-            tin = (float)(o64.uinner - u); tout = (float)(o64.uouter - u);
-            esc = 1u;
-        }
-        if (fabsf(tout - tin) < 1e-12f) Jr = 0;
-        else {
-            o.tb = .5f * (tin + tout);
-            o.Dt = .5f * (tout - tin);
-            const FudgeFn fju{&o, kEvJu};
-            Jr = (double)(rtwo * o.Delta * o.Dt * qags_f(fju, K, 0.f, kPIf, 1e-5f, 1e-3f, fail) / kPIf);
-        }
-        float wt;
-        if (!get_turn_v_f(o, wt, fail)) {  // v at the pole: FP64 (uvOrb.cpp:203-224)
-            if (!have64) fudge64_at_point(o64, P, Delta, Lzsq, E, u, v, shu2, sv, cv, sv2, pu, pv);
-            const double v64 = get_turn_v(o64, .5 * kPIH);
-            fail |= o64.fail;
-            wt = (float)(kPIH - v64);
-            esc = 1u;
-        }
-        if (wt < 1e-12f) Jz = 0;
-        else {
-            o.wt = wt;
-            const FudgeFn fjv{&o, kEvJv};
-            Jz = (double)(2.f * rtwo * o.Delta * wt * qags_f(fjv, K, 0.f, kPIHf, 1e-5f, 1e-3f, fail) / kPIf);
-        }
+    ju = jv = false;
+    if (E >= 0 || isnan(E)) return false;
+    o.P = PF;
+    o.Delta = (float)Delta;
+    o.D2 = (float)D2;
+    o.K = (float)(.5 * (V0 * V0 + V2 * V2) + .5 * Lzsq / R2);
+    o.EC = (float)(.5 * (pu * pu) / D2);
+    o.C0 = (float)(.5 * (pu * pu) / D2 - shu2 * (.5 * (V0 * V0 + V2 * V2) + .5 * Lzsq / R2));
+    o.Lt = (float)(.5 * Lzsq / D2);
+    o.shu2 = (float)shu2;
+    o.sv2 = (float)sv2;
+    o.swp = (float)fabs(cv);
+    o.svp = (float)sqrt(sv2);
+    double sn, cs;
+    sincos(v, &sn, &cs);
+    o.sinv = (float)sn; o.cosv = (float)cs;
+    o.sinhu = (float)shu; o.coshu = (float)chu;
+    o.pvterm = (float)(.5 * (pv * pv) / D2);
+    o.u_pt = u;
+    o.u_f = (float)u;
+    o.rpt = (float)(Delta * sqrt(shu2 + cv2));
+    o.Phipt = pot_phi_f(PF, o.Delta * o.sinhu * o.sinv, o.Delta * o.coshu * o.cosv);
+    Fudge o64;
+    bool have64 = false;
+    float tin, tout;
+    if (!get_turn_u_f(o, 1.0, tin, tout, fail)) {  // u limit: FP64 (uvOrb.cpp:131-201)
+        fudge64_at_point(o64, P, Delta, Lzsq, E, u, v, shu2, sv, cv, sv2, pu, pv);
+        have64 = true;
+        get_turn_u(o64, 1);
+        fail |= o64.fail;
+        tin = (float)(o64.uinner - u); tout = (float)(o64.uouter - u);
+        esc = 1u;
     }
-    if (J) { J[0] = Jr; J[1] = Jz; }
-    const float Jphi = (float)Lz, jr = (float)Jr, jz = (float)Jz, J0 = (float)d.J0;
+    ju = !(fabsf(tout - tin) < 1e-12f);
+    o.tb = .5f * (tin + tout);
+    o.Dt = .5f * (tout - tin);
+    float wt;
+    if (!get_turn_v_f(o, wt, fail)) {  // v at the pole: FP64 (uvOrb.cpp:203-224)
+        if (!have64) fudge64_at_point(o64, P, Delta, Lzsq, E, u, v, shu2, sv, cv, sv2, pu, pv);
+        const double v64 = get_turn_v(o64, .5 * kPIH);
+        fail |= o64.fail;
+        wt = (float)(kPIH - v64);
+        esc = 1u;
+    }
+    jv = !(wt < 1e-12f);
+    o.wt = wt;
+    return true;
+}
+
+// Jr and Jz from their integrals (uvOrb.cpp:238, 256)
+FJ_HD float mixed_jr(float Delta, float Dt, float integral) { return 1.41421356237309505f * Delta * Dt * integral / kPIf; }
+FJ_HD float mixed_jz(float Delta, float wt, float integral)
+{
+    return 2.f * 1.41421356237309505f * Delta * wt * integral / kPIf;
+}
+
+// the double-power-law DF (DF.cpp:65-76,108-119) in FP32 (NaN -> 0 as DF.cpp:105)
+FJ_HD float mixed_df(const DFDev &d, double Lz, float jr, float jz)
+{
+    const float Jphi = (float)Lz, J0 = (float)d.J0;
     const float h = jr + (float)d.dphi_h * fabsf(Jphi) + (float)d.dz_h * jz;
     const float g = jr + (float)d.dphi_g * fabsf(Jphi) + (float)d.dz_g * jz;
     const float ev = (float)d.norm * fmaxf(0.f, powf(1.f + J0 / h, (float)d.alpha) / powf(1.f + g / J0, (float)d.beta)) /
                      (float)d.tpi3;
     float f = d.chi == 0. ? ev : ev + (float)d.k * tanhf((float)d.chi * Jphi / J0) * ev;
     if (isnan(f)) f = 0.f;
-    return (double)f;
+    return f;
+}
+
+// One velocity node on one thread: the turning points, Ju and Jv (uvOrb.cpp:
+// 226-257) with FP32 QAGS, and the DF.  The kernel integrates by groups of lanes
+// instead (fj_moments_mixed.cu), the same panels in the same order.
+// fail gets the kFail* bits, esc = 1 when the FP64 turning-point path ran; J
+// (optional) the actions.
+FJ_HDNI double mixed_node_df(const PotView &P, const PotViewF &PF, const GK21f &K, const DFDev &d, double Delta,
+                             double R, double z, double Phi_h, double V0, double V1, double V2, unsigned &fail,
+                             unsigned &esc, double *J = nullptr)
+{
+    FudgeF o;
+    bool ju, jv;
+    float Jr = 1e31f, Jz = 1e31f;
+    if (mixed_turning_points(P, PF, Delta, R, z, Phi_h, V0, V1, V2, o, ju, jv, fail, esc)) {
+        const FudgeFn fju{&o, kEvJu}, fjv{&o, kEvJv};
+        Jr = ju ? mixed_jr(o.Delta, o.Dt, qags_f(fju, K, 0.f, kPIf, 1e-5f, 1e-3f, fail)) : 0.f;
+        Jz = jv ? mixed_jz(o.Delta, o.wt, qags_f(fjv, K, 0.f, kPIHf, 1e-5f, 1e-3f, fail)) : 0.f;
+    }
+    if (J) { J[0] = (double)Jr; J[1] = (double)Jz; }
+    return (double)mixed_df(d, R * V1, Jr, Jz);
 }
 
 }  // namespace fj

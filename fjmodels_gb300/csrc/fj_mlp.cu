@@ -796,15 +796,19 @@ __global__ void __launch_bounds__(128) k_sg_moments(SgGrid g, const double *wq, 
 // ======================================================================
 // Fused surrogate moments: features, the MLP on the tensor cores and the DF
 // moment sums of one grid point's bound nodes in one kernel.  One CTA per
-// (grid point, node range); two groups of four warps each own a 128-node
+// (grid point, node range); two groups of eight warps each own a 128-node
 // tile in flight (own activation buffer, 128 TMEM columns, mbarrier) and
 // share the five layers' BF16 weights, resident in shared memory in the
-// canonical K-major layout.  Per tile: each thread writes its node's 16
+// canonical K-major layout.  Per tile: a thread per node writes its 16
 // features into the operand buffer; one thread issues the layer's
 // tcgen05.mma chain; after the commit the group reads the accumulators back
 // (tcgen05.ld), applies bias and GELU and writes the BF16 activations into
 // the same buffer as the next layer's operand; the output layer's log h and
 // log g go straight into the DF and the FP64 moment sums.
+// The GELUs are the bound (512 per node against 0.1 Mflop of MMA), and with four
+// warps per group the two warps of a scheduler could not cover their latency:
+// eight warps share a tile, each thread half of its node's columns (80 x 40 grid,
+// 22^3 nodes, with the FP64 work of a node cut: 10.1 -> 8.4 ms).
 // ======================================================================
 namespace fj {
 
@@ -813,7 +817,9 @@ struct SgWeights {
     const float *b[5];
 };
 
-constexpr int kFusedThreads = 256;     // two groups of 128
+constexpr int kFusedGroup = 256;               // threads of a group: 128 nodes x 2 halves of the columns
+constexpr int kFusedThreads = 2 * kFusedGroup;  // two groups
+constexpr int kFusedAxis = 64;         // points of a velocity rule whose squares are tabulated
 constexpr int kFusedMaxNodes = 12288;  // node range of one CTA (bound-node list in shared memory)
 
 // canonical no-swizzle K-major offset (bytes) of element (row, k) of a [rows][K]
@@ -830,18 +836,35 @@ constexpr int kSmActAligned = (kSmAct + 1023) / 1024 * 1024;
 constexpr int kSmList = kSmActAligned + 2 * 32768;
 constexpr size_t fused_smem_bytes() { return (size_t)kSmList + kFusedMaxNodes * 2 + 256; }
 
+// Feature 13, log(H / Phi) / 5 with H = K + Phi, as it enters the network (rounded
+// to BF16 next): in FP32 where every number within the FP32 form's error rounds to
+// the same BF16, else as k_sg_features computes it.  An FP64 logarithm and two
+// divisions per node held the FP64 pipe for as long as the four layers' GELUs take.
+__device__ __forceinline__ float log_energy(double K, double Phi, double iPhi)
+{
+    const float w = (float)(-K * iPhi);                      // 1 - H / Phi
+    const float q = (float)((K + Phi) * iPhi);               // H / Phi, relative precision
+    const float y = (q < 0.5f ? logf(q) : log1pf(-w)) * 0.2f;
+    const float e = 1e-6f * fabsf(y);
+    const uint32_t r = tc::bf16x2(y + e, y - e);
+    if (q > 1e-6f && (r >> 16) == (r & 0xffffu)) return y;
+    return (float)(log(fmax((K + Phi) / Phi, 1e-12)) / 5);
+}
+
 __global__ void __launch_bounds__(kFusedThreads, 1) k_sg_fused(SgGrid g, SgWeights wts, const double *wq, DFDev df,
                                                                int blocks_per_point, double *partial, int *err)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ __align__(8) unsigned long long bars[2];
     __shared__ uint32_t tmem_slot;
-    __shared__ int s_wc[8];
-    __shared__ double s_red[8 * 6];
+    __shared__ float s_v2[kFusedAxis];
+    __shared__ int s_wc[kFusedThreads / 32];
+    __shared__ double s_red[(kFusedThreads / 32) * 6];
     unsigned short *s_list = (unsigned short *)(sm + kSmList);
     float *s_bias = (float *)(sm + kSmBias);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, grp = tid >> 7, gt = tid & 127;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, grp = tid / kFusedGroup, gt = tid % kFusedGroup;
+    const int row = gt & 127, half = gt >> 7;  // the thread's node of the tile and its half of the columns
     const int B = blocks_per_point, p = blockIdx.x / B, chunk = blockIdx.x % B;
     const int nq = g.nq, nq3 = nq * nq * nq;
     const int n0 = (int)((long long)chunk * nq3 / B), n1 = (int)((long long)(chunk + 1) * nq3 / B);
@@ -871,22 +894,41 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_sg_fused(SgGrid g, SgWeigh
         }
         for (int q = tid; q < 4 * 128 + 16; q += kFusedThreads) s_bias[q] = wts.b[q >> 7 < 4 ? q >> 7 : 4][q < 512 ? q & 127 : q - 512];
     }
-    // bound nodes of [n0, n1) in node order
+    // bound nodes of [n0, n1) in node order (the sums as sg_velocity forms them)
     const double Phi_h = g.point[2 * p], Ve = g.point[2 * p + 1];
+    auto velocity = [&](int node, double &V0, double &V1, double &V2) {
+        V0 = 1e-6 + Ve * g.xq[node / (nq * nq)];
+        V1 = 1e-6 + Ve * g.xq[(node / nq) % nq];
+        V2 = 1e-6 + Ve * g.xq[node % nq];
+    };
+    // the sign of H in FP32 from the squared velocities where that is clear of
+    // its rounding, else in FP64 (whose pipe the whole sum would hold for 36 us)
+    const bool tabled = nq <= kFusedAxis;
+    if (tabled && tid < nq) {
+        const double v = 1e-6 + Ve * g.xq[tid];
+        s_v2[tid] = (float)(.5 * v * v);
+    }
+    __syncthreads();
+    const float Phi_f = (float)Phi_h, clear_f = 2e-6f * fabsf(Phi_f);
     int nbound = 0;
     for (int base = n0; base < n1; base += kFusedThreads) {
         const int node = base + tid;
         bool b = false;
         if (node < n1) {
-            double V0, V1, V2, H, R;
-            sg_velocity(g, p, node, V0, V1, V2, H, R);
-            b = H < 0;
+            float h = 0.f;
+            if (tabled) h = s_v2[node / (nq * nq)] + s_v2[(node / nq) % nq] + s_v2[node % nq] + Phi_f;
+            b = h < 0.f;
+            if (!(fabsf(h) > clear_f)) {
+                double V0, V1, V2;
+                velocity(node, V0, V1, V2);
+                b = .5 * (V0 * V0 + V1 * V1 + V2 * V2) + Phi_h < 0;
+            }
         }
         const unsigned bal = __ballot_sync(0xffffffffu, b);
         if (lane == 0) s_wc[warp] = __popc(bal);
         __syncthreads();
         int off = nbound, tot = 0;
-        for (int w = 0; w < 8; w++) {
+        for (int w = 0; w < kFusedThreads / 32; w++) {
             if (w < warp) off += s_wc[w];
             tot += s_wc[w];
         }
@@ -912,16 +954,17 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_sg_fused(SgGrid g, SgWeigh
     fx[5] = (float)(p0v / g.P.phil[0]);
     for (int l = 1; l < 8; l++) fx[5 + l] = l < np_ ? (float)(g.P.phil[n * np_ + l] / fabs(p0v)) : 0.f;
     double m[6] = {0, 0, 0, 0, 0, 0};
+    const double iPhi = 1. / Phi_h;
     uint32_t phase = 0;
     const float J0 = (float)df.J0;
-    auto group_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory"); };
+    auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(kFusedGroup) : "memory"); };
     // true in every thread of the group when v is true in any of them (also a group barrier)
     auto group_any = [&](bool v) {
         uint32_t r;
-        asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.or.pred q, %2, 128, p;\n"
+        asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.or.pred q, %2, %3, p;\n"
                      " selp.u32 %0, 1, 0, q;\n}\n"
                      : "=r"(r)
-                     : "r"((uint32_t)v), "r"(1 + grp)
+                     : "r"((uint32_t)v), "r"(1 + grp), "n"(kFusedGroup)
                      : "memory");
         return r != 0;
     };
@@ -952,24 +995,24 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_sg_fused(SgGrid g, SgWeigh
     const int ntiles = (nbound + 127) / 128;
     bool aborted = false;
     for (int t = grp; t < ntiles && !aborted; t += 2) {
-        const int q = t * 128 + gt;
-        const bool valid = q < nbound;
+        const int q = t * 128 + row;
+        const bool valid = half == 0 && q < nbound;
         const int node = valid ? n0 + s_list[q] : n0;
-        double V0, V1, V2, H, Rr;
-        sg_velocity(g, p, node, V0, V1, V2, H, Rr);
-        // features of this thread's node, row gt of the K = 16 operand
-        {
+        double V0 = 0, V1 = 0, V2 = 0;
+        // features of the node, row `row` of the K = 16 operand
+        if (half == 0) {
+            velocity(node, V0, V1, V2);
             float x[16];
             for (int i = 0; i < 14; i++) x[i] = fx[i];
             x[2] = (float)g.xq[node / (nq * nq)];
             x[3] = (float)g.xq[node % nq];
             x[4] = (float)g.xq[(node / nq) % nq];
-            x[13] = valid ? (float)(log(fmax(H / Phi_h, 1e-12)) / 5) : 0.f;
+            x[13] = valid ? log_energy(.5 * (V0 * V0 + V1 * V1 + V2 * V2), Phi_h, iPhi) : 0.f;
             x[14] = x[15] = 0.f;
             for (int h8 = 0; h8 < 2; h8++) {
                 __align__(16) __nv_bfloat16 v[8];
                 for (int e = 0; e < 8; e++) v[e] = __float2bfloat16_rn(x[h8 * 8 + e]);
-                *reinterpret_cast<uint4 *>(act + kmaj_off(gt, h8 * 8, 128)) = *reinterpret_cast<const uint4 *>(v);
+                *reinterpret_cast<uint4 *>(act + kmaj_off(row, h8 * 8, 128)) = *reinterpret_cast<const uint4 *>(v);
             }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -977,7 +1020,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_sg_fused(SgGrid g, SgWeigh
         // hidden layers: acc -> bias + GELU -> bf16 operand of the next layer
         for (int l = 0; l < 4 && !aborted; l++) {
             if (!mma_chain(l == 0 ? 1 : 8, l == 0 ? kSmW0 : kSmW1 + (l - 1) * 32768, 128)) { aborted = true; break; }
-            for (int c0 = 0; c0 < 128; c0 += 16) {
+            for (int c0 = half * 64; c0 < half * 64 + 64; c0 += 16) {
                 uint32_t r[16];
                 asm volatile(
                     "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
@@ -987,10 +1030,14 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_sg_fused(SgGrid g, SgWeigh
                       "=r"(r[15])
                     : "r"(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0));
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                __align__(16) __nv_bfloat16 v[16];
-                for (int e = 0; e < 16; e++) v[e] = __float2bfloat16_rn(tc::gelu(__uint_as_float(r[e]) + s_bias[l * 128 + c0 + e]));
-                *reinterpret_cast<uint4 *>(act + kmaj_off(gt, c0, 128)) = *reinterpret_cast<const uint4 *>(v);
-                *reinterpret_cast<uint4 *>(act + kmaj_off(gt, c0 + 8, 128)) = *reinterpret_cast<const uint4 *>(v + 8);
+                const float *bias = s_bias + l * 128 + c0;
+                uint32_t v[8];
+#pragma unroll
+                for (int e = 0; e < 8; e++)
+                    v[e] = tc::bf16x2(tc::gelu(__uint_as_float(r[2 * e + 1]) + bias[2 * e + 1]),
+                                      tc::gelu(__uint_as_float(r[2 * e]) + bias[2 * e]));
+                *reinterpret_cast<uint4 *>(act + kmaj_off(row, c0, 128)) = make_uint4(v[0], v[1], v[2], v[3]);
+                *reinterpret_cast<uint4 *>(act + kmaj_off(row, c0 + 8, 128)) = make_uint4(v[4], v[5], v[6], v[7]);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1035,7 +1082,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_sg_fused(SgGrid g, SgWeigh
     __syncthreads();
     if (tid < 6) {
         double sacc = 0;
-        for (int w = 0; w < 8; w++) sacc += s_red[w * 6 + tid];
+        for (int w = 0; w < kFusedThreads / 32; w++) sacc += s_red[w * 6 + tid];
         partial[((size_t)p * B + chunk) * 6 + tid] = sacc;
     }
     if (aborted) {  // let the group's outstanding commit land before TMEM is freed

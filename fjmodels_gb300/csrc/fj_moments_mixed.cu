@@ -8,6 +8,8 @@
 // Built with FMA contraction (the plain form is the rounding-faithful one).
 #include <cstdint>
 
+
+#include "fj_group_qags.cuh"
 #include "fj_internal.h"
 #include "fj_mixed.cuh"
 #include "fj_order.cuh"
@@ -15,32 +17,48 @@
 
 namespace fj {
 
-// Work layout: a block takes one contiguous range of at most a.mixed_chunk
-// nodes of one point (mixed_blocks_per_point blocks per point), compacts the
-// bound ones (H < 0; about 40% of the cube) into a shared-memory list in node
-// order, and its threads take the list round-robin.  So no lane idles on an
-// unbound node, each thread's nodes are summed in a fixed order, and the
-// per-block sums are added in a fixed order by k_moments_finalize.
-// The kernel is built in two forms and each in four register budgets (launch
-// bounds of 3, 4, 6 and 8 resident blocks per SM: 168, 128, 80 and 64
-// registers): kMixedVariants builds.
-//  - static: thread t takes list entries t, t + 128, .. and sums its nodes'
-//    moments as it goes;
-//  - dynamic: a lane that finishes a node takes the next untaken entry
-//    (shared counter), stores the node's DF in a shared array, and after
-//    the list the threads sum the moments of entries t, t + 128, .. from it.
-//    The time per node varies by two orders of magnitude (QAGS takes 1 to
-//    ~60 panels per integral), so with static shares the block waits for its
-//    unluckiest thread; the dynamic form keeps all lanes busy to the end.
-//    Its sums are those of the static form term by term, so both give the
-//    same bits.
-// Which one, and the chunk size, is a per-context setting (fj_autotune_mixed).
+// Work layout: an item is one contiguous range of at most a.mixed_chunk nodes
+// of one point (mixed_blocks_per_point items per point).  Two persistent kernels
+// go through the items of a slice of the launch:
+//   k_mixed_turn       compacts an item's bound nodes (H < 0; about 40% of the
+//                      cube), sorts them by the cost proxy of fj_order.cuh and
+//                      finds their turning points, one node per thread: the FP64
+//                      setup, bracket walks and Brent; a node's constants go to a
+//                      record in device memory;
+//   k_mixed_integrate  kMixedLanes lanes per momentum integral: the first panel of
+//                      every Ju and Jv of the item, then the bisections of those
+//                      that go on, groups taking the next integral as they finish
+//                      (fj_group_qags.cuh); then the DFs and the moment sums.
+// With a node's whole solve on one thread (one kernel) the lanes of a warp sat in
+// different places of it: the evaluator, 3/4 of the instructions, was entered with
+// 13.7 of 32 lanes, and each thread kept its own interval list and call frames in
+// local memory.  The same phases in one kernel executed 22 % fewer instructions
+// but ran no faster: blocks in different phases pushed each other's code out of
+// the instruction caches (4.8 stall cycles per issue waiting for instructions).
+// The integration is built in four register budgets (launch bounds of 3, 4, 6 and
+// 8 resident blocks per SM: 168, 128, 80 and 64 registers), and the turning points
+// in two: kMixedVariants configurations, all with the same bits.  Which one, and
+// the item size, is a per-context setting (fj_autotune_mixed).
 // Shared memory holds only what the node solves read: the FP32 tables, the
 // radii, the focal-distance table, the velocity rule and the node list.  The
 // FP64 potential tables are read from global memory (the point setup, the
-// FP32 table build and the rare FP64 turning-point path): kept out of shared
-// memory they leave L1 to the threads' local memory (QAGS lists, call
-// frames), which took the 80x40 launch from ~347 to ~311 ms.
+// FP32 table build and the rare FP64 turning-point path).
+constexpr int kMixedLanes = 4;                            // lanes per momentum integral
+constexpr int kMixedGroups = kMixedBlock / kMixedLanes;   // integrals in flight per block
+using MixedQags = GroupQags<float, kQagsCapF>;
+
+// What a node's integrals need after its turning points, and its actions
+struct alignas(16) MixedRec {
+    float Delta, D2, K, EC, C0, Lt, shu2, sv2, swp, svp, sinv, cosv, sinhu, coshu, pvterm, rpt, Phipt, u_f, tb, Dt, wt;
+    float Jr, Jz, eu, ev;  // actions; between the passes the first panels' results and errors
+    unsigned word;         // kFail* bits of the turning points, kRecJu, kRecJv, node << kRecNode
+    unsigned pad[2];
+};
+enum : unsigned { kRecJu = 8u, kRecJv = 16u, kRecNode = 8u };  // kRecNode: bit position (node within the item)
+
+size_t mixed_rec_bytes() { return sizeof(MixedRec); }
+size_t mixed_scratch_bytes() { return kMixedGroups * sizeof(MixedQags::List); }
+
 int mixed_blocks_per_point(long long nq3, int chunk) { return (int)((nq3 + chunk - 1) / chunk); }
 
 // capacity of a block's node list: the next power of two >= the node range (the sort pads to it)
@@ -51,216 +69,66 @@ __host__ __device__ static int mixed_list_cap(int chunk)
     return c;
 }
 
-size_t moment_mixed_smem_bytes(const MomentArgs &a)
+// FP32 tables of a model at one grid point in shared memory
+__host__ __device__ static size_t mixed_table_floats(int nr, int npoly, bool grad)
 {
-    const size_t nt = (size_t)a.P.nr * a.P.npoly;
-    return (a.P.nr + 2 * a.ngrid + 2 * a.nq + 6 * (kMixedBlock / 32) + 4) * sizeof(double) +
-           (2 * a.P.nr + 2 * nt + 4 * kQuadIntervals + a.P.npoly) * sizeof(float) + sizeof(GK21f) + 16 +
-           (kMixedBlock / 32) * sizeof(int) + (size_t)mixed_list_cap(a.mixed_chunk) * sizeof(unsigned short) + 16 +
-           (size_t)mixed_list_cap(a.mixed_chunk) * sizeof(float) + sizeof(int);
+    const size_t nt = (size_t)nr * npoly;
+    return 2 * (size_t)nr + (grad ? 4 : 3) * nt + (2 * nt & 1) + 4 * kQuadIntervals + npoly + 2 * kQuadIntervals * npoly + 1;
 }
 
+struct MixedTables {
+    float *ar, *phil, *Pr, *ih, *qc, *pyl, *pd, *pe;
+    // carves the tables out of 8-byte aligned memory; returns the first free float
+    __device__ float *carve(float *f, int nr, int npoly, bool grad)
+    {
+        const int nt = nr * npoly;
+        pd = f; f += 2 * nt;
+        ar = f; f += nr;
+        phil = f; f += nt;
+        Pr = grad ? f : nullptr; if (grad) f += nt;
+        ih = f; f += nr;
+        qc = f; f += 4 * kQuadIntervals;
+        pyl = f; f += npoly;
+        pe = f; f += 2 * kQuadIntervals * npoly;
+        return f;
+    }
+    __device__ PotViewF build(const MomentArgs &a, double Phi_h, double R, double z)
+    {
+        const int nr = a.P.nr, npoly = a.P.npoly;
+        mixed_tables_f(nr, npoly, a.P.ar, a.P.phil, a.P.Pr, Phi_h, R, z, ar, phil, Pr, ih, qc, pyl, threadIdx.x,
+                       blockDim.x);
+        PotViewF v = mixed_view_f(nr, npoly, a.P.ar, a.P.phil, Phi_h, R, z, ar, phil, Pr, ih, qc, pyl);
+        __syncthreads();
+        evaluator_tables_f(v, pd, pe, threadIdx.x, blockDim.x);
+        __syncthreads();
+        v.pd = pd;
+        v.pe = pe;
+        return v;
+    }
+};
 
-// One work item: the node range `bid` (global over the launch's models) of
-// one grid point, as described at the top of the file.
-template <bool DYN>
-__device__ __forceinline__ void mixed_item(const MomentArgs &a0, const MomentBatch &batch, int bid, double *sm,
-                                           unsigned *s_bits, int &s_nleft)
+static size_t mixed_turn_smem(const MomentArgs &a)
 {
-    MomentArgs a = a0;
-    for (int i = threadIdx.x; i < kMixedMaxNodes / 32; i += blockDim.x) s_bits[i] = 0u;
-    if (threadIdx.x == 0) s_nleft = 0;
-    __syncthreads();
-    if (batch.n > 0) {
-        const int m = batch_model(batch.block_start, batch.n, bid);
-        a = batch.args[m];
-        bid -= batch.block_start[m];
-    }
-    const int nr = a.P.nr, npoly = a.P.npoly, nt = nr * npoly;
-    double *s_ar = sm;
-    double *s_Eg = s_ar + nr, *s_Dg = s_Eg + a.ngrid, *s_xq = s_Dg + a.ngrid, *s_wq = s_xq + a.nq;
-    double *s_red = s_wq + a.nq, *s_pt = s_red + 6 * (kMixedBlock / 32);
-    float *f_ar = (float *)(s_pt + 4), *f_phil = f_ar + nr, *f_Pr = f_phil + nt, *f_ih = f_Pr + nt;
-    float *f_qc = f_ih + nr, *f_pyl = f_qc + 4 * kQuadIntervals;
-    GK21f *sK = (GK21f *)(((uintptr_t)(f_pyl + npoly) + 15) & ~(uintptr_t)15);
-    int *s_wc = (int *)(sK + 1);
-    unsigned short *s_list = (unsigned short *)(s_wc + kMixedBlock / 32);
-    const int cap = mixed_list_cap(a.mixed_chunk);
-    float *s_df = (float *)(((uintptr_t)(s_list + cap) + 15) & ~(uintptr_t)15);
-    int *s_next = (int *)(s_df + cap);
-    for (int i = threadIdx.x; i < nr; i += blockDim.x) s_ar[i] = a.P.ar[i];
-    for (int i = threadIdx.x; i < a.ngrid; i += blockDim.x) { s_Eg[i] = a.Eg[i]; s_Dg[i] = a.Dg[i]; }
-    for (int i = threadIdx.x; i < a.nq; i += blockDim.x) { s_xq[i] = a.xq[i]; s_wq[i] = a.wq[i]; }
-    if (threadIdx.x < 11) {
-        sK->xgk[threadIdx.x] = (float)fj_xgk21_d[threadIdx.x];
-        sK->wgk[threadIdx.x] = (float)fj_wgk21_d[threadIdx.x];
-        if (threadIdx.x < 5) sK->wg[threadIdx.x] = (float)fj_wg10_d[threadIdx.x];
-    }
-    const PotView P{nr, npoly, s_ar, a.P.phil, a.P.Pr, a.P.Pr2};
-    const int B = a.blocks_per_point;
-    const int p = bid / B, chunk = bid % B;
-    __syncthreads();
-    if (threadIdx.x == 0) {  // per-point FP64 setup, shared by the block (integ/Integ.cpp:46-62,150-151)
-        double R, z;
-        if (a.Rz) { R = a.Rz[2 * p]; z = a.Rz[2 * p + 1]; }
-        else {
-            const int n = p / a.ngauss, g = p % a.ngauss;
-            const double c = a.ci[g], si = sqrt(1 - c * c);
-            R = s_ar[n] * si; z = s_ar[n] * c;
-        }
-        const double rmax = s_ar[nr - 1];
-        const double Phi_h = pot_phi(P, R, z);
-        s_pt[0] = R; s_pt[1] = z; s_pt[2] = Phi_h;
-        s_pt[3] = sqrt(-2 * (Phi_h - pot_phi(P, 10 * rmax, 10 * rmax)));
-    }
-    __syncthreads();
-    const double R = s_pt[0], z = s_pt[1], Phi_h = s_pt[2], Ve = s_pt[3];
-    mixed_tables_f(nr, npoly, s_ar, a.P.phil, a.P.Pr, Phi_h, R, z, f_ar, f_phil, f_Pr, f_ih, f_qc, f_pyl, threadIdx.x,
-                   blockDim.x);
-    const int nq = a.nq, nq2 = nq * nq;
-    const long long nq3 = (long long)nq2 * nq;
-    const int n0 = (int)(chunk * nq3 / B), n1 = (int)((chunk + 1) * nq3 / B);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-
-    // bound nodes of [n0, n1) in node order
-    int nbound = 0;
-    for (int base = n0; base < n1; base += kMixedBlock) {
-        const int node = base + threadIdx.x;
-        bool b = false;
-        if (node < n1) {
-            const double V0 = 1e-6 + Ve * s_xq[node / nq2], V1 = 1e-6 + Ve * s_xq[(node / nq) % nq],
-                         V2 = 1e-6 + Ve * s_xq[node % nq];
-            b = .5 * (V0 * V0 + V1 * V1 + V2 * V2) + Phi_h < 0;
-        }
-        const unsigned bal = __ballot_sync(0xffffffffu, b);
-        if (lane == 0) s_wc[warp] = __popc(bal);
-        __syncthreads();
-        int off = nbound, tot = 0;
-        for (int w = 0; w < kMixedBlock / 32; w++) {
-            if (w < warp) off += s_wc[w];
-            tot += s_wc[w];
-        }
-        if (b) s_list[off + __popc(bal & ((1u << lane) - 1u))] = (unsigned short)(node - n0);
-        __syncthreads();
-        nbound += tot;
-    }
-    for (int q = threadIdx.x; q < nbound; q += kMixedBlock) {  // cost keys, in s_df until the solves
-        const int node = n0 + s_list[q];
-        s_df[q] = node_cost_key((float)s_xq[node / nq2], (float)s_xq[(node / nq) % nq], (float)s_xq[node % nq]);
-    }
-    sort_list(s_list, s_df, nbound);
-    const PotViewF PF = mixed_view_f(nr, npoly, s_ar, a.P.phil, Phi_h, R, z, f_ar, f_phil, f_Pr, f_ih, f_qc, f_pyl);
-    const double jacob = Ve * Ve * Ve;
-
-    double m[6] = {0, 0, 0, 0, 0, 0};
-    unsigned esc = 0;
-    FailTally tally;
-    // one node's solve; returns the DF that enters the moments.  A node whose
-    // FP32 solve hits a cap (a full QAGS list, a bracket walk or Brent at its
-    // step limit) is marked in the block's bitmap and counts 0 here: k_moments_deferred
-    // solves it again with the plain form's FP64 solve (QAGS lists of kQagsCap
-    // intervals) and adds it to this block's sums.  Only what that solve still
-    // caps is a failure, with the plain form's policy (a capped bracket or root:
-    // DF 0; a full QAGS list: the estimate so far, as QUADPACK returns it).
-    auto solve = [&](int q) {
-        const int node = n0 + s_list[q];
-        const int i = node / nq2, j = (node / nq) % nq, k = node % nq;
-        const double V0 = 1e-6 + Ve * s_xq[i], V1 = 1e-6 + Ve * s_xq[j], V2 = 1e-6 + Ve * s_xq[k];
-        const double H = .5 * (V0 * V0 + V1 * V1 + V2 * V2) + Phi_h;
-        unsigned fail = 0, e = 0;
-        const double Delta = deltafn(s_Eg, s_Dg, a.ngrid, H);
-        double J[2];
-        double f = mixed_node_df(P, PF, *sK, a.df, Delta, R, z, Phi_h, V0, V1, V2, fail, e, J);
-        esc += e;
-        if (fail && a.defer) {
-            atomicOr(&s_bits[(node - n0) >> 5], 1u << ((node - n0) & 31));
-            atomicAdd(&s_nleft, 1);
-            return 0.;
-        }
-        if (a.jout) {
-            float *jo = a.jout + ((size_t)p * nq3 + node) * 2;
-            jo[0] = (float)J[0];
-            jo[1] = (float)J[1];
-        }
-        tally.add(fail);
-        return (fail & (kFailBracket | kFailRoot)) ? 0. : f;
-    };
-    auto accumulate = [&](int q, double DF) {
-        const int node = n0 + s_list[q];
-        const int i = node / nq2, j = (node / nq) % nq, k = node % nq;
-        const double V0 = 1e-6 + Ve * s_xq[i], V1 = 1e-6 + Ve * s_xq[j], V2 = 1e-6 + Ve * s_xq[k];
-        const double jd = (s_wq[i] * s_wq[j] * s_wq[k]) * (jacob * DF);
-        m[0] += jd;
-        m[1] += jd * V1;
-        m[2] += jd * V0 * V0;
-        m[3] += jd * V1 * V1;
-        m[4] += jd * V2 * V2;
-        m[5] += jd * V0 * V2;
-    };
-    if (DYN) {
-        if (threadIdx.x == 0) *s_next = kMixedBlock;
-        __syncthreads();
-        for (int q = threadIdx.x; q < nbound;) {
-            s_df[q] = (float)solve(q);  // the DF is an FP32 value
-            q = atomicAdd(s_next, 1);
-        }
-        __syncthreads();
-        for (int q = threadIdx.x; q < nbound; q += kMixedBlock) accumulate(q, (double)s_df[q]);
-    } else {
-        for (int q = threadIdx.x; q < nbound; q += kMixedBlock) accumulate(q, solve(q));
-    }
-#pragma unroll
-    for (int q = 0; q < 6; q++) {
-        double v = m[q];
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-        if (lane == 0) s_red[warp * 6 + q] = v;
-    }
-    warp_count_fails(a.counters, tally);
-    warp_count(&a.counters[kCntEscalated], esc);
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        double s = 0;
-        for (int w = 0; w < kMixedBlock / 32; w++) s += s_red[w * 6 + threadIdx.x];
-        a.partial[((size_t)p * B + chunk) * 6 + threadIdx.x] = s;
-    }
-    if (a.defer) {  // the block's bitmap of deferred nodes and their number
-        const int nw = defer_words(a.mixed_chunk);
-        for (int i = threadIdx.x; i < nw; i += blockDim.x) a.defer[((size_t)p * B + chunk) * nw + i] = s_bits[i];
-        if (threadIdx.x == 0) a.defer_count[(size_t)p * B + chunk] = s_nleft;
-    }
-    if (threadIdx.x == 0 && nbound) atomicAdd(&a.counters[kCntBound], (unsigned long long)nbound);
+    const size_t cap = mixed_list_cap(a.mixed_chunk);
+    return (a.P.nr + 2 * a.ngrid + a.nq + 4) * sizeof(double) +
+           (mixed_table_floats(a.P.nr, a.P.npoly, true) + 1) * sizeof(float) + (kMixedBlock / 32 + 1) * sizeof(int) +
+           cap * (sizeof(float) + sizeof(unsigned short)) + 16;
 }
 
-// The persistent kernel: a grid of at most as many blocks as fit on the GPU at
-// once takes work items from the queue (an atomic counter) until none is
-// left, in the queue's order (most expensive first, from the previous launch's
-// measured cycles, when the context has them), and records each item's cycles.
-// Blocks free up as their items finish and take the next one, so the uneven
-// cost of the root finding and quadrature is balanced across the GPU.
-template <int MINB, bool DYN>
-__global__ void __launch_bounds__(kMixedBlock, MINB) k_moments_mixed(MomentArgs a0, MomentBatch batch, ItemQueue q)
-{
-    extern __shared__ double sm[];
-    __shared__ unsigned s_bits[kMixedMaxNodes / 32];  // nodes left to the FP64 pass
-    __shared__ int s_nleft, s_item;
-    for (;;) {
-        __syncthreads();  // every thread is done with the previous item's shared data
-        if (threadIdx.x == 0) s_item = (int)atomicAdd(q.next, 1u);
-        __syncthreads();
-        const int it = s_item;
-        if (it >= q.total) return;
-        const int bid = q.order ? q.order[it] : it;
-        const long long t0 = clock64();
-        mixed_item<DYN>(a0, batch, bid, sm, s_bits, s_nleft);
-        if (q.cost && threadIdx.x == 0) q.cost[bid] = (float)(clock64() - t0);
-    }
-}
+// A block's shared memory of the integrals
+struct MixedShared {
+    float vals[kMixedGroups][43];  // panel values
+    GK21f K;
+    int next;
+};
+enum : unsigned char { kIntNone = 0, kIntNew = 1, kIntMore = 2, kIntFull = 3 };  // state of an integral
 
-// ------------------------------------------------------ the FP64 pass
-// Over the nodes the mixed kernel left (launch_deferred): a scan of the
-// blocks' counts, the compact list, one thread per listed node, one thread per
-// block adding its nodes in list order.
+static size_t mixed_integrate_smem(const MomentArgs &a)
+{
+    return (2 * a.nq + 6 * (kMixedBlock / 32)) * sizeof(double) +
+           (mixed_table_floats(a.P.nr, a.P.npoly, false) + 1) * sizeof(float) + sizeof(MixedShared) +
+           defer_words(a.mixed_chunk) * sizeof(unsigned) + 2 * (size_t)a.mixed_chunk + 16;
+}
 
 // the arguments and the model-local index of global block g of a launch
 __device__ __forceinline__ const MomentArgs &block_args(const MomentArgs &a0, const MomentBatch &b, int g, int &bid)
@@ -271,6 +139,333 @@ __device__ __forceinline__ const MomentArgs &block_args(const MomentArgs &a0, co
     bid -= b.block_start[m];
     return b.args[m];
 }
+
+// nodes [n0, n1) of item bid of its model
+__device__ __forceinline__ void item_range(const MomentArgs &a, int bid, int &n0, int &n1)
+{
+    const long long nq3 = (long long)a.nq * a.nq * a.nq;
+    const int B = a.blocks_per_point, chunk = bid % B;
+    n0 = (int)(chunk * nq3 / B);
+    n1 = (int)((chunk + 1) * nq3 / B);
+}
+
+template <int MINB>
+__global__ void __launch_bounds__(kMixedBlock, MINB) k_mixed_turn(MomentArgs a0, MomentBatch batch, ItemQueue q)
+{
+    extern __shared__ double sm[];
+    __shared__ int s_item, s_next;
+    for (;;) {
+        __syncthreads();  // every thread is done with the previous item's shared data
+        if (threadIdx.x == 0) s_item = (int)atomicAdd(q.next, 1u);
+        __syncthreads();
+        const int slot = s_item;
+        if (slot >= q.count) return;
+        const int it = q.first + slot, g = q.order ? q.order[it] : it;
+        const long long t_start = clock64();
+        int bid;
+        const MomentArgs &a = block_args(a0, batch, g, bid);
+        const int nr = a.P.nr, npoly = a.P.npoly;
+        double *s_ar = sm, *s_Eg = s_ar + nr, *s_Dg = s_Eg + a.ngrid, *s_xq = s_Dg + a.ngrid, *s_pt = s_xq + a.nq;
+        MixedTables tab;
+        int *s_wc = (int *)tab.carve((float *)(s_pt + 4), nr, npoly, true);
+        unsigned short *s_list = (unsigned short *)(s_wc + kMixedBlock / 32);
+        const int cap = mixed_list_cap(a.mixed_chunk);
+        float *s_key = (float *)(((uintptr_t)(s_list + cap) + 15) & ~(uintptr_t)15);
+        for (int i = threadIdx.x; i < nr; i += blockDim.x) s_ar[i] = a.P.ar[i];
+        for (int i = threadIdx.x; i < a.ngrid; i += blockDim.x) { s_Eg[i] = a.Eg[i]; s_Dg[i] = a.Dg[i]; }
+        for (int i = threadIdx.x; i < a.nq; i += blockDim.x) s_xq[i] = a.xq[i];
+        const PotView P{nr, npoly, s_ar, a.P.phil, a.P.Pr, a.P.Pr2};
+        const int p = bid / a.blocks_per_point;
+        __syncthreads();
+        if (threadIdx.x == 0) {  // per-point FP64 setup, shared by the block (integ/Integ.cpp:46-62,150-151)
+            double R, z;
+            if (a.Rz) { R = a.Rz[2 * p]; z = a.Rz[2 * p + 1]; }
+            else {
+                const int n = p / a.ngauss, gg = p % a.ngauss;
+                const double c = a.ci[gg], si = sqrt(1 - c * c);
+                R = s_ar[n] * si; z = s_ar[n] * c;
+            }
+            const double rmax = s_ar[nr - 1];
+            const double Phi_h = pot_phi(P, R, z);
+            s_pt[0] = R; s_pt[1] = z; s_pt[2] = Phi_h;
+            s_pt[3] = sqrt(-2 * (Phi_h - pot_phi(P, 10 * rmax, 10 * rmax)));
+        }
+        __syncthreads();
+        const double R = s_pt[0], z = s_pt[1], Phi_h = s_pt[2], Ve = s_pt[3];
+        if (threadIdx.x < 4) q.point[4 * (size_t)slot + threadIdx.x] = s_pt[threadIdx.x];
+        const PotViewF PF = tab.build(a, Phi_h, R, z);
+        const int nq = a.nq, nq2 = nq * nq;
+        int n0, n1;
+        item_range(a, bid, n0, n1);
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        auto velocity = [&](int node, double &V0, double &V1, double &V2) {
+            V0 = 1e-6 + Ve * s_xq[node / nq2]; V1 = 1e-6 + Ve * s_xq[(node / nq) % nq]; V2 = 1e-6 + Ve * s_xq[node % nq];
+        };
+        // bound nodes of [n0, n1) in node order
+        int nbound = 0;
+        for (int base = n0; base < n1; base += kMixedBlock) {
+            const int node = base + threadIdx.x;
+            bool b = false;
+            if (node < n1) {
+                double V0, V1, V2;
+                velocity(node, V0, V1, V2);
+                b = .5 * (V0 * V0 + V1 * V1 + V2 * V2) + Phi_h < 0;
+            }
+            const unsigned bal = __ballot_sync(0xffffffffu, b);
+            if (lane == 0) s_wc[warp] = __popc(bal);
+            __syncthreads();
+            int off = nbound, tot = 0;
+            for (int w = 0; w < kMixedBlock / 32; w++) {
+                if (w < warp) off += s_wc[w];
+                tot += s_wc[w];
+            }
+            if (b) s_list[off + __popc(bal & ((1u << lane) - 1u))] = (unsigned short)(node - n0);
+            __syncthreads();
+            nbound += tot;
+        }
+        for (int k = threadIdx.x; k < nbound; k += kMixedBlock) {
+            const int node = n0 + s_list[k];
+            s_key[k] = node_cost_key((float)s_xq[node / nq2], (float)s_xq[(node / nq) % nq], (float)s_xq[node % nq]);
+        }
+        if (threadIdx.x == 0) { s_next = kMixedBlock; q.nbound[slot] = nbound; }
+        sort_list(s_list, s_key, nbound);
+        __syncthreads();
+        unsigned esc = 0;
+        MixedRec *rec = (MixedRec *)q.rec + (size_t)slot * q.stride;
+        for (int k = threadIdx.x; k < nbound;) {  // nodes taken as threads free up
+            const int node = s_list[k];
+            double V0, V1, V2;
+            velocity(n0 + node, V0, V1, V2);
+            const double H = .5 * (V0 * V0 + V1 * V1 + V2 * V2) + Phi_h;
+            FudgeF o;
+            bool ju, jv;
+            unsigned fail = 0, e = 0;
+            const bool bound = mixed_turning_points(P, PF, deltafn(s_Eg, s_Dg, a.ngrid, H), R, z, Phi_h, V0, V1, V2, o,
+                                                    ju, jv, fail, e);
+            esc += e;
+            MixedRec r;
+            r.Delta = o.Delta; r.D2 = o.D2; r.K = o.K; r.EC = o.EC; r.C0 = o.C0; r.Lt = o.Lt; r.shu2 = o.shu2;
+            r.sv2 = o.sv2; r.swp = o.swp; r.svp = o.svp; r.sinv = o.sinv; r.cosv = o.cosv; r.sinhu = o.sinhu;
+            r.coshu = o.coshu; r.pvterm = o.pvterm; r.rpt = o.rpt; r.Phipt = o.Phipt; r.u_f = o.u_f; r.tb = o.tb;
+            r.Dt = o.Dt; r.wt = o.wt;
+            r.Jr = r.Jz = bound ? 0.f : 1e31f;
+            r.eu = r.ev = 0.f;
+            r.word = fail | (ju ? kRecJu : 0u) | (jv ? kRecJv : 0u) | ((unsigned)node << kRecNode);
+            r.pad[0] = r.pad[1] = 0;
+            rec[k] = r;
+            k = atomicAdd(&s_next, 1);
+        }
+        warp_count(&a.counters[kCntEscalated], esc);
+        if (threadIdx.x == 0 && nbound) atomicAdd(&a.counters[kCntBound], (unsigned long long)nbound);
+        if (q.cost && threadIdx.x == 0) q.cost[g] = (float)(clock64() - t_start);
+    }
+}
+
+// The momentum integrals of an item's n nodes, kMixedLanes lanes to one
+__device__ __forceinline__ void mixed_integrals(const PotViewF &PF, int n, MixedRec *rec, MixedQags::List &L,
+                                                unsigned char *state, MixedShared &sh)
+{
+    const int lane = threadIdx.x & 31, g = threadIdx.x / kMixedLanes, gi = threadIdx.x % kMixedLanes;
+    const int lead = lane & ~(kMixedLanes - 1);
+    const float epsabs = 1e-5f, epsrel = 1e-3f;
+    const GK21f &K = sh.K;
+    float *vals = sh.vals[g];
+    MixedQags st;
+    // pass 0: first panels, item = node (Ju), then n + node (Jv), in order;
+    // pass 1: the bisections of the items that go on, taken as groups free up
+    for (int pass = 0; pass < 2; pass++) {
+        int item = pass == 0 ? g - kMixedGroups : -1;
+        float a1 = 0.f, b2 = 0.f;
+        if (pass == 1) {
+            __syncthreads();
+            if (threadIdx.x == 0) sh.next = 0;
+            __syncthreads();
+        }
+        for (;;) {
+            if (pass == 0) {
+                item += kMixedGroups;
+                a1 = 0.f; b2 = item < n ? kPIf : kPIHf;
+            } else {
+                if (gi == 0 && item < 0) {
+                    do item = atomicAdd(&sh.next, 1);
+                    while (item < 2 * n && state[item] != kIntMore);
+                    if (item < 2 * n) {
+                        const MixedRec &r = rec[item < n ? item : item - n];
+                        a1 = 0.f; b2 = item < n ? kPIf : kPIHf;
+                        st.begin(L, a1, b2, item < n ? r.Jr : r.Jz, item < n ? r.eu : r.ev);
+                    }
+                }
+                item = __shfl_sync(0xffffffffu, item, lead);
+                a1 = __shfl_sync(0xffffffffu, a1, lead);
+                b2 = __shfl_sync(0xffffffffu, b2, lead);
+            }
+            if (!__any_sync(0xffffffffu, item < 2 * n)) break;
+            const bool kv = item >= n;
+            const bool on = item < 2 * n && (pass == 1 || state[item] == kIntNew);
+            const int q = kv ? item - n : item;
+            const float b1 = 0.5f * (a1 + b2);
+            if (on) {
+                const MixedRec &r = rec[q];
+                FudgeF o;
+                o.Delta = r.Delta; o.D2 = r.D2; o.K = r.K; o.EC = r.EC; o.C0 = r.C0; o.Lt = r.Lt; o.shu2 = r.shu2;
+                o.sv2 = r.sv2; o.swp = r.swp; o.svp = r.svp; o.sinv = r.sinv; o.cosv = r.cosv; o.sinhu = r.sinhu;
+                o.coshu = r.coshu; o.pvterm = r.pvterm; o.rpt = r.rpt; o.Phipt = r.Phipt; o.u_f = r.u_f; o.tb = r.tb;
+                o.Dt = r.Dt; o.wt = r.wt;
+                const int npts = pass == 0 ? 21 : 42;
+                for (int e = gi; e < npts; e += kMixedLanes) {
+                    const bool second = e >= 21;
+                    const float x = gk21_abscissa(K, second ? b1 : a1, pass == 0 || second ? b2 : b1, second ? e - 21 : e);
+                    FGeo G;
+                    const int mode = kv ? kEvJv : kEvJu;
+                    fudge_geom(o, mode, x, G);
+                    vals[e] = fudge_finish(mode, G, pot_dphi_f(PF, G.R, G.z, o.rpt, G.dr2, G.dc2, o.Phipt));
+                }
+            }
+            __syncwarp();
+            // the panels' sums on the group's first and third lanes
+            float res = 0.f, err = 0.f, ra = 0.f, rc = 0.f;
+            if (on && (gi == 0 || (gi == 2 && pass == 1)))
+                gk21_sum(K, gi ? b1 : a1, pass == 0 || gi ? b2 : b1, vals + (gi ? 21 : 0), res, err, ra, rc);
+            const float res2 = __shfl_sync(0xffffffffu, res, lead + 2), err2 = __shfl_sync(0xffffffffu, err, lead + 2),
+                        rc2 = __shfl_sync(0xffffffffu, rc, lead + 2);
+            if (on && gi == 0) {
+                bool done, full = false;
+                float r = res;
+                MixedRec &c = rec[q];
+                if (pass == 0) {  // the early exits of QAGS
+                    const float tol = fmaxf(epsabs, epsrel * fabsf(res));
+                    done = (err <= 100 * FLT_EPSILON * ra && err > tol) || (err <= tol && err != rc) || err == 0.0f;
+                    if (!done) {
+                        if (kv) { c.Jz = res; c.ev = err; } else { c.Jr = res; c.eu = err; }
+                        state[item] = kIntMore;
+                    }
+                } else {
+                    done = st.update(L, res, err, rc, res2, err2, rc2, epsabs, epsrel, r, full);
+                    if (!done) { a1 = L.iv[st.maxerr].a; b2 = L.iv[st.maxerr].b; }
+                }
+                if (done) {
+                    if (kv) c.Jz = mixed_jz(c.Delta, c.wt, r); else c.Jr = mixed_jr(c.Delta, c.Dt, r);
+                    state[item] = full ? kIntFull : kIntNone;
+                    if (pass == 1) item = -1;
+                }
+            }
+            __syncwarp();
+        }
+    }
+}
+
+template <int MINB>
+__global__ void __launch_bounds__(kMixedBlock, MINB) k_mixed_integrate(MomentArgs a0, MomentBatch batch, ItemQueue q)
+{
+    extern __shared__ double sm[];
+    __shared__ int s_item, s_nleft;
+    MixedQags::List &L = ((MixedQags::List *)q.scratch)[blockIdx.x * kMixedGroups + threadIdx.x / kMixedLanes];
+    for (;;) {
+        __syncthreads();  // every thread is done with the previous item's shared data
+        if (threadIdx.x == 0) { s_item = (int)atomicAdd(q.next + 1, 1u); s_nleft = 0; }
+        __syncthreads();
+        const int slot = s_item;
+        if (slot >= q.count) return;
+        const int it = q.first + slot, g = q.order ? q.order[it] : it;
+        const long long t_start = clock64();
+        int bid;
+        const MomentArgs &a = block_args(a0, batch, g, bid);
+        const int nr = a.P.nr, npoly = a.P.npoly;
+        double *s_xq = sm, *s_wq = s_xq + a.nq, *s_red = s_wq + a.nq;
+        MixedTables tab;
+        MixedShared &sh = *(MixedShared *)tab.carve((float *)(s_red + 6 * (kMixedBlock / 32)), nr, npoly, false);
+        unsigned *s_bits = (unsigned *)(&sh + 1);  // nodes left to the FP64 pass
+        const int nw = defer_words(a.mixed_chunk);
+        unsigned char *state = (unsigned char *)(s_bits + nw);
+        const double R = q.point[4 * (size_t)slot], z = q.point[4 * (size_t)slot + 1],
+                     Phi_h = q.point[4 * (size_t)slot + 2], Ve = q.point[4 * (size_t)slot + 3];
+        const int n = q.nbound[slot];
+        MixedRec *rec = (MixedRec *)q.rec + (size_t)slot * q.stride;
+        for (int i = threadIdx.x; i < a.nq; i += blockDim.x) { s_xq[i] = a.xq[i]; s_wq[i] = a.wq[i]; }
+        for (int i = threadIdx.x; i < nw; i += blockDim.x) s_bits[i] = 0u;
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            const unsigned w = rec[i].word;
+            state[i] = w & kRecJu ? kIntNew : kIntNone;
+            state[n + i] = w & kRecJv ? kIntNew : kIntNone;
+        }
+        if (threadIdx.x < 11) {
+            sh.K.xgk[threadIdx.x] = (float)fj_xgk21_d[threadIdx.x];
+            sh.K.wgk[threadIdx.x] = (float)fj_wgk21_d[threadIdx.x];
+            if (threadIdx.x < 5) sh.K.wg[threadIdx.x] = (float)fj_wg10_d[threadIdx.x];
+        }
+        const PotViewF PF = tab.build(a, Phi_h, R, z);
+        mixed_integrals(PF, n, rec, L, state, sh);
+        __syncthreads();
+        // The DFs and the moments: thread t sums nodes t, t + 128, .. of the sorted
+        // list.  A node whose FP32 solve hit a cap (a full QAGS list, a bracket walk
+        // or Brent at its step limit) is marked in the item's bitmap and counts 0
+        // here: the FP64 pass solves it again with the plain form's FP64 solve (QAGS
+        // lists of kQagsCap intervals) and adds it to this item's sums.  Only what
+        // that solve still caps is a failure, with the plain form's policy (a capped
+        // bracket or root: DF 0; a full QAGS list: the estimate so far, as QUADPACK
+        // returns it).
+        const int nq = a.nq, nq2 = nq * nq, p = bid / a.blocks_per_point;
+        const long long nq3 = (long long)nq2 * nq;
+        int n0, n1;
+        item_range(a, bid, n0, n1);
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const double jacob = Ve * Ve * Ve;
+        double m[6] = {0, 0, 0, 0, 0, 0};
+        FailTally tally;
+        for (int k = threadIdx.x; k < n; k += kMixedBlock) {
+            const MixedRec &r = rec[k];
+            const int local = (int)(r.word >> kRecNode), node = n0 + local;
+            const int i = node / nq2, j = (node / nq) % nq, l = node % nq;
+            const double V0 = 1e-6 + Ve * s_xq[i], V1 = 1e-6 + Ve * s_xq[j], V2 = 1e-6 + Ve * s_xq[l];
+            const unsigned fail =
+                (r.word & 7u) | (state[k] == kIntFull || state[n + k] == kIntFull ? kFailQuad : 0u);
+            float f = 0.f;
+            if (fail && a.defer) {
+                atomicOr(&s_bits[local >> 5], 1u << (local & 31));
+                atomicAdd(&s_nleft, 1);
+            } else {
+                if (a.jout) {
+                    float *jo = a.jout + ((size_t)p * nq3 + node) * 2;
+                    jo[0] = r.Jr;
+                    jo[1] = r.Jz;
+                }
+                tally.add(fail);
+                if (!(fail & (kFailBracket | kFailRoot))) f = mixed_df(a.df, R * V1, r.Jr, r.Jz);
+            }
+            const double jd = (s_wq[i] * s_wq[j] * s_wq[l]) * (jacob * (double)f);
+            m[0] += jd;
+            m[1] += jd * V1;
+            m[2] += jd * V0 * V0;
+            m[3] += jd * V1 * V1;
+            m[4] += jd * V2 * V2;
+            m[5] += jd * V0 * V2;
+        }
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+            double v = m[c];
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+            if (lane == 0) s_red[warp * 6 + c] = v;
+        }
+        warp_count_fails(a.counters, tally);
+        __syncthreads();
+        if (threadIdx.x < 6) {
+            double s = 0;
+            for (int w = 0; w < kMixedBlock / 32; w++) s += s_red[w * 6 + threadIdx.x];
+            a.partial[(size_t)bid * 6 + threadIdx.x] = s;
+        }
+        if (a.defer) {  // the item's bitmap of deferred nodes and their number
+            for (int i = threadIdx.x; i < nw; i += blockDim.x) a.defer[(size_t)bid * nw + i] = s_bits[i];
+            if (threadIdx.x == 0) a.defer_count[bid] = s_nleft;
+        }
+        if (q.cost && threadIdx.x == 0) q.cost[g] += (float)(clock64() - t_start);
+    }
+}
+
+// ------------------------------------------------------ the FP64 pass
+// Over the nodes the mixed kernel left (launch_deferred): a scan of the
+// blocks' counts, the compact list, one thread per listed node, one thread per
+// block adding its nodes in list order.
 
 // the block's point, its potential and escape speed (as the mixed kernel's setup)
 __device__ void defer_point(const MomentArgs &a, int bid, double &R, double &z, double &Phi_h, double &Ve)
@@ -524,60 +719,73 @@ static cudaError_t launch_deferred(const MomentArgs &a, const MomentBatch &b, lo
 }
 
 namespace {
-template <int MINB, bool DYN>
-cudaError_t launch_variant(const MomentArgs &a, const MomentBatch &b, const ItemQueue &q, size_t smem, cudaStream_t s)
+const void *turn_kernel(int variant)
 {
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_moments_mixed<MINB, DYN>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
+    return variant < 4 ? (const void *)k_mixed_turn<4> : (const void *)k_mixed_turn<8>;
+}
+
+const void *integrate_kernel(int variant)
+{
+    switch (variant & 3) {
+    case 0: return (const void *)k_mixed_integrate<3>;
+    case 1: return (const void *)k_mixed_integrate<4>;
+    case 2: return (const void *)k_mixed_integrate<6>;
+    default: return (const void *)k_mixed_integrate<8>;
     }
+}
+
+int resident(const void *k, size_t smem)
+{
     int dev = 0, nsm = 0, per_sm = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_moments_mixed<MINB, DYN>, kMixedBlock, smem);
-    if (e != cudaSuccess) return e;
-    const long long resident = (long long)(per_sm > 0 ? per_sm : 1) * (nsm > 0 ? nsm : 1);
-    const long long grid = q.total < resident ? q.total : resident;
-    if ((e = cudaMemsetAsync(q.next, 0, sizeof(unsigned), s)) != cudaSuccess) return e;
-    k_moments_mixed<MINB, DYN><<<(unsigned)grid, kMixedBlock, smem, s>>>(a, b, q);
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        (smem > 48 * 1024 &&
+         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kMixedBlock, smem) != cudaSuccess)
+        return 0;
+    return per_sm * nsm;
+}
+
+// the launch's items, a slice of q.per_slice at a time through both kernels
+cudaError_t launch_mixed_any(const MomentArgs &a, const MomentBatch &b, const ItemQueue &q0, size_t smem_t,
+                             size_t smem_i, int variant, cudaStream_t s)
+{
+    if (variant < 0 || variant >= kMixedVariants || q0.grid < 1 || q0.grid_turn < 1) return cudaErrorInvalidValue;
+    for (int first = 0; first < q0.total; first += q0.per_slice) {
+        ItemQueue q = q0;
+        q.first = first;
+        q.count = q0.total - first < q0.per_slice ? q0.total - first : q0.per_slice;
+        cudaError_t e = cudaMemsetAsync(q.next, 0, 2 * sizeof(unsigned), s);
+        if (e != cudaSuccess) return e;
+        void *args[] = {(void *)&a, (void *)&b, (void *)&q};
+        const unsigned gt = (unsigned)(q.count < q.grid_turn ? q.count : q.grid_turn),
+                       gi = (unsigned)(q.count < q.grid ? q.count : q.grid);
+        if ((e = cudaLaunchKernel(turn_kernel(variant), dim3(gt), dim3(kMixedBlock), args, smem_t, s)) != cudaSuccess ||
+            (e = cudaLaunchKernel(integrate_kernel(variant), dim3(gi), dim3(kMixedBlock), args, smem_i, s)) !=
+                cudaSuccess)
+            return e;
+    }
     return cudaGetLastError();
 }
-
-cudaError_t launch_mixed_any(const MomentArgs &a, const MomentBatch &b, const ItemQueue &q, size_t smem, int variant,
-                             cudaStream_t s)
-{
-    switch (variant) {
-    case 0: return launch_variant<3, false>(a, b, q, smem, s);
-    case 1: return launch_variant<4, false>(a, b, q, smem, s);
-    case 2: return launch_variant<6, false>(a, b, q, smem, s);
-    case 3: return launch_variant<8, false>(a, b, q, smem, s);
-    case 4: return launch_variant<3, true>(a, b, q, smem, s);
-    case 5: return launch_variant<4, true>(a, b, q, smem, s);
-    case 6: return launch_variant<6, true>(a, b, q, smem, s);
-    case 7: return launch_variant<8, true>(a, b, q, smem, s);
-    default: return cudaErrorInvalidValue;
-    }
-}
-
-template <int MINB, bool DYN>
-size_t local_bytes()
-{
-    cudaFuncAttributes at;
-    return cudaFuncGetAttributes(&at, k_moments_mixed<MINB, DYN>) == cudaSuccess ? at.localSizeBytes : 0;
-}
 }  // namespace
+
+void mixed_resident(int variant, const MixedSmem &sm, int &turn, int &integrate)
+{
+    turn = resident(turn_kernel(variant), sm.turn);
+    integrate = resident(integrate_kernel(variant), sm.integrate);
+}
+
+MixedSmem mixed_smem(const MomentArgs &a) { return MixedSmem{mixed_turn_smem(a), mixed_integrate_smem(a)}; }
 
 cudaError_t launch_moments_mixed(const MomentArgs &a, int variant, const DeferWork &dw, const ItemQueue &q,
                                  cudaStream_t s)
 {
     if (a.mixed_chunk < kMixedBlock || a.mixed_chunk > kMixedMaxNodes) return cudaErrorInvalidValue;
-    const size_t smem = moment_mixed_smem_bytes(a);
     const MomentBatch none{nullptr, nullptr, nullptr, 0};
     const long long nblocks = (long long)a.npts * a.blocks_per_point;
     if (q.total != nblocks) return cudaErrorInvalidValue;
-    cudaError_t e = launch_mixed_any(a, none, q, smem, variant, s);
+    const MixedSmem sm = mixed_smem(a);
+    cudaError_t e = launch_mixed_any(a, none, q, sm.turn, sm.integrate, variant, s);
     if (e == cudaSuccess) e = launch_deferred(a, none, nblocks, dw, s);
     if (e != cudaSuccess) return e;
     return launch_moments_finalize(a, s);
@@ -586,24 +794,23 @@ cudaError_t launch_moments_mixed(const MomentArgs &a, int variant, const DeferWo
 cudaError_t launch_moments_plain_batch(const MomentArgs &a0, const MomentBatch &b, size_t smem, const PlainWork &w,
                                       cudaStream_t s);
 
-cudaError_t launch_moments_batch(const MomentArgs &a0, const MomentBatch &b, int nblocks, size_t smem, bool mixed,
-                                 int variant, const DeferWork &dw, const ItemQueue &q, const PlainWork &w,
+cudaError_t launch_moments_batch(const MomentArgs &a0, const MomentBatch &b, int nblocks, size_t smem,
+                                 const MixedSmem &msm, bool mixed, int variant, const DeferWork &dw, const ItemQueue &q, const PlainWork &w,
                                  cudaStream_t s)
 {
     if (!mixed) return launch_moments_plain_batch(a0, b, smem, w, s);
     if (q.total != nblocks) return cudaErrorInvalidValue;
-    const cudaError_t e = launch_mixed_any(a0, b, q, smem, variant, s);
+    const cudaError_t e = launch_mixed_any(a0, b, q, msm.turn, msm.integrate, variant, s);
     return e == cudaSuccess ? launch_deferred(a0, b, nblocks, dw, s) : e;
 }
 
 size_t moments_mixed_local_bytes()
 {
-    const size_t v[kMixedVariants] = {local_bytes<3, false>(), local_bytes<4, false>(), local_bytes<6, false>(),
-                                      local_bytes<8, false>(), local_bytes<3, true>(), local_bytes<4, true>(),
-                                      local_bytes<6, true>(), local_bytes<8, true>()};
     size_t m = 0;
-    for (size_t x : v) m = x > m ? x : m;
     cudaFuncAttributes at;
+    for (int v = 0; v < kMixedVariants; v++)
+        for (const void *k : {turn_kernel(v), integrate_kernel(v)})
+            if (cudaFuncGetAttributes(&at, k) == cudaSuccess && at.localSizeBytes > m) m = at.localSizeBytes;
     for (const void *k : {(const void *)k_defer_solve, (const void *)k_defer_add})
         if (cudaFuncGetAttributes(&at, k) == cudaSuccess && at.localSizeBytes > m) m = at.localSizeBytes;
     return m;

@@ -40,20 +40,22 @@ struct OrbitRec {
     __device__ unsigned status() const { return fail | (full[0] | full[1] ? kFailQuad : 0u); }
 };
 
+using OrbitQags = GroupQags<double, kQagsCap, true>;
+
 // A block's scratch in device memory
 struct SolveScratch {
     OrbitRec *rec;                          // [chunk]
     double2 *head;                          // [2 chunk]: first panels of the integrals that go on (result, error)
-    QagsList<double, kQagsCap> *lists;      // [kSolveGroups]
+    OrbitQags::List *lists;      // [kSolveGroups]
 };
 FJ_HD size_t solve_scratch_bytes(int chunk)
 {
-    return chunk * (sizeof(OrbitRec) + 2 * sizeof(double2)) + kSolveGroups * sizeof(QagsList<double, kQagsCap>);
+    return chunk * (sizeof(OrbitRec) + 2 * sizeof(double2)) + kSolveGroups * sizeof(OrbitQags::List);
 }
 FJ_HD SolveScratch solve_scratch(char *base, int chunk)
 {
     SolveScratch s;
-    s.lists = (QagsList<double, kQagsCap> *)base;
+    s.lists = (OrbitQags::List *)base;
     s.head = (double2 *)(s.lists + kSolveGroups);
     s.rec = (OrbitRec *)(s.head + 2 * chunk);
     return s;
@@ -186,8 +188,8 @@ __device__ void solve_orbits64(const PotView &P, const GLRule &gl, const double2
     if (threadIdx.x == 0) sh.next = 0;
     __syncthreads();
     if (sh.nmore > 0) {
-        QagsList<double, kQagsCap> &L = S.lists[g];
-        GroupQags<double, kQagsCap> st;
+        OrbitQags::List &L = S.lists[g];
+        OrbitQags st;
         int item = -1;
         double a1 = 0, b2 = 0;
         unsigned heap = 0;

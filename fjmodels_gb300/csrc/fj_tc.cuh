@@ -61,6 +61,14 @@ __device__ __forceinline__ float gelu_grad(float z)
     return 0.5f * (1.f + t) + 0.5f * z * (1.f - t * t) * 0.7978845608028654f * (1.f + 3.f * 0.044715f * z * z);
 }
 
+// two floats rounded to BF16, lo in the low half
+__device__ __forceinline__ uint32_t bf16x2(float hi, float lo)
+{
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // shared-memory matrix descriptor: start address, leading/stride byte offsets

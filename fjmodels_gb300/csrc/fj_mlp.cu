@@ -795,20 +795,22 @@ __global__ void __launch_bounds__(128) k_sg_moments(SgGrid g, const double *wq, 
 
 // ======================================================================
 // Fused surrogate moments: features, the MLP on the tensor cores and the DF
-// moment sums of one grid point's bound nodes in one kernel.  One CTA per
-// (grid point, node range); two groups of eight warps each own a 128-node
-// tile in flight (own activation buffer, 128 TMEM columns, mbarrier) and
-// share the five layers' BF16 weights, resident in shared memory in the
-// canonical K-major layout.  Per tile: a thread per node writes its 16
-// features into the operand buffer; one thread issues the layer's
-// tcgen05.mma chain; after the commit the group reads the accumulators back
-// (tcgen05.ld), applies bias and GELU and writes the BF16 activations into
-// the same buffer as the next layer's operand; the output layer's log h and
-// log g go straight into the DF and the FP64 moment sums.
-// The GELUs are the bound (512 per node against 0.1 Mflop of MMA), and with four
-// warps per group the two warps of a scheduler could not cover their latency:
-// eight warps share a tile, each thread half of its node's columns (80 x 40 grid,
-// 22^3 nodes, with the FP64 work of a node cut: 10.1 -> 8.4 ms).
+// moment sums of the grid points' bound nodes in one kernel.  One persistent CTA
+// per SM; its three groups of eight warps share the five layers' BF16 weights,
+// resident in shared memory in the canonical K-major layout, and nothing else:
+// each goes through its own items (grid point, node range), collects their bound
+// nodes into 128-node tiles and has its own activation buffer, 128 TMEM columns
+// and mbarrier.  Per tile: a thread per node writes its 16 features into the
+// operand buffer; one thread issues the layer's tcgen05.mma chain; after the
+// commit the group reads the accumulators back (tcgen05.ld), each thread half of
+// its node's columns, applies bias and GELU and writes the BF16 activations into
+// the same buffer as the next layer's operand; the output layer's log h and log g
+// go straight into the DF and the FP64 moment sums.
+// The GELUs are the bound: 512 per node against 0.1 Mflop of MMA.  80 x 40 grid,
+// 22^3 nodes: 10.1 ms with two groups of four warps and the features in FP64 (issue
+// slots 36 % busy), 8.4 ms with eight warps per group and the FP64 work of a node
+// cut, 7.6 ms with packed FP32 pairs in the GELU (gelu2_bf16), 6.8 ms with three
+// independent groups.
 // ======================================================================
 namespace fj {
 
@@ -817,10 +819,12 @@ struct SgWeights {
     const float *b[5];
 };
 
-constexpr int kFusedGroup = 256;               // threads of a group: 128 nodes x 2 halves of the columns
-constexpr int kFusedThreads = 2 * kFusedGroup;  // two groups
+constexpr int kFusedGroup = 256;                         // threads of a group: 128 nodes x 2 halves of the columns
+constexpr int kFusedGroups = 3;
+constexpr int kFusedThreads = kFusedGroups * kFusedGroup;
 constexpr int kFusedAxis = 64;         // points of a velocity rule whose squares are tabulated
-constexpr int kFusedMaxNodes = 12288;  // node range of one CTA (bound-node list in shared memory)
+constexpr int kFusedMaxNodes = 12288;  // most nodes of an item
+constexpr int kFusedBuf = 128 + kFusedGroup;  // bound nodes waiting for a tile
 
 // canonical no-swizzle K-major offset (bytes) of element (row, k) of a [rows][K]
 // bf16 operand: K steps of 16 are rows*32 bytes apart
@@ -829,12 +833,12 @@ __device__ __forceinline__ uint32_t kmaj_off(int row, int k, int rows)
     return (uint32_t)((k >> 4) * rows * 32 + (row >> 3) * 256 + ((k >> 3) & 1) * 128 + (row & 7) * 16 + (k & 7) * 2);
 }
 
-// shared memory: W0 4 KB | W1..W3 96 KB | W4 4 KB | biases 2112 B | 2 x act 32 KB | list | misc
+// shared memory: W0 4 KB | W1..W3 96 KB | W4 4 KB | biases 2112 B | 3 x act 32 KB | 3 x node buffer
 constexpr int kSmW0 = 0, kSmW1 = 4096, kSmW4 = kSmW1 + 3 * 32768, kSmBias = kSmW4 + 4096;
 constexpr int kSmAct = kSmBias + 4 * 128 * 4 + 16 * 4 + 192;  // 1024-aligned below
 constexpr int kSmActAligned = (kSmAct + 1023) / 1024 * 1024;
-constexpr int kSmList = kSmActAligned + 2 * 32768;
-constexpr size_t fused_smem_bytes() { return (size_t)kSmList + kFusedMaxNodes * 2 + 256; }
+constexpr int kSmBuf = kSmActAligned + kFusedGroups * 32768;
+constexpr size_t fused_smem_bytes() { return (size_t)kSmBuf + kFusedGroups * kFusedBuf * 2 + 256; }
 
 // Feature 13, log(H / Phi) / 5 with H = K + Phi, as it enters the network (rounded
 // to BF16 next): in FP32 where every number within the FP32 form's error rounds to
@@ -852,31 +856,33 @@ __device__ __forceinline__ float log_energy(double K, double Phi, double iPhi)
 }
 
 __global__ void __launch_bounds__(kFusedThreads, 1) k_sg_fused(SgGrid g, SgWeights wts, const double *wq, DFDev df,
-                                                               int blocks_per_point, double *partial, int *err)
+                                                               int blocks_per_point, int items, double *partial, int *err)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
-    __shared__ __align__(8) unsigned long long bars[2];
+    __shared__ __align__(8) unsigned long long bars[kFusedGroups];
     __shared__ uint32_t tmem_slot;
-    __shared__ float s_v2[kFusedAxis];
-    __shared__ int s_wc[kFusedThreads / 32];
-    __shared__ double s_red[(kFusedThreads / 32) * 6];
-    unsigned short *s_list = (unsigned short *)(sm + kSmList);
+    __shared__ float g_v2[kFusedGroups][kFusedAxis], g_fx[kFusedGroups][13];  // squared velocities; the point's features (0, 1, 5..12)
+    __shared__ double g_pt[kFusedGroups][2], g_red[kFusedGroups][(kFusedGroup / 32) * 6];  // R, 1 / Phi; the warps' sums
+    __shared__ int g_wc[kFusedGroups][kFusedGroup / 32];
     float *s_bias = (float *)(sm + kSmBias);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, grp = tid / kFusedGroup, gt = tid % kFusedGroup;
+    const int gw = gt >> 5;                    // the warp within the group
     const int row = gt & 127, half = gt >> 7;  // the thread's node of the tile and its half of the columns
-    const int B = blocks_per_point, p = blockIdx.x / B, chunk = blockIdx.x % B;
-    const int nq = g.nq, nq3 = nq * nq * nq;
-    const int n0 = (int)((long long)chunk * nq3 / B), n1 = (int)((long long)(chunk + 1) * nq3 / B);
+    const int B = blocks_per_point, nq = g.nq, nq3 = nq * nq * nq;
+    unsigned short *buf = (unsigned short *)(sm + kSmBuf) + grp * kFusedBuf;
+    float *s_v2 = g_v2[grp], *s_fx = g_fx[grp];
+    double *s_pt = g_pt[grp], *s_red = g_red[grp];
+    int *s_wc = g_wc[grp];
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          tc::smem_addr(&tmem_slot)),
-                     "r"(256)
+                     "r"(512)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (tid < 2) {
+    if (tid < kFusedGroups) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc::smem_addr(&bars[tid])), "r"(1) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -894,48 +900,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_sg_fused(SgGrid g, SgWeigh
         }
         for (int q = tid; q < 4 * 128 + 16; q += kFusedThreads) s_bias[q] = wts.b[q >> 7 < 4 ? q >> 7 : 4][q < 512 ? q & 127 : q - 512];
     }
-    // bound nodes of [n0, n1) in node order (the sums as sg_velocity forms them)
-    const double Phi_h = g.point[2 * p], Ve = g.point[2 * p + 1];
-    auto velocity = [&](int node, double &V0, double &V1, double &V2) {
-        V0 = 1e-6 + Ve * g.xq[node / (nq * nq)];
-        V1 = 1e-6 + Ve * g.xq[(node / nq) % nq];
-        V2 = 1e-6 + Ve * g.xq[node % nq];
-    };
-    // the sign of H in FP32 from the squared velocities where that is clear of
-    // its rounding, else in FP64 (whose pipe the whole sum would hold for 36 us)
-    const bool tabled = nq <= kFusedAxis;
-    if (tabled && tid < nq) {
-        const double v = 1e-6 + Ve * g.xq[tid];
-        s_v2[tid] = (float)(.5 * v * v);
-    }
-    __syncthreads();
-    const float Phi_f = (float)Phi_h, clear_f = 2e-6f * fabsf(Phi_f);
-    int nbound = 0;
-    for (int base = n0; base < n1; base += kFusedThreads) {
-        const int node = base + tid;
-        bool b = false;
-        if (node < n1) {
-            float h = 0.f;
-            if (tabled) h = s_v2[node / (nq * nq)] + s_v2[(node / nq) % nq] + s_v2[node % nq] + Phi_f;
-            b = h < 0.f;
-            if (!(fabsf(h) > clear_f)) {
-                double V0, V1, V2;
-                velocity(node, V0, V1, V2);
-                b = .5 * (V0 * V0 + V1 * V1 + V2 * V2) + Phi_h < 0;
-            }
-        }
-        const unsigned bal = __ballot_sync(0xffffffffu, b);
-        if (lane == 0) s_wc[warp] = __popc(bal);
-        __syncthreads();
-        int off = nbound, tot = 0;
-        for (int w = 0; w < kFusedThreads / 32; w++) {
-            if (w < warp) off += s_wc[w];
-            tot += s_wc[w];
-        }
-        if (b) s_list[off + __popc(bal & ((1u << lane) - 1u))] = (unsigned short)(node - n0);
-        __syncthreads();
-        nbound += tot;
-    }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -944,19 +908,9 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_sg_fused(SgGrid g, SgWeigh
     const uint32_t bar = tc::smem_addr(&bars[grp]);
     unsigned char *act = sm + kSmActAligned + grp * 32768;
     const uint32_t act_a = tc::smem_addr(act), w_a = tc::smem_addr(sm);
-    const int n = p / g.ngauss, np_ = g.P.npoly;
-    const double c = g.ci[p % g.ngauss], R = g.P.ar[n] * sqrt(1 - c * c), jacob = Ve * Ve * Ve;
-    // per-point features
-    float fx[14];
-    fx[0] = (float)((log(g.P.ar[n]) - g.lmu) / g.lsig);
-    fx[1] = (float)c;
-    const double p0v = g.P.phil[n * np_];
-    fx[5] = (float)(p0v / g.P.phil[0]);
-    for (int l = 1; l < 8; l++) fx[5 + l] = l < np_ ? (float)(g.P.phil[n * np_ + l] / fabs(p0v)) : 0.f;
-    double m[6] = {0, 0, 0, 0, 0, 0};
-    const double iPhi = 1. / Phi_h;
-    uint32_t phase = 0;
     const float J0 = (float)df.J0;
+    uint32_t phase = 0;
+    bool aborted = false;
     auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(kFusedGroup) : "memory"); };
     // true in every thread of the group when v is true in any of them (also a group barrier)
     auto group_any = [&](bool v) {
@@ -992,18 +946,82 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_sg_fused(SgGrid g, SgWeigh
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         return !bad;
     };
-    const int ntiles = (nbound + 127) / 128;
-    bool aborted = false;
-    for (int t = grp; t < ntiles && !aborted; t += 2) {
-        const int q = t * 128 + row;
-        const bool valid = half == 0 && q < nbound;
-        const int node = valid ? n0 + s_list[q] : n0;
+    // Every group goes through its own items (grid point, node range); nothing but
+    // the weights is shared.  Bound nodes collect in the group's buffer, in node
+    // order, until they fill a tile.
+    for (int item = blockIdx.x * kFusedGroups + grp; item < items && !aborted; item += gridDim.x * kFusedGroups) {
+        const int p = item / B, chunk = item % B;
+        const int n0 = (int)((long long)chunk * nq3 / B), n1 = (int)((long long)(chunk + 1) * nq3 / B);
+        const double Phi_h = g.point[2 * p], Ve = g.point[2 * p + 1];
+        auto velocity = [&](int node, double &V0, double &V1, double &V2) {
+            V0 = 1e-6 + Ve * g.xq[node / (nq * nq)];
+            V1 = 1e-6 + Ve * g.xq[(node / nq) % nq];
+            V2 = 1e-6 + Ve * g.xq[node % nq];
+        };
+        // the point's features, one per thread (by every thread for itself they held
+        // the FP64 pipe for 19 us per item)
+        {
+            const int n = p / g.ngauss, np_ = g.P.npoly;
+            const double c = g.ci[p % g.ngauss];
+            if (gt == 0) s_fx[0] = (float)((log(g.P.ar[n]) - g.lmu) / g.lsig);
+            if (gt == 32) { s_fx[1] = (float)c; s_pt[0] = g.P.ar[n] * sqrt(1 - c * c); }
+            if (gt == 64) s_pt[1] = 1. / Phi_h;
+            if (gt >= 96 && gt < 104) {
+                const double p0v = g.P.phil[n * np_];
+                const int l = gt - 96;
+                s_fx[5 + l] =
+                    l == 0 ? (float)(p0v / g.P.phil[0]) : l < np_ ? (float)(g.P.phil[n * np_ + l] / fabs(p0v)) : 0.f;
+            }
+        }
+        // the sign of H in FP32 from the squared velocities where that is clear of its
+        // rounding, else in FP64 (the sums as sg_velocity forms them)
+        const bool tabled = nq <= kFusedAxis;
+        if (tabled && gt < nq) {
+            const double v = 1e-6 + Ve * g.xq[gt];
+            s_v2[gt] = (float)(.5 * v * v);
+        }
+        group_sync();
+        const float Phi_f = (float)Phi_h, clear_f = 2e-6f * fabsf(Phi_f);
+        const double R = s_pt[0], iPhi = s_pt[1], jacob = Ve * Ve * Ve;
+        double m[6] = {0, 0, 0, 0, 0, 0};
+        int pos = n0, cnt = 0;
+        for (;;) {
+        while (cnt < 128 && pos < n1) {
+            const int node = pos + gt;
+            bool b = false;
+            if (node < n1) {
+                float h = 0.f;
+                if (tabled) h = s_v2[node / (nq * nq)] + s_v2[(node / nq) % nq] + s_v2[node % nq] + Phi_f;
+                b = h < 0.f;
+                if (!(fabsf(h) > clear_f)) {
+                    double V0, V1, V2;
+                    velocity(node, V0, V1, V2);
+                    b = .5 * (V0 * V0 + V1 * V1 + V2 * V2) + Phi_h < 0;
+                }
+            }
+            const unsigned bal = __ballot_sync(0xffffffffu, b);
+            if (lane == 0) s_wc[gw] = __popc(bal);
+            group_sync();
+            int off = cnt, tot = 0;
+            for (int w = 0; w < kFusedGroup / 32; w++) {
+                if (w < gw) off += s_wc[w];
+                tot += s_wc[w];
+            }
+            if (b) buf[off + __popc(bal & ((1u << lane) - 1u))] = (unsigned short)(node - n0);
+            group_sync();
+            cnt += tot;
+            pos += kFusedGroup;
+        }
+        if (cnt == 0) break;
+        const int nt = min(cnt, 128);
+        const bool valid = half == 0 && row < nt;
+        const int node = valid ? n0 + buf[row] : n0;
         double V0 = 0, V1 = 0, V2 = 0;
         // features of the node, row `row` of the K = 16 operand
         if (half == 0) {
             velocity(node, V0, V1, V2);
             float x[16];
-            for (int i = 0; i < 14; i++) x[i] = fx[i];
+            for (int i = 0; i < 13; i++) x[i] = s_fx[i];
             x[2] = (float)g.xq[node / (nq * nq)];
             x[3] = (float)g.xq[node % nq];
             x[4] = (float)g.xq[(node / nq) % nq];
@@ -1030,12 +1048,14 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_sg_fused(SgGrid g, SgWeigh
                       "=r"(r[15])
                     : "r"(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0));
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                const float *bias = s_bias + l * 128 + c0;
+                const ulonglong2 *bias = reinterpret_cast<const ulonglong2 *>(s_bias + l * 128 + c0);
                 uint32_t v[8];
 #pragma unroll
-                for (int e = 0; e < 8; e++)
-                    v[e] = tc::bf16x2(tc::gelu(__uint_as_float(r[2 * e + 1]) + bias[2 * e + 1]),
-                                      tc::gelu(__uint_as_float(r[2 * e]) + bias[2 * e]));
+                for (int e = 0; e < 4; e++) {
+                    const ulonglong2 b4 = bias[e];
+                    v[2 * e] = tc::gelu2_bf16((uint64_t)r[4 * e + 1] << 32 | r[4 * e], b4.x);
+                    v[2 * e + 1] = tc::gelu2_bf16((uint64_t)r[4 * e + 3] << 32 | r[4 * e + 2], b4.y);
+                }
                 *reinterpret_cast<uint4 *>(act + kmaj_off(row, c0, 128)) = make_uint4(v[0], v[1], v[2], v[3]);
                 *reinterpret_cast<uint4 *>(act + kmaj_off(row, c0 + 8, 128)) = make_uint4(v[4], v[5], v[6], v[7]);
             }
@@ -1072,18 +1092,26 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_sg_fused(SgGrid g, SgWeigh
             m[4] += jd * V2 * V2;
             m[5] += jd * V0 * V2;
         }
-    }
-    for (int qq = 0; qq < 6; qq++) {
-        double v = m[qq];
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-        if (lane == 0) s_red[warp * 6 + qq] = v;
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (tid < 6) {
-        double sacc = 0;
-        for (int w = 0; w < kFusedThreads / 32; w++) sacc += s_red[w * 6 + tid];
-        partial[((size_t)p * B + chunk) * 6 + tid] = sacc;
+        // the nodes past the tile move to the front
+        const int rest = cnt - nt;
+        const unsigned short mv = gt < rest ? buf[nt + gt] : (unsigned short)0;
+        group_sync();
+        if (gt < rest) buf[gt] = mv;
+        group_sync();
+        cnt = rest;
+        }
+        for (int qq = 0; qq < 6; qq++) {
+            double v = m[qq];
+            for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+            if (lane == 0) s_red[gw * 6 + qq] = v;
+        }
+        group_sync();
+        if (gt < 6) {
+            double sacc = 0;
+            for (int w = 0; w < kFusedGroup / 32; w++) sacc += s_red[w * 6 + gt];
+            partial[((size_t)p * B + chunk) * 6 + gt] = sacc;
+        }
+        group_sync();  // the group's sums and features are free for its next item
     }
     if (aborted) {  // let the group's outstanding commit land before TMEM is freed
         tc::mbar_wait(bar, phase ^ 1u);
@@ -1092,12 +1120,29 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_sg_fused(SgGrid g, SgWeigh
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_slot), "r"(256) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_slot), "r"(512) : "memory");
 }
 
 }  // namespace fj
 
 namespace {
+
+// Node ranges per grid point of the fused kernel: what its 16-bit node indices
+// hold, else the split that ends evenly: rounds of the persistent groups times an
+// item's tiles (0.4 of the nodes bound, half a tile lost to the remainder, and
+// about half a tile's time to start an item)
+int sg_fused_blocks(int npts, int nq3, int groups)
+{
+    const int need = (nq3 + fj::kFusedMaxNodes - 1) / fj::kFusedMaxNodes;
+    int best = need;
+    double least = 1e300;
+    for (int B = need; B <= std::max(need, std::min(need + 16, nq3 / 512)); B++) {
+        const double rounds = (double)(((long long)npts * B + groups - 1) / groups);
+        const double t = rounds * (0.4 * nq3 / B / 128 + 1.0);
+        if (t < least) { least = t; best = B; }
+    }
+    return best;
+}
 
 int sg_grid(fj_surrogate *s, const fj_potential *pot, int ngauss, const fj_quad_rule *rule, fj::SgGrid &g)
 {
@@ -1171,7 +1216,11 @@ int fj_surrogate_moments(fj_surrogate *s, const fj_potential *pot, const fj_df_p
     const double *ci, *xq, *wq;
     if ((rc = fj::context_grid_inputs(s->ctx, ngauss, rule, &ci, &xq, &wq))) return rc;
     const int npts = pot->nr * ngauss, nq3 = rule->nq * rule->nq * rule->nq;
-    const int B = fused ? (nq3 + fj::kFusedMaxNodes - 1) / fj::kFusedMaxNodes : 1;
+    int dev = 0, nsm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return FJ_ERR_CUDA;
+    const int B = fused ? sg_fused_blocks(npts, nq3, nsm * fj::kFusedGroups) : 1;
     if ((long long)npts * B > s->partial_cap) {
         void *q;
         if ((rc = sg_alloc(s, &q, (size_t)npts * B * 6 * sizeof(double)))) return rc;
@@ -1194,7 +1243,8 @@ int fj_surrogate_moments(fj_surrogate *s, const fj_potential *pot, const fj_df_p
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
         cudaEventRecord(e0, s->stream);
-        fj::k_sg_fused<<<npts * B, fj::kFusedThreads, smem, s->stream>>>(g, w, wq, dd, B, s->partial, s->err);
+        const int items = npts * B, ctas = std::min((items + fj::kFusedGroups - 1) / fj::kFusedGroups, nsm);
+        fj::k_sg_fused<<<ctas, fj::kFusedThreads, smem, s->stream>>>(g, w, wq, dd, B, items, s->partial, s->err);
         cudaEventRecord(e1, s->stream);
         if (cudaGetLastError() != cudaSuccess) return FJ_ERR_CUDA;
         fj::MomentArgs a{};

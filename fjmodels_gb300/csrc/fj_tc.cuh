@@ -69,6 +69,49 @@ __device__ __forceinline__ uint32_t bf16x2(float hi, float lo)
     return r;
 }
 
+// gelu() of two values (x + b), rounded to BF16 (the first in the low half): the
+// same operations in the same order, the pair's products, sums and FMAs as
+// packed FP32 instructions (half the issue slots)
+__device__ __forceinline__ uint64_t pack2(float a, float b)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float &a, float &b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint32_t gelu2_bf16(uint64_t x, uint64_t b)
+{
+    const uint64_t z = add2(x, b);
+    const uint64_t cz = mul2(pack2(0.044715f, 0.044715f), z);
+    const uint64_t u = mul2(pack2(0.7978845608028654f, 0.7978845608028654f), fma2(mul2(cz, z), z, z));
+    float u0, u1, g0, g1;
+    unpack2(u, u0, u1);
+    const uint64_t t = add2(pack2(1.f, 1.f), pack2(tanhf(u0), tanhf(u1)));
+    unpack2(mul2(mul2(pack2(0.5f, 0.5f), z), t), g0, g1);
+    return bf16x2(g1, g0);
+}
+
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // shared-memory matrix descriptor: start address, leading/stride byte offsets

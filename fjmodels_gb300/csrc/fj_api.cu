@@ -153,7 +153,7 @@ int refresh_queue_order(fj_ctx *ctx)
     return FJ_OK;
 }
 
-int queue_setup(fj_ctx *ctx, long long total, int stride, const MixedSmem &sm, ItemQueue &q)
+int queue_setup(fj_ctx *ctx, long long total, int stride, int np, const MixedSmem &sm, ItemQueue &q)
 {
     if (total < 1 || total > 0x7fffffffLL) return fail(ctx, FJ_ERR_ARG, "moments: too many work items");
     const int n = (int)total;
@@ -175,7 +175,7 @@ int queue_setup(fj_ctx *ctx, long long total, int stride, const MixedSmem &sm, I
     q.cost = (float *)(order + n);
     q.total = n;
     int turn, integrate;
-    mixed_resident(ctx->mixed_variant, sm, turn, integrate);
+    mixed_resident(ctx->mixed_variant, np, sm, turn, integrate);
     if (turn < 1 || integrate < 1) return fail(ctx, FJ_ERR_CUDA, "moments: tables exceed shared memory");
     q.grid_turn = n < turn ? n : turn;
     q.grid = n < integrate ? n : integrate;
@@ -388,7 +388,7 @@ int build_args(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delta
         a.ci = gn;
     }
     const long long nq3 = (long long)rule->nq * rule->nq * rule->nq;
-    a.mixed_chunk = plain_chunk(npts, nq3, ctx->mixed_chunk);
+    a.mixed_chunk = plain_chunk(npts, nq3, ctx->mixed_chunk, kMixedItems);
     if (!mixed && (rc = trig_table(ctx, &a.trig))) return rc;
     a.plain_chunk = plain_chunk(npts, nq3);
     a.blocks_per_point =
@@ -448,7 +448,8 @@ int run_moments(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delt
     FJ_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
     ItemQueue q{};
     if (mixed && (rc = queue_setup(ctx, (long long)npts * a.blocks_per_point,
-                                   (int)((nq3 + a.blocks_per_point - 1) / a.blocks_per_point), mixed_smem(a), q))) return rc;
+                                   (int)((nq3 + a.blocks_per_point - 1) / a.blocks_per_point), a.P.npoly,
+                                   mixed_smem(a), q))) return rc;
     FJ_CUDA(mixed ? launch_moments_mixed(a, ctx->mixed_variant, dw, q, ctx->stream)
                   : launch_moments(a, pw, ctx->stream));
     FJ_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
@@ -572,7 +573,7 @@ int fj_moments_batch(fj_ctx *ctx, int n, const fj_batch_item *items, const fj_qu
     std::vector<int> bs(n + 1, 0), ps(n + 1, 0);
     size_t smem = 0, partial = 0, defer_words_total = 0;
     MixedSmem msm{0, 0};
-    int stride = 1;
+    int stride = 1, np = items[0].pot.npoly;  // the models' multipoles (0: they differ)
     bool mixed = false;
     long long nodes = 0;
     const long long nq3 = (long long)rule->nq * rule->nq * rule->nq;
@@ -603,6 +604,7 @@ int fj_moments_batch(fj_ctx *ctx, int n, const fj_batch_item *items, const fj_qu
         } else {
             smem = std::max(smem, moment_smem_bytes(args[m]));
         }
+        if (it.pot.npoly != np) np = 0;
         nodes += nq3 * npts;
     }
     int rc;
@@ -639,8 +641,8 @@ int fj_moments_batch(fj_ctx *ctx, int n, const fj_batch_item *items, const fj_qu
     if (!mixed && (rc = plain_setup(ctx, bs[n], moments_resident(smem), kPlainChunk, pw))) return rc;
     FJ_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
     ItemQueue q{};
-    if (mixed && (rc = queue_setup(ctx, bs[n], stride, msm, q))) return rc;
-    FJ_CUDA(launch_moments_batch(args[0], b, bs[n], smem, msm, mixed, ctx->mixed_variant, dw, q, pw, ctx->stream));
+    if (mixed && (rc = queue_setup(ctx, bs[n], stride, np, msm, q))) return rc;
+    FJ_CUDA(launch_moments_batch(args[0], b, bs[n], smem, msm, mixed, ctx->mixed_variant, np, dw, q, pw, ctx->stream));
     FJ_CUDA(launch_moments_finalize_batch(b, ps[n], ctx->stream));
     FJ_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
     return stats ? read_stats(ctx, nodes, stats) : FJ_OK;

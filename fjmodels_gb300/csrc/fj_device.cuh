@@ -23,10 +23,12 @@
 #define FJ_HD __host__ __device__ __forceinline__
 #define FJ_HDNI static __host__ __device__ __noinline__
 #define FJ_UNROLL _Pragma("unroll")
+#define FJ_UNROLL1 _Pragma("unroll 1")
 #else
 #define FJ_HD inline
 #define FJ_HDNI static inline
 #define FJ_UNROLL
+#define FJ_UNROLL1
 #endif
 
 namespace fj {

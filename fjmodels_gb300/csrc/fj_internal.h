@@ -28,10 +28,14 @@ constexpr int kPlainChunk = 1024;  // most velocity nodes of one point per work 
 // there are enough items to fill the GPU and balance their uneven cost.  By the
 // model's own size alone, so that a batched launch sums in the same order.
 constexpr int kPlainItems = 1216;  // 8 per SM
-inline int plain_chunk(long long npts, long long nq3, int most = kPlainChunk)
+// Mixed form: twice the blocks of its kernels (24x8 model: 9.9 ms with 1536 items
+// of 512 nodes, 8.1 ms with 3072 of 256; 80x40: 138 ms with 1024-node items, more
+// with shorter or longer ones)
+constexpr int kMixedItems = 2432;
+inline int plain_chunk(long long npts, long long nq3, int most = kPlainChunk, int items = kPlainItems)
 {
     int c = most;
-    while (c > 128 && npts * ((nq3 + c - 1) / c) < kPlainItems) c = c / 2 < 128 ? 128 : c / 2;
+    while (c > 128 && npts * ((nq3 + c - 1) / c) < items) c = c / 2 < 128 ? 128 : c / 2;
     return c;
 }
 // per-thread stack the kernels need: the QAGS interval list (kQagsCap entries
@@ -184,7 +188,7 @@ struct ItemQueue {
 };
 struct MixedSmem { size_t turn, integrate; };  // dynamic shared memory of the two kernels
 cudaError_t launch_moments_batch(const MomentArgs &a0, const MomentBatch &b, int nblocks, size_t smem,
-                                 const MixedSmem &msm, bool mixed, int variant, const DeferWork &dw, const ItemQueue &q, const PlainWork &w,
+                                 const MixedSmem &msm, bool mixed, int variant, int np, const DeferWork &dw, const ItemQueue &q, const PlainWork &w,
                                  cudaStream_t s);
 cudaError_t launch_moments_finalize_batch(const MomentBatch &b, int npoints, cudaStream_t s);
 // dst6[q][idx[t]] = src6[q][t] (moments of n points into a grid of npts)
@@ -218,7 +222,7 @@ constexpr int kMixedVariants = 8;    // builds of the mixed kernel (2 forms x 4 
 MixedSmem mixed_smem(const MomentArgs &a);
 size_t mixed_rec_bytes();      // per node of a slice
 size_t mixed_scratch_bytes();  // per block of the integration kernel
-void mixed_resident(int variant, const MixedSmem &sm, int &turn, int &integrate);  // blocks resident at once
+void mixed_resident(int variant, int np, const MixedSmem &sm, int &turn, int &integrate);  // blocks resident at once
 // nodes whose records a workspace holds: 2.2 GB of records at most per context
 constexpr long long kMixedSliceNodes = 20ll << 20;
 int mixed_blocks_per_point(long long nq3, int chunk);

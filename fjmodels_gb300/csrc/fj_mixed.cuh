@@ -271,42 +271,40 @@ FJ_HDNI void pot_grad_f(const PotViewF &P, float R, float z, float &phi, float &
 //   d_k = C_k ((x - B_k) d_k-1 + (x - y) P_k-1(y) - A_k d_k-2),  x = c^2, y = c2pt,
 // so it keeps its relative precision however close the position is to the
 // point; otherwise it is the direct interpolation (or the r >= ar[nr-1]
-// extrapolation) minus Phipt, the FP32 potential at the point.  All three
-// run in the same loop over the multipoles, each l's term being
-//   vb a_l + (vt - vb) b_l + (v_thr - vb - f3 (vt - vb)) g_l
-// with per-position coefficients selected without branches, so the lanes of
-// a warp do not split between them.  P_k(y) is the point's table P.pyl.
+// extrapolation) minus Phipt, the FP32 potential at the point.  P_k(y) is the
+// point's table P.pyl.
 struct DState {
     int mode;  // 0: difference, 1: direct, 2: extrapolated
     int b, thr;
     bool quad;
-    float f1, f2, f3, f1p, f2p, df1, df2, x, dc2, xe2, xp1, sum0, phipt;
+    float f3, f1p, f2p, df1, df2, x, dc2, xe2, xp1, sum0;
 };
 
 // The arithmetic is written in explicit products, sums and FMAs: the values
 // are the same in the turning-point searches (out of line) and in the momentum
 // integrals (inlined), on any path through the optimiser.
-FJ_HD void dphi_setup(const PotViewF &P, float R, float z, float rpt, float dr2, float dc2, float Phipt, DState &s)
+FJ_HD void dphi_setup(const PotViewF &P, float R, float z, float rpt, float dr2, float dc2, DState &s)
 {
     const float r = sqrtf(fma_rn(R, R, mul_rn(z, z)));
     const float *ar = P.ar;
     const int nr = P.nr;
     const float a0 = ar[0], rmax = ar[nr - 1];
-    s.b = nr - 2; s.thr = 0; s.quad = false;
-    s.f1 = s.f2 = s.f3 = s.f1p = s.f2p = s.df1 = s.df2 = 0.f;
-    s.xe2 = 1.f; s.xp1 = 1.f; s.sum0 = 0.f;
-    s.phipt = Phipt; s.dc2 = dc2;
+    s.dc2 = dc2;
     if (r >= rmax) {  // phi_l = phil[nr-1][l] (rmax/r)^(2l+1); the monopole from the unshifted table value
         s.mode = 2;
+        s.b = nr - 2; s.thr = 0; s.quad = false;
+        s.f3 = s.f1p = s.f2p = s.df1 = s.df2 = 0.f;
         const float xe = rmax / r;
         s.xe2 = mul_rn(xe, xe);
         s.xp1 = mul_rn(xe, s.xe2);
         s.sum0 = fma_rn(P.out0, xe, -P.shift);
     } else {
+        s.xe2 = s.xp1 = 1.f; s.sum0 = 0.f;
         const float re = fmaxf(r, a0), rpe = fmaxf(rpt, a0);
         InterpF I;
         interp_setup_f(P, re, I);
-        s.b = I.bot; s.thr = I.thr; s.quad = I.quad; s.f1 = I.f1; s.f2 = I.f2; s.f3 = I.f3;
+        s.b = I.bot; s.thr = I.thr; s.quad = I.quad; s.f3 = I.f3;
+        s.df1 = I.f1; s.df2 = I.f2; s.f1p = s.f2p = 0.f;
         const float ab = ar[s.b], at = ar[s.b + 1];
         s.mode = 1;
         if (rpt < rmax && rpe >= ab && rpe <= at) {
@@ -325,66 +323,98 @@ FJ_HD void dphi_setup(const PotViewF &P, float R, float z, float rpt, float dr2,
     s.x = s.mode == 0 ? add_rn(P.c2pt, dc2) : mul_rn(z, z) / mul_rn(r, r);
 }
 
-// the term of multipole k: px = P_k(x), dk = P_k(x) - P_k(y), xp the
-// extrapolation factor (1 in the other modes)
-FJ_HD void dphi_acc(const PotViewF &P, const DState &s, float &sum, int k, float px, float dk, float xp)
+// table values of multipole k at the position's interval: phil[b], phil[b+1] -
+// phil[b] and (QUAD) phil[thr] - phil[b] - f3 (phil[b+1] - phil[b])
+template <bool QUAD>
+FJ_HD void dphi_row(const PotViewF &P, const DState &s, int k, float &vb, float &d, float &e)
 {
     const int np_ = P.npoly;
 #ifdef __CUDA_ARCH__
     const float2 vd = *(const float2 *)(P.pd + 2 * (s.b * np_ + k));
-    const float vb = vd.x, d = vd.y;
-    const float e = s.quad ? P.pe[(2 * s.b + (s.thr > s.b ? 1 : 0)) * np_ + k] : 0.f;
+    vb = vd.x; d = vd.y;
+    e = QUAD ? P.pe[(2 * s.b + (s.thr > s.b ? 1 : 0)) * np_ + k] : 0.f;
 #else
     const float *T = P.phil;
-    const float vb = T[s.b * np_ + k], d = T[(s.b + 1) * np_ + k] - vb;
-    const float e = s.quad ? T[s.thr * np_ + k] - vb - s.f3 * d : 0.f;
+    vb = T[s.b * np_ + k]; d = T[(s.b + 1) * np_ + k] - vb;
+    e = QUAD ? T[s.thr * np_ + k] - vb - s.f3 * d : 0.f;
 #endif
-    const float t = mul_rn(xp, px);
-    const bool m0 = s.mode == 0, m1 = s.mode == 1;
-    const float ca = m0 ? dk : t;
-    const float cb = m0 ? (k == 1 ? fma_rn(s.f1p, dk, mul_rn(s.df1, px)) : fma_rn(s.df1, px, mul_rn(s.f1p, dk)))
-                        : (m1 ? mul_rn(s.f1, px) : t);
-    const float cg = m0 ? fma_rn(s.df2, px, mul_rn(s.f2p, dk)) : mul_rn(s.f2, px);
-    sum = add_rn(sum, fma_rn(e, cg, fma_rn(vb, ca, mul_rn(d, cb))));
 }
 
-FJ_HD float dphi_end(const DState &s, float sum) { return s.mode == 0 ? sum : add_rn(sum, -s.phipt); }
-
-// one multipole chain: Legendre recurrences of x and of the difference
-struct DChain {
-    float px1, px2, d1, d2, xp, sum;
-    FJ_HD void begin(const PotViewF &P, const DState &s)
+// The sum over the multipoles of
+//   vb a_l + (vt - vb) b_l + (v_thr - vb - f3 (vt - vb)) g_l,
+// with a_l = d_l (difference) or P_l(x) (direct) and b_l = df1 P_l(x) + f1p d_l,
+// g_l = df2 P_l(x) + f2p d_l (direct: df = f and fp = 0, so b_l = f1 P_l(x)),
+// together with the Legendre recurrences of x and of the difference.  Without
+// the quadratic correction (all but the ten innermost radii) g_l drops out; that
+// and the direct form's share of the coefficients take the loop from 30 to 16
+// instructions per multipole.  NP > 0: npoly known where this is compiled.
+template <int NP, bool QUAD>
+FJ_HD float dphi_chain(const PotViewF &P, const DState &s)
+{
+    const LegCoefF &L = leg_f();
+    const int np_ = NP > 0 ? NP : P.npoly;
+    const bool m0 = s.mode == 0;
+    float vb, d, e;
+    dphi_row<QUAD>(P, s, 0, vb, d, e);
+    float sum = fma_rn(vb, m0 ? 0.f : 1.f, mul_rn(d, s.df1));
+    if (QUAD) sum = fma_rn(e, s.df2, sum);
+    if (np_ < 2) return sum;
+    float px1 = fma_rn(1.5f, s.x, -.5f), px2 = 1.f, d1 = mul_rn(1.5f, s.dc2), d2 = 0.f;
     {
-        sum = s.sum0;
-        dphi_acc(P, s, sum, 0, 1.f, 0.f, s.mode == 2 ? 0.f : 1.f);  // the extrapolated monopole is in sum0
-        px2 = 1.f; d2 = 0.f;
-        if (P.npoly > 1) {
-            px1 = fma_rn(1.5f, s.x, -.5f);
-            d1 = mul_rn(1.5f, s.dc2);
-            dphi_acc(P, s, sum, 1, px1, d1, s.xp1);
-        }
-        xp = mul_rn(s.xp1, s.xe2);
+        dphi_row<QUAD>(P, s, 1, vb, d, e);
+        float t = fma_rn(vb, m0 ? d1 : px1, mul_rn(d, fma_rn(s.f1p, d1, mul_rn(s.df1, px1))));
+        if (QUAD) t = fma_rn(e, fma_rn(s.df2, px1, mul_rn(s.f2p, d1)), t);
+        sum = add_rn(sum, t);
     }
-    FJ_HD void step(const PotViewF &P, const LegCoefF &L, const DState &s, int k)
-    {
+    auto step = [&](int k) {
         const float xb = add_rn(s.x, -L.B[k]), A = L.A[k], C = L.C[k];
         const float px = mul_rn(fma_rn(xb, px1, -mul_rn(A, px2)), C);
         const float dk = mul_rn(fma_rn(-A, d2, fma_rn(xb, d1, mul_rn(s.dc2, P.pyl[k - 1]))), C);
-        dphi_acc(P, s, sum, k, px, dk, xp);
-        xp = mul_rn(xp, s.xe2);
+        dphi_row<QUAD>(P, s, k, vb, d, e);
+        float t = fma_rn(vb, m0 ? dk : px, mul_rn(d, fma_rn(s.df1, px, mul_rn(s.f1p, dk))));
+        if (QUAD) t = fma_rn(e, fma_rn(s.df2, px, mul_rn(s.f2p, dk)), t);
+        sum = add_rn(sum, t);
         px2 = px1; px1 = px; d2 = d1; d1 = dk;
+    };
+    if (NP > 0) {
+FJ_UNROLL
+        for (int k = 2; k < NP; k++) step(k);
+    } else {
+FJ_UNROLL1
+        for (int k = 2; k < np_; k++) step(k);
     }
-};
+    return sum;
+}
 
+// beyond the grid: sum0 + sum_l>0 xp_l P_l(x) phil[nr-1][l], xp_l = (rmax/r)^(2l+1)
+FJ_HD float dphi_outside(const PotViewF &P, const DState &s)
+{
+    const LegCoefF &L = leg_f();
+    float sum = s.sum0, px1 = fma_rn(1.5f, s.x, -.5f), px2 = 1.f, xp = s.xp1;
+FJ_UNROLL1
+    for (int k = 1; k < P.npoly; k++) {
+        float px = px1;
+        if (k > 1) {
+            px = mul_rn(fma_rn(add_rn(s.x, -L.B[k]), px1, -mul_rn(L.A[k], px2)), L.C[k]);
+            px2 = px1; px1 = px;
+        }
+        float vb, d, e;
+        dphi_row<false>(P, s, k, vb, d, e);
+        const float t = mul_rn(xp, px);
+        sum = add_rn(sum, fma_rn(vb, t, mul_rn(d, t)));
+        xp = mul_rn(xp, s.xe2);
+    }
+    return sum;
+}
+
+template <int NP = 0>
 FJ_HD float pot_dphi_f(const PotViewF &P, float R, float z, float rpt, float dr2, float dc2, float Phipt)
 {
     DState s;
-    dphi_setup(P, R, z, rpt, dr2, dc2, Phipt, s);
-    DChain c;
-    c.begin(P, s);
-    const LegCoefF &L = leg_f();
-    for (int k = 2; k < P.npoly; k++) c.step(P, L, s, k);
-    return dphi_end(s, c.sum);
+    dphi_setup(P, R, z, rpt, dr2, dc2, s);
+    if (s.mode == 2) return add_rn(dphi_outside(P, s), -Phipt);
+    const float sum = s.quad ? dphi_chain<0, true>(P, s) : dphi_chain<NP, false>(P, s);
+    return s.mode == 0 ? sum : add_rn(sum, -Phipt);
 }
 
 // Brent root (wrp_GSLroots rule, include/Utils.h:134-167) in FP32; the
@@ -1014,7 +1044,7 @@ FJ_HD void point_legendre_f(float y, int npoly, float *pyl)
 
 // FP32 tables of one grid point (R, z): radii, potential multipoles shifted by
 // Phi_h, interval reciprocals, quadratic-correction constants and P_2k(c2pt)
-// (fPr may be null: the momentum integrals need no radial derivative); threads i0, i0 + stride, ... share the work
+// (fphil and fPr may be null: the momentum integrals read evaluator_tables_f's); threads i0, i0 + stride, ... share the work
 FJ_HD void mixed_tables_f(int nr, int npoly, const double *ar, const double *phil, const double *Pr, double Phi_h,
                           double R, double z, float *far, float *fphil, float *fPr, float *ih, float *qc, float *pyl,
                           int i0, int stride)
@@ -1029,7 +1059,7 @@ FJ_HD void mixed_tables_f(int nr, int npoly, const double *ar, const double *phi
         qc[i] = (float)v;
     }
     for (int i = i0; i < nr * npoly; i += stride) {
-        fphil[i] = (float)(i % npoly == 0 ? phil[i] - Phi_h : phil[i]);
+        if (fphil) fphil[i] = (float)(i % npoly == 0 ? phil[i] - Phi_h : phil[i]);
         if (fPr) fPr[i] = (float)Pr[i];
     }
     if (i0 == 0) point_legendre_f(point_c2_f(R, z), npoly, pyl);
@@ -1052,22 +1082,25 @@ FJ_HD PotViewF mixed_view_f(int nr, int npoly, const double *ar, const double *p
     return v;
 }
 
-// The kernels' evaluator tables of PotViewF (pd, pe) from its FP32 tables, which
-// must be complete; threads i0, i0 + stride, ... share the work
-FJ_HD void evaluator_tables_f(const PotViewF &P, float *pd, float *pe, int i0, int stride)
+// The kernels' evaluator tables of PotViewF (pd, pe) from the FP64 potential
+// multipoles and P's other FP32 tables, which must be complete; threads i0, i0 +
+// stride, ... share the work
+FJ_HD void evaluator_tables_f(const PotViewF &P, const double *phil, double Phi_h, float *pd, float *pe, int i0,
+                              int stride)
 {
     const int nr = P.nr, np_ = P.npoly;
-    const float *T = P.phil;
+    auto T = [&](int i) { return (float)(i % np_ == 0 ? phil[i] - Phi_h : phil[i]); };  // as mixed_tables_f
     for (int i = i0; i < nr * np_; i += stride) {
-        pd[2 * i] = T[i];
-        pd[2 * i + 1] = i < (nr - 1) * np_ ? add_rn(T[i + np_], -T[i]) : 0.f;
+        const float v = T(i);
+        pd[2 * i] = v;
+        pd[2 * i + 1] = i < (nr - 1) * np_ ? add_rn(T(i + np_), -v) : 0.f;
     }
     for (int i = i0; i < 2 * kQuadIntervals * np_; i += stride) {
         const int n = i / (2 * np_), up = (i / np_) & 1, k = i % np_, thr = up ? n + 2 : n - 1;
         float e = 0.f;
         if (thr >= 0 && thr < nr && n + 1 < nr) {
-            const float vb = T[n * np_ + k], d = add_rn(T[(n + 1) * np_ + k], -vb);
-            e = fma_rn(-P.qc[4 * n + (up ? 3 : 1)], d, add_rn(T[thr * np_ + k], -vb));
+            const float vb = T(n * np_ + k), d = add_rn(T((n + 1) * np_ + k), -vb);
+            e = fma_rn(-P.qc[4 * n + (up ? 3 : 1)], d, add_rn(T(thr * np_ + k), -vb));
         }
         pe[i] = e;
     }

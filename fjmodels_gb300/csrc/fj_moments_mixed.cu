@@ -25,7 +25,7 @@ namespace fj {
 //                      finds their turning points, one node per thread: the FP64
 //                      setup, bracket walks and Brent; a node's constants go to a
 //                      record in device memory;
-//   k_mixed_integrate  kMixedLanes lanes per momentum integral: the first panel of
+//   k_mixed_integrate  kMixedLanes (2) lanes per momentum integral: the first panel of
 //                      every Ju and Jv of the item, then the bisections of those
 //                      that go on, groups taking the next integral as they finish
 //                      (fj_group_qags.cuh); then the DFs and the moment sums.
@@ -37,18 +37,25 @@ namespace fj {
 // the instruction caches (4.8 stall cycles per issue waiting for instructions).
 // Measured (GB300, 80x40 grid, 22^3 nodes): 270 ms with the fastest of the earlier
 // one-kernel builds, 361-371 ms with its initial configuration; 284 ms with the
-// phases in one kernel; 171 ms in two, of which the turning points take 40 %.
-// On a 240-point spread of that grid the warp instructions fall from 14.8 G (19.3
-// lanes active) to 3.9 G (17.2) + 7.2 G (25.7), issue slots busy 60 % and 71 %.
-// The integration is built in four register budgets (launch bounds of 3, 4, 6 and
-// 8 resident blocks per SM: 168, 128, 80 and 64 registers), and the turning points
-// in two: kMixedVariants configurations, all with the same bits.  Which one, and
-// the item size, is a per-context setting (fj_autotune_mixed).
+// phases in one kernel; 171 ms in two with four lanes per integral and the
+// multipole loop as it was, 158 ms with it unrolled for the launch's npoly, 144 ms
+// with the terms an evaluation does not need left out (dphi_chain), 138 ms with
+// two lanes per integral (eight: 237 ms; the list upkeep of an integral is serial,
+// so more integrals per warp share it; 24x8 and 33x11 models run 2 % slower with
+// two than with four).  On a 240-point spread of that grid the warp instructions
+// fall from 14.8 G (19.3 lanes active) to 3.4 G (17.3) + 4.9 G (25.1).  Interval
+// lists kept in shared memory instead of behind L1 were slower (144 -> 162 ms at
+// 64 registers: every access selects between the two places).
+// The integration is built in four register budgets (launch bounds of 4, 5, 6 and
+// 8 resident blocks per SM: 128, 96, 80 and 64 registers) and for npoly 3 to 8, the
+// turning points in two budgets (4 and 8 blocks): kMixedVariants configurations,
+// all with the same bits.  Which one, and the item size, is a per-context setting
+// (fj_autotune_mixed).
 // Shared memory holds only what the node solves read: the FP32 tables, the
 // radii, the focal-distance table, the velocity rule and the node list.  The
 // FP64 potential tables are read from global memory (the point setup, the
 // FP32 table build and the rare FP64 turning-point path).
-constexpr int kMixedLanes = 4;                            // lanes per momentum integral
+constexpr int kMixedLanes = 2;                            // lanes per momentum integral
 constexpr int kMixedGroups = kMixedBlock / kMixedLanes;   // integrals in flight per block
 using MixedQags = GroupQags<float, kQagsCapF>;
 
@@ -78,7 +85,7 @@ __host__ __device__ static int mixed_list_cap(int chunk)
 __host__ __device__ static size_t mixed_table_floats(int nr, int npoly, bool grad)
 {
     const size_t nt = (size_t)nr * npoly;
-    return 2 * (size_t)nr + (grad ? 4 : 3) * nt + (2 * nt & 1) + 4 * kQuadIntervals + npoly + 2 * kQuadIntervals * npoly + 1;
+    return 2 * (size_t)nr + (grad ? 4 : 2) * nt + 4 * kQuadIntervals + npoly + 2 * kQuadIntervals * npoly;
 }
 
 struct MixedTables {
@@ -89,7 +96,7 @@ struct MixedTables {
         const int nt = nr * npoly;
         pd = f; f += 2 * nt;
         ar = f; f += nr;
-        phil = f; f += nt;
+        phil = grad ? f : nullptr; if (grad) f += nt;
         Pr = grad ? f : nullptr; if (grad) f += nt;
         ih = f; f += nr;
         qc = f; f += 4 * kQuadIntervals;
@@ -104,7 +111,7 @@ struct MixedTables {
                        blockDim.x);
         PotViewF v = mixed_view_f(nr, npoly, a.P.ar, a.P.phil, Phi_h, R, z, ar, phil, Pr, ih, qc, pyl);
         __syncthreads();
-        evaluator_tables_f(v, pd, pe, threadIdx.x, blockDim.x);
+        evaluator_tables_f(v, a.P.phil, Phi_h, pd, pe, threadIdx.x, blockDim.x);
         __syncthreads();
         v.pd = pd;
         v.pe = pe;
@@ -123,6 +130,7 @@ static size_t mixed_turn_smem(const MomentArgs &a)
 // A block's shared memory of the integrals
 struct MixedShared {
     float vals[kMixedGroups][43];  // panel values
+    float xk[21];                  // panel abscissas in evaluation order: center + half xk (gk21_abscissa)
     GK21f K;
     int next;
 };
@@ -267,9 +275,11 @@ __global__ void __launch_bounds__(kMixedBlock, MINB) k_mixed_turn(MomentArgs a0,
 }
 
 // The momentum integrals of an item's n nodes, kMixedLanes lanes to one
-__device__ __forceinline__ void mixed_integrals(const PotViewF &PF, int n, MixedRec *rec, MixedQags::List &L,
+template <int NP>
+__device__ __forceinline__ void mixed_integrals(PotViewF PF, int n, MixedRec *rec, MixedQags::List &L,
                                                 unsigned char *state, MixedShared &sh)
 {
+    if (NP > 0) PF.npoly = NP;
     const int lane = threadIdx.x & 31, g = threadIdx.x / kMixedLanes, gi = threadIdx.x % kMixedLanes;
     const int lead = lane & ~(kMixedLanes - 1);
     const float epsabs = 1e-5f, epsrel = 1e-3f;
@@ -316,23 +326,28 @@ __device__ __forceinline__ void mixed_integrals(const PotViewF &PF, int n, Mixed
                 o.sv2 = r.sv2; o.swp = r.swp; o.svp = r.svp; o.sinv = r.sinv; o.cosv = r.cosv; o.sinhu = r.sinhu;
                 o.coshu = r.coshu; o.pvterm = r.pvterm; o.rpt = r.rpt; o.Phipt = r.Phipt; o.u_f = r.u_f; o.tb = r.tb;
                 o.Dt = r.Dt; o.wt = r.wt;
+                // the panels' centres and half-lengths, as gk21_abscissa forms them
+                const float hi = pass == 0 ? b2 : b1;
+                const float ce1 = mul_rn(0.5f, add_rn(a1, hi)), ha1 = mul_rn(0.5f, add_rn(hi, -a1)),
+                            ce2 = mul_rn(0.5f, add_rn(b1, b2)), ha2 = mul_rn(0.5f, add_rn(b2, -b1));
                 const int npts = pass == 0 ? 21 : 42;
                 for (int e = gi; e < npts; e += kMixedLanes) {
                     const bool second = e >= 21;
-                    const float x = gk21_abscissa(K, second ? b1 : a1, pass == 0 || second ? b2 : b1, second ? e - 21 : e);
+                    const float x = add_rn(second ? ce2 : ce1, mul_rn(second ? ha2 : ha1, sh.xk[second ? e - 21 : e]));
                     FGeo G;
                     const int mode = kv ? kEvJv : kEvJu;
                     fudge_geom(o, mode, x, G);
-                    vals[e] = fudge_finish(mode, G, pot_dphi_f(PF, G.R, G.z, o.rpt, G.dr2, G.dc2, o.Phipt));
+                    vals[e] = fudge_finish(mode, G, pot_dphi_f<NP>(PF, G.R, G.z, o.rpt, G.dr2, G.dc2, o.Phipt));
                 }
             }
             __syncwarp();
-            // the panels' sums on the group's first and third lanes
+            // the panels' sums on two of the group's lanes
             float res = 0.f, err = 0.f, ra = 0.f, rc = 0.f;
-            if (on && (gi == 0 || (gi == 2 && pass == 1)))
+            if (on && (gi == 0 || (gi == kMixedLanes / 2 && pass == 1)))
                 gk21_sum(K, gi ? b1 : a1, pass == 0 || gi ? b2 : b1, vals + (gi ? 21 : 0), res, err, ra, rc);
-            const float res2 = __shfl_sync(0xffffffffu, res, lead + 2), err2 = __shfl_sync(0xffffffffu, err, lead + 2),
-                        rc2 = __shfl_sync(0xffffffffu, rc, lead + 2);
+            const int lane2 = lead + kMixedLanes / 2;
+            const float res2 = __shfl_sync(0xffffffffu, res, lane2), err2 = __shfl_sync(0xffffffffu, err, lane2),
+                        rc2 = __shfl_sync(0xffffffffu, rc, lane2);
             if (on && gi == 0) {
                 bool done, full = false;
                 float r = res;
@@ -359,7 +374,7 @@ __device__ __forceinline__ void mixed_integrals(const PotViewF &PF, int n, Mixed
     }
 }
 
-template <int MINB>
+template <int MINB, int NP>
 __global__ void __launch_bounds__(kMixedBlock, MINB) k_mixed_integrate(MomentArgs a0, MomentBatch batch, ItemQueue q)
 {
     extern __shared__ double sm[];
@@ -378,7 +393,8 @@ __global__ void __launch_bounds__(kMixedBlock, MINB) k_mixed_integrate(MomentArg
         const int nr = a.P.nr, npoly = a.P.npoly;
         double *s_xq = sm, *s_wq = s_xq + a.nq, *s_red = s_wq + a.nq;
         MixedTables tab;
-        MixedShared &sh = *(MixedShared *)tab.carve((float *)(s_red + 6 * (kMixedBlock / 32)), nr, npoly, false);
+        MixedShared &sh = *(MixedShared *)(((uintptr_t)tab.carve((float *)(s_red + 6 * (kMixedBlock / 32)), nr, npoly, false) +
+                                            15) & ~(uintptr_t)15);
         unsigned *s_bits = (unsigned *)(&sh + 1);  // nodes left to the FP64 pass
         const int nw = defer_words(a.mixed_chunk);
         unsigned char *state = (unsigned char *)(s_bits + nw);
@@ -398,8 +414,13 @@ __global__ void __launch_bounds__(kMixedBlock, MINB) k_mixed_integrate(MomentArg
             sh.K.wgk[threadIdx.x] = (float)fj_wgk21_d[threadIdx.x];
             if (threadIdx.x < 5) sh.K.wg[threadIdx.x] = (float)fj_wg10_d[threadIdx.x];
         }
+        if (threadIdx.x < 21) {
+            const int e = threadIdx.x, jj = e <= 10 ? 2 * ((e - 1) >> 1) + 1 : 2 * ((e - 11) >> 1);
+            const float x = e ? (float)fj_xgk21_d[jj] : 0.f;
+            sh.xk[e] = ((e - 1) & 1) ? x : -x;
+        }
         const PotViewF PF = tab.build(a, Phi_h, R, z);
-        mixed_integrals(PF, n, rec, L, state, sh);
+        mixed_integrals<NP>(PF, n, rec, L, state, sh);
         __syncthreads();
         // The DFs and the moments: thread t sums nodes t, t + 128, .. of the sorted
         // list.  A node whose FP32 solve hit a cap (a full QAGS list, a bracket walk
@@ -729,13 +750,28 @@ const void *turn_kernel(int variant)
     return variant < 4 ? (const void *)k_mixed_turn<4> : (const void *)k_mixed_turn<8>;
 }
 
-const void *integrate_kernel(int variant)
+template <int MINB>
+const void *integrate_kernel_np(int np)
+{
+    switch (np) {
+    case 3: return (const void *)k_mixed_integrate<MINB, 3>;
+    case 4: return (const void *)k_mixed_integrate<MINB, 4>;
+    case 5: return (const void *)k_mixed_integrate<MINB, 5>;
+    case 6: return (const void *)k_mixed_integrate<MINB, 6>;
+    case 7: return (const void *)k_mixed_integrate<MINB, 7>;
+    case 8: return (const void *)k_mixed_integrate<MINB, 8>;
+    default: return (const void *)k_mixed_integrate<MINB, 0>;
+    }
+}
+
+// np: the launch's multipoles per model (0: they differ)
+const void *integrate_kernel(int variant, int np)
 {
     switch (variant & 3) {
-    case 0: return (const void *)k_mixed_integrate<3>;
-    case 1: return (const void *)k_mixed_integrate<4>;
-    case 2: return (const void *)k_mixed_integrate<6>;
-    default: return (const void *)k_mixed_integrate<8>;
+    case 0: return integrate_kernel_np<4>(np);
+    case 1: return integrate_kernel_np<5>(np);
+    case 2: return integrate_kernel_np<6>(np);
+    default: return integrate_kernel_np<8>(np);
     }
 }
 
@@ -753,7 +789,7 @@ int resident(const void *k, size_t smem)
 
 // the launch's items, a slice of q.per_slice at a time through both kernels
 cudaError_t launch_mixed_any(const MomentArgs &a, const MomentBatch &b, const ItemQueue &q0, size_t smem_t,
-                             size_t smem_i, int variant, cudaStream_t s)
+                             size_t smem_i, int variant, int np, cudaStream_t s)
 {
     if (variant < 0 || variant >= kMixedVariants || q0.grid < 1 || q0.grid_turn < 1) return cudaErrorInvalidValue;
     for (int first = 0; first < q0.total; first += q0.per_slice) {
@@ -766,7 +802,7 @@ cudaError_t launch_mixed_any(const MomentArgs &a, const MomentBatch &b, const It
         const unsigned gt = (unsigned)(q.count < q.grid_turn ? q.count : q.grid_turn),
                        gi = (unsigned)(q.count < q.grid ? q.count : q.grid);
         if ((e = cudaLaunchKernel(turn_kernel(variant), dim3(gt), dim3(kMixedBlock), args, smem_t, s)) != cudaSuccess ||
-            (e = cudaLaunchKernel(integrate_kernel(variant), dim3(gi), dim3(kMixedBlock), args, smem_i, s)) !=
+            (e = cudaLaunchKernel(integrate_kernel(variant, np), dim3(gi), dim3(kMixedBlock), args, smem_i, s)) !=
                 cudaSuccess)
             return e;
     }
@@ -774,10 +810,10 @@ cudaError_t launch_mixed_any(const MomentArgs &a, const MomentBatch &b, const It
 }
 }  // namespace
 
-void mixed_resident(int variant, const MixedSmem &sm, int &turn, int &integrate)
+void mixed_resident(int variant, int np, const MixedSmem &sm, int &turn, int &integrate)
 {
     turn = resident(turn_kernel(variant), sm.turn);
-    integrate = resident(integrate_kernel(variant), sm.integrate);
+    integrate = resident(integrate_kernel(variant, np), sm.integrate);
 }
 
 MixedSmem mixed_smem(const MomentArgs &a) { return MixedSmem{mixed_turn_smem(a), mixed_integrate_smem(a)}; }
@@ -790,7 +826,7 @@ cudaError_t launch_moments_mixed(const MomentArgs &a, int variant, const DeferWo
     const long long nblocks = (long long)a.npts * a.blocks_per_point;
     if (q.total != nblocks) return cudaErrorInvalidValue;
     const MixedSmem sm = mixed_smem(a);
-    cudaError_t e = launch_mixed_any(a, none, q, sm.turn, sm.integrate, variant, s);
+    cudaError_t e = launch_mixed_any(a, none, q, sm.turn, sm.integrate, variant, a.P.npoly, s);
     if (e == cudaSuccess) e = launch_deferred(a, none, nblocks, dw, s);
     if (e != cudaSuccess) return e;
     return launch_moments_finalize(a, s);
@@ -800,12 +836,12 @@ cudaError_t launch_moments_plain_batch(const MomentArgs &a0, const MomentBatch &
                                       cudaStream_t s);
 
 cudaError_t launch_moments_batch(const MomentArgs &a0, const MomentBatch &b, int nblocks, size_t smem,
-                                 const MixedSmem &msm, bool mixed, int variant, const DeferWork &dw, const ItemQueue &q, const PlainWork &w,
+                                 const MixedSmem &msm, bool mixed, int variant, int np, const DeferWork &dw, const ItemQueue &q, const PlainWork &w,
                                  cudaStream_t s)
 {
     if (!mixed) return launch_moments_plain_batch(a0, b, smem, w, s);
     if (q.total != nblocks) return cudaErrorInvalidValue;
-    const cudaError_t e = launch_mixed_any(a0, b, q, msm.turn, msm.integrate, variant, s);
+    const cudaError_t e = launch_mixed_any(a0, b, q, msm.turn, msm.integrate, variant, np, s);
     return e == cudaSuccess ? launch_deferred(a0, b, nblocks, dw, s) : e;
 }
 
@@ -814,7 +850,7 @@ size_t moments_mixed_local_bytes()
     size_t m = 0;
     cudaFuncAttributes at;
     for (int v = 0; v < kMixedVariants; v++)
-        for (const void *k : {turn_kernel(v), integrate_kernel(v)})
+        for (const void *k : {turn_kernel(v), integrate_kernel(v, 0), integrate_kernel(v, 7)})
             if (cudaFuncGetAttributes(&at, k) == cudaSuccess && at.localSizeBytes > m) m = at.localSizeBytes;
     for (const void *k : {(const void *)k_defer_solve, (const void *)k_defer_add})
         if (cudaFuncGetAttributes(&at, k) == cudaSuccess && at.localSizeBytes > m) m = at.localSizeBytes;

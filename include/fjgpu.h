@@ -239,7 +239,7 @@ int fj_surrogate_moments(fj_surrogate *s, const fj_potential *pot, const fj_df_p
    counterpart: the reference has one CPU loop).  variant 0..7: 0..3 give
    the turning points the larger register budget (4 resident blocks per SM),
    4..7 the smaller (8); within each, the register budget of the momentum
-   integrals (launch bounds of 3, 4, 6, 8 resident blocks per SM),
+   integrals (launch bounds of 4, 5, 6, 8 resident blocks per SM),
    nodes_per_block = most velocity nodes of one point per work item
    (128..8192; a model too small to fill the GPU with such items is split
    further).  Initially 7 and 1024.

@@ -446,24 +446,52 @@ FJ_HDNI void pot_freqs(const PotView &P, double R, double &kappa, double &nu, do
 // ----------------------------------------------------------------------------
 FJ_HD bool same_sign(double x, double y) { return (x < 0 && y < 0) || (x > 0 && y > 0); }
 
-template <class F>
-FJ_HDNI unsigned brent_root(F &f, double lo, double hi, double &root)
-{
-    const double flo = f(lo);
-    if (fabs(flo) < 5e-4) { root = lo; return 0; }
-    const double fhi = f(hi);
-    if (fabs(fhi) < 5e-4) { root = hi; return 0; }
-    double a = lo, fa = flo, b = hi, fb = fhi, c = hi, fc = fhi, d = hi - lo, e = hi - lo;
-    double xr = 0.5 * (lo + hi), xlo = lo, xhi = hi;
-    for (int it = 0; it < kRootMaxIt; it++) {
-        bool secant = false;
-        if (same_sign(fb, fc)) { secant = true; c = a; fc = fa; d = b - a; e = b - a; }
-        if (fabs(fc) < fabs(fb)) { secant = true; a = b; b = c; c = a; fa = fb; fb = fc; fc = fa; }
-        const double tol = 0.5 * DBL_EPSILON * fabs(b);
-        const double m = 0.5 * (c - b);
-        if (fb == 0) { xr = b; xlo = b; xhi = b; }
-        else if (fabs(m) <= tol) { xr = b; xlo = b < c ? b : c; xhi = b < c ? c : b; }
-        else {
+// The iteration of brent_root as a state that is fed one function value at a time:
+// x is the next abscissa, feed(f(x)) returns true when root (and fail) are final.
+struct BrentState {
+    double a, fa, b, fb, c, fc, d, e, x, root;
+    int it;  // -2: f(lo) awaited, -1: f(hi), >= 0: iterations done
+    unsigned fail;
+    FJ_HD void begin(double lo, double hi)
+    {
+        a = x = lo; b = hi; it = -2; fail = 0;
+        fa = fb = c = fc = d = e = root = 0;
+    }
+    FJ_HD bool feed(double f)
+    {
+        if (it == -2) {
+            if (fabs(f) < 5e-4) { root = a; return true; }
+            fa = f; x = b; it = -1;
+            return false;
+        }
+        if (it == -1) {
+            if (fabs(f) < 5e-4) { root = b; return true; }
+            fb = f; c = b; fc = f; d = b - a; e = d;
+            it = 0;
+        } else {
+            fb = f;
+            const double cc = same_sign(fb, fc) ? a : c;
+            const double xlo = b < cc ? b : cc, xhi = b < cc ? cc : b;
+            const double alo = fabs(xlo), ahi = fabs(xhi);
+            const double mn = ((xlo > 0 && xhi > 0) || (xlo < 0 && xhi < 0)) ? (alo < ahi ? alo : ahi) : 0.0;
+            if (fabs(xhi - xlo) < 1e-8 + 1e-6 * mn && !(xhi - xlo > 1e-8)) { root = b; return true; }
+            it++;
+        }
+        for (;;) {
+            if (it >= kRootMaxIt) { root = b; fail = kFailRoot; return true; }
+            bool secant = false;
+            if (same_sign(fb, fc)) { secant = true; c = a; fc = fa; d = b - a; e = b - a; }
+            if (fabs(fc) < fabs(fb)) { secant = true; a = b; b = c; c = a; fa = fb; fb = fc; fc = fa; }
+            const double tol = 0.5 * DBL_EPSILON * fabs(b);
+            const double m = 0.5 * (c - b);
+            if (fb == 0) { root = b; return true; }
+            if (fabs(m) <= tol) {  // no step left: the wrapper's test on [b, c], which only a huge b fails
+                const double xlo = b < c ? b : c, xhi = b < c ? c : b, alo = fabs(xlo), ahi = fabs(xhi);
+                const double mn = ((xlo > 0 && xhi > 0) || (xlo < 0 && xhi < 0)) ? (alo < ahi ? alo : ahi) : 0.0;
+                if (fabs(xhi - xlo) < 1e-8 + 1e-6 * mn && !(xhi - xlo > 1e-8)) { root = b; return true; }
+                it++;
+                continue;
+            }
             if (fabs(e) < tol || fabs(fa) <= fabs(fb)) { d = m; e = m; }
             else {
                 const double sr = fb / fa;
@@ -482,18 +510,20 @@ FJ_HDNI unsigned brent_root(F &f, double lo, double hi, double &root)
             }
             a = b; fa = fb;
             if (fabs(d) > tol) b += d; else b += (m > 0 ? +tol : -tol);
-            fb = f(b);
-            xr = b;
-            const double cc = same_sign(fb, fc) ? a : c;
-            xlo = b < cc ? b : cc;
-            xhi = b < cc ? cc : b;
+            x = b;
+            return false;
         }
-        const double alo = fabs(xlo), ahi = fabs(xhi);
-        const double mn = ((xlo > 0 && xhi > 0) || (xlo < 0 && xhi < 0)) ? (alo < ahi ? alo : ahi) : 0.0;
-        if (fabs(xhi - xlo) < 1e-8 + 1e-6 * mn && !(xhi - xlo > 1e-8)) { root = xr; return 0; }
     }
-    root = xr;
-    return kFailRoot;
+};
+
+template <class F>
+FJ_HDNI unsigned brent_root(F &f, double lo, double hi, double &root)
+{
+    BrentState s;
+    s.begin(lo, hi);
+    while (!s.feed(f(s.x))) {}
+    root = s.root;
+    return s.fail;
 }
 
 // ----------------------------------------------------------------------------
@@ -1129,18 +1159,17 @@ struct SerialMomInt {
     FJ_HD double operator()(F &f, double b, unsigned &fail) const { return mom_integral(f, b, *gl, fail); }
 };
 
-// One phase-space point: uvOrb ctor (uvOrb.cpp:15-36) and the turning points of
-// Ju and Jv into o (umid, uinner, uouter, ubar, Deltau, vturn; o.fail).
-// Returns false for an unbound orbit.
-FJ_HDNI bool fudge_turning_points(const PotView &P, double Delta, double R, double z, double Phi, double pR,
-                                  double vphi, double pz, Fudge &o)
+// One phase-space point up to the reference point of the u-equation: uvOrb ctor
+// (uvOrb.cpp:15-22), pt (Uvpt.cpp:11-24); pu2, pv2 the squared momenta.  Returns
+// false for an unbound orbit.
+FJ_HDNI bool fudge_point(const PotView &P, double Delta, double R, double z, double Phi, double pR, double vphi,
+                         double pz, Fudge &o, double &pu2, double &pv2)
 {
     o.P = P;
     o.fail = 0;
     o.Delta = Delta;
     const double Lz = R * vphi;
     o.Lzsq = Lz * Lz;
-    // pt(Delta, x, p): Uvpt.cpp:11-24
     const double Delta2 = Delta * Delta, R2 = R * R, z2 = z * z, r2 = R2 + z2;
     const double dmr = Delta2 - r2, dpr = Delta2 + r2;
     const double shu2 = .5 * (r2 - Delta2 + sqrt(dmr * dmr + 4 * Delta2 * R2)) / Delta2;
@@ -1157,32 +1186,50 @@ FJ_HDNI bool fudge_turning_points(const PotView &P, double Delta, double R, doub
     const double p2 = pR * pR + pz * pz;
     const double pu = Delta * (pR * chu * o.sv + pz * shu * cv);
     const double pv = Delta * (pR * shu * cv - pz * chu * o.sv);
+    pu2 = pu * pu;
+    pv2 = pv * pv;
     o.E = .5 * p2 + .5 * o.Lzsq / (R * R) + Phi;
     if (o.E >= 0 || isnan(o.E)) return false;
     sincos(o.v, &o.sinv, &o.cosv);
     o.sinhu = sinh(o.u);
     o.coshu = cosh(o.u);
-    const double us = 58;
-    {
-        const double s = sinh(us), c = cosh(us);
-        o.sh1sq = s * s; o.ch1sq = c * c;
-    }
-    getu0(o, us);
+    return true;
+}
+
+// The rest of the ctor (uvOrb.cpp:22-36) once o.umid is known: Er, Iv and what the
+// equations repeat
+FJ_HDNI void fudge_constants(Fudge &o, double pu2, double pv2)
+{
+    const double Delta2 = o.Delta * o.Delta, shu2 = o.shu2;
     {
         const double s = sinh(o.umid), c = cosh(o.umid);
         o.sh1sq = s * s; o.ch1sq = c * c;
         o.Phiu1 = o.Phiu(s, c);
     }
     o.PhivPIH = o.Phiv(sin(kPIH), cos(kPIH));
-    o.Er = -o.E * (shu2 - o.sh1sq) / o.ch1sq + .5 * (pu * pu) / (Delta2 * o.ch1sq) +
+    o.Er = -o.E * (shu2 - o.sh1sq) / o.ch1sq + .5 * pu2 / (Delta2 * o.ch1sq) +
            .5 * o.Lzsq / (Delta2 * o.ch1sq) * (1 / shu2 - 1 / o.sh1sq) + o.dU(o.u) / o.ch1sq;
     {
         double sn, cs;
         sincos(o.v, &sn, &cs);
         const double dVv = (1 + o.shu2) * o.PhivPIH - (o.shu2 + sn * sn) * o.Phiv(sn, cs);
-        o.Iv = .5 * (pv * pv) / Delta2 - o.E * o.sv2 + .5 * o.Lzsq / (Delta2 * o.sv2) - dVv;
+        o.Iv = .5 * pv2 / Delta2 - o.E * o.sv2 + .5 * o.Lzsq / (Delta2 * o.sv2) - dVv;
     }
     o.prepare();
+}
+
+constexpr double kUmidStart = 58;  // where getu0 starts (uvOrb.cpp:23)
+
+// One phase-space point on one thread: its constants and the turning points of Ju
+// and Jv into o (umid, uinner, uouter, ubar, Deltau, vturn; o.fail).  Returns
+// false for an unbound orbit.
+FJ_HDNI bool fudge_turning_points(const PotView &P, double Delta, double R, double z, double Phi, double pR,
+                                  double vphi, double pz, Fudge &o)
+{
+    double pu2, pv2;
+    if (!fudge_point(P, Delta, R, z, Phi, pR, vphi, pz, o, pu2, pv2)) return false;
+    getu0(o, kUmidStart);
+    fudge_constants(o, pu2, pv2);
     get_turn_u(o, 1);
     o.ubar = .5 * (o.uinner + o.uouter);
     o.Deltau = .5 * (o.uouter - o.uinner);

@@ -83,6 +83,8 @@ struct PlainWork {
     size_t per_block;
     int total, grid;
 };
+// whether the FP64 kernels stage the radial derivative in shared memory too (16 KB)
+FJ_HD bool grad_staged(int nr, int npoly) { return (long long)nr * npoly <= 2048; }
 size_t plain_scratch_bytes(int chunk);  // per block, for items of at most chunk points
 // blocks of a persistent launch resident at once
 int moments_resident(size_t smem);

@@ -77,7 +77,9 @@ __global__ void __launch_bounds__(kLosBlock, 2) k_los(LosArgs a, PlainWork work)
     __shared__ int s_item;
     const MomentArgs &m = a.m;
     const int nr = m.P.nr, npoly = m.P.npoly, nt = nr * npoly;
-    double *s_ar = sm, *s_phil = s_ar + nr, *s_Pr = s_phil + nt, *s_it = s_Pr + nt;
+    const bool grad = grad_staged(nr, npoly);
+    double *s_ar = sm, *s_phil = s_ar + nr, *s_Pr = s_phil + nt, *s_fast = grad ? s_Pr + nt : s_Pr,
+           *s_it = s_fast + fast_table_size(nr, npoly);
     double *s_Eg = s_it + interp_table_size(nr), *s_Dg = s_Eg + m.ngrid, *s_xq = s_Dg + m.ngrid, *s_wq = s_xq + m.nq;
     double *s_glx = s_wq + m.nq, *s_glw = s_glx + m.gl.n, *s_red = s_glw + m.gl.n;
     SolveShared *s_solve = (SolveShared *)(s_red + kLosBlock / 32);
@@ -85,13 +87,18 @@ __global__ void __launch_bounds__(kLosBlock, 2) k_los(LosArgs a, PlainWork work)
     unsigned short *s_list = (unsigned short *)(s_solve + 1);         // [kLosChunk] bound nodes
     int *s_wc = (int *)(s_list + kLosChunk);
     for (int i = threadIdx.x; i < nr; i += blockDim.x) s_ar[i] = m.P.ar[i];
-    for (int i = threadIdx.x; i < nt; i += blockDim.x) { s_phil[i] = m.P.phil[i]; s_Pr[i] = m.P.Pr[i]; }
+    for (int i = threadIdx.x; i < nt; i += blockDim.x) {
+        s_phil[i] = m.P.phil[i];
+        if (grad) s_Pr[i] = m.P.Pr[i];
+    }
     for (int i = threadIdx.x; i < m.ngrid; i += blockDim.x) { s_Eg[i] = m.Eg[i]; s_Dg[i] = m.Dg[i]; }
     for (int i = threadIdx.x; i < m.nq; i += blockDim.x) { s_xq[i] = m.xq[i]; s_wq[i] = m.wq[i]; }
     for (int i = threadIdx.x; i < m.gl.n; i += blockDim.x) { s_glx[i] = m.gl.x01[i]; s_glw[i] = m.gl.w01[i]; }
     __syncthreads();
     interp_table(nr, s_ar, s_it, threadIdx.x, blockDim.x);
-    const PotView P{nr, npoly, s_ar, s_phil, s_Pr, m.P.Pr2, s_it};
+    __syncthreads();
+    const PotView P{nr, npoly, s_ar, s_phil, grad ? s_Pr : m.P.Pr, m.P.Pr2, s_it};
+    const PotFast F = fast_tables(P, s_fast);
     const GLRule gl{m.gl.n, s_glx, s_glw};
     const SolveScratch S = solve_scratch(work.scratch + blockIdx.x * work.per_block, kPlainChunk);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -167,7 +174,7 @@ __global__ void __launch_bounds__(kLosBlock, 2) k_los(LosArgs a, PlainWork work)
         s_key[q] = node_cost_key((float)(V[0] * iVe), (float)(V[1] * iVe), (float)(V[2] * iVe));
     }
     sort_list(s_list, s_key, nbound);
-    solve_orbits64(P, gl, m.trig, nbound, S, *s_solve,
+    solve_orbits64(P, F, gl, m.trig, nbound, S, *s_solve,
                    [&](int q, double &Delta, double &R_, double &z_, double &Phi_, double &V0, double &V1, double &V2) {
                        double V[3], w, jacob;
                        node_vel(n0 + s_list[q], V, w, jacob);
@@ -229,7 +236,8 @@ int los_nodes(int kind, int nq)
 size_t los_smem_bytes(const MomentArgs &m)
 {
     const size_t nt = (size_t)m.P.nr * m.P.npoly;
-    return (m.P.nr + 2 * nt + interp_table_size(m.P.nr) + 2 * m.ngrid + 2 * m.nq + 2 * m.gl.n + kLosBlock / 32) *
+    return (m.P.nr + (grad_staged(m.P.nr, m.P.npoly) ? 2 : 1) * nt + fast_table_size(m.P.nr, m.P.npoly) +
+            interp_table_size(m.P.nr) + 2 * m.ngrid + 2 * m.nq + 2 * m.gl.n + kLosBlock / 32) *
                sizeof(double) +
            sizeof(SolveShared) + kLosChunk * sizeof(unsigned short) + (kLosBlock / 32 + 1) * sizeof(int);
 }

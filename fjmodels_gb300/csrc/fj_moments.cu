@@ -58,12 +58,14 @@ cudaError_t launch_trig_table(double2 *trig, cudaStream_t s)
     return cudaGetLastError();
 }
 
-// shared memory of a model's tables: radii, potential and its radial derivative
-// (the second one, which only the quasi-isothermal DF reads, stays in device
-// memory), interpolation constants, focal distances, velocity and momentum rules
+// shared memory of a model's tables: radii, potential, the integrands' tables,
+// interpolation constants, focal distances, velocity and momentum rules, and of
+// small models the radial derivative (the second one, which only the
+// quasi-isothermal DF reads, stays in device memory)
 static size_t table_doubles(int nr, int npoly, int ngrid, int nq, int ngl)
 {
-    return nr + 2 * (size_t)nr * npoly + interp_table_size(nr) + 2 * ngrid + 2 * nq + 2 * ngl;
+    return nr + (size_t)nr * npoly * (grad_staged(nr, npoly) ? 2 : 1) + fast_table_size(nr, npoly) + interp_table_size(nr) +
+           2 * ngrid + 2 * nq + 2 * ngl;
 }
 
 size_t moment_smem_bytes(const MomentArgs &a)
@@ -91,7 +93,9 @@ __global__ void __launch_bounds__(kMomentBlock, 2) k_moments(MomentArgs a0, Mome
         }
         const MomentArgs &a = batch.n > 0 ? batch.args[m] : a0;
         const int nr = a.P.nr, npoly = a.P.npoly, nt = nr * npoly;
-        double *s_ar = sm, *s_phil = s_ar + nr, *s_Pr = s_phil + nt, *s_it = s_Pr + nt;
+        const bool grad = grad_staged(nr, npoly);
+        double *s_ar = sm, *s_phil = s_ar + nr, *s_Pr = s_phil + nt, *s_fast = grad ? s_Pr + nt : s_Pr,
+               *s_it = s_fast + fast_table_size(nr, npoly);
         double *s_Eg = s_it + interp_table_size(nr), *s_Dg = s_Eg + a.ngrid,
                *s_xq = s_Dg + a.ngrid, *s_wq = s_xq + a.nq;
         double *s_glx = s_wq + a.nq, *s_glw = s_glx + a.gl.n, *s_red = s_glw + a.gl.n;
@@ -103,15 +107,21 @@ __global__ void __launch_bounds__(kMomentBlock, 2) k_moments(MomentArgs a0, Mome
         if (m != model) {
             model = m;
             for (int i = threadIdx.x; i < nr; i += blockDim.x) s_ar[i] = a.P.ar[i];
-            for (int i = threadIdx.x; i < nt; i += blockDim.x) { s_phil[i] = a.P.phil[i]; s_Pr[i] = a.P.Pr[i]; }
+            for (int i = threadIdx.x; i < nt; i += blockDim.x) {
+                s_phil[i] = a.P.phil[i];
+                if (grad) s_Pr[i] = a.P.Pr[i];
+            }
             for (int i = threadIdx.x; i < a.ngrid; i += blockDim.x) { s_Eg[i] = a.Eg[i]; s_Dg[i] = a.Dg[i]; }
             for (int i = threadIdx.x; i < a.nq; i += blockDim.x) { s_xq[i] = a.xq[i]; s_wq[i] = a.wq[i]; }
             for (int i = threadIdx.x; i < a.gl.n; i += blockDim.x) { s_glx[i] = a.gl.x01[i]; s_glw[i] = a.gl.w01[i]; }
             __syncthreads();
             interp_table(nr, s_ar, s_it, threadIdx.x, blockDim.x);
             __syncthreads();
+            fast_tables(PotView{nr, npoly, s_ar, s_phil, s_Pr, a.P.Pr2, s_it}, s_fast);
+            __syncthreads();
         }
-        const PotView P{nr, npoly, s_ar, s_phil, s_Pr, a.P.Pr2, s_it};
+        const PotView P{nr, npoly, s_ar, s_phil, grad ? s_Pr : a.P.Pr, a.P.Pr2, s_it};
+        const PotFast F{nr, npoly, s_ar, s_phil, s_fast, s_fast + nt, s_it};
         const GLRule gl{a.gl.n, s_glx, s_glw};
         const int B = a.blocks_per_point;
         const int p = bid / B, chunk = bid % B;
@@ -164,7 +174,7 @@ __global__ void __launch_bounds__(kMomentBlock, 2) k_moments(MomentArgs a0, Mome
         sort_list(s_list, s_key, nbound);
         // the orbits of the list
         const SolveScratch S = solve_scratch(work.scratch + blockIdx.x * work.per_block, kPlainChunk);
-        solve_orbits64(P, gl, a.trig, nbound, S, *s_solve,
+        solve_orbits64(P, F, gl, a.trig, nbound, S, *s_solve,
                        [&](int q, double &Delta, double &R_, double &z_, double &Phi_, double &V0, double &V1, double &V2) {
                            velocity(n0 + s_list[q], V0, V1, V2);
                            const double H = .5 * (V0 * V0 + V1 * V1 + V2 * V2) + Phi_h;
@@ -310,15 +320,18 @@ __global__ void __launch_bounds__(kSolveBlock, 2) k_actions(PotView P0, const do
     const int nr = P0.nr, npoly = P0.npoly, nt = nr * npoly;
     SolveShared *s_solve = (SolveShared *)sm;
     double *s_ar = (double *)(s_solve + 1), *s_phil = s_ar + nr, *s_Pr = s_phil + nt, *s_it = s_Pr + nt,
-           *s_Eg = s_it + interp_table_size(nr), *s_Dg = s_Eg + ngrid;
+           *s_Eg = s_it + interp_table_size(nr), *s_Dg = s_Eg + ngrid, *s_fast = s_Dg + ngrid;
     PotView P = P0;
+    PotFast F{nr, npoly, P0.ar, P0.phil, nullptr, nullptr, nullptr};
     if (staged) {
         for (int i = threadIdx.x; i < nr; i += blockDim.x) s_ar[i] = P0.ar[i];
         for (int i = threadIdx.x; i < nt; i += blockDim.x) { s_phil[i] = P0.phil[i]; s_Pr[i] = P0.Pr[i]; }
         for (int i = threadIdx.x; i < ngrid; i += blockDim.x) { s_Eg[i] = Eg[i]; s_Dg[i] = Dg[i]; }
         __syncthreads();
         interp_table(nr, s_ar, s_it, threadIdx.x, blockDim.x);
+        __syncthreads();
         P = PotView{nr, npoly, s_ar, s_phil, s_Pr, P0.Pr2, s_it};
+        F = fast_tables(P, s_fast);
         Eg = s_Eg; Dg = s_Dg;
     }
     const SolveScratch S = solve_scratch(work.scratch + blockIdx.x * work.per_block, kActionChunk);
@@ -342,7 +355,7 @@ __global__ void __launch_bounds__(kSolveBlock, 2) k_actions(PotView P0, const do
             }
         }
         __syncthreads();
-        solve_orbits64(P, gl0, trig, s_n, S, *s_solve,
+        solve_orbits64(P, F, gl0, trig, s_n, S, *s_solve,
                        [&](int q, double &Delta, double &R, double &z, double &Phi, double &vR, double &vp, double &vz) {
                            const double *x = pts + 5 * (t0 + s_list[q]);
                            R = x[0]; z = x[1]; vR = x[2]; vp = x[3]; vz = x[4];
@@ -361,7 +374,8 @@ __global__ void __launch_bounds__(kSolveBlock, 2) k_actions(PotView P0, const do
 constexpr size_t kStagedTables = 96 * 1024;
 static size_t actions_table_bytes(int nr, int npoly, int ngrid)
 {
-    return (nr + 2 * (size_t)nr * npoly + interp_table_size(nr) + 2 * (size_t)ngrid) * sizeof(double);
+    return (nr + 2 * (size_t)nr * npoly + fast_table_size(nr, npoly) + interp_table_size(nr) + 2 * (size_t)ngrid) *
+           sizeof(double);
 }
 size_t actions_smem_bytes(int nr, int npoly, int ngrid)
 {

@@ -771,9 +771,7 @@ int fj_actions(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delta
     if (n == 0) return FJ_OK;
     const double2 *trig = nullptr;
     if ((rc = trig_table(ctx, &trig))) return rc;
-    // points per work item: as plain_chunk, a share of the GPU's blocks each
-    int chunk = kActionChunk;
-    while (chunk > 32 && (n + chunk - 1) / chunk < (size_t)kPlainItems) chunk >>= 1;
+    const int chunk = action_chunk(n);
     PlainWork pw{};
     if ((rc = plain_setup(ctx, (long long)((n + chunk - 1) / chunk),
                           actions_resident(actions_smem_bytes(pot->nr, pot->npoly, delta->ngrid)), kActionChunk, pw)))

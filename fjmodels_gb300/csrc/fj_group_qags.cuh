@@ -103,16 +103,20 @@ __device__ __noinline__ void group_qelg(T *tab, int &n_io, T *res3, int &nres, T
 }
 
 // The state of one integral after its first panel (the first lane's registers)
-template <class T, int CAP, bool HEAP = false>
+// IER: also the QUADPACK error class of a finished integral (ier)
+template <class T, int CAP, bool HEAP = false, bool IER = false>
 struct GroupQags {
     using List = QagsList<T, CAP, HEAP>;
+    int ier_class;
+    T res0_, resabs;
     T area, errsum, errmax, res_ext, err_ext, correc, ertest, erlarg, small, len;
     int maxerr, nrmax, last, numrl2, nres, ktmin, ierro, iroff1, iroff2, iroff3;
     bool extrap, noext;
 
     // res0, err0: the first panel on [a, b], which did not finish the integral
-    __device__ void begin(List &L, T a, T b, T res0, T err0)
+    __device__ void begin(List &L, T a, T b, T res0, T err0, T resabs0 = 0)
     {
+        if (IER) { res0_ = res0; resabs = resabs0; ier_class = 0; }
         L.iv[0] = QagsEntry<T>{a, b, res0, err0};
         if (HEAP) L.heap[0] = 1;
         L.iord[0] = 0;
@@ -213,7 +217,11 @@ struct GroupQags {
             errmax = L.iv[maxerr].e;
         }
         bool stop = false;  // the loop ends here
-        if (errsum <= errbnd) { result = list_sum(L, last); return true; }
+        if (errsum <= errbnd) {
+            if (IER) ier_class = ier > 2 ? ier - 1 : ier;
+            result = list_sum(L, last);
+            return true;
+        }
         if (ier) stop = true;
         else if (last == 1) {
             small = len * T(0.375);
@@ -278,6 +286,21 @@ struct GroupQags {
             if (res_ext != 0 && area != 0) {
                 if (err_ext / qabs(res_ext) > errsum / qabs(area)) take_sum = true;
             } else if (err_ext > errsum) take_sum = true;
+        }
+        if (IER) {
+            bool skip_div = false;
+            if (err_ext != HUGE_ && ier + ierro != 0) {
+                if (ier == 0) ier = 3;
+                if (!(res_ext != 0 && area != 0) && !take_sum && area == 0) skip_div = true;
+            }
+            if (!take_sum && !skip_div) {
+                const int ksgn = qabs(res0_) >= (1 - 50 * EPS) * resabs ? 1 : -1;
+                if (!(ksgn == -1 && qmax(qabs(res_ext), qabs(area)) <= resabs * T(0.01))) {
+                    const T ratio = res_ext / area;
+                    if (ratio < T(0.01) || ratio > 100 || errsum > qabs(area)) ier = 6;
+                }
+            }
+            ier_class = ier > 2 ? ier - 1 : ier;
         }
         result = take_sum ? list_sum(L, last) : res_ext;
         return true;

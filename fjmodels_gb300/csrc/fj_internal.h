@@ -231,7 +231,16 @@ int mixed_blocks_per_point(long long nq3, int chunk);
 cudaError_t launch_moments_mixed(const MomentArgs &a, int variant, const DeferWork &dw, const ItemQueue &q,
                                  cudaStream_t s);
 
-constexpr int kActionChunk = 256;  // most points per work item of the action batch
+// Points per work item of the action batch: whole rounds of the two blocks per SM,
+// items of a warp at least (20 001 points: 10.2 ms in items of 32, two rounds of
+// which the second is nearly empty; 6.0 ms in one round of items of 66)
+constexpr int kActionChunk = 256, kActionBlocks = 304;
+inline int action_chunk(size_t n)
+{
+    const size_t most = (size_t)kActionBlocks * kActionChunk, rounds = (n + most - 1) / most;
+    const size_t c = (n + kActionBlocks * rounds - 1) / (kActionBlocks * rounds);
+    return (int)(c < 32 ? 32 : c);
+}
 size_t actions_smem_bytes(int nr, int npoly, int ngrid);
 cudaError_t launch_actions(PotView P, const double *Eg, const double *Dg, int ngrid, GLRule gl, const double2 *trig,
                            const double *pts, size_t n, int chunk, double *out, const PlainWork &w, cudaStream_t s);

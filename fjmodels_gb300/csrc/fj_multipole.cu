@@ -2,8 +2,12 @@
 // projection of the moment grids, the radial Poisson integrals, the sum of
 // component potentials and the tensor-virial sums.  All FP64; each is small
 // next to the phase-space kernel.
+#include <cooperative_groups.h>
+
+#include "fj_group_qags.cuh"
 #include "fj_internal.h"
-#include "fj_qags_warp.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace fj {
 
@@ -40,75 +44,193 @@ cudaError_t launch_project(int nr, int ngauss, int npoly, const double *ar, cons
 }
 
 // ------------------------------------------------------------------ Poisson
-// linear interpolation of one multipole column (include/Utils.h:122-128)
-__device__ __forceinline__ double linterp_col(const double *ar, const double *rhl, int npoly, int l, int nr, double x)
-{
-    if (x <= ar[0]) return rhl[l];
-    if (x >= ar[nr - 1]) return rhl[(nr - 1) * npoly + l];
-    int top = 0, bot = 0;
-    topbottom(ar, nr, x, bot, top);
-    const double yb = rhl[bot * npoly + l], yt = rhl[top * npoly + l];
-    return yb + (x - ar[bot]) / (ar[top] - ar[bot]) * (yt - yb);
-}
+// linear interpolation of one multipole column (include/Utils.h:122-128): rec[n] =
+// 1 / (ar[n+1] - ar[n]), or null to divide; the bracket by the radii's logarithms
+// (lg: log2 of the first and the intervals per unit) corrected by neighbour tests,
+// the interval that topbottom's bisection finds (the upper one on a node)
+struct RadialTab {
+    const double *ar, *rhl, *rec;
+    int npoly, col, nr;
+    float2 lg;
+    __device__ __forceinline__ double linterp(double x) const
+    {
+        if (x <= ar[0]) return rhl[col];
+        if (x >= ar[nr - 1]) return rhl[(nr - 1) * npoly + col];
+        const long long xb = __double_as_longlong(x);
+        const int hi = (int)(xb >> 32);
+        const float m = __int_as_float(0x3f800000 | ((hi & 0xfffff) << 3) | (int)(((unsigned)xb) >> 29));
+        int b = (int)(((float)((hi >> 20) - 1023) + __log2f(m) - lg.x) * lg.y);
+        b = b < 0 ? 0 : (b > nr - 2 ? nr - 2 : b);
+        while (b > 0 && xb < __double_as_longlong(ar[b])) --b;
+        while (b < nr - 2 && xb >= __double_as_longlong(ar[b + 1])) ++b;
+        const double ab = ar[b], yb = rhl[b * npoly + col], yt = rhl[(b + 1) * npoly + col];
+        const double f = rec ? div_by(x - ab, ar[b + 1] - ab, rec[b]) : (x - ab) / (ar[b + 1] - ab);
+        return yb + f * (yt - yb);
+    }
+};
 
 struct IInternal {  // I_internal (pot/Potential.cpp:83-89); multipole column col, degree l = 2*col
-    const double *ar, *rhl; int npoly, col, l, nr;
-    __device__ double operator()(double x) const { return pow(x, l + 2) * linterp_col(ar, rhl, npoly, col, nr, x); }
+    RadialTab T; int l;
+    __device__ double operator()(double x) const { return pow(x, l + 2) * T.linterp(x); }
 };
 struct IExternalT {  // I_external (pot/Potential.cpp:90-101) on x = a + (1-t)/t, divided by t^2
-    const double *ar, *rhl; int npoly, col, l, nr; double a;
+    RadialTab T; int l; double a;
     __device__ double operator()(double t) const
     {
         const double x = a + (1 - t) / t;
         double rhol;
-        if (x > ar[nr - 1]) rhol = dmax(0., rhl[(nr - 1) * npoly + col] * pow(ar[nr - 1] / x, 4));
-        else rhol = linterp_col(ar, rhl, npoly, col, nr, x);
+        if (x > T.ar[T.nr - 1]) rhol = dmax(0., T.rhl[(T.nr - 1) * T.npoly + T.col] * pow(T.ar[T.nr - 1] / x, 4));
+        else rhol = T.linterp(x);
         const double y = rhol / pow(x, l - 1);
         return (y / t) / t;
     }
 };
 
-// One warp per (n, l) pair.  The QAGS calls of a pair run on all 32 lanes
-// at once: the function values of each Gauss-Kronrod panel (21 or 15, 42 or
-// 30 per bisection) are spread over the lanes and exchanged through shared
-// memory, every lane forms the panel sums from them in the same order, and
-// the adaptive bookkeeping runs uniformly on every lane over an interval
-// list in the warp's shared memory (identical values, identical writes).
-// The results are those of one thread running the same QAGS: the same
-// function values enter the same sums in the same order.  With one thread
-// per pair the 2 nr npoly integrals (560 on 80 x 7) sat on a few SMs, each
-// thread evaluating its thousands of integrand values one after another.
-constexpr int kPoissonWarps = 4;
+// A warp per integral (2 nr npoly of them: internal, then external).  The function
+// values of each Gauss-Kronrod panel (21 or 15, 42 or 30 per bisection) are spread
+// over the lanes and summed in the order of one thread running the same QAGS: the
+// same function values enter the same sums.  The bookkeeping (fj_group_qags.cuh) is
+// over an interval list in shared memory: no device workspace.
+// The solve lasts as long as its longest integrals, which are FP64 latency: up to
+// 213 bisections on 80 x 7, an external integral tried again with doubled
+// tolerances up to four times.  A new try bisects the same intervals until its
+// tolerance tells, so the panels of the last try's bisections are kept (kPoissonLog
+// of them) and only new intervals are evaluated.  80 x 7: 2.7-2.9 ms; 3.6 ms without
+// that, half a warp per integral and bracket searches by bisection; 3.9-4.4 ms with a
+// warp per (n, l) pair taking its two integrals one after the other and the panel
+// sums on every lane; 33 ms with one thread per pair.
+constexpr int kPoissonLanes = 32;
+constexpr int kPoissonBlock = 64;
+constexpr int kPoissonGroups = kPoissonBlock / kPoissonLanes;
+constexpr int kPoissonLog = 64;
+constexpr int kPoissonTabled = 2048;  // radii whose reciprocals fit shared memory beside the lists
+using PoissonQags = GroupQags<double, kPoissonCap, false, true>;
+struct PoissonPanels { double a, b, res, err, rc, res2, err2, rc2; };  // one bisection's two panels
 
-// computeInts + computePhil (pot/Potential.cpp:110-200)
-__global__ void __launch_bounds__(32 * kPoissonWarps) k_poisson(int nr, int npoly, const double *ar,
-                                                                 const double *rhl, double *phil, double *Pr,
-                                                                 double *Pr2, unsigned long long *counters)
+// QAGS of f on [a, b] by the group's lanes (every lane of the warp calls it; `on`
+// per group); retry: with doubled tolerances until it succeeds (computeInts,
+// pot/Potential.cpp:146-150).  The result is valid on the group's first lane.
+template <int RULE, class F>
+__device__ double poisson_integral(const F &f, bool on, double a, double b, bool retry, PoissonQags::List &L,
+                                   PoissonPanels *log, double *vals, bool &full)
 {
-    __shared__ double s_list[kPoissonWarps][4 * kPoissonCap];
-    __shared__ int s_iord[kPoissonWarps][kPoissonCap];
-    __shared__ double s_vals[kPoissonWarps][42];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t = blockIdx.x * kPoissonWarps + warp;
-    const int nt = nr * npoly;
-    if (t >= nt) return;  // the whole warp
-    const int n = t / npoly, np = t % npoly, l = 2 * np;
-    double *dws = s_list[warp];
-    const QagsWs W{dws, dws + kPoissonCap, dws + 2 * kPoissonCap, dws + 3 * kPoissonCap, s_iord[warp], kPoissonCap};
-    unsigned fail = 0;
-    double Iint, Iext, err;
-    IInternal fi{ar, rhl, npoly, np, l, nr};
-    qags_warp<21>(fi, 0., ar[n], 1e-4, 1e-3, 1000, Iint, err, fail, W, s_vals[warp], lane);
-    IExternalT fe{ar, rhl, npoly, np, l, nr, ar[n]};
-    double epsabs = 1e-4, epsrel = 1e-3;
-    int status = 1, tries = 0;
-    while (status != 0 && tries < 60) {
-        status = qags_warp<15>(fe, 0.0, 1.0, epsabs, epsrel, 1000, Iext, err, fail, W, s_vals[warp], lane);
-        epsabs *= 2; epsrel *= 2; tries++;
+    constexpr int N = GKRule<RULE>::npts, G = kPoissonLanes;
+    const int lane = threadIdx.x & 31, gi = lane % G, lead = lane - gi;
+    double epsabs = 1e-4, epsrel = 1e-3, result = 0, res0 = 0, err0 = 0, ra0 = 0, rc0 = 0, a1 = 0, b2 = 0;
+    int tries = 0, step = 0, logged = 0;  // the bisection of this try; bisections logged
+    bool run = false;
+    PoissonQags st;
+    if (on) {
+        for (int e = gi; e < N; e += G) vals[e] = f(gk_abscissa<RULE>(a, b, e));
     }
-    if (lane != 0) return;
-    if (fail && counters) atomicAdd(&counters[kCntPoisson], 1ull);
-    const double r = ar[n];
+    __syncwarp();
+    // the next call: finished by its first panel, or the bisections begin
+    auto start = [&]() {
+        for (;;) {
+            double r, ae;
+            const int h = qags_head(res0, err0, ra0, rc0, epsabs, epsrel, 1000, r, ae);
+            if (h < 0) {
+                st.begin(L, a, b, res0, err0, ra0);
+                a1 = a; b2 = b;
+                step = 0;
+                run = true;
+                return;
+            }
+            result = r;
+            run = false;
+            if (!retry || h == 0 || ++tries >= 60) return;
+            epsabs *= 2; epsrel *= 2;
+        }
+    };
+    if (on && gi == 0) {
+        gk_sum<RULE>(a, b, vals, res0, err0, ra0, rc0);
+        start();
+    }
+    for (;;) {
+        // 0: finished, 1: evaluate, 2: logged
+        const bool known = gi == 0 && run && step < logged && log[step].a == a1 && log[step].b == b2;
+        const int go = __shfl_sync(0xffffffffu, run ? (known ? 2 : 1) : 0, lead);
+        if (!__any_sync(0xffffffffu, go)) return result;
+        a1 = __shfl_sync(0xffffffffu, a1, lead);
+        b2 = __shfl_sync(0xffffffffu, b2, lead);
+        const double b1 = 0.5 * (a1 + b2);
+        double res = 0, err = 0, ra, rc = 0;
+        if (go == 1) {
+            for (int e = gi; e < 2 * N; e += G) {
+                const bool second = e >= N;
+                vals[e] = f(gk_abscissa<RULE>(second ? b1 : a1, second ? b2 : b1, second ? e - N : e));
+            }
+        }
+        __syncwarp();
+        if (go == 1 && gi % (G / 2) == 0)
+            gk_sum<RULE>(gi ? b1 : a1, gi ? b2 : b1, vals + (gi ? N : 0), res, err, ra, rc);
+        double res2 = __shfl_sync(0xffffffffu, res, lead + G / 2), err2 = __shfl_sync(0xffffffffu, err, lead + G / 2),
+               rc2 = __shfl_sync(0xffffffffu, rc, lead + G / 2);
+        if (go && gi == 0) {
+            if (go == 2) {
+                const PoissonPanels &p = log[step];
+                res = p.res; err = p.err; rc = p.rc; res2 = p.res2; err2 = p.err2; rc2 = p.rc2;
+            } else if (retry && step < kPoissonLog) {
+                log[step] = PoissonPanels{a1, b2, res, err, rc, res2, err2, rc2};
+                if (logged == step) logged = step + 1;
+            }
+            step++;
+        }
+        if (go && gi == 0) {
+            double r = 0;
+            if (st.update(L, res, err, rc, res2, err2, rc2, epsabs, epsrel, r, full)) {
+                result = r;
+                run = false;
+                if (retry && st.ier_class != 0 && ++tries < 60) {
+                    epsabs *= 2; epsrel *= 2;
+                    start();
+                }
+            } else {
+                a1 = L.iv[st.maxerr].a;
+                b2 = L.iv[st.maxerr].b;
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// computeInts (pot/Potential.cpp:110-155): the internal integrals into phil, the
+// external ones into Pr, for k_poisson_tables
+__global__ void __launch_bounds__(kPoissonBlock) k_poisson(int nr, int npoly, const double *ar, const double *rhl,
+                                                           double *phil, double *Pr, unsigned long long *counters)
+{
+    __shared__ PoissonQags::List s_list[kPoissonGroups];
+    __shared__ PoissonPanels s_log[kPoissonGroups][kPoissonLog];
+    __shared__ double s_vals[kPoissonGroups][43];
+    extern __shared__ double s_rec[];  // of grids that fit: 1 / (ar[n+1] - ar[n])
+    const bool tabled = nr <= kPoissonTabled;
+    for (int i = threadIdx.x; tabled && i < nr - 1; i += kPoissonBlock) s_rec[i] = recip(ar[i + 1] - ar[i]);
+    __syncthreads();
+    const int g = threadIdx.x / kPoissonLanes, nt = nr * npoly;
+    const int i = blockIdx.x * kPoissonGroups + g;  // [0, nt): external (the longer ones), then internal
+    const bool ext = i < nt;
+    const int t = ext ? i : i - nt;
+    const bool on = t < nt;
+    const int n = on ? t / npoly : 0, np = on ? t % npoly : 0, l = 2 * np;
+    bool full = false;
+    double v;
+    const float l0 = log2f((float)ar[0]);
+    const RadialTab T{ar, rhl, tabled ? s_rec : nullptr, npoly, np, nr, make_float2(l0, (nr - 1) / (log2f((float)ar[nr - 1]) - l0))};
+    if (!ext) v = poisson_integral<21>(IInternal{T, l}, on, 0., ar[n], false, s_list[g], s_log[g], s_vals[g], full);
+    else v = poisson_integral<15>(IExternalT{T, l, ar[n]}, on, 0., 1., true, s_list[g], s_log[g], s_vals[g], full);
+    if (!on || threadIdx.x % kPoissonLanes) return;
+    if (full && counters) atomicAdd(&counters[kCntPoisson], 1ull);
+    (ext ? Pr : phil)[t] = v;
+}
+
+// computePhil (pot/Potential.cpp:157-200) from the integrals, in place
+__global__ void k_poisson_tables(int nr, int npoly, const double *ar, const double *rhl, double *phil, double *Pr,
+                                 double *Pr2)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nr * npoly) return;
+    const int n = t / npoly, l = 2 * (t % npoly);
+    const double r = ar[n], Iint = phil[t], Iext = Pr[t];
     const double G = 1;
     phil[t] = -kTPI * G * (Iint / pow(r, l + 1) + Iext * pow(r, l));
     Pr[t] = -kTPI * G * (-(l + 1) * Iint / pow(r, l + 2) + l * Iext * pow(r, l - 1));
@@ -120,8 +242,10 @@ cudaError_t launch_poisson(int nr, int npoly, const double *ar, const double *rh
                            double *Pr, double *Pr2, unsigned long long *counters, cudaStream_t s)
 {
     const int nt = nr * npoly;
-    k_poisson<<<(nt + kPoissonWarps - 1) / kPoissonWarps, 32 * kPoissonWarps, 0, s>>>(nr, npoly, ar, rhl, phil, Pr,
-                                                                                      Pr2, counters);
+    const size_t smem = nr <= kPoissonTabled ? (nr - 1) * sizeof(double) : 0;
+    k_poisson<<<(2 * nt + kPoissonGroups - 1) / kPoissonGroups, kPoissonBlock, smem, s>>>(nr, npoly, ar, rhl, phil, Pr,
+                                                                                         counters);
+    k_poisson_tables<<<(nt + 63) / 64, 64, 0, s>>>(nr, npoly, ar, rhl, phil, Pr, Pr2);
     return cudaGetLastError();
 }
 
@@ -135,36 +259,65 @@ cudaError_t launch_poisson(int nr, int npoly, const double *ar, const double *rh
 // a fixed order.  No adaptive decisions: the potential is a smooth function of
 // the density, where the reference's QAGS (epsabs 1e-4, epsrel 1e-3) moves it
 // by up to ~1e-3 when a small change of the density flips a subdivision.
-// One block per multipole l, a thread per interval, then one thread per radius.
+// One cluster of kCumCluster blocks per multipole l.  The powers of the radii are
+// most of the work (nine per radius, ~190 FP64 instructions each): the cluster's
+// blocks, on SMs of their own, share them, a thread per power, into the first
+// block's shared memory; that block goes on with a thread per interval, the two
+// prefix sums on a thread each, and a thread per radius.  40 radii, l <= 8: 16.4 us;
+// 22.4 us with one block taking all powers, ~58 us with a thread per interval taking
+// its own eight and a thread per radius seven.
 
-// int_a^b x^m (c0 + c1 x) dx
-__device__ __forceinline__ double seg_power_integral(double a, double b, int m, double c0, double c1)
+// int_a^b x^m (c0 + c1 x) dx from a^(m+1), b^(m+1) (p0) and a^(m+2), b^(m+2) (p1)
+__device__ __forceinline__ double seg_power_integral(double a, double b, int m, double c0, double c1, double p0a,
+                                                     double p0b, double p1a, double p1b)
 {
-    const double t0 = m == -1 ? log(b / a) : (pow(b, m + 1) - pow(a, m + 1)) / (m + 1);
-    const double t1 = m == -2 ? log(b / a) : (pow(b, m + 2) - pow(a, m + 2)) / (m + 2);
+    const double t0 = m == -1 ? log(b / a) : (p0b - p0a) / (m + 1);
+    const double t1 = m == -2 ? log(b / a) : (p1b - p1a) / (m + 2);
     return c0 * t0 + c1 * t1;
 }
 
-__global__ void k_poisson_cumulative(int nr, int npoly, const double *ar, const double *rhl, double *phil,
-                                     double *Pr, double *Pr2)
+constexpr int kCumPowers = 9, kCumBlock = 128, kCumCluster = 8;
+
+__global__ void __launch_bounds__(kCumBlock) __cluster_dims__(kCumCluster, 1, 1)
+    k_poisson_cumulative(int nr, int npoly, const double *ar,
+                                                                  const double *rhl, double *phil, double *Pr,
+                                                                  double *Pr2, bool tabled)
 {
     extern __shared__ double sh[];
     double *s_in = sh, *s_ex = sh + nr;  // interval i = [ar[i], ar[i+1]] (s_in[nr-1]: [0, ar[0]]; s_ex[nr-1]: tail)
-    const int np = blockIdx.x, l = 2 * np;
-    for (int i = threadIdx.x; i < nr; i += blockDim.x) {
+    const int np = blockIdx.x / kCumCluster, l = 2 * np;
+    cg::cluster_group cluster = cg::this_cluster();
+    // pw[j][n] = ar[n]^(l - 2 + j), j < 7; pw[7][n] = ar[n]^(2 - l), pw[8][n] = ar[n]^(3 - l); of grids too large
+    // for shared memory where they are used
+    double *pw = sh + 2 * nr;
+    auto power = [&](int j, int n) { return pow(ar[n], j < 7 ? l - 2 + j : j == 7 ? 2 - l : 3 - l); };
+    const int rank = (int)cluster.block_rank();
+    if (tabled) {
+        double *first = cluster.map_shared_rank(pw, 0);
+        for (int i = rank * kCumBlock + threadIdx.x; i < kCumPowers * nr; i += kCumCluster * kCumBlock)
+            first[i] = power(i / nr, i % nr);
+        cluster.sync();  // the powers are in the first block's shared memory
+    }
+    if (rank != 0) return;
+    auto q = [&](int j, int n) { return tabled ? pw[j * nr + n] : power(j, n); };
+    for (int t = threadIdx.x; t < 2 * nr; t += blockDim.x) {
+        const int i = t % nr;
+        const bool ex = t >= nr;
         if (i < nr - 1) {
             const double a = ar[i], b = ar[i + 1], ya = rhl[i * npoly + np], yb = rhl[(i + 1) * npoly + np];
             const double s = (yb - ya) / (b - a), c0 = ya - s * a;
-            s_in[i] = seg_power_integral(a, b, l + 2, c0, s);
-            s_ex[i] = seg_power_integral(a, b, 1 - l, c0, s);
+            if (!ex) s_in[i] = seg_power_integral(a, b, l + 2, c0, s, q(5, i), q(5, i + 1), q(6, i), q(6, i + 1));
+            else s_ex[i] = seg_power_integral(a, b, 1 - l, c0, s, q(7, i), q(7, i + 1), q(8, i), q(8, i + 1));
+        } else if (!ex) {
+            s_in[i] = rhl[np] * q(5, 0) / (l + 3);
         } else {
-            const double a0 = ar[0], R = ar[nr - 1], yN = rhl[(nr - 1) * npoly + np];
-            s_in[i] = rhl[np] * pow(a0, l + 3) / (l + 3);
-            s_ex[i] = (yN > 0 ? yN : 0.) * pow(R, 2 - l) / (l + 2);
+            const double yN = rhl[(nr - 1) * npoly + np];
+            s_ex[i] = (yN > 0 ? yN : 0.) * q(7, nr - 1) / (l + 2);
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {  // prefix sums in place: s_in[n] = I_int(ar[n]), s_ex[n] = I_ext(ar[n])
+    // prefix sums in place: s_in[n] = I_int(ar[n]), s_ex[n] = I_ext(ar[n])
+    if (threadIdx.x == 0) {
         double acc = s_in[nr - 1], seg = s_in[0];
         s_in[0] = acc;
         for (int n = 1; n < nr; n++) {
@@ -172,7 +325,8 @@ __global__ void k_poisson_cumulative(int nr, int npoly, const double *ar, const 
             seg = s_in[n];
             s_in[n] = acc;
         }
-        acc = s_ex[nr - 1];
+    } else if (threadIdx.x == 32) {
+        double acc = s_ex[nr - 1];
         for (int n = nr - 1; n >= 0; n--) {
             const double cur = n < nr - 1 ? s_ex[n] : 0.;
             if (n < nr - 1) acc += cur;
@@ -181,12 +335,11 @@ __global__ void k_poisson_cumulative(int nr, int npoly, const double *ar, const 
     }
     __syncthreads();
     for (int n = threadIdx.x; n < nr; n += blockDim.x) {  // computePhil (Potential.cpp:163-200)
-        const double r = ar[n], Ii = s_in[n], Ie = s_ex[n], G = 1;
+        const double Ii = s_in[n], Ie = s_ex[n], G = 1;
         const int t = n * npoly + np;
-        phil[t] = -kTPI * G * (Ii / pow(r, l + 1) + Ie * pow(r, l));
-        Pr[t] = -kTPI * G * (-(l + 1) * Ii / pow(r, l + 2) + l * Ie * pow(r, l - 1));
-        Pr2[t] = -kTPI * G * ((l + 2) * (l + 1) * Ii / pow(r, l + 3) + (l - 1) * l * Ie * pow(r, l - 2) -
-                              (2 * l + 1) * rhl[t]);
+        phil[t] = -kTPI * G * (Ii / q(3, n) + Ie * q(2, n));
+        Pr[t] = -kTPI * G * (-(l + 1) * Ii / q(4, n) + l * Ie * q(1, n));
+        Pr2[t] = -kTPI * G * ((l + 2) * (l + 1) * Ii / q(5, n) + (l - 1) * l * Ie * q(0, n) - (2 * l + 1) * rhl[t]);
     }
 }
 
@@ -194,7 +347,9 @@ cudaError_t launch_poisson_cumulative(int nr, int npoly, const double *ar, const
                                       double *Pr, double *Pr2, cudaStream_t s)
 {
     if (nr < 2 || nr > kPoissonCumulativeMaxNr) return cudaErrorInvalidValue;
-    k_poisson_cumulative<<<npoly, 128, 2 * nr * sizeof(double), s>>>(nr, npoly, ar, rhl, phil, Pr, Pr2);
+    const bool tabled = (2 + kCumPowers) * nr * sizeof(double) <= 48 * 1024;
+    k_poisson_cumulative<<<npoly * kCumCluster, kCumBlock, (tabled ? 2 + kCumPowers : 2) * nr * sizeof(double), s>>>(
+        nr, npoly, ar, rhl, phil, Pr, Pr2, tabled);
     return cudaGetLastError();
 }
 

@@ -28,7 +28,7 @@
 namespace fj {
 
 constexpr int kSolveBlock = 128;                        // threads of a solving block
-constexpr int kSolveLanes = 4;                          // lanes per momentum integral
+constexpr int kSolveLanes = 4;                          // lanes per momentum integral (2: large launches 3-9 % faster, 6 points 20 % slower)
 constexpr int kSolveGroups = kSolveBlock / kSolveLanes;  // integrals in flight
 constexpr int kTrigPanels = 1024;                       // bisection tree down to 1/512 of the range
 
@@ -595,12 +595,12 @@ __device__ void solve_orbits64(const PotView &P, const PotFast &F, const GLRule 
                 }
             }
             __syncwarp();
-            // the panels' sums on the group's first and third lanes
+            // the panels' sums on two of the group's lanes
             double res = 0, err = 0, ra, rc = 0;
-            if (on && (gi & 1) == 0)
+            if (on && gi % (kSolveLanes / 2) == 0)
                 gk_sum<21>(gi ? b1 : a1, gi ? b2 : b1, vals + (gi ? 21 : 0), res, err, ra, rc);
-            const double res2 = __shfl_sync(0xffffffffu, res, lead + 2), err2 = __shfl_sync(0xffffffffu, err, lead + 2),
-                         rc2 = __shfl_sync(0xffffffffu, rc, lead + 2);
+            const double res2 = __shfl_sync(0xffffffffu, res, lead + kSolveLanes / 2), err2 = __shfl_sync(0xffffffffu, err, lead + kSolveLanes / 2),
+                         rc2 = __shfl_sync(0xffffffffu, rc, lead + kSolveLanes / 2);
             if (on && gi == 0) {
                 double r = 0;
                 bool full = false;

@@ -494,9 +494,8 @@ int fj_ctx_create(int device, fj_ctx **out)
         return FJ_ERR_CUDA;
     }
     c->stream = c->own;
-    // The phase-space kernels keep the QAGS interval list on the per-thread
-    // call stack (about 5.5 KB, ptxas "cumulative stack size"); the function
-    // attributes do not report call-stack frames, so the floor is explicit.
+    // The function attributes do not report the frames of called device
+    // functions, so the floor is explicit.
     size_t need = moments_local_bytes();
     for (size_t n2 : {multipole_local_bytes(), moments_mixed_local_bytes(), delta_local_bytes(), los_local_bytes()})
         if (n2 > need) need = n2;

@@ -2,10 +2,9 @@
 // multipole potential and gradient, Brent roots, QUADPACK QAGS, the Staeckel
 // fudge and the distribution function.
 //
-// Written for one thread per (meridional point, velocity node).  Everything
-// a thread needs lives in registers; the only indexed per-thread storage is
-// the QAGS interval list, which the compiler keeps in local memory and only
-// touches when an integral is subdivided.
+// The building blocks of the kernels: which threads work on an orbit, and where
+// its interval lists live, is theirs (fj_solve64.cuh: groups of lanes;
+// fj_qags_warp.cuh: a warp).
 //
 // Arithmetic follows the reference's expression order where that is free,
 // so FP64 results agree with the reference to rounding level.  Deliberate
@@ -43,7 +42,7 @@ constexpr double kTINY = 1e-12;
 constexpr int kMaxPoly = 24;      // largest supported npoly (l_max = 46)
 constexpr int kLoopCap = 4096;    // cap on every bracketing loop (unbounded in the reference)
 constexpr int kRootMaxIt = 200;   // cap on Brent iterations
-constexpr int kQagsCap = 128;     // interval capacity of the per-thread QAGS list
+constexpr int kQagsCap = 128;     // interval capacity of a momentum integral's QAGS list
 
 // status bits of one phase-space evaluation
 constexpr unsigned kFailBracket = 1u;  // a bracketing loop hit kLoopCap
@@ -645,15 +644,6 @@ FJ_UNROLL
     abserr = rescale_err(err, ra, rasc);
 }
 
-template <int RULE, class F>
-FJ_HD void gk_panel(F &f, double a, double b, double &res, double &abserr, double &resabs, double &resasc)
-{
-    double v[GKRule<RULE>::npts];
-FJ_UNROLL
-    for (int e = 0; e < GKRule<RULE>::npts; e++) v[e] = f(gk_abscissa<RULE>(a, b, e));
-    gk_sum<RULE>(a, b, v, res, abserr, resabs, resasc);
-}
-
 // Wynn epsilon step (DQELG); tab[0..n-1] with room for n+2
 FJ_HD void qelg(double *tab, int &n_io, double *res3, int &nres, double &result, double &abserr)
 {
@@ -732,7 +722,7 @@ FJ_HD int qags_head(double res0, double err0, double resabs0, double resasc0, do
 
 // The rest of QAGS after a first panel (res0, err0, resabs0) that did not
 // finish it: Pn::two evaluates the two half-interval panels of each bisection
-// (LanePanels64: one thread; the Poisson kernel's warp form: one warp).
+// (fj_qags_warp.cuh: a warp).
 template <int RULE, class Pn>
 FJ_HDNI int qags_rest(Pn &pn, double a, double b, double res0, double err0, double resabs0, double epsabs,
                       double epsrel, int limit, double &result, double &abserr, unsigned &fail, const QagsWs &ws)
@@ -914,29 +904,6 @@ FJ_HDNI int qags_rest(Pn &pn, double a, double b, double res0, double err0, doub
     }
     if (ier > 2) ier--;
     return ier;
-}
-
-template <int RULE, class F>
-struct LanePanels64 {
-    F &f;
-    FJ_HD void two(double a1, double b1, double a2, double b2, double &r1, double &e1, double &ra1, double &rc1,
-                   double &r2, double &e2, double &ra2, double &rc2)
-    {
-        gk_panel<RULE>(f, a1, b1, r1, e1, ra1, rc1);
-        gk_panel<RULE>(f, a2, b2, r2, e2, ra2, rc2);
-    }
-};
-
-template <int RULE, class F>
-FJ_HDNI int qags(F &f, double a, double b, double epsabs, double epsrel, int limit, double &result,
-               double &abserr, unsigned &fail, const QagsWs &ws)
-{
-    double res0, err0, resabs0, resasc0;
-    gk_panel<RULE>(f, a, b, res0, err0, resabs0, resasc0);
-    const int h = qags_head(res0, err0, resabs0, resasc0, epsabs, epsrel, limit, result, abserr);
-    if (h >= 0) return h;
-    LanePanels64<RULE, F> pn{f};
-    return qags_rest<RULE>(pn, a, b, res0, err0, resabs0, epsabs, epsrel, limit, result, abserr, fail, ws);
 }
 
 // ----------------------------------------------------------------------------
@@ -1129,34 +1096,12 @@ FJ_HDNI double get_turn_v(Fudge &o, double vtry)
     return r;
 }
 
-// Momentum-integral rule: QAGS as wrp_GSLinteg (include/Utils.h:173-185) or fixed GL.
+// Momentum-integral rule: QAGS as wrp_GSLinteg (include/Utils.h:173-185) or fixed
+// Gauss-Legendre.
 struct GLRule {
     int n;              // 0 = QAGS
     const double *x01;  // nodes on (0,1)
     const double *w01;  // weights on (0,1)
-};
-
-template <class F>
-FJ_HDNI double mom_integral(F &f, double b, const GLRule &gl, unsigned &fail)
-{
-    if (gl.n <= 0) {
-        double al[kQagsCap], bl[kQagsCap], rl[kQagsCap], el[kQagsCap];
-        int io[kQagsCap];
-        const QagsWs ws{al, bl, rl, el, io, kQagsCap};
-        double r, e;
-        qags<21>(f, 0.0, b, 1e-5, 1e-3, 1000, r, e, fail, ws);
-        return r;
-    }
-    double s = 0;
-    for (int i = 0; i < gl.n; i++) s += (b * gl.w01[i]) * f(b * gl.x01[i]);
-    return s;
-}
-
-// The momentum integrals of one thread: QAGS or fixed Gauss-Legendre (mom_integral)
-struct SerialMomInt {
-    const GLRule *gl;
-    template <class F>
-    FJ_HD double operator()(F &f, double b, unsigned &fail) const { return mom_integral(f, b, *gl, fail); }
 };
 
 // One phase-space point up to the reference point of the u-equation: uvOrb ctor
@@ -1265,12 +1210,6 @@ FJ_HDNI bool fudge_actions_with(const PotView &P, double Delta, double R, double
     }
     fail |= o.fail;
     return true;
-}
-
-FJ_HDNI bool fudge_actions(const PotView &P, double Delta, double R, double z, double Phi, double pR,
-                         double vphi, double pz, const GLRule &gl, double &Jr, double &Jz, unsigned &fail)
-{
-    return fudge_actions_with(P, Delta, R, z, Phi, pR, vphi, pz, SerialMomInt{&gl}, Jr, Jz, fail);
 }
 
 // ----------------------------------------------------------------------------

@@ -38,11 +38,10 @@ inline int plain_chunk(long long npts, long long nq3, int most = kPlainChunk, in
     while (c > 128 && npts * ((nq3 + c - 1) / c) < items) c = c / 2 < 128 ? 128 : c / 2;
     return c;
 }
-// per-thread stack the kernels need: the QAGS interval list (kQagsCap entries
-// of four doubles and an int), the epsilon table and the call frames
+// per-thread stack floor: the function attributes do not report the frames of the
+// device functions a kernel calls (4.1 KB at most, by ptxas' "cumulative
+// stack size")
 constexpr size_t kStackBytes = 8192;
-static_assert(kQagsCap * (4 * sizeof(double) + sizeof(int)) + 52 * sizeof(double) + 1024 < kStackBytes,
-              "stack floor below the QAGS workspace");
 
 // Arguments of the phase-space (moment) kernel.  All pointers are device memory.
 struct MomentArgs {
@@ -220,7 +219,7 @@ struct DeferWork {
 constexpr int kScanChunk = 1024;  // blocks per chunk of the count scan
 constexpr int kMixedMaxNodes = 8192; // largest node range of one block (shared-memory list)
 FJ_HD int defer_words(int chunk) { return (chunk + 31) / 32; }  // bitmap words of one block
-constexpr int kMixedVariants = 8;    // builds of the mixed kernel (2 forms x 4 register budgets)
+constexpr int kMixedVariants = 8;    // configurations of the mixed kernels (2 turning-point x 4 integral builds)
 MixedSmem mixed_smem(const MomentArgs &a);
 size_t mixed_rec_bytes();      // per node of a slice
 size_t mixed_scratch_bytes();  // per block of the integration kernel

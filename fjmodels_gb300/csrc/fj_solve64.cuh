@@ -505,7 +505,7 @@ __device__ void solve_orbits64(const PotView &P, const PotFast &F, const GLRule 
         r.fjv = fudge_jv_factor(o);
         const unsigned todo = (fudge_ju_zero(o) ? 0u : kOrbitJu) | (fudge_jv_zero(o) ? 0u : kOrbitJv);
         r.todo = todo;
-        for (int kv = 0; kv < 2 && gl.n > 0; kv++) {  // fixed Gauss-Legendre integrals: on the spot (mom_integral)
+        for (int kv = 0; kv < 2 && gl.n > 0; kv++) {  // fixed Gauss-Legendre integrals: on the spot
             if (!(todo & (kv ? kOrbitJv : kOrbitJu))) continue;
             const double b = kv ? kPIH : kPI;
             double s = 0;

@@ -105,7 +105,7 @@ int ensure(fj_ctx *ctx, DevBuf &b, size_t bytes)
 // buffer: bitmaps | counts | offsets | scan carries | list (nodes, blocks,
 // moments).  The list holds 1/256 of the nodes (at least 64 Ki, at most 4 Mi
 // entries); a launch that leaves more is still exact (the extra nodes are
-// solved by their block's adding thread), only slower.
+// solved one after another by their item's block), only slower.
 int defer_setup(fj_ctx *ctx, long long nblocks, size_t words, long long nodes, DeferWork &dw, unsigned *&bitmaps)
 {
     const long long nchunks = (nblocks + kScanChunk - 1) / kScanChunk;
@@ -389,7 +389,7 @@ int build_args(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delta
     }
     const long long nq3 = (long long)rule->nq * rule->nq * rule->nq;
     a.mixed_chunk = plain_chunk(npts, nq3, ctx->mixed_chunk, kMixedItems);
-    if (!mixed && (rc = trig_table(ctx, &a.trig))) return rc;
+    if ((rc = trig_table(ctx, &a.trig))) return rc;
     a.plain_chunk = plain_chunk(npts, nq3);
     a.blocks_per_point =
         mixed ? mixed_blocks_per_point(nq3, a.mixed_chunk) : (int)((nq3 + a.plain_chunk - 1) / a.plain_chunk);

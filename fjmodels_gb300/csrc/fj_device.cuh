@@ -3,8 +3,7 @@
 // fudge and the distribution function.
 //
 // The building blocks of the kernels: which threads work on an orbit, and where
-// its interval lists live, is theirs (fj_solve64.cuh: groups of lanes;
-// fj_qags_warp.cuh: a warp).
+// its interval lists live, is theirs (fj_solve64.cuh).
 //
 // Arithmetic follows the reference's expression order where that is free,
 // so FP64 results agree with the reference to rounding level.  Deliberate
@@ -526,10 +525,10 @@ FJ_HDNI unsigned brent_root(F &f, double lo, double hi, double &root)
 }
 
 // ----------------------------------------------------------------------------
-// QUADPACK QAGS (Piessens et al. 1983: DQAGSE, DQK21/DQK15, DQPSRT, DQELG;
-// the epsilon table's result count advances only on completed updates, as in
-// GSL).  The interval list holds kQagsCap entries; a full list stops the
-// refinement, keeps the current estimate and sets kFailQuad.
+// QUADPACK QAGS (Piessens et al. 1983: DQAGSE, DQK21/DQK15): the panels and the
+// decision on the first one.  The bisections (fj_group_qags.cuh) keep a list of
+// kQagsCap intervals; a full list stops the refinement, keeps the current estimate
+// and sets kFailQuad.
 // ----------------------------------------------------------------------------
 FJ_HD double rescale_err(double err, double resabs, double resasc)
 {
@@ -644,72 +643,9 @@ FJ_UNROLL
     abserr = rescale_err(err, ra, rasc);
 }
 
-// Wynn epsilon step (DQELG); tab[0..n-1] with room for n+2
-FJ_HD void qelg(double *tab, int &n_io, double *res3, int &nres, double &result, double &abserr)
-{
-    const int n = n_io - 1;
-    const double current = tab[n];
-    result = current;
-    abserr = DBL_MAX;
-    if (n < 2) return;
-    tab[n + 2] = tab[n];
-    tab[n] = DBL_MAX;
-    const int newelm = n / 2;
-    int n_final = n;
-    for (int i = 0; i < newelm; i++) {
-        double res = tab[n - 2 * i + 2];
-        const double e0 = tab[n - 2 * i - 2], e1 = tab[n - 2 * i - 1], e2 = res;
-        const double e1abs = fabs(e1);
-        const double delta2 = e2 - e1, err2 = fabs(delta2);
-        const double tol2 = (fabs(e2) > e1abs ? fabs(e2) : e1abs) * DBL_EPSILON;
-        const double delta3 = e1 - e0, err3 = fabs(delta3);
-        const double tol3 = (e1abs > fabs(e0) ? e1abs : fabs(e0)) * DBL_EPSILON;
-        if (err2 <= tol2 && err3 <= tol3) {
-            const double rel = 5 * DBL_EPSILON * fabs(res);
-            result = res;
-            abserr = (err2 + err3) > rel ? (err2 + err3) : rel;
-            return;
-        }
-        const double e3 = tab[n - 2 * i];
-        tab[n - 2 * i] = e1;
-        const double delta1 = e1 - e3, err1 = fabs(delta1);
-        const double tol1 = (e1abs > fabs(e3) ? e1abs : fabs(e3)) * DBL_EPSILON;
-        if (err1 <= tol1 || err2 <= tol2 || err3 <= tol3) { n_final = 2 * i; break; }
-        const double ss = (1 / delta1 + 1 / delta2) - 1 / delta3;
-        if (fabs(ss * e1) <= 0.0001) { n_final = 2 * i; break; }
-        res = e1 + 1 / ss;
-        tab[n - 2 * i] = res;
-        const double error = err2 + fabs(res - e2) + err3;
-        if (error <= abserr) { abserr = error; result = res; }
-    }
-    if (n_final == 49) n_final = 48;
-    if (n % 2 == 1) { for (int i = 0; i <= newelm; i++) tab[1 + 2 * i] = tab[2 * i + 3]; }
-    else { for (int i = 0; i <= newelm; i++) tab[2 * i] = tab[2 * i + 2]; }
-    if (n != n_final) for (int i = 0; i <= n_final; i++) tab[i] = tab[n - n_final + i];
-    n_io = n_final + 1;
-    if (nres < 3) { res3[nres] = result; abserr = DBL_MAX; }
-    else {
-        abserr = fabs(result - res3[2]) + fabs(result - res3[1]) + fabs(result - res3[0]);
-        res3[0] = res3[1]; res3[1] = res3[2]; res3[2] = result;
-    }
-    nres += 1;
-    const double rel = 5 * DBL_EPSILON * fabs(result);
-    if (rel > abserr) abserr = rel;
-}
-
-// Interval list of one QAGS call: per-thread local arrays in the phase-space
-// kernel, a slice of context scratch in the Poisson kernel.
-struct QagsWs {
-    double *alist, *blist, *rlist, *elist;
-    int *iord;
-    int cap;
-};
-
-// QAGS on [a,b].  limit is the reference's nominal limit (it only enters the
-// ordering rule of DQPSRT); ws.cap is the storage actually available.
-// Returns the QUADPACK error class (0 = success); fail gets kFailQuad on overflow.
-// The first panel's early exits: returns the QUADPACK error class of a
-// finished call (result and abserr set), or -1 when the bisection goes on.
+// QAGS on [a,b] after its first panel: returns the QUADPACK error class of a call
+// that the panel finishes (result and abserr set), or -1 when bisections follow
+// (fj_group_qags.cuh).  limit is the reference's nominal limit.
 FJ_HD int qags_head(double res0, double err0, double resabs0, double resasc0, double epsabs, double epsrel, int limit,
                     double &result, double &abserr)
 {
@@ -718,192 +654,6 @@ FJ_HD int qags_head(double res0, double err0, double resabs0, double resasc0, do
     if ((err0 <= tol && err0 != resasc0) || err0 == 0.0) { result = res0; abserr = err0; return 0; }
     if (limit == 1) { result = res0; abserr = err0; return 1; }
     return -1;
-}
-
-// The rest of QAGS after a first panel (res0, err0, resabs0) that did not
-// finish it: Pn::two evaluates the two half-interval panels of each bisection
-// (fj_qags_warp.cuh: a warp).
-template <int RULE, class Pn>
-FJ_HDNI int qags_rest(Pn &pn, double a, double b, double res0, double err0, double resabs0, double epsabs,
-                      double epsrel, int limit, double &result, double &abserr, unsigned &fail, const QagsWs &ws)
-{
-    const int CAP = ws.cap;
-    double *alist = ws.alist, *blist = ws.blist, *rlist = ws.rlist, *elist = ws.elist;
-    int *iord = ws.iord;
-    double rlist2[52], res3la[3];
-    int nres = 0, numrl2 = 1;
-    alist[0] = a; blist[0] = b; rlist[0] = res0; elist[0] = err0; iord[0] = 0;
-    rlist2[0] = res0;
-    double area = res0, errsum = err0, errmax = err0;
-    int maxerr = 0, nrmax = 0, last = 1, ier = 0;
-    double res_ext = res0, err_ext = DBL_MAX, correc = 0, ertest = 0, erlarg = 0, small = 0;
-    int ktmin = 0, ierro = 0;
-    bool extrap = false, noext = false, done_sum = false;
-    int iroff1 = 0, iroff2 = 0, iroff3 = 0;
-    const int ksgn = fabs(res0) >= (1 - 50 * DBL_EPSILON) * resabs0 ? 1 : -1;
-
-    for (last = 1; last < limit; last++) {
-        if (last >= CAP) { fail |= kFailQuad; last = CAP - 1; done_sum = true; break; }
-        const double a1 = alist[maxerr], b1 = 0.5 * (alist[maxerr] + blist[maxerr]);
-        const double a2 = b1, b2 = blist[maxerr];
-        const double erlast = errmax;
-        double area1, error1, ra1, rasc1, area2, error2, ra2, rasc2;
-        pn.two(a1, b1, a2, b2, area1, error1, ra1, rasc1, area2, error2, ra2, rasc2);
-        const double area12 = area1 + area2, erro12 = error1 + error2;
-        errsum = errsum + erro12 - errmax;
-        area = area + area12 - rlist[maxerr];
-        if (!(rasc1 == error1 || rasc2 == error2)) {
-            if (fabs(rlist[maxerr] - area12) <= 1e-5 * fabs(area12) && erro12 >= 0.99 * errmax) {
-                if (extrap) iroff2++; else iroff1++;
-            }
-            if (last > 9 && erro12 > errmax) iroff3++;
-        }
-        rlist[maxerr] = area1;
-        rlist[last] = area2;
-        const double errbnd = epsabs > epsrel * fabs(area) ? epsabs : epsrel * fabs(area);
-        if (iroff1 + iroff2 >= 10 || iroff3 >= 20) ier = 2;
-        if (iroff2 >= 5) ierro = 3;
-        if (last == limit - 1) ier = 1;
-        const double mx = fabs(a1) > fabs(b2) ? fabs(a1) : fabs(b2);
-        if (mx <= (1 + 100 * DBL_EPSILON) * (fabs(a2) + 1000 * DBL_MIN)) ier = 4;
-        if (!(error2 > error1)) {
-            alist[last] = a2; blist[maxerr] = b1; blist[last] = b2;
-            elist[maxerr] = error1; elist[last] = error2;
-        } else {
-            alist[maxerr] = a2; alist[last] = a1; blist[last] = b1;
-            rlist[maxerr] = area2; rlist[last] = area1;
-            elist[maxerr] = error2; elist[last] = error1;
-        }
-        {   // DQPSRT with 1-based positions
-            const int L = last + 1;
-            if (L <= 2) { iord[0] = 0; iord[1] = 1; }
-            else {
-                const double em = elist[maxerr];
-                int nr1 = nrmax + 1;
-                if (nr1 != 1) {
-                    const int ido = nr1 - 1;
-                    for (int i = 1; i <= ido; i++) {
-                        const int isucc = iord[nr1 - 2];
-                        if (em <= elist[isucc]) break;
-                        iord[nr1 - 1] = isucc;
-                        nr1--;
-                    }
-                }
-                int jupbn = L;
-                if (L > limit / 2 + 2) jupbn = limit + 3 - L;
-                const double errmin = elist[L - 1];
-                const int jbnd = jupbn - 1, ibeg = nr1 + 1;
-                int i = ibeg;
-                bool found = false;
-                if (ibeg <= jbnd) {
-                    for (i = ibeg; i <= jbnd; i++) {
-                        const int isucc = iord[i - 1];
-                        if (em >= elist[isucc]) { found = true; break; }
-                        iord[i - 2] = isucc;
-                    }
-                }
-                if (!found) { iord[jbnd - 1] = maxerr; iord[jupbn - 1] = L - 1; }
-                else {
-                    iord[i - 2] = maxerr;
-                    int k = jbnd;
-                    bool ins = false;
-                    for (int j = i; j <= jbnd; j++) {
-                        const int isucc = iord[k - 1];
-                        if (errmin < elist[isucc]) { iord[k] = L - 1; ins = true; break; }
-                        iord[k] = isucc;
-                        k--;
-                    }
-                    if (!ins) iord[i - 1] = L - 1;
-                }
-                nrmax = nr1 - 1;
-            }
-            maxerr = iord[nrmax];
-            errmax = elist[maxerr];
-        }
-        if (errsum <= errbnd) { done_sum = true; break; }
-        if (ier) break;
-        if (last == 1) {
-            small = fabs(b - a) * 0.375;
-            erlarg = errsum;
-            ertest = errbnd;
-            rlist2[1] = area; numrl2 = 2;
-            continue;
-        }
-        if (noext) continue;
-        erlarg -= erlast;
-        if (fabs(b1 - a1) > small) erlarg += erro12;
-        if (!extrap) {
-            if (fabs(blist[maxerr] - alist[maxerr]) > small) continue;
-            extrap = true;
-            nrmax = 1;
-        }
-        bool do_ext = true;
-        if (!(ierro == 3 || erlarg <= ertest)) {
-            int jupbnd = last + 1;
-            if (last + 1 > 2 + limit / 2) jupbnd = limit + 3 - (last + 1);
-            for (int k = nrmax + 1; k <= jupbnd; k++) {
-                maxerr = iord[nrmax];
-                errmax = elist[maxerr];
-                if (fabs(blist[maxerr] - alist[maxerr]) > small) { do_ext = false; break; }
-                nrmax++;
-            }
-        }
-        if (!do_ext) continue;
-        rlist2[numrl2] = area; numrl2++;
-        double reseps, abseps;
-        qelg(rlist2, numrl2, res3la, nres, reseps, abseps);
-        ktmin++;
-        if (ktmin > 5 && err_ext < 1e-3 * errsum) ier = 5;
-        if (abseps < err_ext) {
-            ktmin = 0;
-            err_ext = abseps;
-            res_ext = reseps;
-            correc = erlarg;
-            ertest = epsabs > epsrel * fabs(reseps) ? epsabs : epsrel * fabs(reseps);
-            if (err_ext <= ertest) break;
-        }
-        if (numrl2 == 1) noext = true;
-        if (ier == 5) break;
-        maxerr = iord[0];
-        errmax = elist[maxerr];
-        nrmax = 0;
-        extrap = false;
-        small *= 0.5;
-        erlarg = errsum;
-    }
-    bool take_sum = done_sum;
-    if (!done_sum) {
-        result = res_ext;
-        abserr = err_ext;
-        if (err_ext == DBL_MAX) take_sum = true;
-        else {
-            bool skip_div = false;
-            if (ier + ierro != 0) {
-                if (ierro == 3) err_ext += correc;
-                if (ier == 0) ier = 3;
-                if (res_ext != 0.0 && area != 0.0) {
-                    if (err_ext / fabs(res_ext) > errsum / fabs(area)) take_sum = true;
-                } else if (err_ext > errsum) take_sum = true;
-                else if (area == 0.0) skip_div = true;
-                abserr = err_ext;
-            }
-            if (!take_sum && !skip_div) {
-                const double mxa = fabs(res_ext) > fabs(area) ? fabs(res_ext) : fabs(area);
-                if (!(ksgn == -1 && mxa <= resabs0 * 0.01)) {
-                    const double ratio = res_ext / area;
-                    if (ratio < 0.01 || ratio > 100.0 || errsum > fabs(area)) ier = 6;
-                }
-            }
-        }
-    }
-    if (take_sum) {
-        double s = 0;
-        for (int k = 0; k <= last; k++) s += rlist[k];
-        result = s;
-        abserr = errsum;
-    }
-    if (ier > 2) ier--;
-    return ier;
 }
 
 // ----------------------------------------------------------------------------
@@ -968,47 +718,6 @@ struct Fudge {
 struct UturnF { const Fudge *o; FJ_HD double operator()(double x) const { return o->uturnfn(x); } };
 struct DuturnF { const Fudge *o; FJ_HD double operator()(double x) const { return o->duturnfn(x); } };
 struct VturnF { const Fudge *o; FJ_HD double operator()(double x) const { return o->vturnfn(x); } };
-struct JuIntF {
-    const Fudge *o;
-    FJ_HD double operator()(double psi) const
-    {
-        double sn, cs;
-        sincos(psi, &sn, &cs);
-        return sqrt(dmax(0., o->uturnfn(o->ubar - o->Deltau * cs))) * sn;
-    }
-};
-struct JvIntF {
-    const Fudge *o;
-    FJ_HD double operator()(double psi) const
-    {
-        double sn, cs;
-        sincos(psi, &sn, &cs);
-        return sqrt(dmax(0., o->vturnfn(kPIH - (kPIH - o->vturn) * cs))) * sn;
-    }
-};
-
-// uvOrb::Getu0 (uvOrb.cpp:109-129)
-FJ_HDNI void getu0(Fudge &o, double utry)
-{
-    DuturnF f{&o};
-    double ui = utry, uo = utry, dut = f(utry);
-    int it = 0;
-    if (dut > 0) {
-        while (dut > 0) {
-            ui = utry; utry *= 1.2; dut = f(utry);
-            if (++it > kLoopCap) { o.fail |= kFailBracket; break; }
-        }
-        uo = utry;
-    } else {
-        while (dut < 0) {
-            uo = utry; utry *= .8; dut = f(utry);
-            if (++it > kLoopCap) { o.fail |= kFailBracket; break; }
-        }
-        ui = utry;
-    }
-    o.fail |= brent_root(f, ui, uo, o.umid);
-}
-
 // uvOrb::GetTurnu (uvOrb.cpp:131-201)
 FJ_HDNI void get_turn_u(Fudge &o, double utry)
 {
@@ -1165,52 +874,12 @@ FJ_HDNI void fudge_constants(Fudge &o, double pu2, double pv2)
 
 constexpr double kUmidStart = 58;  // where getu0 starts (uvOrb.cpp:23)
 
-// One phase-space point on one thread: its constants and the turning points of Ju
-// and Jv into o (umid, uinner, uouter, ubar, Deltau, vturn; o.fail).  Returns
-// false for an unbound orbit.
-FJ_HDNI bool fudge_turning_points(const PotView &P, double Delta, double R, double z, double Phi, double pR,
-                                  double vphi, double pz, Fudge &o)
-{
-    double pu2, pv2;
-    if (!fudge_point(P, Delta, R, z, Phi, pR, vphi, pz, o, pu2, pv2)) return false;
-    getu0(o, kUmidStart);
-    fudge_constants(o, pu2, pv2);
-    get_turn_u(o, 1);
-    o.ubar = .5 * (o.uinner + o.uouter);
-    o.Deltau = .5 * (o.uouter - o.uinner);
-    o.vturn = get_turn_v(o, .5 * kPIH);
-    return true;
-}
-
 // whether Ju and Jv vanish (uvOrb.cpp:226-229, 247-249), and their factors
 // before the integrals (uvOrb.cpp:238, 256)
 FJ_HD bool fudge_ju_zero(const Fudge &o) { return fabs(o.uouter - o.uinner) < kTINY; }
 FJ_HD bool fudge_jv_zero(const Fudge &o) { return fabs(o.vturn - kPIH) < kTINY; }
 FJ_HD double fudge_ju_factor(const Fudge &o) { return sqrt(2.0) * o.Delta * o.Deltau; }
 FJ_HD double fudge_jv_factor(const Fudge &o) { return 2 * sqrt(2.0) * o.Delta * (kPIH - o.vturn); }
-
-// Actions of one phase-space point: the turning points, Ju and Jv with the
-// momentum integrals by mi(integrand, upper limit, fail).
-// Returns false for an unbound orbit (Jr = Jz = 1e31).
-template <class MI>
-FJ_HDNI bool fudge_actions_with(const PotView &P, double Delta, double R, double z, double Phi, double pR,
-                                double vphi, double pz, const MI &mi, double &Jr, double &Jz, unsigned &fail)
-{
-    Fudge o;
-    if (!fudge_turning_points(P, Delta, R, z, Phi, pR, vphi, pz, o)) { Jr = Jz = 1e31; return false; }
-    if (fudge_ju_zero(o)) Jr = 0;
-    else {
-        JuIntF fju{&o};
-        Jr = fudge_ju_factor(o) * mi(fju, kPI, o.fail) / kPI;
-    }
-    if (fudge_jv_zero(o)) Jz = 0;
-    else {
-        JvIntF fjv{&o};
-        Jz = fudge_jv_factor(o) * mi(fjv, kPIH, o.fail) / kPI;
-    }
-    fail |= o.fail;
-    return true;
-}
 
 // ----------------------------------------------------------------------------
 // focal distance and DF

@@ -10,7 +10,7 @@
 // With G = 4 the 42 points are 11 rounds (95 % of the lanes busy), an integral's
 // serial chain is a quarter as long, and a warp keeps 8 interval lists instead
 // of 32.  The function values enter the same sums in the same order as in the
-// one-thread forms (qags, qags_f), and the bookkeeping is theirs statement by
+// one-thread form (qags_f), and the bookkeeping is its, statement by
 // statement, so an integral has the same bits.
 //
 // The bookkeeping runs on the group's first lane only; the others receive the
@@ -48,7 +48,8 @@ struct QagsList {
     unsigned char iord[CAP];
 };
 
-// Wynn epsilon step (DQELG), as qelg / qelg_f
+// Wynn epsilon step (DQELG; tab[0..n-1] with room for n+2; the result count advances
+// only on completed updates, as in GSL), as qelg_f
 template <class T>
 __device__ __noinline__ void group_qelg(T *tab, int &n_io, T *res3, int &nres, T &result, T &abserr)
 {

@@ -58,7 +58,7 @@ struct MomentArgs {
     int npts;
     int blocks_per_point;
     int plain_chunk;         // FP64 form: nodes per work item (<= kPlainChunk)
-    const double2 *trig;     // FP64 form: sines and cosines of the quadrature angles (launch_trig_table)
+    const double2 *trig;     // sines and cosines of the FP64 quadrature angles (launch_trig_table)
     int mixed_chunk;         // mixed form: nodes per block (<= kMixedMaxNodes)
     float *jout;             // mixed form, optional: (Jr, Jz) of every bound node [npts][nq^3][2]
     double *partial;         // [npts][blocks_per_point][6]
@@ -205,8 +205,8 @@ constexpr int kMixedBlock = 128;     // threads per block of the mixed kernel
 // sums and records how many it left.  The FP64 pass (launch_deferred) then lists
 // every launch's left nodes compactly, block by block in node order (an
 // exclusive scan of the counts gives each block its offset), solves them all in
-// parallel, one thread per node, and adds each block's nodes to its partial
-// sums in list order: the same sums whatever order the threads ran in.
+// parallel, a block of two warps per node, and adds each item's nodes to its
+// partial sums in list order: the same sums whatever order the blocks ran in.
 struct DeferWork {
     int *count;      // [nblocks] the blocks' counts (the launch's defer_count arrays, in block order)
     int *offset;     // [nblocks] exclusive prefix of the blocks' counts
@@ -214,7 +214,7 @@ struct DeferWork {
     int *node;       // [cap] listed nodes (index within the point's nq^3 rule)
     int *block;      // [cap] global block index of each listed node
     double *mom;     // [cap][6] moment contributions of the listed nodes
-    int cap;         // list capacity; nodes beyond it are solved by their block's adding thread
+    int cap;         // list capacity; nodes beyond it are solved item by item
 };
 constexpr int kScanChunk = 1024;  // blocks per chunk of the count scan
 constexpr int kMixedMaxNodes = 8192; // largest node range of one block (shared-memory list)

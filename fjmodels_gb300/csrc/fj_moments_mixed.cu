@@ -13,7 +13,7 @@
 #include "fj_internal.h"
 #include "fj_mixed.cuh"
 #include "fj_order.cuh"
-#include "fj_qags_warp.cuh"
+#include "fj_solve64.cuh"
 
 namespace fj {
 
@@ -489,71 +489,232 @@ __global__ void __launch_bounds__(kMixedBlock, MINB) k_mixed_integrate(MomentArg
 }
 
 // ------------------------------------------------------ the FP64 pass
-// Over the nodes the mixed kernel left (launch_deferred): a scan of the
-// blocks' counts, the compact list, one thread per listed node, one thread per
-// block adding its nodes in list order.
+// Over the nodes the mixed kernels left (launch_deferred): a scan of the items'
+// counts, the compact list, a block of two warps per listed node, a warp per item
+// adding its nodes in list order.
+//
+// The pass lasts as long as its slowest node (64 to a few thousand of them, most
+// integrals of which fill an FP32 list: up to 127 bisections), so a node's solve is
+// built for latency: the two warps take the u and the v turning points and then
+// the Ju and the Jv integral side by side, the two u roots are two lanes', a
+// panel's values go over the lanes and its two sums over two of them, and the
+// integrands are those of fj_solve64.cuh (tables in shared memory, one
+// exponential, tabulated angles).  Measured (GB300): 1.5 ms for a 24x8 model's launch
+// (16^3 nodes), 4.1 ms for one of six 40x16 models; 2.2 and 5.5 ms with one warp per
+// node, its integrals one after the other in the reference's expressions.
 
-// the block's point, its potential and escape speed (as the mixed kernel's setup)
-__device__ void defer_point(const MomentArgs &a, int bid, double &R, double &z, double &Phi_h, double &Ve)
-{
-    const int nr = a.P.nr, p = bid / a.blocks_per_point;
-    if (a.Rz) { R = a.Rz[2 * p]; z = a.Rz[2 * p + 1]; }
-    else {
-        const int n = p / a.ngauss, gg = p % a.ngauss;
-        const double c = a.ci[gg], si = sqrt(1 - c * c);
-        R = a.P.ar[n] * si; z = a.P.ar[n] * c;
-    }
-    const PotView P{nr, a.P.npoly, a.P.ar, a.P.phil, a.P.Pr, a.P.Pr2};
-    const double rmax = a.P.ar[nr - 1];
-    Phi_h = pot_phi(P, R, z);
-    Ve = sqrt(-2 * (Phi_h - pot_phi(P, 10 * rmax, 10 * rmax)));
-}
+constexpr int kDeferBlock = 64;
+// FP64 tables of a model staged in shared memory: 80 radii with 8 multipoles fit;
+// a block of 32 KB leaves room for seven per SM.  A larger model's potential is
+// read from global memory and its integrands are the reference's expressions.
+constexpr int kDeferTable = 2560;
 
-// The momentum integrals of a warp: QAGS with the panels spread over the lanes
-struct WarpMomInt {
-    WarpQagsWs w;
-    int lane;
-    template <class F>
-    FJ_HD double operator()(F &f, double b, unsigned &fail) const
-    {
-#ifdef __CUDA_ARCH__
-        double r, e;
-        qags_warp<21>(f, 0.0, b, 1e-5, 1e-3, 1000, r, e, fail, w.ws(), w.buf, lane);
-        return r;
-#else
-        (void)f; (void)b; (void)fail;
-        return 0.;
-#endif
-    }
+struct DeferShared {
+    double tab[kDeferTable];
+    OrbitQags::List list[2];
+    double vals[2][43];
+    double pt[4];  // R, z, Phi, escape speed
+    OrbitRec rec;
 };
 
-// one left node with the plain form's FP64 solve (the actions with QAGS lists
-// of kQagsCap intervals, df_value) by a whole warp (every lane calls it with the
-// same node; the turning points run on every lane, the momentum integrals
-// spread their panels over the lanes): its six moment contributions
-__device__ void defer_solve(const MomentArgs &a, int bid, int node, double *c6, FailTally &tally,
-                            const WarpQagsWs &w, int lane)
+// the potential of item arguments a: staged unless cur is a's already (all threads)
+__device__ void defer_model(const MomentArgs &a, DeferShared &s, const MomentArgs *&cur, PotView &P, PotFast &F)
 {
-    double R, z, Phi_h, Ve;
-    defer_point(a, bid, R, z, Phi_h, Ve);
-    const PotView P{a.P.nr, a.P.npoly, a.P.ar, a.P.phil, a.P.Pr, a.P.Pr2};
+    if (cur == &a) return;
+    cur = &a;
+    const int nr = a.P.nr, npoly = a.P.npoly, nt = nr * npoly;
+    P = PotView{nr, npoly, a.P.ar, a.P.phil, a.P.Pr, a.P.Pr2, nullptr};
+    F = PotFast{nr, npoly, P.ar, P.phil, nullptr, nullptr, nullptr};
+    if (nr + 2 * nt + fast_table_size(nr, npoly) + interp_table_size(nr) > kDeferTable) return;
+    double *s_ar = s.tab, *s_phil = s_ar + nr, *s_Pr = s_phil + nt, *s_fast = s_Pr + nt,
+           *s_it = s_fast + fast_table_size(nr, npoly);
+    __syncthreads();
+    for (int i = threadIdx.x; i < nr; i += kDeferBlock) s_ar[i] = a.P.ar[i];
+    for (int i = threadIdx.x; i < nt; i += kDeferBlock) { s_phil[i] = a.P.phil[i]; s_Pr[i] = a.P.Pr[i]; }
+    __syncthreads();
+    interp_table(nr, s_ar, s_it, threadIdx.x, kDeferBlock);
+    __syncthreads();
+    P = PotView{nr, npoly, s_ar, s_phil, s_Pr, a.P.Pr2, s_it};
+    F = fast_tables(P, s_fast);
+    __syncthreads();
+}
+
+// QAGS of r's Ju or Jv integrand by a warp (all lanes; valid on lane 0)
+__device__ double warp_orbit_integral(const PotView &P, const PotFast &F, const OrbitRec &r, bool kv, const double2 *trig,
+                                      OrbitQags::List &L, double *vals, bool &full)
+{
+    const int lane = threadIdx.x & 31;
+    const double epsabs = 1e-5, epsrel = 1e-3;  // wrp_GSLinteg, include/Utils.h:173-185
+    double a1 = 0., b2 = kv ? kPIH : kPI, result = 0;
+    unsigned heap = 1;
+    bool run = false;
+    OrbitQags st;
+    if (lane < 21) {
+        double sn, cs;
+        panel_sincos(trig, kv, 1u, a1, b2, lane, sn, cs);
+        vals[lane] = orbit_integrand(P, F, r, kv, sn, cs);
+    }
+    __syncwarp();
+    if (lane == 0) {
+        double res, err, ra, rc, ae;
+        gk_sum<21>(a1, b2, vals, res, err, ra, rc);
+        run = qags_head(res, err, ra, rc, epsabs, epsrel, 1000, result, ae) < 0;
+        if (run) st.begin(L, a1, b2, res, err);
+    }
+    for (;;) {
+        if (!__shfl_sync(0xffffffffu, run ? 1 : 0, 0)) return result;
+        a1 = __shfl_sync(0xffffffffu, a1, 0);
+        b2 = __shfl_sync(0xffffffffu, b2, 0);
+        heap = __shfl_sync(0xffffffffu, heap, 0);
+        const double b1 = 0.5 * (a1 + b2);
+        const unsigned h1 = heap < (1u << 30) ? 2 * heap : 0u, h2 = h1 ? h1 + 1u : 0u;
+        for (int e = lane; e < 42; e += 32) {
+            const bool second = e >= 21;
+            double sn, cs;
+            panel_sincos(trig, kv, second ? h2 : h1, second ? b1 : a1, second ? b2 : b1, second ? e - 21 : e, sn, cs);
+            vals[e] = orbit_integrand(P, F, r, kv, sn, cs);
+        }
+        __syncwarp();
+        double res = 0, err = 0, ra, rc = 0;
+        if (lane < 2) gk_sum<21>(lane ? b1 : a1, lane ? b2 : b1, vals + 21 * lane, res, err, ra, rc);
+        const double res2 = __shfl_sync(0xffffffffu, res, 1), err2 = __shfl_sync(0xffffffffu, err, 1),
+                     rc2 = __shfl_sync(0xffffffffu, rc, 1);
+        if (lane == 0) {
+            if (st.update(L, res, err, rc, res2, err2, rc2, epsabs, epsrel, result, full)) run = false;
+            else {
+                a1 = L.iv[st.maxerr].a;
+                b2 = L.iv[st.maxerr].b;
+                heap = L.heap[st.maxerr];
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// one left node's FP64 solve (the turning points of the plain form, QAGS lists of
+// kQagsCap intervals, df_value) by the block: its six moment contributions and
+// status on thread 0
+__device__ void defer_solve(const MomentArgs &a, int bid, int node, const PotView &P, const PotFast &F, DeferShared &s,
+                            double *c6, FailTally &tally)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, p = bid / a.blocks_per_point;
+    OrbitRec &rec = s.rec;
+    __syncthreads();  // the previous node's record is free
+    if (warp == 0) {
+        double R, z;  // the point, as the mixed kernels' setup
+        if (a.Rz) { R = a.Rz[2 * p]; z = a.Rz[2 * p + 1]; }
+        else {
+            const int n = p / a.ngauss, gg = p % a.ngauss;
+            const double c = a.ci[gg], si = sqrt(1 - c * c);
+            R = P.ar[n] * si; z = P.ar[n] * c;
+        }
+        const double far = 10 * P.ar[P.nr - 1];
+        const double phi = pot_phi(P, lane == 1 ? far : R, lane == 1 ? far : z);
+        const double Phi_h = __shfl_sync(0xffffffffu, phi, 0), Ve = sqrt(-2 * (Phi_h - __shfl_sync(0xffffffffu, phi, 1)));
+        if (lane == 0) { s.pt[0] = R; s.pt[1] = z; s.pt[2] = Phi_h; s.pt[3] = Ve; }
+    }
+    __syncthreads();
+    const double R = s.pt[0], z = s.pt[1], Phi_h = s.pt[2], Ve = s.pt[3];
     const int nq = a.nq, nq2 = nq * nq;
     const int i = node / nq2, j = (node / nq) % nq, l = node % nq;
     const double V0 = 1e-6 + Ve * a.xq[i], V1 = 1e-6 + Ve * a.xq[j], V2 = 1e-6 + Ve * a.xq[l];
-    const double H = .5 * (V0 * V0 + V1 * V1 + V2 * V2) + Phi_h;
-    unsigned fail = 0;
-    double Jr, Jz;
-    fudge_actions_with(P, deltafn(a.Eg, a.Dg, a.ngrid, H), R, z, Phi_h, V0, V1, V2, WarpMomInt{w, lane}, Jr, Jz,
-                       fail);
+    if (warp == 0) {  // the constants of its equations
+        Fudge o;
+        double pu2, pv2;
+        const double H = .5 * (V0 * V0 + V1 * V1 + V2 * V2) + Phi_h;
+        const bool bound = fudge_point(P, deltafn(a.Eg, a.Dg, a.ngrid, H), R, z, Phi_h, V0, V1, V2, o, pu2, pv2);
+        if (bound) {
+            U0Walk w;
+            w.begin();
+            while (!w.step(o)) {}
+            BrentState b;
+            b.begin(w.ui, w.uo);
+            while (!b.feed(o.duturnfn(b.x))) {}
+            o.umid = b.root;
+            o.fail |= b.fail;
+            fudge_constants(o, pu2, pv2);
+        }
+        if (lane == 0) {
+            rec.o = o;
+            rec.todo = bound ? kOrbitBound : 0u;
+            rec.Jr = rec.Jz = bound ? 0. : 1e31;
+            rec.rootfail[0] = rec.rootfail[1] = rec.rootfail[2] = 0;
+            rec.full[0] = rec.full[1] = 0;
+        }
+    }
+    __syncthreads();
+    if (rec.todo & kOrbitBound) {
+        {
+            Fudge o = rec.o;
+            o.fail = 0;
+            __syncthreads();  // the turning points below go to the record
+            if (warp == 0) {
+                UWalk w;
+                w.begin();
+                while (!w.step(o)) {}
+                double root = w.uin;
+                unsigned fail = o.fail;
+                if (!w.degenerate) {  // the inner root on even lanes, the outer one on odd lanes
+                    BrentState b;
+                    b.begin(lane & 1 ? w.u2 : w.uin, lane & 1 ? w.uout : w.u1);
+                    while (!b.feed(o.uturnfn(b.x))) {}
+                    root = b.root;
+                    fail |= b.fail;
+                }
+                __syncwarp();
+                const double outer = __shfl_sync(0xffffffffu, root, 1);
+                fail |= __shfl_sync(0xffffffffu, fail, 1);
+                if (lane == 0) {
+                    Fudge &c = rec.o;
+                    c.uinner = root; c.uouter = outer;
+                    c.ubar = .5 * (root + outer);
+                    c.Deltau = .5 * (outer - root);
+                    rec.fju = fudge_ju_factor(c);
+                    rec.rootfail[0] = fail;
+                }
+            } else {
+                VWalk v;
+                v.begin();
+                while (!v.step(o)) {}
+                double vt = v.turn;
+                unsigned fail = o.fail;
+                if (!v.limit) {
+                    BrentState b;
+                    b.begin(v.vbot < v.vtop ? v.vbot : v.vtop, v.vbot < v.vtop ? v.vtop : v.vbot);
+                    while (!b.feed(o.vturnfn(b.x))) {}
+                    vt = b.root;
+                    fail |= b.fail;
+                }
+                if (lane == 0) {
+                    rec.o.vturn = vt;
+                    rec.w = kPIH - vt;
+                    rec.fjv = fudge_jv_factor(rec.o);
+                    rec.rootfail[2] = fail;
+                }
+            }
+        }
+        __syncwarp();  // a warp's integral needs its own turning points only
+        const bool kv = warp != 0;
+        if (!(kv ? fudge_jv_zero(rec.o) : fudge_ju_zero(rec.o))) {
+            bool full = false;
+            const double r = warp_orbit_integral(P, F, rec, kv, a.trig, s.list[warp], s.vals[warp], full);
+            if (lane == 0) {
+                if (kv) rec.Jz = rec.fjv * r / kPI; else rec.Jr = rec.fju * r / kPI;
+                if (full) rec.full[warp] = 1;
+            }
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x > 0) return;
+    const double Jr = rec.Jr, Jz = rec.Jz;
+    unsigned fail = rec.todo & kOrbitBound ? rec.status() : 0u;
     double DF = df_value(a.df, P, R, Jr, Jz, R * V1, fail);
     if (fail & (kFailBracket | kFailRoot)) DF = 0.;
-    if (lane == 0) {
-        tally.add(fail);
-        if (a.jout) {
-            float *jo = a.jout + ((size_t)(bid / a.blocks_per_point) * nq2 * nq + node) * 2;
-            jo[0] = (float)Jr;
-            jo[1] = (float)Jz;
-        }
+    tally.add(fail);
+    if (a.jout) {
+        float *jo = a.jout + ((size_t)p * nq2 * nq + node) * 2;
+        jo[0] = (float)Jr;
+        jo[1] = (float)Jz;
     }
     const double jd = (a.wq[i] * a.wq[j] * a.wq[l]) * (Ve * Ve * Ve * DF);
     c6[0] = jd; c6[1] = jd * V1; c6[2] = jd * V0 * V0;
@@ -652,80 +813,77 @@ __global__ void __launch_bounds__(32 * kListWarps) k_defer_list(MomentArgs a0, M
     }
 }
 
-// one warp per listed node (grid-stride over the launch's total)
-constexpr int kSolveWarps = 4;
-__global__ void __launch_bounds__(32 * kSolveWarps) k_defer_solve(MomentArgs a0, MomentBatch batch, DeferWork dw,
-                                                                   int nchunks)
+// a block per listed node (grid-stride over the launch's total); nodes beyond the
+// list's capacity by their item, in node order, into its partial sums
+__global__ void __launch_bounds__(kDeferBlock) k_defer_solve(MomentArgs a0, MomentBatch batch, DeferWork dw, int nblocks,
+                                                             int nchunks)
 {
-    __shared__ double s_list[kSolveWarps][4 * kQagsCap];
-    __shared__ int s_iord[kSolveWarps][kQagsCap];
-    __shared__ double s_buf[kSolveWarps][42];
-    const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
-    const WarpQagsWs w{s_list[wq], s_iord[wq], s_buf[wq], kQagsCap};
-    const int total = min(dw.chunk_sum[nchunks], dw.cap);
+    __shared__ __align__(128) unsigned char raw[sizeof(DeferShared)];
+    DeferShared &s = *(DeferShared *)raw;
+    const int total = dw.chunk_sum[nchunks], listed = min(total, dw.cap);
+    const MomentArgs *cur = nullptr;
+    PotView P;
+    PotFast F;
     FailTally tally;
     unsigned solved = 0;
     unsigned long long *counters = a0.counters;
-    for (int e = blockIdx.x * kSolveWarps + wq; e < total; e += gridDim.x * kSolveWarps) {
+    for (int e = blockIdx.x; e < listed; e += gridDim.x) {
         int bid;
         const MomentArgs &a = block_args(a0, batch, dw.block[e], bid);
         counters = a.counters;
+        defer_model(a, s, cur, P, F);
         double c6[6];
-        defer_solve(a, bid, dw.node[e], c6, tally, w, lane);
-        if (lane == 0) {
+        defer_solve(a, bid, dw.node[e], P, F, s, c6, tally);
+        if (threadIdx.x == 0) {
             for (int q = 0; q < 6; q++) dw.mom[(size_t)e * 6 + q] = c6[q];
             solved++;
         }
     }
-    if (lane == 0) add_tally(counters, tally, solved);
+    for (int g = blockIdx.x; total > dw.cap && g < nblocks; g += gridDim.x) {
+        const int cnt = dw.count[g], off = dw.offset[g];
+        if (off + cnt <= dw.cap) continue;
+        int bid;
+        const MomentArgs &a = block_args(a0, batch, g, bid);
+        counters = a.counters;
+        defer_model(a, s, cur, P, F);
+        const long long nq3 = (long long)a.nq * a.nq * a.nq;
+        const int n0 = (int)((bid % a.blocks_per_point) * nq3 / a.blocks_per_point);
+        const unsigned *bits = a.defer + (size_t)bid * defer_words(a.mixed_chunk);
+        double msum[6] = {0, 0, 0, 0, 0, 0};
+        for (int k = max(0, dw.cap - off); k < cnt; k++) {  // the item's k-th left node, from its bitmap
+            int r = k, wd = 0;
+            while (r >= __popc(bits[wd])) r -= __popc(bits[wd++]);
+            unsigned word = bits[wd];
+            for (int t = 0; t < r; t++) word &= word - 1;
+            double c6[6];
+            defer_solve(a, bid, n0 + wd * 32 + (__ffs((int)word) - 1), P, F, s, c6, tally);
+            if (threadIdx.x == 0) {
+                for (int q = 0; q < 6; q++) msum[q] += c6[q];
+                solved++;
+            }
+        }
+        if (threadIdx.x == 0)
+            for (int q = 0; q < 6; q++) a.partial[(size_t)bid * 6 + q] += msum[q];
+    }
+    if (threadIdx.x == 0) add_tally(counters, tally, solved);
 }
 
-// one warp per block: its listed nodes added in list order by lane 0 (nodes
-// beyond the list's capacity solved here by the warp, in node order)
+// a warp per item: its listed nodes added in list order, a moment per lane
 constexpr int kAddWarps = 4;
 __global__ void __launch_bounds__(32 * kAddWarps) k_defer_add(MomentArgs a0, MomentBatch batch, DeferWork dw,
                                                                int nblocks)
 {
-    __shared__ double s_list[kAddWarps][4 * kQagsCap];
-    __shared__ int s_iord[kAddWarps][kQagsCap];
-    __shared__ double s_buf[kAddWarps][42];
-    const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
-    const int g = blockIdx.x * kAddWarps + wq;
-    if (g >= nblocks) return;  // the whole warp
+    const int lane = threadIdx.x & 31;
+    const int g = blockIdx.x * kAddWarps + (threadIdx.x >> 5);
+    if (g >= nblocks) return;
     const int cnt = dw.count[g];
-    if (cnt == 0) return;
+    if (cnt == 0 || lane >= 6) return;
     int bid;
     const MomentArgs &a = block_args(a0, batch, g, bid);
-    const int off = dw.offset[g];
-    const WarpQagsWs w{s_list[wq], s_iord[wq], s_buf[wq], kQagsCap};
-    double msum[6] = {0, 0, 0, 0, 0, 0};
-    FailTally tally;
-    unsigned solved = 0;
-    for (int k = 0; k < cnt; k++) {
-        const int e = off + k;
-        if (e < dw.cap) {
-            for (int q = 0; q < 6; q++) msum[q] += dw.mom[(size_t)e * 6 + q];
-            continue;
-        }
-        // past the list: the block's k-th left node, from its bitmap
-        const int nw = defer_words(a.mixed_chunk), B = a.blocks_per_point;
-        const long long nq3 = (long long)a.nq * a.nq * a.nq;
-        const int n0 = (int)((bid % B) * nq3 / B);
-        const unsigned *bits = a.defer + (size_t)bid * nw;
-        int r = k, wd = 0;
-        while (r >= __popc(bits[wd])) r -= __popc(bits[wd++]);
-        unsigned word = bits[wd];
-        for (int t = 0; t < r; t++) word &= word - 1;
-        double c6[6];
-        defer_solve(a, bid, n0 + wd * 32 + (__ffs((int)word) - 1), c6, tally, w, lane);
-        solved++;
-        for (int q = 0; q < 6; q++) msum[q] += c6[q];
-    }
-    if (lane == 0) {
-        double *pt = a.partial + (size_t)bid * 6;
-        for (int q = 0; q < 6; q++) pt[q] += msum[q];
-        add_tally(a.counters, tally, solved);
-    }
+    const int off = dw.offset[g], last = min(off + cnt, dw.cap);
+    double msum = 0;
+    for (int e = off; e < last; e++) msum += dw.mom[(size_t)e * 6 + lane];
+    a.partial[(size_t)bid * 6 + lane] += msum;
 }
 
 static cudaError_t launch_deferred(const MomentArgs &a, const MomentBatch &b, long long nblocks, const DeferWork &dw,
@@ -739,7 +897,7 @@ static cudaError_t launch_deferred(const MomentArgs &a, const MomentBatch &b, lo
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    k_defer_solve<<<4 * (nsm > 0 ? nsm : 1), 32 * kSolveWarps, 0, s>>>(a, b, dw, nchunks);
+    k_defer_solve<<<16 * (nsm > 0 ? nsm : 1), kDeferBlock, 0, s>>>(a, b, dw, nb, nchunks);
     k_defer_add<<<(nb + kAddWarps - 1) / kAddWarps, 32 * kAddWarps, 0, s>>>(a, b, dw, nb);
     return cudaGetLastError();
 }

@@ -13,7 +13,7 @@
 //    bisection tree (its panels are the same for every orbit), the divisions of
 //    the potential by grid constants from reciprocals (PotView::itab), and what
 //    an orbit's equations repeat is computed once (Fudge::prepare).
-// The turning points are those of fudge_actions bit for bit (up to div_by's
+// The turning points are those of a point on one thread bit for bit (up to div_by's
 // rounding), the integrals to rounding (PotFast).
 // Measured (GB300), one thread per orbit with in-place divisions before, this
 // after: one iteration of a 16x6 model with 22^3 nodes 556 -> 160 ms, moments at

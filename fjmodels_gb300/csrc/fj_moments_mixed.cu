@@ -495,13 +495,16 @@ __global__ void __launch_bounds__(kMixedBlock, MINB) k_mixed_integrate(MomentArg
 //
 // The pass lasts as long as its slowest node (64 to a few thousand of them, most
 // integrals of which fill an FP32 list: up to 127 bisections), so a node's solve is
-// built for latency: the two warps take the u and the v turning points and then
-// the Ju and the Jv integral side by side, the two u roots are two lanes', a
+// built for latency: a bracket walk evaluates its next 32 positions at once
+// (warp_walk; walks had been three quarters of the time before the integrals), the
+// two warps take the u and the v turning points and then the Ju and the Jv integral
+// side by side, the two u roots are two lanes', a
 // panel's values go over the lanes and its two sums over two of them, and the
 // integrands are those of fj_solve64.cuh (tables in shared memory, one
-// exponential, tabulated angles).  Measured (GB300): 1.5 ms for a 24x8 model's launch
-// (16^3 nodes), 4.1 ms for one of six 40x16 models; 2.2 and 5.5 ms with one warp per
-// node, its integrals one after the other in the reference's expressions.
+// exponential, tabulated angles).  Measured (GB300): 0.72 ms for a 24x8 model's
+// launch (16^3 nodes), 2.0 ms for one of six 40x16 models; 1.5 and 4.1 ms with the
+// walks a step at a time, 2.2 and 5.5 ms with one warp per node, its integrals one
+// after the other in the reference's expressions.
 
 constexpr int kDeferBlock = 64;
 // FP64 tables of a model staged in shared memory: 80 radii with 8 multipoles fit;
@@ -591,6 +594,139 @@ __device__ double warp_orbit_integral(const PotView &P, const PotFast &F, const 
     }
 }
 
+// A bracket walk by a warp: the positions x, next(x), next(next(x)), .. one per
+// lane, each reached by the walk's own steps, up to the first where stop holds.
+// x becomes that position, kept the one before it (unchanged if there is none), at
+// the lane that holds it; it counts the steps.  False beyond kLoopCap steps.
+template <class Next, class Stop>
+__device__ bool warp_walk(double &x, double &kept, int &at, int &it, Next next, Stop stop)
+{
+    const int lane = threadIdx.x & 31;
+    for (;;) {
+        double p = x;
+        for (int i = 0; i < lane; i++) p = next(p);
+        const unsigned m = __ballot_sync(0xffffffffu, stop(p));
+        if (m) {
+            at = __ffs((int)m) - 1;
+            if (at > 0) kept = __shfl_sync(0xffffffffu, p, at - 1);
+            x = __shfl_sync(0xffffffffu, p, at);
+            it += at;
+            return it <= kLoopCap;
+        }
+        kept = __shfl_sync(0xffffffffu, p, 31);
+        x = next(kept);
+        it += 32;
+        if (it > kLoopCap) return false;
+    }
+}
+
+// U0Walk by a warp: the bracket [ui, uo] of u0; false beyond kLoopCap steps
+__device__ bool warp_u0_bracket(const Fudge &o, double &ui, double &uo)
+{
+    double x = kUmidStart, dut;
+    int at, it = 0;
+    ui = uo = x;
+    bool ok = warp_walk(x, uo, at, it, [](double p) { return p * .8; },
+                        [&](double p) { dut = o.duturnfn(p); return !(dut < 0); });
+    ui = x;
+    if (it == 0 && __shfl_sync(0xffffffffu, dut, 0) > 0) {
+        ok = warp_walk(x, ui, at, it, [](double p) { return p * 1.2; },
+                       [&](double p) { return !(o.duturnfn(p) > 0); });
+        uo = x;
+    }
+    return ok;
+}
+
+// UWalk by a warp (its results; fails beyond kLoopCap steps)
+struct UBrackets {
+    double u1, u2, uin, uout;
+    bool degenerate, capped;
+};
+__device__ UBrackets warp_u_brackets(const Fudge &o)
+{
+    UBrackets w{1., 1., 1., 1., false, false};
+    double x = 1., ut = o.uturnfn(x), dut = ut < 0 ? o.duturnfn(x) : 0.;
+    int at, it = 0;
+    auto out = [](double p) { return p * 1.1; };
+    auto in = [](double p) { return p * .9; };
+    auto positive_ends = [&](double p) { return !(o.uturnfn(p) > 0); };
+    bool ok = true;
+    if (ut < 0) {
+        const bool climb = dut > 0;
+        double eps = .1;
+        for (;;) {
+            const double f = 1 + eps;
+            if (climb)
+                ok = warp_walk(x, w.uin, at, it, [=](double p) { return p * f; },
+                               [&](double p) {
+                                   ut = o.uturnfn(p);
+                                   return !(ut < 0 && o.duturnfn(p) > 0);
+                               });
+            else
+                ok = warp_walk(x, w.uout, at, it, [=](double p) { return p / f; },
+                               [&](double p) {
+                                   ut = o.uturnfn(p);
+                                   return !(ut < 0 && o.duturnfn(p) < 0);
+                               });
+            if (!ok || __shfl_sync(0xffffffffu, ut, at) >= 0) break;
+            x = climb ? x / f : x * f;
+            eps *= .2;
+            if (eps < kTINY) {
+                w.uin = w.uout = x;
+                w.degenerate = true;
+                return w;
+            }
+            x = climb ? x * (1 + eps) : x / (1 + eps);
+        }
+        if (ok && climb) {
+            w.u1 = x;
+            ok = warp_walk(x, w.u2, at, it, out, positive_ends);
+            w.uout = x;
+        } else if (ok) {
+            w.u2 = x;
+            ok = warp_walk(x, w.u1, at, it, in, positive_ends);
+            w.uin = x;
+        }
+    } else {
+        const double fu1 = ut;
+        ok = warp_walk(x, w.u2, at, it, out, positive_ends);
+        w.uout = x;
+        if (ok && fu1 > 0) {
+            w.u1 = x;
+            x *= .9;
+            ok = warp_walk(x, w.u1, at, it, in, positive_ends);
+        }
+        w.uin = x;
+    }
+    if (!ok) {
+        w.uin = w.uout = x;
+        w.degenerate = w.capped = true;
+    }
+    return w;
+}
+
+// VWalk by a warp: the bracket [lo, hi] of the v root, or true with the turning
+// point at a limit in lo
+__device__ bool warp_v_bracket(const Fudge &o, double &lo, double &hi, bool &capped)
+{
+    double x = .5 * kPIH, f;
+    int at, it = 0;
+    lo = hi = x;
+    bool ok = warp_walk(x, hi, at, it, [](double p) { return .5 * (kPIH + p); },
+                        [&](double p) { f = o.vturnfn(p); return kPIH - p < kTINY || !(f < 0); });
+    if (it > 0) {
+        if (!ok || kPIH - x < kTINY) { capped = !ok; lo = kPIH; return true; }
+        lo = .5 * kPIH; hi = x;
+        return false;
+    }
+    x = .5 * kPIH;
+    ok = warp_walk(x, lo, at, it, [](double p) { return p * .5; },
+                   [&](double p) { return p < kTINY || !(o.vturnfn(p) > 0); });
+    if (!ok || x < kTINY) { capped = !ok; lo = 0; return true; }
+    lo = x; hi = .5 * kPIH;
+    return false;
+}
+
 // one left node's FP64 solve (the turning points of the plain form, QAGS lists of
 // kQagsCap intervals, df_value) by the block: its six moment contributions and
 // status on thread 0
@@ -624,11 +760,10 @@ __device__ void defer_solve(const MomentArgs &a, int bid, int node, const PotVie
         const double H = .5 * (V0 * V0 + V1 * V1 + V2 * V2) + Phi_h;
         const bool bound = fudge_point(P, deltafn(a.Eg, a.Dg, a.ngrid, H), R, z, Phi_h, V0, V1, V2, o, pu2, pv2);
         if (bound) {
-            U0Walk w;
-            w.begin();
-            while (!w.step(o)) {}
+            double ui, uo;
+            if (!warp_u0_bracket(o, ui, uo)) o.fail |= kFailBracket;
             BrentState b;
-            b.begin(w.ui, w.uo);
+            b.begin(ui, uo);
             while (!b.feed(o.duturnfn(b.x))) {}
             o.umid = b.root;
             o.fail |= b.fail;
@@ -645,15 +780,12 @@ __device__ void defer_solve(const MomentArgs &a, int bid, int node, const PotVie
     __syncthreads();
     if (rec.todo & kOrbitBound) {
         {
-            Fudge o = rec.o;
-            o.fail = 0;
+            const Fudge o = rec.o;
             __syncthreads();  // the turning points below go to the record
             if (warp == 0) {
-                UWalk w;
-                w.begin();
-                while (!w.step(o)) {}
+                const UBrackets w = warp_u_brackets(o);
                 double root = w.uin;
-                unsigned fail = o.fail;
+                unsigned fail = w.capped ? kFailBracket : 0u;
                 if (!w.degenerate) {  // the inner root on even lanes, the outer one on odd lanes
                     BrentState b;
                     b.begin(lane & 1 ? w.u2 : w.uin, lane & 1 ? w.uout : w.u1);
@@ -673,14 +805,13 @@ __device__ void defer_solve(const MomentArgs &a, int bid, int node, const PotVie
                     rec.rootfail[0] = fail;
                 }
             } else {
-                VWalk v;
-                v.begin();
-                while (!v.step(o)) {}
-                double vt = v.turn;
-                unsigned fail = o.fail;
-                if (!v.limit) {
+                double vt, hi;
+                bool capped = false;
+                const bool limit = warp_v_bracket(o, vt, hi, capped);
+                unsigned fail = capped ? kFailBracket : 0u;
+                if (!limit) {
                     BrentState b;
-                    b.begin(v.vbot < v.vtop ? v.vbot : v.vtop, v.vbot < v.vtop ? v.vtop : v.vbot);
+                    b.begin(vt, hi);
                     while (!b.feed(o.vturnfn(b.x))) {}
                     vt = b.root;
                     fail |= b.fail;

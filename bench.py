@@ -73,11 +73,11 @@ UNIT = "s/model"
 ALG_FLOPS_PER_EVAL = 1.33e5
 # FLOPs executed by active lanes (ncu: fadd + fmul + 2*ffma, resp. the FP64 ones) per
 # evaluation in each form's kernel, from captures of the same workload
-EXEC_FLOPS_PER_EVAL = {"mixed": 4.68e4, "plain": 1.21e5}
+EXEC_FLOPS_PER_EVAL = {"mixed": 3.23e4, "plain": 3.85e4}
 # DRAM bytes (read + write) per phase-space evaluation from ncu captures of the same workload
-# (mixed: a 240-point spread, 2,555,520 evaluations; plain: 24 points): local-memory and
-# partial-sum traffic, the inputs are < 16 KB; a launch's traffic scales with its evaluations
-DRAM_BYTES_PER_EVAL = {"mixed": 1416.7e6 / 2555520, "plain": 7.58e6 / 255552}
+# (mixed: a 240-point spread, 2,555,520 evaluations; plain: 24 points): node records, interval
+# lists and local memory, the inputs are < 16 KB; a launch's traffic scales with its evaluations
+DRAM_BYTES_PER_EVAL = {"mixed": 1011.5e6 / 2555520, "plain": 41.5e6 / 255552}
 L2_NOTE = "256 MiB buffer written between steps"
 
 
@@ -340,6 +340,9 @@ def run_ours(args, rank, world):
     achieved = ALG_FLOPS_PER_EVAL * nodes / (k_ms * 1e-3) / 1e12
     executed = EXEC_FLOPS_PER_EVAL[args.form] * nodes / (k_ms * 1e-3) / 1e12
     tot = lambda f: int(sum(getattr(st, f) for st in stats))  # noqa: E731
+    # per step: finalize, projection, Poisson; the phase-space kernels (mixed: two per slice of
+    # at most 20 M nodes, five of the capped nodes' pass)
+    launches = (2 * -(-nodes // (20 << 20)) + 5 if fp32 else 1) + (3 if args.poisson == "cumulative" else 4)
     out = {
         "metric": METRIC, "value": None, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_per_step, "higher_is_better": False, "scaling": "weak",
@@ -353,13 +356,13 @@ def run_ours(args, rank, world):
         "kernel_ms_per_step": k_ms,
         "tol": CFG["tol"], "potential_change_per_timed_step": [float(f"{c:.3g}") for c in ch],
         "iterations_to_converge_timed": conv_timed,
-        "gpu_launches": 4 * args.steps,
+        "gpu_launches": launches * args.steps,
         "failed_evals_timed": tot("failures"), "failed_by_kind_timed": {"quad": tot("fail_quad"),
                                                                         "bracket": tot("fail_bracket"),
                                                                         "root": tot("fail_root")},
         "resolved_fp64_evals_per_step": tot("resolved64") / len(stats), "escalated_evals_timed": tot("escalated"),
         "mixed_kernel_config": tuned,
-        "roofline": {"bound": "fp32" if fp32 else "fp64", "kernel": "k_moments_mixed" if fp32 else "k_moments",
+        "roofline": {"bound": "fp32" if fp32 else "fp64", "kernel": "k_mixed_turn + k_mixed_integrate" if fp32 else "k_moments",
                      "achieved": achieved, "peak": float(peak[0]),
                      "unit": "TFLOP/s", "frac": achieved / peak[0],
                      "peak_source": f"fj_measure_fma_peak ({'FP32' if fp32 else 'FP64'} FMA chains, this GPU; "

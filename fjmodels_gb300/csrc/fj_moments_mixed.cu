@@ -493,14 +493,14 @@ __global__ void __launch_bounds__(kMixedBlock, MINB) k_mixed_integrate(MomentArg
 // counts, the compact list, a block of two warps per listed node, a warp per item
 // adding its nodes in list order.
 //
-// The pass lasts as long as its slowest node (64 to a few thousand of them, most
-// integrals of which fill an FP32 list: up to 127 bisections), so a node's solve is
-// built for latency: a bracket walk evaluates its next 32 positions at once
-// (warp_walk; walks had been three quarters of the time before the integrals), the
-// two warps take the u and the v turning points and then the Ju and the Jv integral
-// side by side, the two u roots are two lanes', a
-// panel's values go over the lanes and its two sums over two of them, and the
-// integrands are those of fj_solve64.cuh (tables in shared memory, one
+// The pass lasts as long as its slowest nodes (tens to a few thousand nodes, whose
+// FP32 lists were full; in FP64 their integrals take up to some 30 bisections), so a
+// node's solve is built for latency: a bracket walk evaluates its next 32 positions
+// at once (warp_walk; walks were two thirds of a node's time), the two warps take
+// the u and the v turning points and then the Ju and the Jv integral side by side,
+// the two u roots are two lanes', a panel's values go over the lanes and its two
+// sums over two of them, and the integrands are those of fj_solve64.cuh (tables in
+// shared memory, one
 // exponential, tabulated angles).  Measured (GB300): 0.72 ms for a 24x8 model's
 // launch (16^3 nodes), 2.0 ms for one of six 40x16 models; 1.5 and 4.1 ms with the
 // walks a step at a time, 2.2 and 5.5 ms with one warp per node, its integrals one

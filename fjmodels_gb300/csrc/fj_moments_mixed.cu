@@ -48,9 +48,13 @@ namespace fj {
 // 64 registers: every access selects between the two places).
 // The integration is built in four register budgets (launch bounds of 4, 5, 6 and
 // 8 resident blocks per SM: 128, 96, 80 and 64 registers) and for npoly 3 to 8, the
-// turning points in two budgets (4 and 8 blocks): kMixedVariants configurations,
-// all with the same bits.  Which one, and the item size, is a per-context setting
-// (fj_autotune_mixed).
+// turning points in two (10 and 7 blocks: 48 and 72 registers): kMixedVariants
+// configurations, all with the same bits.  Turning points at 4, 5, 6, 7, 8 and 10
+// blocks, the integration at 8: 141.1, 134.7, 131.8, 130.6, 135.2 and 135.0 ms on
+// 80x40, 29.6, 28.5, 27.5, 26.8, 26.9 and 26.7 ms on four iterations of a 33x11 model,
+// 53.3, 51.5, 50.6, 50.2, 50.0 and 49.5 ms on six 40x16 ones.  The integration at 6,
+// 7, 8, 9 and 10 blocks: 135.3, 131.2, 130.9, 146.2 and 159.2 ms on 80x40.  Which
+// configuration, and the item size, is a per-context setting (fj_autotune_mixed).
 // Shared memory holds only what the node solves read: the FP32 tables, the
 // radii, the focal-distance table, the velocity rule and the node list.  The
 // FP64 potential tables are read from global memory (the point setup, the
@@ -1036,7 +1040,7 @@ static cudaError_t launch_deferred(const MomentArgs &a, const MomentBatch &b, lo
 namespace {
 const void *turn_kernel(int variant)
 {
-    return variant < 4 ? (const void *)k_mixed_turn<4> : (const void *)k_mixed_turn<8>;
+    return variant < 4 ? (const void *)k_mixed_turn<10> : (const void *)k_mixed_turn<7>;
 }
 
 template <int MINB>

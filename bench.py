@@ -77,7 +77,7 @@ EXEC_FLOPS_PER_EVAL = {"mixed": 3.23e4, "plain": 3.85e4}
 # DRAM bytes (read + write) per phase-space evaluation from ncu captures of the same workload
 # (mixed: a 240-point spread, 2,555,520 evaluations; plain: 24 points): node records, interval
 # lists and local memory, the inputs are < 16 KB; a launch's traffic scales with its evaluations
-DRAM_BYTES_PER_EVAL = {"mixed": 1011.5e6 / 2555520, "plain": 41.5e6 / 255552}
+DRAM_BYTES_PER_EVAL = {"mixed": 922.6e6 / 2555520, "plain": 41.5e6 / 255552}
 L2_NOTE = "256 MiB buffer written between steps"
 
 

@@ -42,7 +42,8 @@ namespace fj {
 // with the terms an evaluation does not need left out (dphi_chain), 138 ms with
 // two lanes per integral (eight: 237 ms; the list upkeep of an integral is serial,
 // so more integrals per warp share it; 24x8 and 33x11 models run 2 % slower with
-// two than with four).  On a 240-point spread of that grid the warp instructions
+// two than with four), 131 ms with the capped nodes' pass and the turning points'
+// registers as below.  On a 240-point spread of that grid the warp instructions
 // fall from 14.8 G (19.3 lanes active) to 3.4 G (17.3) + 4.9 G (25.1).  Interval
 // lists kept in shared memory instead of behind L1 were slower (144 -> 162 ms at
 // 64 registers: every access selects between the two places).

@@ -18,7 +18,7 @@
 // Measured (GB300), one thread per orbit with in-place divisions before, this
 // after: one iteration of a 16x6 model with 22^3 nodes 556 -> 160 ms, moments at
 // 6 points 95-111 -> 12.2 ms, 40 line-profile values 171 -> 39.8 ms, 20 001 actions
-// 33.4 -> 10.2 ms.  Of these steps, the integrals by groups, the table and the
+// 33.4 -> 6.0 ms (10.2 before its items were cut to whole rounds).  Of these steps, the integrals by groups, the table and the
 // reciprocals gave 581 -> 230 ms on the first, the turning points phase by phase
 // 230 -> 216 ms, the integrands' own potential and exponential 216 -> 160 ms.
 #pragma once

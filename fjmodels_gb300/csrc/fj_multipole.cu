@@ -293,8 +293,15 @@ __global__ void __launch_bounds__(kCumBlock) __cluster_dims__(kCumCluster, 1, 1)
     auto power = [&](int j, int n) { return pow(ar[n], j < 7 ? l - 2 + j : j == 7 ? 2 - l : 3 - l); };
     const int rank = (int)cluster.block_rank();
     if (tabled) {
+        // The first block's shared memory may be written only once that block runs: every block
+        // arrives at the cluster's barrier as it starts and waits there with its first power at hand.
+        cluster.barrier_arrive();
         double *first = cluster.map_shared_rank(pw, 0);
-        for (int i = rank * kCumBlock + threadIdx.x; i < kCumPowers * nr; i += kCumCluster * kCumBlock)
+        int i = rank * kCumBlock + threadIdx.x;
+        const double p0 = i < kCumPowers * nr ? power(i / nr, i % nr) : 0.;
+        cluster.barrier_wait();
+        if (i < kCumPowers * nr) first[i] = p0;
+        for (i += kCumCluster * kCumBlock; i < kCumPowers * nr; i += kCumCluster * kCumBlock)
             first[i] = power(i / nr, i % nr);
         cluster.sync();  // the powers are in the first block's shared memory
     }

@@ -85,7 +85,12 @@ struct PlainWork {
 // whether the FP64 kernels stage the radial derivative in shared memory too (16 KB)
 FJ_HD bool grad_staged(int nr, int npoly) { return (long long)nr * npoly <= 2048; }
 size_t plain_scratch_bytes(int chunk);  // per block, for items of at most chunk points
-// blocks of a persistent launch resident at once
+// Blocks of a kernel that the current device holds at once, with `threads` threads and
+// `smem` bytes of dynamic shared memory each; 0 if not one fits.  More than 48 KB (the
+// static part included) needs an opt-in, a limit that belongs to the kernel in the
+// whole process: it is only ever set to the device's maximum, so that a thread with
+// a small model cannot lower it between another's call of this and its launch.
+int resident_blocks(const void *kernel, int threads, size_t smem);
 int moments_resident(size_t smem);
 int los_resident(size_t smem);
 int actions_resident(size_t smem);

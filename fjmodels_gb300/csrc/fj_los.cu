@@ -242,17 +242,7 @@ size_t los_smem_bytes(const MomentArgs &m)
            sizeof(SolveShared) + kLosChunk * sizeof(unsigned short) + (kLosBlock / 32 + 1) * sizeof(int);
 }
 
-int los_resident(size_t smem)
-{
-    int dev = 0, nsm = 0, per_sm = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        (smem > 48 * 1024 &&
-         cudaFuncSetAttribute(k_los, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_los, kLosBlock, smem) != cudaSuccess)
-        return 0;
-    return per_sm * nsm;
-}
+int los_resident(size_t smem) { return resident_blocks((const void *)k_los, kLosBlock, smem); }
 
 size_t los_local_bytes()
 {

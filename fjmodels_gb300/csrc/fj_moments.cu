@@ -219,19 +219,24 @@ __global__ void __launch_bounds__(kMomentBlock, 2) k_moments(MomentArgs a0, Mome
     }
 }
 
-static int resident_blocks(const void *kernel, size_t smem)
+int resident_blocks(const void *kernel, int threads, size_t smem)
 {
-    int dev = 0, nsm = 0, per_sm = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        (smem > 48 * 1024 &&
-         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSolveBlock, smem) != cudaSuccess)
-        return 0;
-    return per_sm * nsm;
+    int dev = 0, nsm = 0, per_sm = 0, optin = 0;
+    cudaFuncAttributes at;
+    if (cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
+        cudaFuncGetAttributes(&at, kernel) == cudaSuccess && smem + at.sharedSizeBytes <= (size_t)optin &&
+        (smem + at.sharedSizeBytes <= 48 * 1024 ||
+         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              optin - (int)at.sharedSizeBytes) == cudaSuccess) &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) == cudaSuccess)
+        return per_sm * nsm;
+    cudaGetLastError();  // the caller refuses the call; a later launch must not report this
+    return 0;
 }
 
-int moments_resident(size_t smem) { return resident_blocks((const void *)k_moments, smem); }
+int moments_resident(size_t smem) { return resident_blocks((const void *)k_moments, kMomentBlock, smem); }
 
 // sums the per-block partials of each point and normalises as rhofDF does
 // (integ/Integ.cpp:160-162)
@@ -383,7 +388,7 @@ size_t actions_smem_bytes(int nr, int npoly, int ngrid)
     return sizeof(SolveShared) + (t <= kStagedTables ? t : 0);
 }
 
-int actions_resident(size_t smem) { return resident_blocks((const void *)k_actions, smem); }
+int actions_resident(size_t smem) { return resident_blocks((const void *)k_actions, kSolveBlock, smem); }
 
 cudaError_t launch_actions(PotView P, const double *Eg, const double *Dg, int ngrid, GLRule gl, const double2 *trig,
                            const double *pts, size_t n, int chunk, double *out, const PlainWork &w, cudaStream_t s)

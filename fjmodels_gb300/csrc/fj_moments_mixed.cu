@@ -1069,18 +1069,6 @@ const void *integrate_kernel(int variant, int np)
     }
 }
 
-int resident(const void *k, size_t smem)
-{
-    int dev = 0, nsm = 0, per_sm = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        (smem > 48 * 1024 &&
-         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kMixedBlock, smem) != cudaSuccess)
-        return 0;
-    return per_sm * nsm;
-}
-
 // the launch's items, a slice of q.per_slice at a time through both kernels
 cudaError_t launch_mixed_any(const MomentArgs &a, const MomentBatch &b, const ItemQueue &q0, size_t smem_t,
                              size_t smem_i, int variant, int np, cudaStream_t s)
@@ -1106,8 +1094,8 @@ cudaError_t launch_mixed_any(const MomentArgs &a, const MomentBatch &b, const It
 
 void mixed_resident(int variant, int np, const MixedSmem &sm, int &turn, int &integrate)
 {
-    turn = resident(turn_kernel(variant), sm.turn);
-    integrate = resident(integrate_kernel(variant, np), sm.integrate);
+    turn = resident_blocks(turn_kernel(variant), kMixedBlock, sm.turn);
+    integrate = resident_blocks(integrate_kernel(variant, np), kMixedBlock, sm.integrate);
 }
 
 MixedSmem mixed_smem(const MomentArgs &a) { return MixedSmem{mixed_turn_smem(a), mixed_integrate_smem(a)}; }

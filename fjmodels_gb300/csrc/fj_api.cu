@@ -49,6 +49,7 @@ struct fj_ctx {
     std::map<int, DevBuf> gl_rules;                    // jquad -> [2][n]
     std::vector<double> rule_host;                     // last uploaded velocity rule
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t used = nullptr;                        // the last use of the buffers above and below (SharedUse)
     int mixed_variant = 7, mixed_chunk = 1024;         // mixed kernel configuration (fj_autotune_mixed)
     int poisson = FJ_POISSON_QAGS;                     // radial integrals of fj_poisson (fj_set_poisson)
     float *jout = nullptr;                             // mixed form: actions of every bound node (fj_set_action_output)
@@ -87,6 +88,25 @@ int cuda_fail(fj_ctx *c, cudaError_t e, const char *what)
         cudaError_t e_ = (call);                           \
         if (e_ != cudaSuccess) return cuda_fail(ctx, e_, #call); \
     } while (0)
+
+// A call's use of the context's buffers.  fj_ctx_set_stream may have moved the
+// context to another stream with the previous call still running on the old one: the
+// call waits for that one's last work, and leaves an event for the next (1 us of host
+// time together).  A captured launch does neither: when it runs is up to whoever
+// launches the graph.
+struct SharedUse {
+    fj_ctx *ctx;
+    bool on;
+    explicit SharedUse(fj_ctx *c) : ctx(c), on(false)
+    {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(c->stream, &cs) != cudaSuccess) cudaGetLastError();  // the call's own work reports it
+        else on = cs == cudaStreamCaptureStatusNone && cudaStreamWaitEvent(c->stream, c->used, 0) == cudaSuccess;
+    }
+    ~SharedUse() { if (on) cudaEventRecord(ctx->used, ctx->stream); }
+    SharedUse(const SharedUse &) = delete;
+    SharedUse &operator=(const SharedUse &) = delete;
+};
 
 int ensure(fj_ctx *ctx, DevBuf &b, size_t bytes)
 {
@@ -196,7 +216,7 @@ int queue_setup(fj_ctx *ctx, long long total, int stride, int np, const MixedSme
 
 // Work queue and block scratch of a persistent FP64 launch of `total` items whose
 // kernel fits `resident` blocks on the GPU at once.  One buffer per context,
-// grown on demand: a context's launches are ordered on its stream.
+// grown on demand: a context's calls are ordered (SharedUse).
 int plain_setup(fj_ctx *ctx, long long total, int resident, int chunk, PlainWork &w)
 {
     if (total < 1 || total > 0x7fffffffLL) return fail(ctx, FJ_ERR_ARG, "moments: too many work items");
@@ -421,6 +441,7 @@ int run_moments(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delt
                 const fj_quad_rule *rule, int ngauss, const double *Rz, int npts, double *out6,
                 fj_moment_stats *stats)
 {
+    const SharedUse use(ctx);
     MomentArgs a;
     bool mixed = false;
     int rc = build_args(ctx, pot, delta, df, rule, ngauss, Rz, npts, out6, a, mixed);
@@ -462,6 +483,7 @@ namespace fj {
 int context_grid_inputs(fj_ctx *ctx, int ngauss, const fj_quad_rule *rule, const double **ci, const double **xq,
                         const double **wq)
 {
+    const SharedUse use(ctx);
     int rc = gauss_nodes(ctx, ngauss, ci);
     if (rc) return rc;
     return upload_rule(ctx, rule, xq, wq);
@@ -489,7 +511,8 @@ int fj_ctx_create(int device, fj_ctx **out)
     fj_ctx *c = new fj_ctx;
     c->device = device;
     if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&c->own, cudaStreamDefault) != cudaSuccess ||
-        cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess) {
+        cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->used, cudaEventDisableTiming) != cudaSuccess) {
         delete c;
         return FJ_ERR_CUDA;
     }
@@ -506,6 +529,7 @@ int fj_ctx_create(int device, fj_ctx **out)
         (cur < need && cudaDeviceSetLimit(cudaLimitStackSize, need) != cudaSuccess)) {
         cudaEventDestroy(c->ev0);
         cudaEventDestroy(c->ev1);
+        cudaEventDestroy(c->used);
         cudaStreamDestroy(c->own);
         delete c;
         return FJ_ERR_CUDA;
@@ -519,6 +543,7 @@ int fj_ctx_destroy(fj_ctx *ctx)
     if (!ctx) return FJ_OK;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
+    cudaEventSynchronize(ctx->used);
     for (DevBuf *b : {&ctx->partial, &ctx->counters, &ctx->rule, &ctx->misc, &ctx->defer, &ctx->queue, &ctx->trig,
                       &ctx->plain, &ctx->mixed_ws, &ctx->batch, &ctx->delta_ws})
         if (b->p) cudaFree(b->p);
@@ -527,6 +552,7 @@ int fj_ctx_destroy(fj_ctx *ctx)
     for (auto &kv : ctx->gl_rules) cudaFree(kv.second.p);
     cudaEventDestroy(ctx->ev0);
     cudaEventDestroy(ctx->ev1);
+    cudaEventDestroy(ctx->used);
     if (ctx->own) cudaStreamDestroy(ctx->own);
     delete ctx;
     return FJ_OK;
@@ -568,6 +594,7 @@ int fj_moments_batch(fj_ctx *ctx, int n, const fj_batch_item *items, const fj_qu
                      fj_moment_stats *stats)
 {
     if (!ctx || n < 1 || !items || !rule) return fail(ctx, FJ_ERR_ARG, "moments_batch: bad arguments");
+    const SharedUse use(ctx);
     std::vector<MomentArgs> args(n);
     std::vector<int> bs(n + 1, 0), ps(n + 1, 0);
     size_t smem = 0, partial = 0, defer_words_total = 0;
@@ -765,6 +792,7 @@ int fj_actions(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delta
     if (rc) return rc;
     if (!delta || delta->ngrid < 2 || !pts || !out || jquad < 0 || jquad > 64)
         return fail(ctx, FJ_ERR_ARG, "actions: bad arguments");
+    const SharedUse use(ctx);
     GLRule gl;
     if ((rc = gl_rule(ctx, jquad, &gl))) return rc;
     if (n == 0) return FJ_OK;
@@ -834,6 +862,7 @@ int fj_los(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delta, co
     if ((kind == FJ_LOS_SIGMA || kind == FJ_LOS_LINE) && !rhl)
         return fail(ctx, FJ_ERR_ARG, "los: SigmaDF needs the density multipoles");
     if (!rule || rule->precision != FJ_PREC_FP64) return fail(ctx, FJ_ERR_ARG, "los: FP64 rule only");
+    const SharedUse use(ctx);
     LosArgs a;
     bool mixed = false;
     int rc = build_args(ctx, pot, delta, df, rule, 0, Rzv, n, out, a.m, mixed);

@@ -116,7 +116,10 @@ int fj_ctx_destroy(fj_ctx *ctx);
 /* Order subsequent work on the given cudaStream_t (passed as void*, used as
    is: NULL is the legacy default stream).  A new context works on its own
    stream, which is a blocking stream and so also orders after work on the
-   legacy default stream. */
+   legacy default stream.  Calls of one context share its buffers: each waits on
+   the device for the previous one's work on them, whatever stream that ran on.
+   Launches of a graph captured from a context's calls are ordered by whoever
+   launches it. */
 int fj_ctx_set_stream(fj_ctx *ctx, void *stream);
 /* The context's own stream (to go back to it with fj_ctx_set_stream). */
 void *fj_ctx_own_stream(fj_ctx *ctx);

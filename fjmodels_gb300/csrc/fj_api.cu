@@ -11,6 +11,7 @@
 #include <cstring>
 #include <fstream>
 #include <map>
+#include <mutex>
 #include <new>
 #include <string>
 #include <thread>
@@ -28,6 +29,7 @@ using namespace fj;
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
+    bool captured = false;  // a captured launch holds the address: kept when a larger buffer takes its place
 };
 
 // The history of one Anderson-mixed iteration (fj_anderson_step, fj_anderson_host_step)
@@ -56,9 +58,10 @@ struct fj_ctx {
     DevBuf batch;                                      // batched launch: MomentArgs[n] | block_start | point_start
     std::vector<char> batch_host;                      // what `batch` holds (re-uploaded only when it changes)
     DevBuf delta_ws;                                   // GPU focal-distance tables: views | Eg ptrs | Dg ptrs | flags
-    DevBuf trig;                                       // FP64 form: quadrature-angle table (MomentArgs::trig)
+    DevBuf trig;                                       // FP64 form: quadrature-angle table (MomentArgs::trig), made with the context
     DevBuf mixed_ws;                                   // mixed form: blocks' scratch
     DevBuf plain;                                      // FP64 form: work counter | blocks' scratch (PlainWork)
+    std::vector<DevBuf> retired;                       // outgrown buffers that captured launches hold
     DevBuf queue;                                      // mixed kernel's work queue: counter | order | costs
     int q_total = 0;                                   // items of the launch whose costs the queue holds
     bool q_costs = false, q_order = false;             // costs recorded / order taken from them
@@ -111,12 +114,113 @@ struct SharedUse {
 int ensure(fj_ctx *ctx, DevBuf &b, size_t bytes)
 {
     if (b.bytes >= bytes) return FJ_OK;
-    if (b.p) cudaFree(b.p);
-    b.p = nullptr;
-    b.bytes = 0;
+    if (b.p && b.captured) ctx->retired.push_back(b);
+    else if (b.p) cudaFree(b.p);
+    b = DevBuf{};
     cudaError_t e = cudaMalloc(&b.p, bytes);
     if (e != cudaSuccess) return fail(ctx, FJ_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     b.bytes = bytes;
+    return FJ_OK;
+}
+
+// Workspaces of captured launches.  A graph runs whenever its owner launches it,
+// beside any other call, so a captured FP64 launch (fj_actions above all, which
+// shares nothing else of the context) has a workspace of its own.  It belongs to the
+// graph as a user object and comes back here, from a thread of the CUDA runtime that
+// may not call CUDA, once the graph and its executables are gone; the next capture
+// takes it from here, and the end of any context frees what is left.
+struct GraphBuffer {
+    int device;
+    DevBuf b;
+};
+struct GraphBuffers {
+    std::mutex m;
+    std::vector<GraphBuffer> idle;
+};
+GraphBuffers &graph_buffers()
+{
+    static GraphBuffers *g = new GraphBuffers;  // outlives every graph
+    return *g;
+}
+
+void CUDART_CB graph_buffer_back(void *p)
+{
+    GraphBuffer *gb = (GraphBuffer *)p;
+    try {
+        GraphBuffers &g = graph_buffers();
+        const std::lock_guard<std::mutex> lock(g.m);
+        g.idle.push_back(*gb);
+    } catch (...) {  // no host memory for the list: the buffer stays allocated
+    }
+    delete gb;
+}
+
+void free_idle_graph_buffers()
+{
+    std::vector<GraphBuffer> idle;
+    {
+        GraphBuffers &g = graph_buffers();
+        const std::lock_guard<std::mutex> lock(g.m);
+        idle.swap(g.idle);
+    }
+    for (GraphBuffer &gb : idle) cudaFree(gb.b.p);
+}
+
+// a workspace for the launch that the context's stream is capturing
+int graph_buffer(fj_ctx *ctx, size_t bytes, void **p)
+{
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cudaGraph_t graph = nullptr;
+    FJ_CUDA(cudaStreamGetCaptureInfo(ctx->stream, &cs, nullptr, &graph));
+    if (cs != cudaStreamCaptureStatusActive) return fail(ctx, FJ_ERR_CUDA, "capture: not active");
+    GraphBuffer *gb = new (std::nothrow) GraphBuffer{ctx->device, DevBuf{}};
+    if (!gb) return fail(ctx, FJ_ERR_NOMEM, "capture: no host memory");
+    {   // the smallest idle one that is large enough
+        GraphBuffers &g = graph_buffers();
+        const std::lock_guard<std::mutex> lock(g.m);
+        size_t best = g.idle.size();
+        for (size_t i = 0; i < g.idle.size(); i++)
+            if (g.idle[i].device == ctx->device && g.idle[i].b.bytes >= bytes &&
+                (best == g.idle.size() || g.idle[i].b.bytes < g.idle[best].b.bytes))
+                best = i;
+        if (best < g.idle.size()) {
+            gb->b = g.idle[best].b;
+            g.idle.erase(g.idle.begin() + best);
+        }
+    }
+    if (!gb->b.p) {  // an allocation is no part of the captured work
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        const cudaError_t e = cudaMalloc(&gb->b.p, bytes);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) {
+            delete gb;
+            cudaGetLastError();
+            return fail(ctx, FJ_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+        }
+        gb->b.bytes = bytes;
+    }
+    *p = gb->b.p;
+    cudaUserObject_t obj;
+    cudaError_t e = cudaUserObjectCreate(&obj, gb, graph_buffer_back, 1, cudaUserObjectNoDestructorSync);
+    if (e != cudaSuccess) {
+        graph_buffer_back(gb);
+        return cuda_fail(ctx, e, "cudaUserObjectCreate");
+    }
+    e = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove);
+    if (e != cudaSuccess) {
+        cudaUserObjectRelease(obj, 1);  // gives the buffer back
+        return cuda_fail(ctx, e, "cudaGraphRetainUserObject");
+    }
+    return FJ_OK;
+}
+
+// whether the context's stream is capturing
+int capturing(fj_ctx *ctx, bool &on)
+{
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    FJ_CUDA(cudaStreamIsCapturing(ctx->stream, &cs));
+    on = cs != cudaStreamCaptureStatusNone;
     return FJ_OK;
 }
 
@@ -183,12 +287,11 @@ int queue_setup(fj_ctx *ctx, long long total, int stride, int np, const MixedSme
         ctx->q_total = n;
         ctx->q_costs = ctx->q_order = false;
     }
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    FJ_CUDA(cudaStreamIsCapturing(ctx->stream, &cs));
-    if (cs == cudaStreamCaptureStatusNone && ctx->q_costs && (!ctx->q_order || ctx->q_launches >= kReorderEvery)) {
-        int rc = refresh_queue_order(ctx);
-        if (rc) return rc;
-    }
+    bool captured;
+    int rc = capturing(ctx, captured);
+    if (rc) return rc;
+    if (!captured && ctx->q_costs && (!ctx->q_order || ctx->q_launches >= kReorderEvery))
+        if ((rc = refresh_queue_order(ctx))) return rc;
     int *order = (int *)((char *)ctx->queue.p + 16);
     q.next = (unsigned *)ctx->queue.p;
     q.order = ctx->q_order ? order : nullptr;
@@ -203,8 +306,8 @@ int queue_setup(fj_ctx *ctx, long long total, int stride, int np, const MixedSme
     q.per_slice = (int)std::min<long long>(n, std::max<long long>(1, kMixedSliceNodes / stride));
     const size_t rec = (size_t)q.per_slice * stride * mixed_rec_bytes(), pt = (size_t)q.per_slice * 4 * sizeof(double),
                  nb = ((size_t)q.per_slice * sizeof(int) + 15) / 16 * 16;
-    int rc = ensure(ctx, ctx->mixed_ws, rec + pt + nb + q.grid * mixed_scratch_bytes());
-    if (rc) return rc;
+    if ((rc = ensure(ctx, ctx->mixed_ws, rec + pt + nb + q.grid * mixed_scratch_bytes()))) return rc;
+    ctx->mixed_ws.captured |= captured;
     q.rec = (char *)ctx->mixed_ws.p;
     q.point = (double *)(q.rec + rec);
     q.nbound = (int *)(q.rec + rec + pt);
@@ -216,7 +319,8 @@ int queue_setup(fj_ctx *ctx, long long total, int stride, int np, const MixedSme
 
 // Work queue and block scratch of a persistent FP64 launch of `total` items whose
 // kernel fits `resident` blocks on the GPU at once.  One buffer per context,
-// grown on demand: a context's calls are ordered (SharedUse).
+// grown on demand: a context's calls are ordered (SharedUse).  A captured launch
+// has its own (graph_buffer).
 int plain_setup(fj_ctx *ctx, long long total, int resident, int chunk, PlainWork &w)
 {
     if (total < 1 || total > 0x7fffffffLL) return fail(ctx, FJ_ERR_ARG, "moments: too many work items");
@@ -224,23 +328,19 @@ int plain_setup(fj_ctx *ctx, long long total, int resident, int chunk, PlainWork
     w.total = (int)total;
     w.grid = (int)(total < resident ? total : resident);
     w.per_block = plain_scratch_bytes(chunk);
-    int rc = ensure(ctx, ctx->plain, 256 + w.grid * w.per_block);
+    const size_t bytes = 256 + w.grid * w.per_block;
+    bool captured;
+    void *ws = nullptr;
+    int rc = capturing(ctx, captured);
     if (rc) return rc;
-    w.next = (unsigned *)ctx->plain.p;
-    w.scratch = (char *)ctx->plain.p + 256;
-    return FJ_OK;
-}
-
-// the FP64 solver's angle table, made on first use
-int trig_table(fj_ctx *ctx, const double2 **t)
-{
-    if (!ctx->trig.p) {
-        int rc = ensure(ctx, ctx->trig, kTrigTableEntries * sizeof(double2));
-        if (rc) return rc;
-        FJ_CUDA(launch_trig_table((double2 *)ctx->trig.p, ctx->stream));
-        FJ_CUDA(cudaStreamSynchronize(ctx->stream));  // a later call may use another stream
+    if (captured) {
+        if ((rc = graph_buffer(ctx, bytes, &ws))) return rc;
+    } else {
+        if ((rc = ensure(ctx, ctx->plain, bytes))) return rc;
+        ws = ctx->plain.p;
     }
-    *t = (const double2 *)ctx->trig.p;
+    w.next = (unsigned *)ws;
+    w.scratch = (char *)ws + 256;
     return FJ_OK;
 }
 
@@ -409,7 +509,7 @@ int build_args(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delta
     }
     const long long nq3 = (long long)rule->nq * rule->nq * rule->nq;
     a.mixed_chunk = plain_chunk(npts, nq3, ctx->mixed_chunk, kMixedItems);
-    if ((rc = trig_table(ctx, &a.trig))) return rc;
+    a.trig = (const double2 *)ctx->trig.p;
     a.plain_chunk = plain_chunk(npts, nq3);
     a.blocks_per_point =
         mixed ? mixed_blocks_per_point(nq3, a.mixed_chunk) : (int)((nq3 + a.plain_chunk - 1) / a.plain_chunk);
@@ -524,9 +624,14 @@ int fj_ctx_create(int device, fj_ctx **out)
         if (n2 > need) need = n2;
     need = (need + 1024 + 1023) / 1024 * 1024;
     if (need < kStackBytes) need = kStackBytes;
+    // and the FP64 solver's angle table (0.7 MB), so that no later call, which may be
+    // under capture, has to make it
     size_t cur = 0;
     if (cudaDeviceGetLimit(&cur, cudaLimitStackSize) != cudaSuccess ||
-        (cur < need && cudaDeviceSetLimit(cudaLimitStackSize, need) != cudaSuccess)) {
+        (cur < need && cudaDeviceSetLimit(cudaLimitStackSize, need) != cudaSuccess) ||
+        ensure(c, c->trig, kTrigTableEntries * sizeof(double2)) != FJ_OK ||
+        launch_trig_table((double2 *)c->trig.p, c->own) != cudaSuccess || cudaStreamSynchronize(c->own) != cudaSuccess) {
+        if (c->trig.p) cudaFree(c->trig.p);
         cudaEventDestroy(c->ev0);
         cudaEventDestroy(c->ev1);
         cudaEventDestroy(c->used);
@@ -547,6 +652,8 @@ int fj_ctx_destroy(fj_ctx *ctx)
     for (DevBuf *b : {&ctx->partial, &ctx->counters, &ctx->rule, &ctx->misc, &ctx->defer, &ctx->queue, &ctx->trig,
                       &ctx->plain, &ctx->mixed_ws, &ctx->batch, &ctx->delta_ws})
         if (b->p) cudaFree(b->p);
+    for (DevBuf &b : ctx->retired) cudaFree(b.p);
+    free_idle_graph_buffers();
     for (auto &kv : ctx->gauss_nodes) cudaFree(kv.second.p);
     for (auto &kv : ctx->poly) cudaFree(kv.second.p);
     for (auto &kv : ctx->gl_rules) cudaFree(kv.second.p);
@@ -796,8 +903,7 @@ int fj_actions(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delta
     GLRule gl;
     if ((rc = gl_rule(ctx, jquad, &gl))) return rc;
     if (n == 0) return FJ_OK;
-    const double2 *trig = nullptr;
-    if ((rc = trig_table(ctx, &trig))) return rc;
+    const double2 *trig = (const double2 *)ctx->trig.p;
     const int chunk = action_chunk(n);
     PlainWork pw{};
     if ((rc = plain_setup(ctx, (long long)((n + chunk - 1) / chunk),

@@ -277,7 +277,7 @@ int refresh_queue_order(fj_ctx *ctx)
     return FJ_OK;
 }
 
-int queue_setup(fj_ctx *ctx, long long total, int stride, int np, const MixedSmem &sm, ItemQueue &q)
+int queue_setup(fj_ctx *ctx, long long total, int stride, int np, const MixedSize &size, ItemQueue &q)
 {
     if (total < 1 || total > 0x7fffffffLL) return fail(ctx, FJ_ERR_ARG, "moments: too many work items");
     const int n = (int)total;
@@ -297,21 +297,21 @@ int queue_setup(fj_ctx *ctx, long long total, int stride, int np, const MixedSme
     q.order = ctx->q_order ? order : nullptr;
     q.cost = (float *)(order + n);
     q.total = n;
-    int turn, integrate;
-    mixed_resident(ctx->mixed_variant, np, sm, turn, integrate);
-    if (turn < 1 || integrate < 1) return fail(ctx, FJ_ERR_CUDA, "moments: tables exceed shared memory");
-    q.grid_turn = n < turn ? n : turn;
-    q.grid = n < integrate ? n : integrate;
+    if (!mixed_place(ctx->mixed_variant, np, size, q))
+        return fail(ctx, FJ_ERR_CUDA, "moments: tables exceed shared memory");
     q.stride = stride;
     q.per_slice = (int)std::min<long long>(n, std::max<long long>(1, kMixedSliceNodes / stride));
     const size_t rec = (size_t)q.per_slice * stride * mixed_rec_bytes(), pt = (size_t)q.per_slice * 4 * sizeof(double),
-                 nb = ((size_t)q.per_slice * sizeof(int) + 15) / 16 * 16;
-    if ((rc = ensure(ctx, ctx->mixed_ws, rec + pt + nb + q.grid * mixed_scratch_bytes()))) return rc;
+                 nb = ((size_t)q.per_slice * sizeof(int) + 15) / 16 * 16,
+                 lists = (q.grid * mixed_scratch_bytes() + 15) / 16 * 16,
+                 far = std::max(q.grid_turn, q.grid) * q.far_floats * sizeof(float);
+    if ((rc = ensure(ctx, ctx->mixed_ws, rec + pt + nb + lists + far))) return rc;
     ctx->mixed_ws.captured |= captured;
     q.rec = (char *)ctx->mixed_ws.p;
     q.point = (double *)(q.rec + rec);
     q.nbound = (int *)(q.rec + rec + pt);
     q.scratch = q.rec + rec + pt + nb;
+    q.far = (float *)(q.scratch + lists);
     ctx->q_costs = true;  // this launch records them
     ctx->q_launches++;
     return FJ_OK;
@@ -570,7 +570,7 @@ int run_moments(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delt
     ItemQueue q{};
     if (mixed && (rc = queue_setup(ctx, (long long)npts * a.blocks_per_point,
                                    (int)((nq3 + a.blocks_per_point - 1) / a.blocks_per_point), a.P.npoly,
-                                   mixed_smem(a), q))) return rc;
+                                   mixed_size(a), q))) return rc;
     FJ_CUDA(mixed ? launch_moments_mixed(a, ctx->mixed_variant, dw, q, ctx->stream)
                   : launch_moments(a, pw, ctx->stream));
     FJ_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
@@ -705,7 +705,7 @@ int fj_moments_batch(fj_ctx *ctx, int n, const fj_batch_item *items, const fj_qu
     std::vector<MomentArgs> args(n);
     std::vector<int> bs(n + 1, 0), ps(n + 1, 0);
     size_t smem = 0, partial = 0, defer_words_total = 0;
-    MixedSmem msm{0, 0};
+    MixedSize size;
     int stride = 1, np = items[0].pot.npoly;  // the models' multipoles (0: they differ)
     bool mixed = false;
     long long nodes = 0;
@@ -730,9 +730,7 @@ int fj_moments_batch(fj_ctx *ctx, int n, const fj_batch_item *items, const fj_qu
             defer_words_total += (size_t)nb * defer_words(args[m].mixed_chunk);
         }
         if (mixed) {
-            const MixedSmem sm = mixed_smem(args[m]);
-            msm.turn = std::max(msm.turn, sm.turn);
-            msm.integrate = std::max(msm.integrate, sm.integrate);
+            size.cover(mixed_size(args[m]));
             stride = std::max(stride, (int)((nq3 + args[m].blocks_per_point - 1) / args[m].blocks_per_point));
         } else {
             smem = std::max(smem, moment_smem_bytes(args[m]));
@@ -774,8 +772,8 @@ int fj_moments_batch(fj_ctx *ctx, int n, const fj_batch_item *items, const fj_qu
     if (!mixed && (rc = plain_setup(ctx, bs[n], moments_resident(smem), kPlainChunk, pw))) return rc;
     FJ_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
     ItemQueue q{};
-    if (mixed && (rc = queue_setup(ctx, bs[n], stride, np, msm, q))) return rc;
-    FJ_CUDA(launch_moments_batch(args[0], b, bs[n], smem, msm, mixed, ctx->mixed_variant, np, dw, q, pw, ctx->stream));
+    if (mixed && (rc = queue_setup(ctx, bs[n], stride, np, size, q))) return rc;
+    FJ_CUDA(launch_moments_batch(args[0], b, bs[n], smem, mixed, ctx->mixed_variant, np, dw, q, pw, ctx->stream));
     FJ_CUDA(launch_moments_finalize_batch(b, ps[n], ctx->stream));
     FJ_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
     return stats ? read_stats(ctx, nodes, stats) : FJ_OK;

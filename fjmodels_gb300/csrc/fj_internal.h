@@ -189,12 +189,31 @@ struct ItemQueue {
     int *nbound;       // [per_slice] bound nodes of the items
     int stride;        // most nodes of an item
     int total, per_slice;
-    int grid_turn, grid;  // blocks of the two kernels
+    int grid_turn, grid;        // blocks of the two kernels,
+    size_t smem_turn, smem;     // their dynamic shared memory
+    bool far_turn, far_integrate;  // and whether their tables are in device memory (mixed_place):
+    float *far;                    // far_floats for each block
+    size_t far_floats;
     int first, count;     // the slice (set per launch)
 };
-struct MixedSmem { size_t turn, integrate; };  // dynamic shared memory of the two kernels
-cudaError_t launch_moments_batch(const MomentArgs &a0, const MomentBatch &b, int nblocks, size_t smem,
-                                 const MixedSmem &msm, bool mixed, int variant, int np, const DeferWork &dw, const ItemQueue &q, const PlainWork &w,
+// What a model needs with near and with far tables: dynamic shared memory of the two
+// kernels, floats per block in device memory
+struct MixedSize {
+    size_t turn[2] = {0, 0}, integrate[2] = {0, 0}, far = 0;
+    void cover(const MixedSize &o)  // both models in one launch
+    {
+        for (int p = 0; p < 2; p++) {
+            turn[p] = turn[p] > o.turn[p] ? turn[p] : o.turn[p];
+            integrate[p] = integrate[p] > o.integrate[p] ? integrate[p] : o.integrate[p];
+        }
+        far = far > o.far ? far : o.far;
+    }
+};
+MixedSize mixed_size(const MomentArgs &a);
+// where the launch's tables go (q.total set), and its grids; false: they do not fit either way
+bool mixed_place(int variant, int np, const MixedSize &z, ItemQueue &q);
+cudaError_t launch_moments_batch(const MomentArgs &a0, const MomentBatch &b, int nblocks, size_t smem, bool mixed,
+                                 int variant, int np, const DeferWork &dw, const ItemQueue &q, const PlainWork &w,
                                  cudaStream_t s);
 cudaError_t launch_moments_finalize_batch(const MomentBatch &b, int npoints, cudaStream_t s);
 // dst6[q][idx[t]] = src6[q][t] (moments of n points into a grid of npts)
@@ -225,10 +244,8 @@ constexpr int kScanChunk = 1024;  // blocks per chunk of the count scan
 constexpr int kMixedMaxNodes = 8192; // largest node range of one block (shared-memory list)
 FJ_HD int defer_words(int chunk) { return (chunk + 31) / 32; }  // bitmap words of one block
 constexpr int kMixedVariants = 8;    // configurations of the mixed kernels (2 turning-point x 4 integral builds)
-MixedSmem mixed_smem(const MomentArgs &a);
 size_t mixed_rec_bytes();      // per node of a slice
 size_t mixed_scratch_bytes();  // per block of the integration kernel
-void mixed_resident(int variant, int np, const MixedSmem &sm, int &turn, int &integrate);  // blocks resident at once
 // nodes whose records a workspace holds: 2.2 GB of records at most per context
 constexpr long long kMixedSliceNodes = 20ll << 20;
 int mixed_blocks_per_point(long long nq3, int chunk);

@@ -6,8 +6,8 @@
 // FP32 for the turning-point searches, the QAGS momentum integrals and the
 // DF, FP64 again for turning points at the u/v limits and for the moments.
 // Built with FMA contraction (the plain form is the rounding-faithful one).
+#include <algorithm>
 #include <cstdint>
-
 
 #include "fj_group_qags.cuh"
 #include "fj_internal.h"
@@ -86,23 +86,32 @@ __host__ __device__ static int mixed_list_cap(int chunk)
     return c;
 }
 
-// FP32 tables of a model at one grid point in shared memory
-__host__ __device__ static size_t mixed_table_floats(int nr, int npoly, bool grad)
+// FP32 tables of a model at one grid point.  Near: all in shared memory.  Far: the
+// evaluator's table (pd) and the turning points' own copy of the potential and its
+// derivative in device memory, one set per block, the rest in shared memory
+// (kernels of their own, FAR: the near ones keep their shared-memory loads); the
+// same values, so the same bits.  mixed_place chooses.
+__host__ __device__ static size_t mixed_table_floats(int nr, int npoly, bool grad, bool far)
 {
-    const size_t nt = (size_t)nr * npoly;
-    return 2 * (size_t)nr + (grad ? 4 : 2) * nt + 4 * kQuadIntervals + npoly + 2 * kQuadIntervals * npoly;
+    return 2 * (size_t)nr + (far ? 0 : (grad ? 4 : 2) * (size_t)nr * npoly) + 4 * kQuadIntervals + npoly +
+           2 * kQuadIntervals * npoly;
 }
+// floats of a block's tables in device memory
+static size_t mixed_far_floats(int nr, int npoly) { return 4 * (size_t)nr * npoly; }
 
 struct MixedTables {
     float *ar, *phil, *Pr, *ih, *qc, *pyl, *pd, *pe;
-    // carves the tables out of 8-byte aligned memory; returns the first free float
-    __device__ float *carve(float *f, int nr, int npoly, bool grad)
+    // carves the tables out of 8-byte aligned memory f and, FAR, the block's set in
+    // device memory; returns the first free float of f
+    template <bool FAR>
+    __device__ float *carve(float *f, int nr, int npoly, bool grad, float *far)
     {
         const int nt = nr * npoly;
-        pd = f; f += 2 * nt;
+        float *&g = FAR ? far : f;
+        pd = g; g += 2 * nt;
+        phil = Pr = nullptr;
+        if (grad) { phil = g; Pr = g + nt; g += 2 * nt; }
         ar = f; f += nr;
-        phil = grad ? f : nullptr; if (grad) f += nt;
-        Pr = grad ? f : nullptr; if (grad) f += nt;
         ih = f; f += nr;
         qc = f; f += 4 * kQuadIntervals;
         pyl = f; f += npoly;
@@ -124,11 +133,11 @@ struct MixedTables {
     }
 };
 
-static size_t mixed_turn_smem(const MomentArgs &a)
+static size_t mixed_turn_smem(const MomentArgs &a, bool far)
 {
     const size_t cap = mixed_list_cap(a.mixed_chunk);
     return (a.P.nr + 2 * a.ngrid + a.nq + 4) * sizeof(double) +
-           (mixed_table_floats(a.P.nr, a.P.npoly, true) + 1) * sizeof(float) + (kMixedBlock / 32 + 1) * sizeof(int) +
+           (mixed_table_floats(a.P.nr, a.P.npoly, true, far) + 1) * sizeof(float) + (kMixedBlock / 32 + 1) * sizeof(int) +
            cap * (sizeof(float) + sizeof(unsigned short)) + 16;
 }
 
@@ -141,10 +150,10 @@ struct MixedShared {
 };
 enum : unsigned char { kIntNone = 0, kIntNew = 1, kIntMore = 2, kIntFull = 3 };  // state of an integral
 
-static size_t mixed_integrate_smem(const MomentArgs &a)
+static size_t mixed_integrate_smem(const MomentArgs &a, bool far)
 {
     return (2 * a.nq + 6 * (kMixedBlock / 32)) * sizeof(double) +
-           (mixed_table_floats(a.P.nr, a.P.npoly, false) + 1) * sizeof(float) + sizeof(MixedShared) +
+           (mixed_table_floats(a.P.nr, a.P.npoly, false, far) + 1) * sizeof(float) + sizeof(MixedShared) +
            defer_words(a.mixed_chunk) * sizeof(unsigned) + 2 * (size_t)a.mixed_chunk + 16;
 }
 
@@ -167,7 +176,7 @@ __device__ __forceinline__ void item_range(const MomentArgs &a, int bid, int &n0
     n1 = (int)((chunk + 1) * nq3 / B);
 }
 
-template <int MINB>
+template <int MINB, bool FAR>
 __global__ void __launch_bounds__(kMixedBlock, MINB) k_mixed_turn(MomentArgs a0, MomentBatch batch, ItemQueue q)
 {
     extern __shared__ double sm[];
@@ -185,7 +194,7 @@ __global__ void __launch_bounds__(kMixedBlock, MINB) k_mixed_turn(MomentArgs a0,
         const int nr = a.P.nr, npoly = a.P.npoly;
         double *s_ar = sm, *s_Eg = s_ar + nr, *s_Dg = s_Eg + a.ngrid, *s_xq = s_Dg + a.ngrid, *s_pt = s_xq + a.nq;
         MixedTables tab;
-        int *s_wc = (int *)tab.carve((float *)(s_pt + 4), nr, npoly, true);
+        int *s_wc = (int *)tab.carve<FAR>((float *)(s_pt + 4), nr, npoly, true, q.far + blockIdx.x * q.far_floats);
         unsigned short *s_list = (unsigned short *)(s_wc + kMixedBlock / 32);
         const int cap = mixed_list_cap(a.mixed_chunk);
         float *s_key = (float *)(((uintptr_t)(s_list + cap) + 15) & ~(uintptr_t)15);
@@ -379,7 +388,7 @@ __device__ __forceinline__ void mixed_integrals(PotViewF PF, int n, MixedRec *re
     }
 }
 
-template <int MINB, int NP>
+template <int MINB, int NP, bool FAR>
 __global__ void __launch_bounds__(kMixedBlock, MINB) k_mixed_integrate(MomentArgs a0, MomentBatch batch, ItemQueue q)
 {
     extern __shared__ double sm[];
@@ -398,8 +407,9 @@ __global__ void __launch_bounds__(kMixedBlock, MINB) k_mixed_integrate(MomentArg
         const int nr = a.P.nr, npoly = a.P.npoly;
         double *s_xq = sm, *s_wq = s_xq + a.nq, *s_red = s_wq + a.nq;
         MixedTables tab;
-        MixedShared &sh = *(MixedShared *)(((uintptr_t)tab.carve((float *)(s_red + 6 * (kMixedBlock / 32)), nr, npoly, false) +
-                                            15) & ~(uintptr_t)15);
+        float *const free = tab.carve<FAR>((float *)(s_red + 6 * (kMixedBlock / 32)), nr, npoly, false,
+                                           q.far + blockIdx.x * q.far_floats);
+        MixedShared &sh = *(MixedShared *)(((uintptr_t)free + 15) & ~(uintptr_t)15);
         unsigned *s_bits = (unsigned *)(&sh + 1);  // nodes left to the FP64 pass
         const int nw = defer_words(a.mixed_chunk);
         unsigned char *state = (unsigned char *)(s_bits + nw);
@@ -1039,28 +1049,30 @@ static cudaError_t launch_deferred(const MomentArgs &a, const MomentBatch &b, lo
 }
 
 namespace {
-const void *turn_kernel(int variant)
+const void *turn_kernel(int variant, bool far)
 {
-    return variant < 4 ? (const void *)k_mixed_turn<10> : (const void *)k_mixed_turn<7>;
+    if (far) return (const void *)k_mixed_turn<7, true>;
+    return variant < 4 ? (const void *)k_mixed_turn<10, false> : (const void *)k_mixed_turn<7, false>;
 }
 
 template <int MINB>
 const void *integrate_kernel_np(int np)
 {
     switch (np) {
-    case 3: return (const void *)k_mixed_integrate<MINB, 3>;
-    case 4: return (const void *)k_mixed_integrate<MINB, 4>;
-    case 5: return (const void *)k_mixed_integrate<MINB, 5>;
-    case 6: return (const void *)k_mixed_integrate<MINB, 6>;
-    case 7: return (const void *)k_mixed_integrate<MINB, 7>;
-    case 8: return (const void *)k_mixed_integrate<MINB, 8>;
-    default: return (const void *)k_mixed_integrate<MINB, 0>;
+    case 3: return (const void *)k_mixed_integrate<MINB, 3, false>;
+    case 4: return (const void *)k_mixed_integrate<MINB, 4, false>;
+    case 5: return (const void *)k_mixed_integrate<MINB, 5, false>;
+    case 6: return (const void *)k_mixed_integrate<MINB, 6, false>;
+    case 7: return (const void *)k_mixed_integrate<MINB, 7, false>;
+    case 8: return (const void *)k_mixed_integrate<MINB, 8, false>;
+    default: return (const void *)k_mixed_integrate<MINB, 0, false>;
     }
 }
 
 // np: the launch's multipoles per model (0: they differ)
-const void *integrate_kernel(int variant, int np)
+const void *integrate_kernel(int variant, int np, bool far)
 {
+    if (far) return (const void *)k_mixed_integrate<8, 0, true>;
     switch (variant & 3) {
     case 0: return integrate_kernel_np<4>(np);
     case 1: return integrate_kernel_np<5>(np);
@@ -1070,8 +1082,8 @@ const void *integrate_kernel(int variant, int np)
 }
 
 // the launch's items, a slice of q.per_slice at a time through both kernels
-cudaError_t launch_mixed_any(const MomentArgs &a, const MomentBatch &b, const ItemQueue &q0, size_t smem_t,
-                             size_t smem_i, int variant, int np, cudaStream_t s)
+cudaError_t launch_mixed_any(const MomentArgs &a, const MomentBatch &b, const ItemQueue &q0, int variant, int np,
+                             cudaStream_t s)
 {
     if (variant < 0 || variant >= kMixedVariants || q0.grid < 1 || q0.grid_turn < 1) return cudaErrorInvalidValue;
     for (int first = 0; first < q0.total; first += q0.per_slice) {
@@ -1083,8 +1095,8 @@ cudaError_t launch_mixed_any(const MomentArgs &a, const MomentBatch &b, const It
         void *args[] = {(void *)&a, (void *)&b, (void *)&q};
         const unsigned gt = (unsigned)(q.count < q.grid_turn ? q.count : q.grid_turn),
                        gi = (unsigned)(q.count < q.grid ? q.count : q.grid);
-        if ((e = cudaLaunchKernel(turn_kernel(variant), dim3(gt), dim3(kMixedBlock), args, smem_t, s)) != cudaSuccess ||
-            (e = cudaLaunchKernel(integrate_kernel(variant, np), dim3(gi), dim3(kMixedBlock), args, smem_i, s)) !=
+        if ((e = cudaLaunchKernel(turn_kernel(variant, q.far_turn), dim3(gt), dim3(kMixedBlock), args, q.smem_turn, s)) != cudaSuccess ||
+            (e = cudaLaunchKernel(integrate_kernel(variant, np, q.far_integrate), dim3(gi), dim3(kMixedBlock), args, q.smem, s)) !=
                 cudaSuccess)
             return e;
     }
@@ -1092,13 +1104,40 @@ cudaError_t launch_mixed_any(const MomentArgs &a, const MomentBatch &b, const It
 }
 }  // namespace
 
-void mixed_resident(int variant, int np, const MixedSmem &sm, int &turn, int &integrate)
+// The line between near and far tables, by the blocks that an SM holds: a launch
+// that near tables hold below the far kernel's residency runs faster from device
+// memory (the tables stay in L1 and L2), the turning points with any block less, the
+// integrals, which read little else, with a third less.  1500 points, 14^3 nodes (ms,
+// near / turning points far / integrals far; one kernel with everything near before
+// these two): 40x24 40.4 / 38.9 / 43.0, before 89; 80x24 39.1 / 33.5 / 40.0, 89; 100x24
+// 36.2 / 31.6 / 35.9, 81; 130x24 37.6 / 29.9 / 36.0, 69; 250x24 49.1 / 27.9 / 44.5, 62;
+// 500x24 83.2 / 41.0 / 65.4, 70; 80x7 15.3 / 15.5 / 16.9, 38; 400x7 15.4 / 11.5 / 15.3,
+// 23; 1000x7 34.7 / 15.5 / 33.1, 36.  As chosen: 33.5, 28.7 (130x24), 23.6, 23.3 (500x24),
+// 11.4 and 13.9 (1000x7).  Models beyond the near tables' limit (13 000 to 14 000
+// entries) have the far ones only: 700x24 24.6 (one kernel before: 52 for 1000 points).  Few
+// items take the near tables where these fit and hold every item at once.
+bool mixed_place(int variant, int np, const MixedSize &z, ItemQueue &q)
 {
-    turn = resident_blocks(turn_kernel(variant), kMixedBlock, sm.turn);
-    integrate = resident_blocks(integrate_kernel(variant, np), kMixedBlock, sm.integrate);
+    const int nt = resident_blocks(turn_kernel(variant, false), kMixedBlock, z.turn[0]),
+              ni = resident_blocks(integrate_kernel(variant, np, false), kMixedBlock, z.integrate[0]),
+              ft = resident_blocks(turn_kernel(variant, true), kMixedBlock, z.turn[1]),
+              fi = resident_blocks(integrate_kernel(variant, np, true), kMixedBlock, z.integrate[1]);
+    q.far_turn = ft > nt && q.total > nt;
+    q.far_integrate = 2 * fi >= 3 * ni && q.total > ni;
+    q.smem_turn = z.turn[q.far_turn];
+    q.smem = z.integrate[q.far_integrate];
+    q.grid_turn = std::min(q.total, q.far_turn ? ft : nt);
+    q.grid = std::min(q.total, q.far_integrate ? fi : ni);
+    q.far_floats = q.far_turn || q.far_integrate ? z.far : 0;
+    return q.grid_turn > 0 && q.grid > 0;
 }
 
-MixedSmem mixed_smem(const MomentArgs &a) { return MixedSmem{mixed_turn_smem(a), mixed_integrate_smem(a)}; }
+MixedSize mixed_size(const MomentArgs &a)
+{
+    return MixedSize{{mixed_turn_smem(a, false), mixed_turn_smem(a, true)},
+                     {mixed_integrate_smem(a, false), mixed_integrate_smem(a, true)},
+                     mixed_far_floats(a.P.nr, a.P.npoly)};
+}
 
 cudaError_t launch_moments_mixed(const MomentArgs &a, int variant, const DeferWork &dw, const ItemQueue &q,
                                  cudaStream_t s)
@@ -1107,8 +1146,7 @@ cudaError_t launch_moments_mixed(const MomentArgs &a, int variant, const DeferWo
     const MomentBatch none{nullptr, nullptr, nullptr, 0};
     const long long nblocks = (long long)a.npts * a.blocks_per_point;
     if (q.total != nblocks) return cudaErrorInvalidValue;
-    const MixedSmem sm = mixed_smem(a);
-    cudaError_t e = launch_mixed_any(a, none, q, sm.turn, sm.integrate, variant, a.P.npoly, s);
+    cudaError_t e = launch_mixed_any(a, none, q, variant, a.P.npoly, s);
     if (e == cudaSuccess) e = launch_deferred(a, none, nblocks, dw, s);
     if (e != cudaSuccess) return e;
     return launch_moments_finalize(a, s);
@@ -1118,12 +1156,12 @@ cudaError_t launch_moments_plain_batch(const MomentArgs &a0, const MomentBatch &
                                       cudaStream_t s);
 
 cudaError_t launch_moments_batch(const MomentArgs &a0, const MomentBatch &b, int nblocks, size_t smem,
-                                 const MixedSmem &msm, bool mixed, int variant, int np, const DeferWork &dw, const ItemQueue &q, const PlainWork &w,
-                                 cudaStream_t s)
+                                 bool mixed, int variant, int np, const DeferWork &dw, const ItemQueue &q,
+                                 const PlainWork &w, cudaStream_t s)
 {
     if (!mixed) return launch_moments_plain_batch(a0, b, smem, w, s);
     if (q.total != nblocks) return cudaErrorInvalidValue;
-    const cudaError_t e = launch_mixed_any(a0, b, q, msm.turn, msm.integrate, variant, np, s);
+    const cudaError_t e = launch_mixed_any(a0, b, q, variant, np, s);
     return e == cudaSuccess ? launch_deferred(a0, b, nblocks, dw, s) : e;
 }
 
@@ -1132,9 +1170,10 @@ size_t moments_mixed_local_bytes()
     size_t m = 0;
     cudaFuncAttributes at;
     for (int v = 0; v < kMixedVariants; v++)
-        for (const void *k : {turn_kernel(v), integrate_kernel(v, 0), integrate_kernel(v, 7)})
+        for (const void *k : {turn_kernel(v, false), integrate_kernel(v, 0, false), integrate_kernel(v, 7, false)})
             if (cudaFuncGetAttributes(&at, k) == cudaSuccess && at.localSizeBytes > m) m = at.localSizeBytes;
-    for (const void *k : {(const void *)k_defer_solve, (const void *)k_defer_add})
+    for (const void *k : {turn_kernel(0, true), integrate_kernel(0, 0, true), (const void *)k_defer_solve,
+                          (const void *)k_defer_add})
         if (cudaFuncGetAttributes(&at, k) == cudaSuccess && at.localSizeBytes > m) m = at.localSizeBytes;
     return m;
 }

@@ -59,8 +59,10 @@ struct fj_ctx {
     std::vector<char> batch_host;                      // what `batch` holds (re-uploaded only when it changes)
     DevBuf delta_ws;                                   // GPU focal-distance tables: views | Eg ptrs | Dg ptrs | flags
     DevBuf trig;                                       // FP64 form: quadrature-angle table (MomentArgs::trig), made with the context
-    DevBuf mixed_ws;                                   // mixed form: blocks' scratch
+    DevBuf mixed_ws;                                   // mixed form: records of a slice's nodes | blocks' scratch
+    size_t mixed_refused = (size_t)-1;                 // a size of mixed_ws that the device refused
     DevBuf plain;                                      // FP64 form: work counter | blocks' scratch (PlainWork)
+    size_t plain_refused = (size_t)-1;                 // a size of plain that the device refused
     std::vector<DevBuf> retired;                       // outgrown buffers that captured launches hold
     DevBuf queue;                                      // mixed kernel's work queue: counter | order | costs
     int q_total = 0;                                   // items of the launch whose costs the queue holds
@@ -118,7 +120,10 @@ int ensure(fj_ctx *ctx, DevBuf &b, size_t bytes)
     else if (b.p) cudaFree(b.p);
     b = DevBuf{};
     cudaError_t e = cudaMalloc(&b.p, bytes);
-    if (e != cudaSuccess) return fail(ctx, FJ_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // reported here, not by a later launch
+        return fail(ctx, FJ_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    }
     b.bytes = bytes;
     return FJ_OK;
 }
@@ -300,12 +305,32 @@ int queue_setup(fj_ctx *ctx, long long total, int stride, int np, const MixedSiz
     if (!mixed_place(ctx->mixed_variant, np, size, q))
         return fail(ctx, FJ_ERR_CUDA, "moments: tables exceed shared memory");
     q.stride = stride;
+    // Slices of kMixedSliceNodes nodes (80x40 grid, 22^3 nodes: 131 ms; 134, 141 and 162 ms
+    // with slices of a half, a quarter and a tenth) and all the blocks that the GPU
+    // holds, or what the device has room for: a refusal halves the larger of the slice's
+    // records and the blocks' scratch, and a size once refused is not asked for again
     q.per_slice = (int)std::min<long long>(n, std::max<long long>(1, kMixedSliceNodes / stride));
-    const size_t rec = (size_t)q.per_slice * stride * mixed_rec_bytes(), pt = (size_t)q.per_slice * 4 * sizeof(double),
-                 nb = ((size_t)q.per_slice * sizeof(int) + 15) / 16 * 16,
-                 lists = (q.grid * mixed_scratch_bytes() + 15) / 16 * 16,
-                 far = std::max(q.grid_turn, q.grid) * q.far_floats * sizeof(float);
-    if ((rc = ensure(ctx, ctx->mixed_ws, rec + pt + nb + lists + far))) return rc;
+    size_t rec, pt, nb, lists;
+    for (;;) {
+        rec = (size_t)q.per_slice * stride * mixed_rec_bytes();
+        pt = (size_t)q.per_slice * 4 * sizeof(double);
+        nb = ((size_t)q.per_slice * sizeof(int) + 15) / 16 * 16;
+        lists = (q.grid * mixed_scratch_bytes() + 15) / 16 * 16;
+        const size_t far = std::max(q.grid_turn, q.grid) * q.far_floats * sizeof(float);
+        const size_t bytes = rec + pt + nb + lists + far;
+        if (bytes < ctx->mixed_refused) {
+            if ((rc = ensure(ctx, ctx->mixed_ws, bytes)) == FJ_OK) break;
+            if (rc != FJ_ERR_NOMEM) return rc;
+            ctx->mixed_refused = bytes;
+        }
+        const bool blocks = q.grid > 1 || q.grid_turn > 1;
+        if (q.per_slice == 1 && !blocks) return fail(ctx, FJ_ERR_NOMEM, "moments: no device memory for the workspace");
+        if (q.per_slice > 1 && (rec > lists + far || !blocks)) q.per_slice = (q.per_slice + 1) / 2;
+        else {
+            q.grid = (q.grid + 1) / 2;
+            q.grid_turn = (q.grid_turn + 1) / 2;
+        }
+    }
     ctx->mixed_ws.captured |= captured;
     q.rec = (char *)ctx->mixed_ws.p;
     q.point = (double *)(q.rec + rec);
@@ -328,17 +353,19 @@ int plain_setup(fj_ctx *ctx, long long total, int resident, int chunk, PlainWork
     w.total = (int)total;
     w.grid = (int)(total < resident ? total : resident);
     w.per_block = plain_scratch_bytes(chunk);
-    const size_t bytes = 256 + w.grid * w.per_block;
     bool captured;
     void *ws = nullptr;
     int rc = capturing(ctx, captured);
     if (rc) return rc;
-    if (captured) {
-        if ((rc = graph_buffer(ctx, bytes, &ws))) return rc;
-    } else {
-        if ((rc = ensure(ctx, ctx->plain, bytes))) return rc;
-        ws = ctx->plain.p;
+    for (;; w.grid = (w.grid + 1) / 2) {  // fewer blocks where the device has no room for all of them
+        const size_t bytes = 256 + w.grid * w.per_block;
+        if (bytes >= ctx->plain_refused && w.grid > 1) continue;
+        rc = captured ? graph_buffer(ctx, bytes, &ws) : ensure(ctx, ctx->plain, bytes);
+        if (rc == FJ_OK) break;
+        if (rc != FJ_ERR_NOMEM || w.grid == 1) return rc;
+        ctx->plain_refused = bytes;
     }
+    if (!captured) ws = ctx->plain.p;
     w.next = (unsigned *)ws;
     w.scratch = (char *)ws + 256;
     return FJ_OK;

@@ -53,6 +53,7 @@ struct fj_ctx {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t used = nullptr;                        // the last use of the buffers above and below (SharedUse)
     int mixed_variant = 7, mixed_chunk = 1024;         // mixed kernel configuration (fj_autotune_mixed)
+    bool tuning = false;                               // fj_autotune_mixed: item sizes as set, not cut to the launch
     int poisson = FJ_POISSON_QAGS;                     // radial integrals of fj_poisson (fj_set_poisson)
     float *jout = nullptr;                             // mixed form: actions of every bound node (fj_set_action_output)
     DevBuf batch;                                      // batched launch: MomentArgs[n] | block_start | point_start
@@ -535,7 +536,7 @@ int build_args(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delta
         a.ci = gn;
     }
     const long long nq3 = (long long)rule->nq * rule->nq * rule->nq;
-    a.mixed_chunk = plain_chunk(npts, nq3, ctx->mixed_chunk, kMixedItems);
+    a.mixed_chunk = ctx->tuning ? ctx->mixed_chunk : plain_chunk(npts, nq3, ctx->mixed_chunk, kMixedItems);
     a.trig = (const double2 *)ctx->trig.p;
     a.plain_chunk = plain_chunk(npts, nq3);
     a.blocks_per_point =
@@ -830,24 +831,32 @@ int fj_autotune_mixed(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table
 {
     if (!ctx || !rule || rule->precision != FJ_PREC_MIXED || !Rz || npts < 1 || !out6)
         return fail(ctx, FJ_ERR_ARG, "autotune_mixed: needs a mixed-precision rule and sample points");
+    // Items of the sizes as named, as a grid of many points has them: cut to the sample
+    // (plain_chunk), launches under different names would be one and the same.
     static const int chunks[] = {1024, 2048, 4096};
     const int v0 = ctx->mixed_variant, c0 = ctx->mixed_chunk;
-    int bv = v0, bc = c0;
+    int bv = v0, bc = c0, rc = FJ_OK;
     double best = -1;
-    for (int v = 0; v < kMixedVariants; v++)
-        for (int ci = 0; ci < 3; ci++) {
+    ctx->tuning = true;
+    for (int v = 0; v < kMixedVariants && rc == FJ_OK; v++)
+        for (int ci = 0; ci < 3 && rc == FJ_OK; ci++) {
             ctx->mixed_variant = v;
             ctx->mixed_chunk = chunks[ci];
             double ms = -1;
-            for (int rep = 0; rep < 2; rep++) {  // the faster of two launches (the first may pay one-time costs)
+            for (int rep = 0; rep < 2 && rc == FJ_OK; rep++) {  // the faster of two launches (the first may pay one-time costs)
                 fj_moment_stats st;
-                int rc = run_moments(ctx, pot, delta, df, rule, 0, Rz, npts, out6, &st);
-                if (rc) { ctx->mixed_variant = v0; ctx->mixed_chunk = c0; return rc; }
-                if (ms < 0 || st.kernel_ms < ms) ms = st.kernel_ms;
+                rc = run_moments(ctx, pot, delta, df, rule, 0, Rz, npts, out6, &st);
+                if (rc == FJ_OK && (ms < 0 || st.kernel_ms < ms)) ms = st.kernel_ms;
             }
-            if (all_ms) all_ms[v * 3 + ci] = ms;
-            if (best < 0 || ms < best) { best = ms; bv = v; bc = chunks[ci]; }
+            if (rc == FJ_OK && all_ms) all_ms[v * 3 + ci] = ms;
+            if (rc == FJ_OK && (best < 0 || ms < best)) { best = ms; bv = v; bc = chunks[ci]; }
         }
+    ctx->tuning = false;
+    if (rc) {
+        ctx->mixed_variant = v0;
+        ctx->mixed_chunk = c0;
+        return rc;
+    }
     ctx->mixed_variant = bv;
     ctx->mixed_chunk = bc;
     if (best_ms) *best_ms = best;

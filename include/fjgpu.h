@@ -238,21 +238,22 @@ int fj_surrogate_fit(fj_surrogate *s, const fj_potential *pot, const fj_df_param
 int fj_surrogate_moments(fj_surrogate *s, const fj_potential *pot, const fj_df_params *df, const fj_quad_rule *rule,
                          int ngauss, double *grids6, double *ms, int fused);
 
-/* Configuration of the mixed-precision phase-space kernel (no reference
-   counterpart: the reference has one CPU loop).  variant 0..7: 0..3 give
-   the turning points the larger register budget (4 resident blocks per SM),
-   4..7 the smaller (8); within each, the register budget of the momentum
-   integrals (launch bounds of 4, 5, 6, 8 resident blocks per SM),
-   nodes_per_block = most velocity nodes of one point per work item
-   (128..8192; a model too small to fill the GPU with such items is split
-   further).  Initially 7 and 1024.
+/* Configuration of the mixed-precision phase-space kernels (no reference
+   counterpart: the reference has one CPU loop).  variant 0..7: 0..3 build the
+   turning points for 10 resident blocks per SM (48 registers), 4..7 for 7 (72
+   registers); within each, the register budget of the momentum integrals (4, 5,
+   6, 8 resident blocks per SM: 128, 96, 80, 64 registers).  Models whose tables
+   do not fit shared memory beside that many blocks have a build of their own,
+   whatever the variant.  nodes_per_block = most velocity nodes of one point per
+   work item (128..8192; a launch of too few points to fill the GPU with such
+   items is split further).  Initially 7 and 1024.
    fj_autotune_mixed times every variant x {1024, 2048, 4096} with
    fj_moments_points on the given device sample points (out6 device
-   [6][npts] scratch), keeps the fastest in the context and returns its
-   kernel time (all_ms, if not NULL: host [8][3] times of every variant x
-   {1024, 2048, 4096}); results are the same in every configuration up to
-   the summation order of the per-thread sums (the variants give the same bits
-   at the same nodes_per_block). */
+   [6][npts] scratch; items of the size named, not split further), keeps the
+   fastest in the context and returns its kernel time (all_ms, if not NULL: host
+   [8][3] times of every variant x {1024, 2048, 4096}).  Results are the same in
+   every configuration up to the summation order of the per-item sums (the
+   variants give the same bits at the same item size). */
 int fj_set_mixed_config(fj_ctx *ctx, int variant, int nodes_per_block);
 int fj_get_mixed_config(fj_ctx *ctx, int *variant, int *nodes_per_block);
 int fj_autotune_mixed(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delta, const fj_df_params *df,

@@ -133,6 +133,44 @@ FJ_HD int topbottom(const double *xm, int n, double x, int &bot, int &top)
     return 1;
 }
 
+// The interval b with ar[b] <= x < ar[b + 1] (b <= nr - 2) of an increasing grid of
+// positive radii, ar[0] <= x <= ar[nr - 1], from a guess: doubling steps away from it until
+// x is enclosed, then halving.  A guess that is right costs two reads of the grid
+// (at(i)), one that is d intervals off 2 log2(d) + 4: on a grid that is not the guess's
+// (which assumes a logarithmic one) never much more than a search without it.
+template <class At>
+FJ_HD int bracket_near(const At &at, int nr, double x, int guess)
+{
+#ifdef __CUDA_ARCH__
+    // the bit patterns of positive values are ordered as they are, and leave the FP64 pipe alone
+    const long long v = __double_as_longlong(x);
+    auto below = [&](int i) { return v < __double_as_longlong(at(i)); };
+#else
+    auto below = [&](int i) { return x < at(i); };
+#endif
+    int lo = guess, hi = guess + 1;
+    if (lo > 0 && below(lo)) {
+        int step = 1;
+        do {
+            hi = lo;
+            lo = lo - step > 0 ? lo - step : 0;
+            step *= 2;
+        } while (lo > 0 && below(lo));
+    } else {
+        int step = 1;
+        while (hi < nr - 1 && !below(hi)) {
+            lo = hi;
+            hi = hi + step < nr - 1 ? hi + step : nr - 1;
+            step *= 2;
+        }
+    }
+    while (hi - lo > 1) {
+        const int m = (lo + hi) >> 1;
+        if (below(m)) hi = m; else lo = m;
+    }
+    return lo;
+}
+
 // interpolation weights of intpo2 (include/UtilsLeg.h:96-158) at one radius
 struct Interp {
     int bot, top, thr;

@@ -938,7 +938,7 @@ int fj_actions(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delta
     if ((rc = gl_rule(ctx, jquad, &gl))) return rc;
     if (n == 0) return FJ_OK;
     const double2 *trig = (const double2 *)ctx->trig.p;
-    const int chunk = action_chunk(n);
+    const int chunk = action_chunk(n, sm_count());
     PlainWork pw{};
     if ((rc = plain_setup(ctx, (long long)((n + chunk - 1) / chunk),
                           actions_resident(actions_smem_bytes(pot->nr, pot->npoly, delta->ngrid)), kActionChunk, pw)))

@@ -91,6 +91,7 @@ size_t plain_scratch_bytes(int chunk);  // per block, for items of at most chunk
 // whole process: it is only ever set to the device's maximum, so that a thread with
 // a small model cannot lower it between another's call of this and its launch.
 int resident_blocks(const void *kernel, int threads, size_t smem);
+int sm_count();  // of the current device; 0 if there is none
 int moments_resident(size_t smem);
 int los_resident(size_t smem);
 int actions_resident(size_t smem);
@@ -252,14 +253,14 @@ int mixed_blocks_per_point(long long nq3, int chunk);
 cudaError_t launch_moments_mixed(const MomentArgs &a, int variant, const DeferWork &dw, const ItemQueue &q,
                                  cudaStream_t s);
 
-// Points per work item of the action batch: whole rounds of the two blocks per SM,
-// items of a warp at least (20 001 points: 10.2 ms in items of 32, two rounds of
+// Points per work item of the action batch: whole rounds of two blocks per SM, items of
+// a warp at least (20 001 points on 152 SMs: 10.2 ms in items of 32, two rounds of
 // which the second is nearly empty; 6.0 ms in one round of items of 66)
-constexpr int kActionChunk = 256, kActionBlocks = 304;
-inline int action_chunk(size_t n)
+constexpr int kActionChunk = 256;
+inline int action_chunk(size_t n, int sms)
 {
-    const size_t most = (size_t)kActionBlocks * kActionChunk, rounds = (n + most - 1) / most;
-    const size_t c = (n + kActionBlocks * rounds - 1) / (kActionBlocks * rounds);
+    const size_t blocks = 2 * (size_t)(sms > 0 ? sms : 1), most = blocks * kActionChunk, rounds = (n + most - 1) / most;
+    const size_t c = (n + blocks * rounds - 1) / (blocks * rounds);
     return (int)(c < 32 ? 32 : c);
 }
 size_t actions_smem_bytes(int nr, int npoly, int ngrid);

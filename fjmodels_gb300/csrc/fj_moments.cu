@@ -11,6 +11,7 @@
 // (fj_solve64.cuh), and thread t sums the moments of entries t, t + 128, .. in
 // order.  The per-item sums go to a scratch array and a second kernel adds them
 // in a fixed order, so results are deterministic run to run.
+#include <algorithm>
 #include <cstdint>
 
 #include "fj_internal.h"
@@ -219,12 +220,21 @@ __global__ void __launch_bounds__(kMomentBlock, 2) k_moments(MomentArgs a0, Mome
     }
 }
 
+int sm_count()
+{
+    int dev = 0, nsm = 0;
+    return cudaGetDevice(&dev) == cudaSuccess &&
+                   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess
+               ? nsm
+               : 0;
+}
+
 int resident_blocks(const void *kernel, int threads, size_t smem)
 {
-    int dev = 0, nsm = 0, per_sm = 0, optin = 0;
+    const int nsm = sm_count();
+    int dev = 0, per_sm = 0, optin = 0;
     cudaFuncAttributes at;
     if (cudaGetDevice(&dev) == cudaSuccess &&
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
         cudaFuncGetAttributes(&at, kernel) == cudaSuccess && smem + at.sharedSizeBytes <= (size_t)optin &&
         (smem + at.sharedSizeBytes <= 48 * 1024 ||
@@ -444,7 +454,7 @@ cudaError_t launch_potential_eval(PotView P, const double *Rz, size_t n, double 
     if (n == 0) return cudaSuccess;
     const size_t tab = potential_smem_bytes(P), blocks = (n + kPotBlock - 1) / kPotBlock;
     const bool staged = tab <= kPotStaged;
-    const size_t most = staged ? 4 * 152 : 0x7fffffff;  // staged: one wave, each block's tables serve all its points
+    const size_t most = staged ? 4 * (size_t)std::max(1, sm_count()) : 0x7fffffff;  // staged: one wave, each block's tables serve all its points
     k_potential_eval<<<(unsigned)(blocks < most ? blocks : most), kPotBlock, staged ? tab : 0, s>>>(P, Rz, n, out,
                                                                                                  staged);
     return cudaGetLastError();

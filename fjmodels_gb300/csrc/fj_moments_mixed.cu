@@ -1040,10 +1040,7 @@ static cudaError_t launch_deferred(const MomentArgs &a, const MomentBatch &b, lo
     k_defer_scan_chunks<<<nchunks, kScanChunk, 0, s>>>(dw, nb);
     k_defer_scan_carries<<<1, kScanChunk, 0, s>>>(dw, nchunks);
     k_defer_list<<<(nb + kListWarps - 1) / kListWarps, 32 * kListWarps, 0, s>>>(a, b, dw, nb);
-    int dev = 0, nsm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    k_defer_solve<<<16 * (nsm > 0 ? nsm : 1), kDeferBlock, 0, s>>>(a, b, dw, nb, nchunks);
+    k_defer_solve<<<16 * std::max(1, sm_count()), kDeferBlock, 0, s>>>(a, b, dw, nb, nchunks);
     k_defer_add<<<(nb + kAddWarps - 1) / kAddWarps, 32 * kAddWarps, 0, s>>>(a, b, dw, nb);
     return cudaGetLastError();
 }

@@ -236,11 +236,14 @@ int capturing(fj_ctx *ctx, bool &on)
 // moments).  The list holds 1/256 of the nodes (at least 64 Ki, at most 4 Mi
 // entries); a launch that leaves more is still exact (the extra nodes are
 // solved one after another by their item's block), only slower.
+#ifndef FJ_DEFER_LIST
+#define FJ_DEFER_LIST 65536  // least entries of the list (tests make it overflow)
+#endif
 int defer_setup(fj_ctx *ctx, long long nblocks, size_t words, long long nodes, DeferWork &dw, unsigned *&bitmaps)
 {
     const long long nchunks = (nblocks + kScanChunk - 1) / kScanChunk;
     long long cap = nodes / 256;
-    cap = cap < 65536 ? 65536 : (cap > (4ll << 20) ? (4ll << 20) : cap);
+    cap = cap < FJ_DEFER_LIST ? FJ_DEFER_LIST : (cap > (4ll << 20) ? (4ll << 20) : cap);
     const size_t ints = words + 2 * (size_t)nblocks + nchunks + 2 + 2 * (size_t)cap;
     const size_t off_mom = (ints * sizeof(int) + 15) / 16 * 16;
     int rc = ensure(ctx, ctx->defer, off_mom + (size_t)cap * 6 * sizeof(double));

@@ -60,6 +60,9 @@ namespace fj {
 // radii, the focal-distance table, the velocity rule and the node list.  The
 // FP64 potential tables are read from global memory (the point setup, the
 // FP32 table build and the rare FP64 turning-point path).
+#ifndef FJ_MIXED_LEAVE_ALL
+#define FJ_MIXED_LEAVE_ALL 0  // 1: every bound node goes to the FP64 pass (tests)
+#endif
 constexpr int kMixedLanes = 2;                            // lanes per momentum integral
 constexpr int kMixedGroups = kMixedBlock / kMixedLanes;   // integrals in flight per block
 using MixedQags = GroupQags<float, kQagsCapF>;
@@ -459,7 +462,7 @@ __global__ void __launch_bounds__(kMixedBlock, MINB) k_mixed_integrate(MomentArg
             const int i = node / nq2, j = (node / nq) % nq, l = node % nq;
             const double V0 = 1e-6 + Ve * s_xq[i], V1 = 1e-6 + Ve * s_xq[j], V2 = 1e-6 + Ve * s_xq[l];
             const unsigned fail =
-                (r.word & 7u) | (state[k] == kIntFull || state[n + k] == kIntFull ? kFailQuad : 0u);
+                (FJ_MIXED_LEAVE_ALL ? kFailQuad : 0u) | (r.word & 7u) | (state[k] == kIntFull || state[n + k] == kIntFull ? kFailQuad : 0u);
             float f = 0.f;
             if (fail && a.defer) {
                 atomicOr(&s_bits[local >> 5], 1u << (local & 31));

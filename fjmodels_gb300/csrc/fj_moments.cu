@@ -418,7 +418,10 @@ cudaError_t launch_actions(PotView P, const double *Eg, const double *Dg, int ng
 // shared memory once per block where they fit (the FP64 pipe is the bound: ~400
 // FP64 instructions per point at l <= 12).  200 003 points, 80 x 7 tables: 367
 // us with a division per recurrence step and a bisection search per point, 253
-// us with the reciprocals and the interval guess of interp_setup.
+// us with the reciprocals and the interval guess of interp_setup.  Fewer points than
+// the threads of the two blocks that an SM holds (94 registers) go to as many blocks, a
+// warp of points or more to each: 1000 points 50.6 us at first, 52.3 in whole blocks of
+// 256, 35.7 so; 10 000 points 50.8, 53, 38.2.
 constexpr int kPotBlock = 256;
 constexpr size_t kPotStaged = 40 * 1024;
 static size_t potential_smem_bytes(const PotView &P)
@@ -426,8 +429,8 @@ static size_t potential_smem_bytes(const PotView &P)
     return (P.nr + 2 * (size_t)P.nr * P.npoly + interp_table_size(P.nr)) * sizeof(double);
 }
 
-__global__ void __launch_bounds__(kPotBlock) k_potential_eval(PotView P, const double *Rz, size_t n, double *out,
-                                                              bool staged)
+__global__ void __launch_bounds__(kPotBlock) k_potential_eval(PotView P, const double *Rz, size_t n, size_t per,
+                                                              double *out, bool staged)
 {
     extern __shared__ double sm[];
     if (staged) {
@@ -440,7 +443,10 @@ __global__ void __launch_bounds__(kPotBlock) k_potential_eval(PotView P, const d
         __syncthreads();
         P = PotView{nr, P.npoly, s_ar, s_phil, s_Pr, P.Pr2, s_it};
     }
-    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
+    // blocks of a small batch take `per` consecutive points each, of a larger one (per = 0) all in strides
+    const size_t first = blockIdx.x * (per ? per : (size_t)blockDim.x), end = per && first + per < n ? first + per : n,
+                 stride = per ? blockDim.x : (size_t)gridDim.x * blockDim.x;
+    for (size_t t = first + threadIdx.x; t < end; t += stride) {
         double phi, dR, dz;
         pot_grad(P, Rz[2 * t], Rz[2 * t + 1], phi, dR, dz);
         out[3 * t] = phi;
@@ -452,11 +458,17 @@ __global__ void __launch_bounds__(kPotBlock) k_potential_eval(PotView P, const d
 cudaError_t launch_potential_eval(PotView P, const double *Rz, size_t n, double *out, cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
-    const size_t tab = potential_smem_bytes(P), blocks = (n + kPotBlock - 1) / kPotBlock;
+    const size_t tab = potential_smem_bytes(P), sms = std::max(1, sm_count()), held = 2 * sms, wave = 4 * sms;
     const bool staged = tab <= kPotStaged;
-    const size_t most = staged ? 4 * (size_t)std::max(1, sm_count()) : 0x7fffffff;  // staged: one wave, each block's tables serve all its points
-    k_potential_eval<<<(unsigned)(blocks < most ? blocks : most), kPotBlock, staged ? tab : 0, s>>>(P, Rz, n, out,
-                                                                                                 staged);
+    size_t per = 0, blocks = (n + kPotBlock - 1) / kPotBlock;
+    if (blocks <= held) {  // a warp or more for each of the blocks that the SMs hold at once
+        per = ((n + held - 1) / held + 31) / 32 * 32;
+        blocks = (n + per - 1) / per;
+    } else if (staged && blocks > wave) {
+        blocks = wave;  // each block's tables serve all its points
+    }
+    k_potential_eval<<<(unsigned)std::min(blocks, (size_t)0x7fffffff), kPotBlock, staged ? tab : 0, s>>>(P, Rz, n, per,
+                                                                                                      out, staged);
     return cudaGetLastError();
 }
 

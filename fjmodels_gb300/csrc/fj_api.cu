@@ -1023,7 +1023,8 @@ int fj_los(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delta, co
     }
     if ((long long)n * a.blocks_per_item > 0x7fffffffLL) return fail(ctx, FJ_ERR_ARG, "los: too many values");
     PlainWork pw{};
-    if ((rc = plain_setup(ctx, (long long)n * a.blocks_per_item, los_resident(los_smem_bytes(a.m)), kLosChunk, pw)))
+    if (kind != FJ_LOS_SIGMA &&
+        (rc = plain_setup(ctx, (long long)n * a.blocks_per_item, los_resident(los_smem_bytes(a.m)), kLosChunk, pw)))
         return rc;
     if ((rc = ensure(ctx, ctx->partial, (size_t)n * a.blocks_per_item * sizeof(double)))) return rc;
     a.partial = (double *)ctx->partial.p;

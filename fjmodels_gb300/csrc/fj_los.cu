@@ -110,10 +110,6 @@ __global__ void __launch_bounds__(kLosBlock, 2) k_los(LosArgs a, PlainWork work)
     if (bid >= work.total) return;
     const int B = a.blocks_per_item, item = bid / B, chunk = bid % B;
     const double R = a.Rzv[3 * item], z = a.Rzv[3 * item + 1], v = a.Rzv[3 * item + 2];
-    if (a.kind == FJ_LOS_SIGMA) {
-        if (threadIdx.x == 0) a.out[item] = sigma_df(P, a.rhl, a, R, z);
-        continue;
-    }
     const double rmax = s_ar[nr - 1];
     const double Phi = pot_phi(P, R, z), Ve = sqrt(-2 * (Phi - pot_phi(P, 10 * rmax, 10 * rmax)));
     const int nq = m.nq;
@@ -213,12 +209,26 @@ __global__ void __launch_bounds__(kLosBlock, 2) k_los(LosArgs a, PlainWork work)
     }
 }
 
+// FJ_LOS_SIGMA: a warp per value, its 22 nodes on a lane each, added in sigma_df's order.
+// (In k_los, one thread of a block after the orbit solver's tables: 12x1 114 us, 40x5 167;
+// with fewer tables before that 102 and 224; so 59 and 59.)
+__global__ void __launch_bounds__(128) k_los_sigma(LosArgs a)
+{
+    const int item = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) / 32), lane = threadIdx.x & 31;
+    if (item >= a.n) return;  // the whole warp
+    const double R = a.Rzv[3 * item], z = a.Rzv[3 * item + 1], jac = a.m.P.ar[a.m.P.nr - 1] - R;
+    double t = 0, s = 0;
+    if (lane < kLos01) t = a.w01[lane] * (jac * ev_dens1(a.m.P, a.rhl, R + a.x01[lane] * jac, z));
+    for (int i = 0; i < kLos01; i++) s += __shfl_sync(0xffffffffu, t, i);
+    if (lane == 0) a.out[item] = 2 * s;
+}
+
 // a value's block sums in order; a line profile is divided by SigmaDF at the
 // point (Integ.cpp:92), from the tables in global memory
 __global__ void k_los_finalize(LosArgs a)
 {
     const int item = blockIdx.x * blockDim.x + threadIdx.x;
-    if (item >= a.n || a.kind == FJ_LOS_SIGMA) return;
+    if (item >= a.n) return;
     const int B = a.blocks_per_item;
     double s = 0;
     for (int c = 0; c < B; c++) s += a.partial[(size_t)item * B + c];
@@ -247,17 +257,24 @@ int los_resident(size_t smem) { return resident_blocks((const void *)k_los, kLos
 size_t los_local_bytes()
 {
     cudaFuncAttributes at;
-    return cudaFuncGetAttributes(&at, k_los) == cudaSuccess ? at.localSizeBytes : 0;
+    size_t m = 0;
+    for (const void *k : {(const void *)k_los, (const void *)k_los_sigma, (const void *)k_los_finalize})
+        if (cudaFuncGetAttributes(&at, k) == cudaSuccess && at.localSizeBytes > m) m = at.localSizeBytes;
+    return m;
 }
 
 cudaError_t launch_los(const LosArgs &a, const PlainWork &w, cudaStream_t s)
 {
+    if (a.kind == FJ_LOS_SIGMA) {
+        k_los_sigma<<<(unsigned)((32 * (size_t)a.n + 127) / 128), 128, 0, s>>>(a);
+        return cudaGetLastError();
+    }
     if (w.grid < 1) return cudaErrorInvalidConfiguration;
     cudaError_t e = cudaMemsetAsync(w.next, 0, sizeof(unsigned), s);
     if (e != cudaSuccess) return e;
     k_los<<<(unsigned)w.grid, kLosBlock, los_smem_bytes(a.m), s>>>(a, w);
     e = cudaGetLastError();
-    if (e != cudaSuccess || a.kind == FJ_LOS_SIGMA) return e;
+    if (e != cudaSuccess) return e;
     k_los_finalize<<<(a.n + 127) / 128, 128, 0, s>>>(a);
     return cudaGetLastError();
 }

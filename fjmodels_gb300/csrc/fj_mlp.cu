@@ -949,8 +949,14 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_sg_fused(SgGrid g, SgWeigh
     // Every group goes through its own items (grid point, node range); nothing but
     // the weights is shared.  Bound nodes collect in the group's buffer, in node
     // order, until they fill a tile.
-    for (int item = blockIdx.x * kFusedGroups + grp; item < items && !aborted; item += gridDim.x * kFusedGroups) {
-        const int p = item / B, chunk = item % B;
+    // Consecutive items are the same node range of successive points, dealt to the CTAs
+    // before their groups: few items spread over the SMs, and a group's items go
+    // through the ranges one after the other (range by range of a point, a stride that
+    // is a multiple of B gave some groups nothing but the ranges where most nodes are
+    // bound: 60 x 2 points, 64^3 nodes 9.9 ms, in two groups per point 9.5, so 6.1).
+    const int points = items / B;
+    for (int item = grp * gridDim.x + blockIdx.x; item < items && !aborted; item += gridDim.x * kFusedGroups) {
+        const int p = item % points, chunk = item / points;
         const int n0 = (int)((long long)chunk * nq3 / B), n1 = (int)((long long)(chunk + 1) * nq3 / B);
         const double Phi_h = g.point[2 * p], Ve = g.point[2 * p + 1];
         auto velocity = [&](int node, double &V0, double &V1, double &V2) {
@@ -1136,7 +1142,7 @@ int sg_fused_blocks(int npts, int nq3, int groups)
     const int need = (nq3 + fj::kFusedMaxNodes - 1) / fj::kFusedMaxNodes;
     int best = need;
     double least = 1e300;
-    for (int B = need; B <= std::max(need, std::min(need + 16, nq3 / 512)); B++) {
+    for (int B = need; B <= std::max(need, std::min(need + 16, nq3 / 128)); B++) {
         const double rounds = (double)(((long long)npts * B + groups - 1) / groups);
         const double t = rounds * (0.4 * nq3 / B / 128 + 1.0);
         if (t < least) { least = t; best = B; }
@@ -1243,7 +1249,7 @@ int fj_surrogate_moments(fj_surrogate *s, const fj_potential *pot, const fj_df_p
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
         cudaEventRecord(e0, s->stream);
-        const int items = npts * B, ctas = std::min((items + fj::kFusedGroups - 1) / fj::kFusedGroups, nsm);
+        const int items = npts * B, ctas = std::min(items, nsm);
         fj::k_sg_fused<<<ctas, fj::kFusedThreads, smem, s->stream>>>(g, w, wq, dd, B, items, s->partial, s->err);
         cudaEventRecord(e1, s->stream);
         if (cudaGetLastError() != cudaSuccess) return FJ_ERR_CUDA;

@@ -97,8 +97,8 @@ int cuda_fail(fj_ctx *c, cudaError_t e, const char *what)
 
 // A call's use of the context's buffers.  fj_ctx_set_stream may have moved the
 // context to another stream with the previous call still running on the old one: the
-// call waits for that one's last work, and leaves an event for the next (1 us of host
-// time together).  A captured launch does neither: when it runs is up to whoever
+// call waits for that one's last work, and leaves an event for the next (under 1 us
+// of host time together).  A captured launch does neither: when it runs is up to whoever
 // launches the graph.
 struct SharedUse {
     fj_ctx *ctx;

@@ -27,7 +27,7 @@ constexpr int kPlainChunk = 1024;  // most velocity nodes of one point per work 
 // possible (a long node list keeps the lanes of a block busy to its end) while
 // there are enough items to fill the GPU and balance their uneven cost.  By the
 // model's own size alone, so that a batched launch sums in the same order.
-constexpr int kPlainItems = 1216;  // 8 per SM
+constexpr int kPlainItems = 1216;  // 8 per SM of 152 (a constant: the sums keep their order on any device)
 // Mixed form: twice the blocks of its kernels (24x8 model: 9.9 ms with 1536 items
 // of 512 nodes, 8.1 ms with 3072 of 256; 80x40: 138 ms with 1024-node items, more
 // with shorter or longer ones)
@@ -69,10 +69,6 @@ struct MomentArgs {
     double *out6;            // [6][npts]
 };
 
-// Projected density, line profiles and velocity distributions (fj_los.cu):
-// n values at Rzv [n][3] (R, z, v) of one kind (FJ_LOS_*), on m's potential,
-// focal-distance table, [-1,1] rule and DF, with the 22-point [0,1] table
-constexpr int kLos01 = 22;
 // Work queue and scratch of a persistent FP64 launch (k_moments, k_los,
 // k_actions): items 0 .. total-1 from a device counter that the launch zeroes,
 // scratch of per_block bytes for each of its blocks
@@ -99,6 +95,10 @@ int actions_resident(size_t smem);
 constexpr size_t kTrigTableEntries = 2 * 1024 * 21;
 cudaError_t launch_trig_table(double2 *trig, cudaStream_t s);
 
+// Projected density, line profiles and velocity distributions (fj_los.cu):
+// n values at Rzv [n][3] (R, z, v) of one kind (FJ_LOS_*), on m's potential,
+// focal-distance table, [-1,1] rule and DF, with the 22-point [0,1] table
+constexpr int kLos01 = 22;
 struct LosArgs {
     MomentArgs m;
     const double *rhl;  // [nr*npoly] density multipoles (SigmaDF)
@@ -175,7 +175,6 @@ __device__ __forceinline__ int batch_model(const int *start, int n, int i)
 
 size_t moment_smem_bytes(const MomentArgs &a);
 cudaError_t launch_moments(const MomentArgs &a, const PlainWork &w, cudaStream_t s);
-// batched forms: grid = total blocks, smem = the largest model's
 // Work queue and workspace of the mixed form's persistent kernels.  Item i is
 // block order[i] (order NULL: block i) of the launch's layout; cost[b] receives
 // block b's cycles.  The launch goes through its items in slices of per_slice,
@@ -213,6 +212,7 @@ struct MixedSize {
 MixedSize mixed_size(const MomentArgs &a);
 // where the launch's tables go (q.total set), and its grids; false: they do not fit either way
 bool mixed_place(int variant, int np, const MixedSize &z, ItemQueue &q);
+// a batch: nblocks = items of all models, smem = the largest model's (FP64 form)
 cudaError_t launch_moments_batch(const MomentArgs &a0, const MomentBatch &b, int nblocks, size_t smem, bool mixed,
                                  int variant, int np, const DeferWork &dw, const ItemQueue &q, const PlainWork &w,
                                  cudaStream_t s);
@@ -271,7 +271,7 @@ cudaError_t launch_potential_eval(PotView P, const double *Rz, size_t n, double 
 // projection: poly [npoly][ngauss] = 2 P_2l(c_g) w_g
 cudaError_t launch_project(int nr, int ngauss, int npoly, const double *ar, const double *poly,
                            const double *grids6, double *coef6, cudaStream_t s);
-// Poisson: one warp per (n, l), QAGS interval lists of kPoissonCap entries in
+// Poisson: a warp per radial integral, QAGS interval lists of kPoissonCap entries in
 // shared memory (no device workspace)
 constexpr int kPoissonCap = 256;
 cudaError_t launch_poisson(int nr, int npoly, const double *ar, const double *rhl, double *phil,

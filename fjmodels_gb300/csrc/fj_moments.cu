@@ -1,7 +1,6 @@
-// fj_moments.cu -- the phase-space kernel: one thread per (meridional point,
-// velocity node) evaluates the Staeckel-fudge actions and the DF and the
-// block reduces the six velocity moments; plus the batched action and
-// potential kernels.
+// fj_moments.cu -- the FP64 phase-space kernel: the Staeckel-fudge actions of
+// every (meridional point, velocity node), the DF and the six velocity moments;
+// plus the batched action and potential kernels.
 //
 // Work unit: node q = (i, j, k) of the nq^3 tensor rule (integ/GaussQuad.cpp:
 // 160-180), velocity V = 1e-6 + Ve*(x_i, x_j, x_k) (integ/Integ.cpp:46-62).

@@ -47,6 +47,8 @@ namespace fj {
 // fall from 14.8 G (19.3 lanes active) to 3.4 G (17.3) + 4.9 G (25.1).  Interval
 // lists kept in shared memory instead of behind L1 were slower (144 -> 162 ms at
 // 64 registers: every access selects between the two places).
+// (The unrolled range, npoly 3 to 8, is that of the models in use here; what larger ones
+// or a batch of differing models would gain from builds of their own is not measured.)
 // The integration is built in four register budgets (launch bounds of 4, 5, 6 and
 // 8 resident blocks per SM: 128, 96, 80 and 64 registers) and for npoly 3 to 8, the
 // turning points in two (10 and 7 blocks: 48 and 72 registers): kMixedVariants
@@ -56,8 +58,9 @@ namespace fj {
 // 53.3, 51.5, 50.6, 50.2, 50.0 and 49.5 ms on six 40x16 ones.  The integration at 6,
 // 7, 8, 9 and 10 blocks: 135.3, 131.2, 130.9, 146.2 and 159.2 ms on 80x40.  Which
 // configuration, and the item size, is a per-context setting (fj_autotune_mixed).
-// Shared memory holds only what the node solves read: the FP32 tables, the
-// radii, the focal-distance table, the velocity rule and the node list.  The
+// Shared memory holds only what the node solves read: the FP32 tables (of a model
+// too large for that, device memory: mixed_place), the radii, the focal-distance
+// table, the velocity rule and the node list.  The
 // FP64 potential tables are read from global memory (the point setup, the
 // FP32 table build and the rare FP64 turning-point path).
 #ifndef FJ_MIXED_LEAVE_ALL

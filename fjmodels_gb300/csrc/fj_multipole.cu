@@ -264,7 +264,7 @@ cudaError_t launch_poisson(int nr, int npoly, const double *ar, const double *rh
 // most of the work (nine per radius, ~190 FP64 instructions each): the cluster's
 // blocks, on SMs of their own, share them, a thread per power, into the first
 // block's shared memory; that block goes on with a thread per interval, the two
-// prefix sums on a thread each, and a thread per radius.  40 radii, l <= 8: 16.4 us;
+// prefix sums on a thread each, and a thread per radius.  40 radii, l <= 8: 16.9 us;
 // 22.4 us with one block taking all powers, ~58 us with a thread per interval taking
 // its own eight and a thread per radius seven.
 

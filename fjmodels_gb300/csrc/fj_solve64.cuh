@@ -84,7 +84,8 @@ struct SolveShared {
 // exponential.  Measured against 113-bit values (4000 orbits of an 80-radius, l <=
 // 12 potential, focal distances 1e-3 to 1, errors relative to the orbit's
 // integrand): Ju median 1.2e-15, rms 3.6e-14 (the plain form 1.35e-15, 4.1e-14), Jv
-// 8.4e-16, 4.7e-13 (9.6e-16, 4.6e-13).  One iteration of the 16x6 model 216 -> 160
+// 8.4e-16, 4.7e-13 (9.6e-16, 4.6e-13: the one figure of the four that is not smaller,
+// by 2 %, one orbit's cancellation).  One iteration of the 16x6 model 216 -> 160
 // ms, 40 line-profile values 65 -> 39.8 ms.
 struct PotFast {
     int nr, npoly;

@@ -133,6 +133,10 @@ const char *fj_last_error(fj_ctx *ctx);
    integ/Integ.cpp:150-163) as called by computeRhl's grid loop
    (pot/potLeg.cpp:54-58).  The grid points are (ar[n]*sqrt(1-c_g^2), ar[n]*c_g)
    with c_g the ngauss Gauss-Legendre nodes on (0,1) (potLeg.cpp:43-47).
+   A point's sums run over ranges of its velocity nodes whose length follows from
+   the number of points of the call (few points: shorter ranges), so a point alone
+   and the same point in a grid agree to rounding, not bit for bit; a call gives the
+   same bits every time, by itself or in fj_moments_batch.
    grids6: device [6][nr*ngauss] = rho, vrot, sigR, sigp, sigz, sigRz. */
 int fj_moments(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delta,
                const fj_df_params *df, const fj_quad_rule *rule, int ngauss, double *grids6,
@@ -327,7 +331,9 @@ int fj_compute_new_phi(fj_ctx *ctx, const fj_potential *pot, const fj_delta_tabl
    (include/uvOrb.h:15,23-24; uvOrb/uvOrb.cpp:15-262) for n phase points
    pts device [n][5] = (R, z, vR, vphi, vz), with Delta = Deltafn(H)
    (delta/tabulate.cpp:40-44) as df() does.  out device [n][2] = (Jr, Jz);
-   (-1,-1) marks H >= 0, 1e31 an unbound orbit.  jquad: FJ_JQUAD_QAGS or GL order. */
+   (-1,-1) marks H >= 0, 1e31 an unbound orbit.  jquad: FJ_JQUAD_QAGS or GL order.
+   Can be captured (with FJ_JQUAD_QAGS as a context's first call too): the captured
+   launch has a workspace of its own, which lives as long as its graph. */
 int fj_actions(fj_ctx *ctx, const fj_potential *pot, const fj_delta_table *delta,
                const double *pts, size_t n, int jquad, double *out);
 

@@ -334,6 +334,11 @@ FJ_HD void dphi_row(const PotViewF &P, const DState &s, int k, float &vb, float 
     vb = vd.x; d = vd.y;
     e = QUAD ? P.pe[(2 * s.b + (s.thr > s.b ? 1 : 0)) * np_ + k] : 0.f;
 #else
+    if (P.pd) {  // the kernels' tables, where a host build has made them
+        vb = P.pd[2 * (s.b * np_ + k)]; d = P.pd[2 * (s.b * np_ + k) + 1];
+        e = QUAD ? P.pe[(2 * s.b + (s.thr > s.b ? 1 : 0)) * np_ + k] : 0.f;
+        return;
+    }
     const float *T = P.phil;
     vb = T[s.b * np_ + k]; d = T[(s.b + 1) * np_ + k] - vb;
     e = QUAD ? T[s.thr * np_ + k] - vb - s.f3 * d : 0.f;
